@@ -1201,7 +1201,8 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
   int rc = ensure_device(H);
   if (rc) return rc;
   ZState& Z = H->z;
-  Z.assembled = Z.valid32 = Z.table = false;
+  Z.assembled = false;
+  Z.drop_table();
   Z.elems = 0;
   Z.k = wavenumber;
   Z.h = h;

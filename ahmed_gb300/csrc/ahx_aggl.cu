@@ -483,7 +483,7 @@ int agglomerate_impl(ahx_hmat* H, double eps, uint32_t max_rank, uint32_t* nmerg
     Z.arena.release();
     Z.arena = fresh;
     Z.elems = total;
-    Z.valid32 = Z.table = false;
+    Z.drop_table();
     Z.arena32.release();
     Z.rank = nrank;
     Z.aca_rank = nrank;

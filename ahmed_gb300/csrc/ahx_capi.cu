@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 
 #include "ahx_aca.cuh"
+#include "ahx_dg.cuh"
 #include "ahx_hmat.hpp"
 #include "ahx_umma.cuh"
 
@@ -162,6 +163,8 @@ int arena_append(ahx_hmat* H, uint64_t count, uint64_t& off) {
 
 void invalidate_products(ahx_hmat* H) {
   for (auto& pc : H->prod) pc.release_all();
+  for (auto& d : H->dg) d.release();
+  H->finite = 0;
 }
 
 void set_error(const std::string& msg) { g_err = msg; }
@@ -590,6 +593,20 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     AHX_CUDA(launch_matvec_um(pl, d, p, X, ldX, Y, ldY, H->stream));
     return AHX_OK;
   }
+  // FP64 and its double-float stand-in: the digit-sliced product where it is the
+  // faster one; the plain kernel then only runs when X was not finite
+  const int* guard = nullptr;
+  if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) {
+    bool usable = false;
+    if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
+    if (usable) {
+      const DgPlan pl = dg_plan(H->dg[transposed ? 1 : 0], H->tree.n, H->arena64.p, H->dg_work);
+      const DgArgs da{false, d, 0.0, p, X, ldX, Y, ldY};
+      AHX_CUDA(launch_matvec_dg(pl, da, H->stream));
+      guard = dg_flag(pl);
+      prec = kFP64;
+    }
+  }
   rc = prepare_product(H, prec);
   if (rc) return rc;
   ProdCopy& pc = H->prod[prec];
@@ -617,6 +634,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   a.Y = Y;
   a.ldY = ldY;
   a.transposed = transposed ? 1u : 0u;
+  a.guard = guard;
   AHX_CUDA(launch_matvec(prec, a, H->stream));
   if (pc.ntleaves) {
     // symmetric tree: the blocks below the diagonal are the upper ones transposed
@@ -626,6 +644,32 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     a.transposed = 1u;
     AHX_CUDA(launch_matvec(prec, a, H->stream));
   }
+  return AHX_OK;
+}
+
+int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable) {
+  usable = false;
+  if (H->finite == 2) return AHX_OK;
+  DgState& D = H->dg[transposed ? 1 : 0];
+  int rc;
+  if (!D.valid) {
+    const auto& Ls = H->tree.leaves;
+    std::vector<DgLeaf> lv;
+    lv.reserve(Ls.size());
+    for (uint32_t l = 0; l < (uint32_t)Ls.size(); ++l) {
+      const Leaf& L = Ls[l];
+      if (H->rank[l] == 0) continue;
+      lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, H->rank[l], transposed ? kDgT : kDgN, H->off[l]});
+      // symmetric tree: the blocks below the diagonal are the upper ones transposed
+      if (H->tree.sym && L.b1 != L.b2)
+        lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, H->rank[l], kDgT, H->off[l]});
+    }
+    if ((rc = dg_prepare_state(D, lv, H->tree.n, H->arena64.p, H->arena64_elems, kDgK, H->finite, H->device, H->stream)))
+      return rc;
+  }
+  if (!D.usable || H->finite == 2) return AHX_OK;
+  if ((rc = H->dg_work.reserve(dg_work_bytes(false, H->tree.n, D.t_rows, p)))) return rc;
+  usable = true;
   return AHX_OK;
 }
 
@@ -719,6 +763,7 @@ int ahx_hmat_destroy(ahx_hmat* H) {
   H->stage_x.release();
   H->stage_y.release();
   H->scratch.release();
+  H->dg_work.release();
   H->z.release_all();
   if (H->own_stream && H->stream) cudaStreamDestroy(H->stream);
   delete H;
@@ -1132,7 +1177,9 @@ int ahx_hmat_prepare(ahx_hmat* H, int precision) {
   int rc = ensure_device(H);
   if (rc) return rc;
   if (precision == kFP32 && um_enabled()) return prepare_um(H);
-  return prepare_product(H, precision);
+  if ((rc = prepare_product(H, precision)) || precision != kFP64) return rc;
+  bool usable;
+  return prepare_dg(H, 1, false, usable);
 }
 
 int ahx_hmat_release(ahx_hmat* H, int precision) {

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/ahx.h"
+#include "ahx_dg.cuh"
 #include "ahx_matvec.cuh"
 #include "ahx_tree.hpp"
 
@@ -79,6 +80,19 @@ struct ProdCopy {
   }
 };
 
+// Device layout of a digit-sliced product (ahx_dg.cuh) over one block tree and op.
+struct DgState {
+  bool valid = false;   // built (usable or not)
+  bool usable = false;  // the layout's indices fit
+  DevBuf vpieces, rpieces, rowptr, pos;
+  uint32_t nv = 0, nr = 0, t_rows = 0, t_split = 0;
+  bool rs1 = true;
+  void release() {
+    for (DevBuf* b : {&vpieces, &rpieces, &rowptr, &pos}) b->release();
+    valid = usable = false;
+  }
+};
+
 // Complex (Helmholtz) leaves of a handle's block tree in the mblock<dcomp>
 // layout (low rank: U (n1 x k) then V (n2 x k), the block U V^H; dense: n1 x n2
 // column-major), complex elements interleaved (re, im).
@@ -98,9 +112,18 @@ struct ZState {
   bool table = false;
   DevBuf gm;                            // GMRES workspace
   DevBuf xc;                            // conjugated right-hand sides (adjoint of a symmetric matrix)
+  DgState dg[3];                        // digit-sliced products: A, A^H, A^T (ZOp)
+  int finite = 0;                       // elements: 0 not looked at, 1 fit for digits, 2 not
+  // the leaf table and everything built from the leaves
+  void drop_table() {
+    valid32 = table = false;
+    for (auto& d : dg) d.release();
+    finite = 0;
+  }
   void release_all() {
+    drop_table();
     for (DevBuf* b : {&arena, &arena32, &leaves, &order, &tleaves, &torder, &gm, &xc}) b->release();
-    assembled = valid32 = table = false;
+    assembled = false;
     elems = 0;
     nleaves = ntleaves = 0;
   }
@@ -169,6 +192,9 @@ struct ahx_hmat {
   uint64_t arena64_elems = 0;
   ahx::ProdCopy prod[ahx::kNumPrecisions];
   ahx::ZState z;  // Helmholtz (complex) leaves, when assembled
+  ahx::DgState dg[2];     // digit-sliced FP64 products: A, A^T
+  int finite = 0;         // FP64 leaf elements: 0 not looked at, 1 fit for digits, 2 not
+  ahx::DevBuf dg_work;    // their work buffer (real and complex)
   // staging buffers for host vectors
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch
@@ -183,6 +209,17 @@ int prepare_product(ahx_hmat* H, int prec);
 // FP32 leaves as tcgen05 streams (ahx_umma.cuh); AHX_UMMA=0 keeps every FP32 product on the mma.sync sweeps
 int prepare_um(ahx_hmat* H);
 bool um_enabled();
+// Whether p right-hand sides on leaves of `elems` real elements go through the
+// digit-sliced product.
+bool dg_wanted(uint64_t elems, uint32_t p);
+// Builds the layout of `leaves`; looks at the arena's elements once (finite).
+// count: its doubles.
+int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,
+                     uint32_t kmax, int& finite, int device, cudaStream_t s);
+DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& work);
+// FP64 leaves: layout and work buffer ahead of products with p right-hand sides
+// (and of graph capture); sets usable.
+int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable);
 // kDF64 product scratch for p right-hand sides (the split X), ahead of graph capture
 int prepare_df_x(ahx::ProdCopy& pc, uint64_t n, uint32_t p);
 // Y += d A X in double-float over a leaf table and pc.lr (the split FP64 arena)

@@ -298,7 +298,8 @@ int load_impl(ahx_hmat* H, Reader& rd, double* eta_out, uint32_t* bmin_out, bool
     est += L.adm ? (uint64_t)(L.n1 + L.n2) * 16 : (uint64_t)L.n1 * L.n2;
   if (cplx) {
     ZState& Z = H->z;
-    Z.assembled = Z.valid32 = Z.table = false;
+    Z.assembled = false;
+    Z.drop_table();
     Z.k = Z.h = Z.eps = 0.0;
     Z.elems = 0;
     Z.arena.release();

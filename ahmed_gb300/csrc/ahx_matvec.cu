@@ -9,6 +9,8 @@
 // the V-phase T = V^T X splits each output over several threads and sums the
 // partial results in a fixed order (run-to-run deterministic per leaf).
 // Contributions are added to Y with FP64 atomics (leaves sharing rows).
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include "ahx_matvec.cuh"
@@ -45,11 +47,8 @@ __device__ __forceinline__ void stage_x(A (*Xs)[PG + 1], const MvArgs& a, uint32
 // roles of the factors and of the row / column ranges swap); a dense leaf D
 // acts as D^T, one warp per column of D.
 template <typename SL, typename SD, typename A, int PG, bool TR>
-__global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
-  __shared__ A Xs[kCh][PG + 1];
-  __shared__ A Ts[kKt][PG];
-  __shared__ A red[kThreads];
-  MvLeaf L = a.leaves[a.order[blockIdx.x]];
+__device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[PG + 1], A (*Ts)[PG], A* red) {
+  MvLeaf L = a.leaves[a.order[leaf]];
   const uint32_t tid = threadIdx.x;
   const double d = a.d;
   uint64_t voff = L.off + (uint64_t)L.n1 * (L.rank > 0 ? (uint32_t)L.rank : 0u);  // V of U V^T
@@ -210,15 +209,33 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
   }
 }
 
+template <typename SL, typename SD, typename A, int PG, bool TR, bool GUARD>
+__global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
+  __shared__ A Xs[kCh][PG + 1];
+  __shared__ A Ts[kKt][PG];
+  __shared__ A red[kThreads];
+  if (GUARD) {
+    if (*a.guard == 0) return;
+    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) mv_leaf<SL, SD, A, PG, TR>(a, l, Xs, Ts, red);
+  } else {
+    mv_leaf<SL, SD, A, PG, TR>(a, blockIdx.x, Xs, Ts, red);
+  }
+}
+
 template <typename SL, typename SD, typename A, bool TR>
 cudaError_t launch_typed(const MvArgs& a, cudaStream_t s) {
   if (a.nleaves == 0 || a.p == 0) return cudaSuccess;
+  if (a.guard) {
+    mv_kernel<SL, SD, A, 8, TR, true><<<std::min(a.nleaves, 1024u), kThreads, 0, s>>>(a);
+    count_product_launches(1);
+    return cudaGetLastError();
+  }
   const uint32_t grid = a.nleaves;
-  if (a.p == 1) mv_kernel<SL, SD, A, 1, TR><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) mv_kernel<SL, SD, A, 2, TR><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) mv_kernel<SL, SD, A, 4, TR><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 8) mv_kernel<SL, SD, A, 8, TR><<<grid, kThreads, 0, s>>>(a);
-  else mv_kernel<SL, SD, A, 16, TR><<<grid, kThreads, 0, s>>>(a);
+  if (a.p == 1) mv_kernel<SL, SD, A, 1, TR, false><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p == 2) mv_kernel<SL, SD, A, 2, TR, false><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 4) mv_kernel<SL, SD, A, 4, TR, false><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 8) mv_kernel<SL, SD, A, 8, TR, false><<<grid, kThreads, 0, s>>>(a);
+  else mv_kernel<SL, SD, A, 16, TR, false><<<grid, kThreads, 0, s>>>(a);
   count_product_launches(1);
   return cudaGetLastError();
 }

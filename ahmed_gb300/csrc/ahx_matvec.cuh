@@ -39,6 +39,8 @@ struct MvArgs {
   double* Y;
   uint64_t ldY;
   uint32_t transposed = 0;  // 1: Y += d A^T X (H/mltaGeHVec.cpp:62-150)
+  // when set: the product runs only if *guard is not zero (few CTAs, a leaf loop)
+  const int* guard = nullptr;
 };
 
 cudaError_t launch_matvec(int prec, const MvArgs& a, cudaStream_t s);
@@ -80,6 +82,7 @@ struct ZArgs {
   double2* Y;
   uint64_t ldY;
   int op;
+  const int* guard = nullptr;  // as MvArgs::guard
 };
 cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s);
 // dst[i] = (float) src[i], complex128 -> complex64

@@ -1,0 +1,1027 @@
+// Digit-sliced H-matrix product on mma.sync (see ahx_dg.cuh): Y += d op(A) X
+// for FP64 and complex128 leaves and two or more right-hand sides (mltaGeHGeM /
+// mltaGeHhGeM / mltaGeHtGeM, H/mltaGeHVec.cpp:16-150, 770-805).
+//
+// Two sweeps, each a GEMM D[m][n] = sum_k A[m][k] B[k][n] with the leaf data
+// on M x K and the right-hand sides on N:
+//   V sweep     T = Q^T X: m = factor columns of all leaves of one column
+//               cluster (48 per tile), k = the cluster's rows
+//   rows sweep  Y += P T + D X: m = the rows of one finest row block (<= 48),
+//               k = every rank column and dense column of the leaves over it
+// One CTA of three warps per piece (tile x K range), a warp per 16 rows: the
+// finest clusters of the default leaf size hold 33 to 64 points, 45 on average,
+// so that a fourth warp would mostly idle (128 threads: 1.47 ms instead of 1.42,
+// 65,536 points, 16 right-hand sides).  A lane loads its eight elements of a
+// 16 x 16 fragment straight from the arena (full 32-byte sectors in both
+// orientations: the K positions of a fragment are permuted so that a lane quad
+// reads four consecutive ones) one step ahead, cuts them into digits in registers
+// and multiplies with the Z rows' digits, which the CTA stages in shared memory
+// by cp.async.
+//
+// A complex leaf is the real matrix of its interleaved (re, im) storage: its K
+// is twice as long (position 2k: re, 2k + 1: im) and a complex Z row becomes
+// the two real rows (x.re | x.im) and (-x.im | x.re), columns 2r and 2r + 1;
+// conjugated factors flip the sign of their im elements.
+//
+// Accuracy.  Digit products are integers of at most 2^16; the sums of the
+// weights 2^0, 2^-9, 2^-18, 2^-27 over one step (16 positions, at most four
+// digit pairs: <= 2^22) leave the MMA exactly, as offsets from 1.5 * 2^23, and
+// are added up in 32-bit integers; those of 2^-36 gather in FP32 for one chunk
+// and are then moved to the integers too; those of 2^-45 and 2^-54 stay in FP32.
+// Pairs below are left out (2^-63).  So the error is that of the digits: 2^-58 of
+// the row's largest term so far per entry, below what the FP64 kernel rounds away
+// in its own sums.  Against long double on the same leaves (2,000 to 4,096 points,
+// 2 to 20 right-hand sides): 0.9e-16 to 2.7e-16 per right-hand side, the FP64
+// kernel 1.5e-16 to 5.0e-16.
+//
+// What bounds it: the ALU work of cutting (about 30 integer operations per
+// element; ALU pipe 53%, issue 48%, tensor pipe 22% to 31% busy at 32,768 points).
+// 65,536 points (2.09 GB): 8.35 -> 1.41 ms with 16 right-hand sides, 4.21 -> 0.99
+// ms with 8 (2.1 TB/s); 8,300 us of it were the FP64 pipe.
+#include <algorithm>
+#include <cstdlib>
+
+#include <cuda_fp16.h>
+
+#include "ahx_dg.cuh"
+#include "ahx_hmat.hpp"
+
+namespace ahx {
+namespace {
+
+constexpr int kThreads = 2 * kDgRows;  // a warp per 16 rows
+constexpr int kChunk = 64;          // real K positions staged at a time
+constexpr int S = 6;                // digits of a value
+constexpr int kMagic = 0x4B400000;  // 1.5 * 2^23
+
+// Exponents.  Leaf elements other than zero lie in [2^-500, 2^500] and the
+// exponents of the Z rows in [-200, 200] (anything else is left to the plain
+// kernel: dg_scan_kernel, the flag), zero Z rows have kZeroZ.  So exponent + Z
+// exponent is at least 323 for a term that counts, at most 200 for a zero element
+// and at most 123 for a zero Z row: neither moves a row's exponent, and both are
+// more than 63 bits below it.
+constexpr int kLeafMin = 523, kLeafMax = 1523;  // double exponent fields
+constexpr int kZMin = -200, kZMax = 200;
+constexpr int kZeroZ = -1400;
+// a row's scale before its first element: above every zero, below every term
+constexpr int kFloor = 260 * (1 << 20) + 0xfffff;
+
+// fixed-point words: the digits' fields, 1.0 of the row's scale at 2^58
+struct Dig {  // 64-bit: d5 [3,12], d4 [13,22], d3 [23,31] | d2 [0,8], d1 [9,17], d0 [18,28]
+  uint32_t lo, hi;
+};
+
+// offsets that make the balanced digits non-negative fields, and half a unit of the last one
+constexpr unsigned long long kBias = ((((256ull << 18) + (256ull << 9) + 256ull) << 32) |
+                                       ((256ull << 23) + (512ull << 13) + (512ull << 3))) + 4ull;
+
+// fixed-point word of a double (hi, lo words) sh = E - its exponent >= 0 bits below the scale
+__device__ __forceinline__ Dig fix_f64(uint32_t hi, uint32_t lo, uint32_t sh) {
+  const uint32_t mh = (__funnelshift_l(lo, hi, 5) & 0x1ffffffu) | 0x2000000u;
+  const unsigned long long m = ((unsigned long long)mh << 32) | (lo << 5);
+  unsigned long long v;
+  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(sh));  // (past 63: zero)
+  // one's complement for negative values: an eighth of the last digit's unit off
+  const uint32_t sg = (uint32_t)((int)hi >> 31);
+  v = (v ^ (((unsigned long long)sg << 32) | sg)) + kBias;
+  return {(uint32_t)v, (uint32_t)(v >> 32)};
+}
+__device__ __forceinline__ uint32_t h2sub(uint32_t v, float off) {
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), __float2half2_rn(off));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t h2fma(uint32_t v, float a, float b) {
+  const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&v), __float2half2_rn(a), __float2half2_rn(b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// digit pairs (x low half, y high half) as FP16: a field f < 1024 becomes 1024 + f
+// by its bits alone, then the offset comes off; d4 / 2 and d5 / 4 bring both to
+// multiples of the weights 2^-36 and 2^-45
+__device__ __forceinline__ void digits(const Dig& x, const Dig& y, uint32_t (&d)[S]) {
+  constexpr uint32_t k = 0x64006400u;
+  d[0] = h2sub(((x.hi >> 18) & 0x3ffu) | ((y.hi >> 2) & 0x03ff0000u) | k, 1280.f);
+  d[1] = h2sub(((x.hi >> 9) & 0x1ffu) | ((y.hi << 7) & 0x01ff0000u) | k, 1280.f);
+  d[2] = h2sub((x.hi & 0x1ffu) | ((y.hi << 16) & 0x01ff0000u) | k, 1280.f);
+  d[3] = h2sub((x.lo >> 23) | ((y.lo >> 7) & 0x01ff0000u) | k, 1280.f);
+  d[4] = h2fma(((x.lo >> 13) & 0x3ffu) | ((y.lo << 3) & 0x03ff0000u) | k, 0.5f, -768.f);
+  d[5] = h2fma(((x.lo >> 3) & 0x3ffu) | ((y.lo << 13) & 0x03ff0000u) | k, 0.25f, -384.f);
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+// d = a b + c
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
+                                    const float (&c)[4]) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c[0]), "f"(c[1]), "f"(c[2]),
+        "f"(c[3]));
+}
+
+struct KArgs {
+  const DgPiece* pieces;
+  const uint64_t* rowptr;
+  const DgPos* pos;
+  const void* arena;
+  const unsigned char* z;  // Z rows: S digits x NP FP16 values, then the exponent << 20
+  const int* xexp;         // rows sweep: exponent of every column of X
+  const int* flag;
+  double* T;               // V sweep: T rows, NP doubles each
+  double* Y;               // rows sweep (complex: interleaved), first column of the pass
+  uint64_t ldY;            // in elements (complex: double2)
+  double dre, dim;
+  uint32_t pc;             // columns in use (real; <= NP)
+};
+
+// Partial sums of one accumulator element: integers (exact) and FP32, in units
+// of a product of leading digits; wide(): the integers as one, units of 2^-kU.
+constexpr int kU = 36;
+struct Acc {
+  int i0, i1, i2, i3;
+  float f4, f;  // units of 2^-36, 2^-45
+  __device__ __forceinline__ void clear() {
+    i0 = i1 = i2 = i3 = 0;
+    f4 = f = 0.f;
+  }
+  // the whole units of f4, which keeps the rest: FP32 never holds a long sum
+  __device__ __forceinline__ int drain() {
+    const float r = rintf(f4);
+    f4 -= r;
+    return __float2int_rn(r);
+  }
+  __device__ __forceinline__ long long wide() {
+    return ((long long)i0 << 36) + ((long long)i1 << 27) + ((long long)i2 << 18) + ((long long)i3 << 9) +
+           (long long)drain();
+  }
+  __device__ __forceinline__ float rest() const { return fmaf(f4, 512.f, f); }
+};
+__device__ __forceinline__ void mma_step(const uint32_t (&A)[S][4], const uint32_t (&B)[S][2], Acc (&acc)[4]) {
+  const float mg = __int_as_float(kMagic);
+  const float C[4] = {mg, mg, mg, mg}, zero[4] = {0.f, 0.f, 0.f, 0.f};
+  float t0[4], t1[4], t2[4], t3[4], t4[4], f5[4], f6[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    t4[j] = acc[j].f4;
+    f5[j] = acc[j].f;
+  }
+  mma(t0, A[0], B[0], C);
+  mma(t1, A[0], B[1], C);
+  mma(t2, A[0], B[2], C);
+  mma(t3, A[0], B[3], C);
+  mma(t4, A[0], B[4], t4);
+  mma(f5, A[0], B[5], f5);
+  mma(f6, A[1], B[5], zero);
+  mma(t1, A[1], B[0], t1);
+  mma(t2, A[1], B[1], t2);
+  mma(t3, A[1], B[2], t3);
+  mma(t4, A[1], B[3], t4);
+  mma(f5, A[1], B[4], f5);
+  mma(f6, A[2], B[4], f6);
+  mma(t2, A[2], B[0], t2);
+  mma(t3, A[2], B[1], t3);
+  mma(t4, A[2], B[2], t4);
+  mma(f5, A[2], B[3], f5);
+  mma(f6, A[3], B[3], f6);
+  mma(t3, A[3], B[0], t3);
+  mma(t4, A[3], B[1], t4);
+  mma(f5, A[3], B[2], f5);
+  mma(f6, A[4], B[2], f6);
+  mma(t4, A[4], B[0], t4);
+  mma(f5, A[4], B[1], f5);
+  mma(f6, A[5], B[1], f6);
+  mma(f5, A[5], B[0], f5);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    acc[j].i0 += __float_as_int(t0[j]) - kMagic;
+    acc[j].i1 += __float_as_int(t1[j]) - kMagic;
+    acc[j].i2 += __float_as_int(t2[j]) - kMagic;
+    acc[j].i3 += __float_as_int(t3[j]) - kMagic;
+    acc[j].f4 = t4[j];
+    acc[j].f = fmaf(f6[j], 0x1p-9f, f5[j]);
+  }
+}
+// 16-byte pieces of a Z row (digits, exponent): an odd number, so that ldmatrix
+// reads 8 rows x 16 bytes without bank conflicts
+template <int NT>
+constexpr int kPR = S * NT + 1;
+static_assert(S % 2 == 0, "odd row pitch");
+
+template <int NT, int CW>
+struct Smem {
+  alignas(16) unsigned char z[2][kChunk * kPR<NT> * 16];
+  alignas(16) DgPos pos[3][kChunk / CW];
+  // sums at a row's earlier exponents, brought to its present one: units of
+  // 2^-kU and 2^-(kU + 9)
+  long long bi[NT * 4][kThreads];
+  float bf[NT * 4][kThreads];
+};
+
+// v 2^e without the FP64 pipe where the result is a normal number
+__device__ __forceinline__ double scale2(double v, int e) {
+  const int hi = __double2hiint(v);
+  const int x = ((hi >> 20) & 0x7ff) + e;
+  if (v == 0.0) return v;
+  if (x < 1 || x > 2046 || e < -2000 || e > 2000) return scalbn(v, e);
+  return __hiloint2double(hi + (e << 20), __double2loint(v));
+}
+
+// RS1: every position's rows are
+// consecutive in the arena (rows sweep of A; not the dense leaves of A^T).
+template <int NT, int CW, bool ROWS, bool RS1>
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 5 : 4) dg_sweep_kernel(const KArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& sm = *reinterpret_cast<Smem<NT, CW>*>(smem_raw);
+  constexpr int NP = 8 * NT;
+  constexpr uint32_t kCE = kChunk / CW;  // elements (complex: pairs) per chunk
+  constexpr uint32_t kRow = kPR<NT> * 16;
+  if (*a.flag) return;                   // X not fit for digits: the plain kernel runs instead
+  const DgPiece pc = a.pieces[blockIdx.x];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+  const uint32_t nch = (pc.kn + kCE - 1) / kCE;
+
+  // this lane's rows of the fragment (rows past the tile repeat its last one)
+  const bool active = warp * 16 < pc.nrows;
+  const uint32_t ra = min(warp * 16 + g, pc.nrows - 1), rb = min(warp * 16 + g + 8, pc.nrows - 1);
+  uint64_t pa = 0, pb = 0;
+  uint32_t cja = 0, cjb = 0;
+  if (!ROWS) {
+    pa = a.rowptr[pc.row0 + ra];
+    pb = a.rowptr[pc.row0 + rb];
+    cja = (uint32_t)(pa >> 63) << 31;
+    cjb = (uint32_t)(pb >> 63) << 31;
+    pa = (pa & ~kDgConj) + pc.k0;
+    pb = (pb & ~kDgConj) + pc.k0;
+  } else if (RS1) {
+    pa = ra;
+    pb = rb;
+  }
+  const uint2* const Aa = reinterpret_cast<const uint2*>(a.arena) + pa * CW + (CW == 2 ? (c & 1) : 0);
+  const uint2* const Ab = reinterpret_cast<const uint2*>(a.arena) + pb * CW + (CW == 2 ? (c & 1) : 0);
+
+  auto copy_pos = [&](uint32_t ch) {
+    // (past the piece: its last position again; zero Z rows meet it)
+    if (ROWS && tid < kCE)
+      cp16(su32(&sm.pos[ch % 3][tid]), a.pos + pc.k0 + min(ch * kCE + tid, pc.kn - 1));
+  };
+  // kLR lanes to a row, a lane per piece
+  auto copy_z = [&](uint32_t ch) {
+    constexpr uint32_t kLR = kPR<NT> <= 8 ? 8 : kPR<NT> <= 16 ? 16 : 32;
+    const uint32_t w = lane % kLR, zb = su32(sm.z[ch & 1]);
+    const DgPos* ps = sm.pos[ch % 3];
+    if (w < kPR<NT>) {
+#pragma unroll 4
+      for (uint32_t q = warp * (32 / kLR) + lane / kLR; q < (uint32_t)kChunk; q += kThreads / 32 * (32 / kLR)) {
+        const uint32_t k = ch * kCE + q / CW;
+        if (k < pc.kn) {
+          const uint32_t zr = CW * (ROWS ? ps[q / CW].z : pc.in0 + pc.k0 + k) + q % CW;
+          cp16(zb + q * kRow + w * 16, a.z + (uint64_t)zr * kRow + w * 16);
+        } else {
+          // past the piece: zero A digits meet these rows, which must be numbers
+          *reinterpret_cast<uint4*>(sm.z[ch & 1] + q * kRow + w * 16) =
+              make_uint4(w == S * NT ? (uint32_t)(kZeroZ * (1 << 20)) : 0u, 0u, 0u, 0u);
+        }
+      }
+    }
+  };
+  // the eight elements of step s of chunk ch: row ra / rb, positions c + 4 i
+  uint32_t raw[8][2];
+  auto load_a = [&](uint32_t ch, uint32_t s) {
+    const DgPos* ps = sm.pos[ch % 3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t q = s * 16 + c + 4 * i;
+      uint2 va, vb;
+      uint32_t sa = cja, sb = cjb;
+      if (ROWS) {
+        const DgPos& P = ps[q / CW];
+        if (CW == 2) sa = sb = P.rsf & 0x80000000u;
+        if (RS1) {
+          va = __ldg(Aa + P.off * CW);
+          vb = __ldg(Ab + P.off * CW);
+        } else {
+          const uint64_t rs = P.rsf & 0x7fffffffu;
+          va = __ldg(Aa + (P.off + ra * rs) * CW);
+          vb = __ldg(Aa + (P.off + rb * rs) * CW);
+        }
+      } else {
+        const uint64_t k = min(ch * kCE + q / CW, pc.kn - 1);
+        va = __ldg(Aa + k * CW);
+        vb = __ldg(Ab + k * CW);
+      }
+      raw[2 * i][0] = va.y;
+      raw[2 * i][1] = va.x;
+      raw[2 * i + 1][0] = vb.y;
+      raw[2 * i + 1][1] = vb.x;
+      if (CW == 2 && (c & 1)) {
+        raw[2 * i][0] ^= sa;
+        raw[2 * i + 1][0] ^= sb;
+      }
+    }
+  };
+
+  Acc acc[NT][4];
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[t][j].clear();
+      sm.bi[t * 4 + j][tid] = 0;
+      sm.bf[t * 4 + j][tid] = 0.f;
+    }
+  // row scale 2^E as its limit (E << 20) + 0xfffff: the largest key that fits
+  int La = kFloor, Lb = kFloor;
+
+  copy_pos(0);
+  copy_pos(1);
+  cp_commit();
+  cp_wait_all();
+  __syncthreads();
+  copy_z(0);
+  cp_commit();
+  if (active) load_a(0, 0);
+
+  for (uint32_t ch = 0; ch < nch; ++ch) {
+    cp_wait_all();
+    __syncthreads();
+    if (ch + 1 < nch) copy_z(ch + 1);
+    if (ch + 2 < nch) copy_pos(ch + 2);
+    cp_commit();
+    if (!active) continue;
+    const uint32_t left = (pc.kn - ch * kCE) * CW;  // real positions from this chunk on
+    const uint32_t steps = min((left + 15) / 16, (uint32_t)kChunk / 16);
+#pragma unroll 1
+    for (uint32_t s = 0; s < steps; ++s) {
+      // ---- exponents: keys = (exponent << 20) + leading mantissa bits
+      int ka[4], kb[4];
+      const unsigned char* zq = sm.z[ch & 1] + (s * 16 + c) * kRow + S * NT * 16;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int zx = *reinterpret_cast<const int*>(zq + 4 * i * kRow);
+        const uint32_t ha = raw[2 * i][0] & 0x7fffffffu, hb = raw[2 * i + 1][0] & 0x7fffffffu;
+        ka[i] = (int)ha + zx;
+        kb[i] = (int)hb + zx;
+      }
+      int ma = max(max(ka[0], ka[1]), max(ka[2], ka[3])), mb = max(max(kb[0], kb[1]), max(kb[2], kb[3]));
+      if (__any_sync(0xffffffffu, ma > La || mb > Lb)) {
+        // a row meets a larger exponent: its sums so far are banked at the new scale
+        ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, 1));
+        ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, 2));
+        mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+        mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          int& L = h ? Lb : La;
+          const int m = h ? mb : ma;
+          if (m > L) {
+            const int N = m | 0xfffff;
+            {
+              const uint32_t sh = (uint32_t)(N - L) >> 20;
+#pragma unroll
+              for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int j = 2 * h; j < 2 * h + 2; ++j) {
+                  const long long v = sh < 64 ? sm.bi[t * 4 + j][tid] + acc[t][j].wide() : 0;
+                  const float f = sm.bf[t * 4 + j][tid] + acc[t][j].rest();
+                  // the bits shifted out, as a fraction of the new unit (sh >= 1)
+                  const unsigned long long lost = (unsigned long long)v << ((64u - sh) & 63u);
+                  sm.bi[t * 4 + j][tid] = v >> min(sh, 63u);
+                  sm.bf[t * 4 + j][tid] = f * __int_as_float((127 - (int)min(sh, 126u)) << 23) +
+                                          __uint2float_rn((uint32_t)(lost >> 32)) * 0x1p-23f;
+                  acc[t][j].clear();
+                }
+            }
+            L = N;
+          }
+        }
+      }
+      // ---- digits of the fragment: a0 (row ra, first half of K), a1 (rb), a2 (ra, second half), a3 (rb)
+      uint32_t A[S][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        Dig x[2], y[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int i = 2 * h + e;
+          const uint32_t sa = (uint32_t)(La - ka[i]) >> 20, sb = (uint32_t)(Lb - kb[i]) >> 20;
+          x[e] = fix_f64(raw[2 * i][0], raw[2 * i][1], sa);
+          y[e] = fix_f64(raw[2 * i + 1][0], raw[2 * i + 1][1], sb);
+        }
+        uint32_t da[S], db[S];
+        digits(x[0], x[1], da);
+        digits(y[0], y[1], db);
+#pragma unroll
+        for (int d = 0; d < S; ++d) {
+          A[d][2 * h] = da[d];
+          A[d][2 * h + 1] = db[d];
+        }
+      }
+      // ---- the next step's elements
+      if (s + 1 < steps) load_a(ch, s + 1);
+      else if (ch + 1 < nch) load_a(ch + 1, 0);
+      // ---- multiply.  Matrix rows of ldmatrix in the lanes' K order: i -> (i >> 1) + 4 (i & 1)
+      const uint32_t li = lane & 7, krow = (li >> 1) + 4 * (li & 1) + 8 * ((lane >> 3) & 1);
+      const uint32_t zrow = su32(sm.z[ch & 1]) + (s * 16 + krow) * kRow;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        uint32_t B[S][2];
+#pragma unroll
+        for (int d = 0; d + 1 < S; d += 2) {
+          uint32_t r[4];
+          ldsm4t(zrow + ((d + (lane >> 4)) * NT + t) * 16, r);
+          B[d][0] = r[0];
+          B[d][1] = r[1];
+          B[d + 1][0] = r[2];
+          B[d + 1][1] = r[3];
+        }
+        mma_step(A, B, acc[t]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sm.bi[t * 4 + j][tid] += acc[t][j].drain();
+  }
+  if (!active) return;
+  // ---- output: lane holds rows g, g + 8, columns 8 t + 2 c, + 1
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t row = warp * 16 + g + 8 * h;
+      if (row >= pc.nrows) continue;
+      const int L = h ? Lb : La;
+      const int ex = (L >> 20) - 1022 - 16;  // a product of leading digits: 2^-16
+      const uint32_t col = 8 * t + 2 * c;
+      double v[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int e = t * 4 + 2 * h + j;
+        const long long i = sm.bi[e][tid] + acc[t][2 * h + j].wide();
+        v[j] = fma((double)i, 512.0, (double)(sm.bf[e][tid] + acc[t][2 * h + j].rest()));  // units of 2^-(U + 9)
+      }
+      if (!ROWS) {
+        double* T = a.T + (uint64_t)(pc.row0 + row) * NP + col;
+        const double t0 = scale2(v[0], ex - kU - 9), t1 = scale2(v[1], ex - kU - 9);
+        if (pc.add) {
+          atomicAdd(T, t0);
+          atomicAdd(T + 1, t1);
+        } else {
+          *reinterpret_cast<double2*>(T) = make_double2(t0, t1);
+        }
+      } else if (CW == 2) {
+        if (col < a.pc) {
+          const int x = a.xexp[col] + ex - kU - 9;
+          const double re = scale2(v[0], x), im = scale2(v[1], x);
+          double* y = a.Y + 2 * ((uint64_t)(col / 2) * a.ldY + pc.row0 + row);
+          atomicAdd(y, a.dre * re - a.dim * im);
+          atomicAdd(y + 1, a.dre * im + a.dim * re);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (col + j < a.pc)
+            atomicAdd(a.Y + (uint64_t)(col + j) * a.ldY + pc.row0 + row,
+                      a.dre * scale2(v[j], a.xexp[col + j] + ex - kU - 9));
+      }
+    }
+  }
+}
+
+// ---- Z rows --------------------------------------------------------------
+
+// exponent field of the largest |X_r| per column (complex: of both parts), and
+// the flag of a value that is not finite
+template <int CW>
+__global__ void dg_xmax_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, int* __restrict__ xmax,
+                               int* __restrict__ flag) {
+  const double* x = X + (uint64_t)blockIdx.y * ldX * CW;
+  uint32_t m = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)n * CW;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    m = max(m, ((uint32_t)__double2hiint(x[i]) >> 20) & 0x7ffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(xmax + blockIdx.y, (int)m);
+    if (m == 0x7ffu) atomicOr(flag, 1);
+  }
+}
+
+__device__ __forceinline__ bool subnormal(double v) {
+  const uint32_t hi = (uint32_t)__double2hiint(v);
+  return (hi & 0x7ff00000u) == 0u && ((hi << 1) | (uint32_t)__double2loint(v)) != 0u;
+}
+
+// Digits of one Z row (8 NT columns of real values v(col), exponents rel(col)
+// relative to the columns' scales), written at z with the row's exponent.
+// Exponents out of range raise the flag.
+template <int NT, typename V>
+__device__ __forceinline__ void z_row(unsigned char* z, const V& val, uint32_t pc, int* flag) {
+  constexpr int NP = 8 * NT;
+  int m = kZeroZ;
+#pragma unroll 4
+  for (int j = 0; j < NP; ++j) {
+    if ((uint32_t)j >= pc) break;
+    int sc;
+    const double v = val(j, sc);
+    const int e = ((uint32_t)__double2hiint(v) >> 20) & 0x7ffu;
+    if (e) m = max(m, e - sc);
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    uint32_t o[S][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      Dig f[2];
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const int j = 8 * t + 2 * u + w;
+        int sc = 0;
+        const double v = (uint32_t)j < pc ? val(j, sc) : 0.0;
+        const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+        const int e = (hi >> 20) & 0x7ffu;
+        f[w] = fix_f64(hi, lo, e ? (uint32_t)(m - (e - sc)) : 64u);
+      }
+      uint32_t d[S];
+      digits(f[0], f[1], d);
+#pragma unroll
+      for (int k = 0; k < S; ++k) o[k][u] = d[k];
+    }
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+      *reinterpret_cast<uint4*>(z + (k * NT + t) * 16) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+  }
+  if (m != kZeroZ && (m < kZMin || m > kZMax)) atomicOr(flag, 1);
+  *reinterpret_cast<uint4*>(z + S * NT * 16) = make_uint4((uint32_t)(m * (1 << 20)), 0u, 0u, 0u);
+}
+
+// X rows (blocks past them do nothing); real row CW i + e of a complex row: e = 0
+// (re | im), e = 1 (-im | re)
+template <int NT, int CW>
+__global__ void dg_xprep_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t pc,
+                                const int* __restrict__ xmax, int* __restrict__ xexp, unsigned char* __restrict__ z,
+                                int* __restrict__ flag) {
+  const uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  // unit of column col: 2^(xexp - 0), xexp = field - 1022 (complex: the column pair shares it)
+  if (q < (uint64_t)8 * NT) xexp[q] = q < pc ? xmax[q / CW] - 1022 : 0;
+  const uint64_t total = (uint64_t)n * CW;
+  if (q >= total) return;
+  // e-major order: consecutive threads read consecutive rows of X
+  const uint32_t e = (uint32_t)(q / n), i = (uint32_t)(q - (uint64_t)e * n);
+  bool bad = false;
+  auto val = [&](int col, int& sc) -> double {
+    sc = __ldg(xmax + col / CW);
+    double r;
+    if (CW == 1) {
+      r = __ldg(X + (uint64_t)col * ldX + i);
+    } else {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(X) + (uint64_t)(col / 2) * ldX + i);
+      r = e == 0 ? ((col & 1) ? v.y : v.x) : ((col & 1) ? v.x : -v.y);
+    }
+    // a subnormal entry counts as zero: only beside entries 2^99 times larger
+    bad = bad || (sc < 100 && subnormal(r));
+    return r;
+  };
+  const uint64_t zr = (uint64_t)CW * i + e;
+  z_row<NT>(z + zr * (kPR<NT> * 16), val, pc, flag);
+  if (bad) atomicOr(flag, 1);
+}
+
+template <int NT, int CW>
+__global__ void dg_tprep_kernel(const double* __restrict__ T, uint32_t t_rows, uint32_t pc,
+                                unsigned char* __restrict__ z, int* __restrict__ flag) {
+  constexpr int NP = 8 * NT;
+  const uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (q >= (uint64_t)t_rows * CW) return;
+  const uint64_t i = q / CW;
+  const uint32_t e = (uint32_t)(q % CW);
+  const double* t = T + i * NP;
+  bool bad = false;
+  auto val = [&](int col, int& sc) -> double {
+    sc = 1022;
+    double v;
+    if (CW == 1 || e == 0) v = t[col];
+    else v = (col & 1) ? t[col - 1] : -t[col + 1];
+    bad = bad || (((uint32_t)__double2hiint(v) >> 20) & 0x7ffu) == 0x7ffu || subnormal(v);
+    return v;
+  };
+  z_row<NT>(z + q * (kPR<NT> * 16), val, pc, flag);
+  if (bad) atomicOr(flag, 1);
+}
+
+__global__ void dg_expand_kernel(const DgSeg* __restrict__ segs, uint32_t nsegs, DgPos* __restrict__ pos) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, l = threadIdx.x & 7;
+  if (s >= nsegs) return;
+  const DgSeg g = segs[s];
+  for (uint32_t k = l; k < g.kn; k += 8) pos[(uint64_t)g.pos0 + k] = DgPos{g.base + (uint64_t)k * g.ldk, g.z + k, g.rsf};
+}
+
+__global__ void dg_scan_kernel(const uint2* __restrict__ a, uint64_t count, int* __restrict__ bad) {
+  bool b = false;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint2 u = __ldg(a + i);
+    const uint32_t e = (u.y >> 20) & 0x7ffu;
+    b = b || (((u.y << 1) | u.x) != 0 && (e < kLeafMin || e > kLeafMax));
+  }
+  if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
+}
+
+size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+
+struct Work {
+  size_t xmax, xexp, z, t, end;  // the flag word is at 0
+};
+
+// n-tiles of 8 columns per pass.  More than two per warp measured slower than
+// more passes (64 right-hand sides, 65,536 points: 6.2 ms with four, 5.6 ms with
+// two): their sums take the registers of half the warps.
+constexpr uint32_t kMaxCols = 16;
+int nt_of(uint32_t cols) { return cols <= 8 ? 1 : 2; }
+
+Work work_of(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p) {
+  const size_t cw = cplx ? 2 : 1, nt = nt_of(p * (uint32_t)cw);
+  Work w;
+  w.xmax = 256;
+  w.xexp = align256(w.xmax + (size_t)p * 4);
+  w.z = align256(w.xexp + kMaxCols * 4);
+  w.t = align256(w.z + ((size_t)n + t_rows) * cw * (S * nt + 1) * 16);
+  w.end = align256(w.t + (size_t)t_rows * nt * 64);
+  return w;
+}
+
+template <int NT, int CW, bool ROWS, bool RS1>
+cudaError_t sweep(const KArgs& k, uint32_t n, cudaStream_t s) {
+  if (!n) return cudaSuccess;
+  auto f = dg_sweep_kernel<NT, CW, ROWS, RS1>;
+  constexpr size_t smem = sizeof(Smem<NT, CW>);
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  f<<<n, kThreads, smem, s>>>(k);
+  count_product_launches(1);
+  return cudaGetLastError();
+}
+
+template <int NT, int CW>
+cudaError_t run_pass(const DgPlan& pl, const DgArgs& a, const Work& w, uint32_t r0, uint32_t pr, cudaStream_t s) {
+  unsigned char* wk = pl.work;
+  int* flag = reinterpret_cast<int*>(wk);
+  int* xmax = reinterpret_cast<int*>(wk + w.xmax) + r0;
+  int* xexp = reinterpret_cast<int*>(wk + w.xexp);
+  unsigned char* z = wk + w.z;
+  double* T = reinterpret_cast<double*>(wk + w.t);
+  const uint32_t pc = pr * CW;
+  const double* X = static_cast<const double*>(a.X) + (uint64_t)r0 * a.ldX * CW;
+  const uint64_t xr = (uint64_t)pl.n * CW, tr = (uint64_t)pl.t_rows * CW;
+  dg_xprep_kernel<NT, CW><<<(unsigned)((std::max<uint64_t>(xr, 32) + 127) / 128), 128, 0, s>>>(
+      X, a.ldX, pl.n, pc, xmax, xexp, z, flag);
+  KArgs k;
+  k.arena = pl.arena;
+  k.rowptr = pl.rowptr;
+  k.pos = pl.pos;
+  k.z = z;
+  k.xexp = xexp;
+  k.flag = flag;
+  k.T = T;
+  k.Y = static_cast<double*>(a.Y) + (uint64_t)r0 * a.ldY * CW;
+  k.ldY = a.ldY;
+  k.dre = a.dre;
+  k.dim = a.dim;
+  k.pc = pc;
+  cudaError_t e;
+  if (pl.nv) {
+    if (pl.t_split && (e = cudaMemsetAsync(T, 0, (size_t)pl.t_split * NT * 64, s)) != cudaSuccess) return e;
+    k.pieces = pl.vpieces;
+    if ((e = sweep<NT, CW, false, false>(k, pl.nv, s)) != cudaSuccess) return e;
+    dg_tprep_kernel<NT, CW><<<(unsigned)((tr + 127) / 128), 128, 0, s>>>(T, pl.t_rows, pc,
+                                                                            z + xr * (kPR<NT> * 16), flag);
+    count_product_launches(1);
+  }
+  k.pieces = pl.rpieces;
+  e = pl.rs1 ? sweep<NT, CW, true, true>(k, pl.nr, s) : sweep<NT, CW, true, false>(k, pl.nr, s);
+  if (e != cudaSuccess) return e;
+  count_product_launches(1);
+  return cudaGetLastError();
+}
+
+template <int CW>
+cudaError_t run_all(const DgPlan& pl, const DgArgs& a, const Work& w, cudaStream_t s) {
+  unsigned char* wk = pl.work;
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(wk, 0, w.xexp, s)) != cudaSuccess) return e;  // flag, column maxima
+  const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.n * CW + 1023) / 1024, 64));
+  for (uint32_t r0 = 0; r0 < a.p; r0 += 65535) {
+    const uint32_t pr = std::min<uint32_t>(a.p - r0, 65535);
+    dg_xmax_kernel<CW><<<dim3(gx, pr), 256, 0, s>>>(static_cast<const double*>(a.X) + (uint64_t)r0 * a.ldX * CW,
+                                                    a.ldX, pl.n, reinterpret_cast<int*>(wk + w.xmax) + r0,
+                                                    reinterpret_cast<int*>(wk));
+  }
+  count_product_launches(1);
+  const uint32_t per = kMaxCols / CW;
+  for (uint32_t r0 = 0; r0 < a.p; r0 += per) {
+    const uint32_t pr = std::min(per, a.p - r0);
+    e = nt_of(pr * CW) == 1 ? run_pass<1, CW>(pl, a, w, r0, pr, s) : run_pass<2, CW>(pl, a, w, r0, pr, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
+size_t dg_work_bytes(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p) { return work_of(cplx, n, t_rows, p).end; }
+
+cudaError_t launch_matvec_dg(const DgPlan& pl, const DgArgs& a, cudaStream_t s) {
+  if (a.p == 0) return cudaSuccess;
+  const Work w = work_of(a.cplx, pl.n, pl.t_rows, a.p);
+  return a.cplx ? run_all<2>(pl, a, w, s) : run_all<1>(pl, a, w, s);
+}
+
+cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cudaStream_t s) {
+  if (!nsegs) return cudaSuccess;
+  dg_expand_kernel<<<(unsigned)(((uint64_t)nsegs * 8 + 255) / 256), 256, 0, s>>>(segs, nsegs, pos);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStream_t s) {
+  if (!count) return cudaSuccess;
+  const unsigned grid = (unsigned)std::min<uint64_t>((count + 1023) / 1024, 152ull * 16);
+  dg_scan_kernel<<<grid, 256, 0, s>>>(static_cast<const uint2*>(arena), count, bad);
+  return cudaGetLastError();
+}
+
+// Two right-hand sides and 10^7 (elements x right-hand sides) on.  Below, the six
+// launches of the sliced product (34 us at least) outlast the plain kernel: 1,000
+// points (10^6 elements) take 35 us against 20 (p = 2), 38 against 41 (p = 8) and
+// 43 against 69 (p = 16).  One right-hand side leaves the FP64 pipe less work per
+// byte than the digits take: 0.99 ms against 0.64 ms (65,536 points; p = 2: 0.99
+// against 1.11 ms, p = 8: 0.99 against 4.2, p = 16: 1.41 against 8.35).
+// AHX_DG_MIN overrides the 10^7.
+bool dg_wanted(uint64_t elems, uint32_t p) {
+  const char* e = std::getenv("AHX_DG_MIN");
+  const uint64_t least = e && *e ? std::strtoull(e, nullptr, 10) : 10000000ull;
+  return p >= 2 && elems * p >= least;
+}
+
+int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,
+                     uint32_t kmax, int& finite, int device, cudaStream_t s) {
+  int rc;
+  if (finite == 0) {
+    ScopedBuf bad;
+    int b = 0;
+    if ((rc = bad.reserve(sizeof(int)))) return rc;
+    AHX_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
+    AHX_CUDA(launch_dg_scan(arena, count, bad.as<int>(), s));
+    AHX_CUDA(cudaMemcpyAsync(&b, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AHX_CUDA(cudaStreamSynchronize(s));
+    finite = b ? 2 : 1;
+  }
+  if (D.valid) return AHX_OK;
+  int sms = 0;
+  AHX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  DgHost L;
+  D.release();
+  D.valid = true;
+  if (!build_dg_layout(leaves, n, (uint32_t)std::max(sms, 1) * 16, kmax, L)) return AHX_OK;
+  D.valid = false;
+  ScopedBuf segs;
+  if ((rc = upload(D.vpieces, L.vpieces, s))) return rc;
+  if ((rc = upload(D.rpieces, L.rpieces, s))) return rc;
+  if ((rc = upload(D.rowptr, L.rowptr, s))) return rc;
+  if ((rc = upload(segs, L.segs, s))) return rc;
+  if ((rc = D.pos.reserve(std::max<uint64_t>(L.npos, 1) * sizeof(DgPos)))) return rc;
+  AHX_CUDA(launch_dg_expand(segs.as<DgSeg>(), (uint32_t)L.segs.size(), D.pos.as<DgPos>(), s));
+  AHX_CUDA(cudaStreamSynchronize(s));
+  D.nv = (uint32_t)L.vpieces.size();
+  D.nr = (uint32_t)L.rpieces.size();
+  D.t_rows = L.t_rows;
+  D.t_split = L.t_split;
+  D.rs1 = L.rs1;
+  D.valid = D.usable = true;
+  return AHX_OK;
+}
+
+DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& work) {
+  DgPlan p;
+  p.vpieces = D.vpieces.as<DgPiece>();
+  p.rpieces = D.rpieces.as<DgPiece>();
+  p.rowptr = D.rowptr.as<uint64_t>();
+  p.pos = D.pos.as<DgPos>();
+  p.nv = D.nv;
+  p.nr = D.nr;
+  p.t_rows = D.t_rows;
+  p.t_split = D.t_split;
+  p.rs1 = D.rs1;
+  p.n = n;
+  p.arena = arena;
+  p.work = static_cast<unsigned char*>(work.p);
+  return p;
+}
+
+// ---- layout --------------------------------------------------------------
+
+bool build_dg_layout(const std::vector<DgLeaf>& leaves, uint32_t n, uint32_t ctas, uint32_t kmax, DgHost& L) {
+  L = DgHost();
+  // the side a leaf reads (in) and writes (out), by its mode
+  struct Side {
+    uint32_t ib, in, ob, on;
+    uint64_t q, p;  // factor on the input / output side
+  };
+  auto side = [](const DgLeaf& l) -> Side {
+    const uint64_t u = l.off, v = l.off + (uint64_t)l.n1 * (uint32_t)std::max(l.rank, 0);
+    return l.mode == kDgN ? Side{l.b2, l.n2, l.b1, l.n1, v, u} : Side{l.b1, l.n1, l.b2, l.n2, u, v};
+  };
+  // ---- V sweep: factor columns by column cluster, long clusters first (their
+  // tiles are split along K, so their T rows come first)
+  std::vector<uint32_t> lr;
+  for (uint32_t l = 0; l < leaves.size(); ++l)
+    if (leaves[l].rank > 0) lr.push_back(l);
+  std::stable_sort(lr.begin(), lr.end(), [&](uint32_t x, uint32_t y) {
+    const Side a = side(leaves[x]), b = side(leaves[y]);
+    return a.in != b.in ? a.in > b.in : a.ib < b.ib;
+  });
+  std::vector<uint32_t> trow(leaves.size(), 0);
+  uint64_t t_rows = 0, vwork = 0;
+  for (uint32_t l : lr) t_rows += (uint32_t)leaves[l].rank;
+  if (t_rows + n > 0x3fffffffull) return false;
+  L.rowptr.reserve(t_rows);
+  struct Tile {
+    uint32_t row0, nrows, in0, K;
+  };
+  std::vector<Tile> vt;
+  for (size_t i = 0; i < lr.size();) {
+    const Side s = side(leaves[lr[i]]);
+    const uint32_t t0 = (uint32_t)L.rowptr.size();
+    for (; i < lr.size(); ++i) {
+      const DgLeaf& q = leaves[lr[i]];
+      const Side b = side(q);
+      if (b.in != s.in || b.ib != s.ib) break;
+      trow[lr[i]] = (uint32_t)L.rowptr.size();
+      // U V^H: the input factor is conjugated unless the leaf acts transposed
+      const uint64_t cj = q.mode == kDgT ? 0ull : kDgConj;
+      for (int32_t k = 0; k < q.rank; ++k) L.rowptr.push_back((b.q + (uint64_t)k * b.in) | cj);
+    }
+    const uint32_t t1 = (uint32_t)L.rowptr.size();
+    for (uint32_t t = t0; t < t1; t += kDgRows) {
+      vt.push_back({t, std::min(kDgRows, t1 - t), s.ib, s.in});
+      vwork += s.in;
+    }
+  }
+  L.t_rows = (uint32_t)t_rows;
+  // K range of a piece: enough pieces to fill the GPU several times over, long
+  // enough that a piece's start-up and its additions to T or Y stay small
+  auto piece_len = [&](uint64_t work) {
+    const uint64_t k = work / std::max<uint32_t>(ctas, 1);
+    // (the integer sums of a piece have room for 1024 real positions)
+    return (uint32_t)std::min<uint64_t>(kmax, std::max<uint64_t>(std::min(256u, kmax), (k + 63) / 64 * 64));
+  };
+  const uint32_t kv = piece_len(vwork);
+  for (const Tile& t : vt) {
+    const uint32_t np = (t.K + kv - 1) / kv;
+    if (np > 1) L.t_split = t.row0 + t.nrows;
+    for (uint32_t p = 0; p < np; ++p) {
+      const uint32_t k0 = p * kv;
+      L.vpieces.push_back({t.row0, t.nrows, k0, std::min(kv, t.K - k0), t.in0, np > 1 ? 1u : 0u, {0, 0}});
+    }
+  }
+  // ---- rows sweep: the finest row blocks, at most kDgRows rows each
+  std::vector<uint32_t> bd{0u, n};
+  for (const DgLeaf& q : leaves)
+    if (q.rank != 0) {
+      const Side s = side(q);
+      bd.push_back(s.ob);
+      bd.push_back(s.ob + s.on);
+    }
+  std::sort(bd.begin(), bd.end());
+  bd.erase(std::unique(bd.begin(), bd.end()), bd.end());
+  std::vector<uint32_t> bs;
+  for (size_t i = 0; i + 1 < bd.size(); ++i) {
+    const uint32_t len = bd[i + 1] - bd[i];
+    // parts of whole 16-row fragments (only the last one ragged)
+    const uint32_t np = (len + kDgRows - 1) / kDgRows, fr = ((len + 15) / 16 + np - 1) / np * 16;
+    for (uint32_t r = 0; r < len; r += fr) bs.push_back(bd[i] + r);
+  }
+  bs.push_back(n);
+  const size_t nb = bs.size() - 1;
+  std::vector<uint32_t> first(nb + 1, 0);
+  auto each_block = [&](auto&& f) {
+    // low-rank leaves first: the dense ones hold a row's largest entries, and
+    // what a row has met before them keeps its own, finer scale
+    for (int pass = 0; pass < 2; ++pass)
+      for (uint32_t l = 0; l < leaves.size(); ++l) {
+        if (leaves[l].rank == 0 || (leaves[l].rank < 0) != (pass == 1)) continue;
+        const Side s = side(leaves[l]);
+        size_t i = (size_t)(std::lower_bound(bs.begin(), bs.end(), s.ob) - bs.begin());
+        for (; i < nb && bs[i] < s.ob + s.on; ++i) f(l, s, i);
+      }
+  };
+  each_block([&](uint32_t, const Side&, size_t i) { ++first[i + 1]; });
+  for (size_t i = 0; i < nb; ++i) first[i + 1] += first[i];
+  L.segs.resize(first[nb]);
+  {
+    std::vector<uint32_t> at(first.begin(), first.end() - 1);
+    each_block([&](uint32_t l, const Side& s, size_t i) {
+      const DgLeaf& q = leaves[l];
+      const uint32_t r = bs[i] - s.ob;
+      DgSeg g{};
+      if (q.rank > 0) {
+        // U V^H: only the transposed leaf conj(V) U^T conjugates its output factor
+        g = DgSeg{s.p + r, s.on, 1u | (q.mode == kDgT ? 0x80000000u : 0u), (uint32_t)q.rank, n + trow[l], 0u, 0u};
+      } else if (q.mode == kDgN) {
+        g = DgSeg{q.off + r, q.n1, 1u, q.n2, q.b2, 0u, 0u};
+      } else {
+        L.rs1 = false;
+        g = DgSeg{q.off + (uint64_t)r * q.n1, 1u, q.n1 | (q.mode == kDgH ? 0x80000000u : 0u), q.n1, q.b1, 0u, 0u};
+      }
+      L.segs[at[i]++] = g;
+    });
+  }
+  uint64_t npos = 0;
+  std::vector<uint64_t> bpos(nb + 1, 0);
+  for (size_t i = 0; i < nb; ++i) {
+    for (uint32_t s = first[i]; s < first[i + 1]; ++s) {
+      L.segs[s].pos0 = (uint32_t)npos;
+      npos += L.segs[s].kn;
+      if (npos > 0xffffffffull) return false;
+    }
+    bpos[i + 1] = npos;
+  }
+  L.npos = npos;
+  const uint32_t kr = piece_len(npos);
+  for (size_t i = 0; i < nb; ++i)
+    for (uint64_t k = bpos[i]; k < bpos[i + 1]; k += kr)
+      L.rpieces.push_back({bs[i], bs[i + 1] - bs[i], (uint32_t)k, (uint32_t)std::min<uint64_t>(kr, bpos[i + 1] - k),
+                           0u, 0u, {0, 0}});
+  return true;
+}
+
+}  // namespace ahx
+
+// Test hook (not part of the drop-in interface): Y += op(A) X through the layout
+// of the digit-sliced product, evaluated on the host in FP64 piece by piece as the
+// sweeps do.  leaves: 6 words per leaf (b1, n1, b2, n2, rank, DgMode), offs:
+// element offsets, cplx: complex elements (re, im).  info[4] = {V pieces, rows
+// pieces, T rows, rows of the widest tile}.
+extern "C" int ahx_dg_host_product(uint32_t n, uint32_t nleaves, const uint32_t* leaves, const uint64_t* offs,
+                                   const double* arena, int cplx, uint32_t p, const double* X, double* Y,
+                                   uint64_t* info, uint32_t ctas) {
+  if (!leaves || !offs || !arena || !X || !Y || !info) return 2;
+  std::vector<ahx::DgLeaf> lv(nleaves);
+  for (uint32_t l = 0; l < nleaves; ++l) {
+    const uint32_t* w = leaves + 6 * (size_t)l;
+    lv[l] = ahx::DgLeaf{w[0], w[1], w[2], w[3], (int32_t)w[4], w[5], offs[l]};
+  }
+  ahx::DgHost L;
+  if (!ahx::build_dg_layout(lv, n, ctas, cplx ? ahx::kDgK / 2 : ahx::kDgK, L)) return 1;
+  const uint32_t cw = cplx ? 2 : 1;
+  // z (re, im) += op(element) * x, op: conjugation
+  auto madd = [&](double* z, uint64_t e, bool cj, const double* x) {
+    if (!cplx) {
+      z[0] += arena[e] * x[0];
+      return;
+    }
+    const double re = arena[2 * e], im = cj ? -arena[2 * e + 1] : arena[2 * e + 1];
+    z[0] += re * x[0] - im * x[1];
+    z[1] += re * x[1] + im * x[0];
+  };
+  std::vector<double> T((size_t)L.t_rows * p * cw, 0.0);
+  std::vector<ahx::DgPos> pos(L.npos);
+  for (const ahx::DgSeg& g : L.segs)
+    for (uint32_t k = 0; k < g.kn; ++k) pos[g.pos0 + k] = ahx::DgPos{g.base + (uint64_t)k * g.ldk, g.z + k, g.rsf};
+  for (const ahx::DgPiece& q : L.vpieces) {
+    if (!q.add && q.row0 < L.t_split) return 3;  // rows that are stored, not added to
+    for (uint32_t r = 0; r < q.nrows; ++r) {
+      const uint64_t w = L.rowptr[q.row0 + r];
+      for (uint32_t k = q.k0; k < q.k0 + q.kn; ++k)
+        for (uint32_t j = 0; j < p; ++j)
+          madd(&T[((size_t)(q.row0 + r) * p + j) * cw], (w & ~ahx::kDgConj) + k, (w & ahx::kDgConj) != 0,
+               X + ((size_t)j * n + q.in0 + k) * cw);
+    }
+  }
+  info[3] = 0;
+  for (const ahx::DgPiece& q : L.rpieces) {
+    info[3] = std::max<uint64_t>(info[3], q.nrows);
+    for (uint32_t k = q.k0; k < q.k0 + q.kn; ++k)
+      for (uint32_t r = 0; r < q.nrows; ++r)
+        for (uint32_t j = 0; j < p; ++j) {
+          const ahx::DgPos& P = pos[k];
+          if (L.rs1 && (P.rsf & 0x7fffffffu) != 1) return 4;
+          const double* x = P.z < n ? X + ((size_t)j * n + P.z) * cw : &T[((size_t)(P.z - n) * p + j) * cw];
+          madd(Y + ((size_t)j * n + q.row0 + r) * cw, P.off + (uint64_t)r * (P.rsf & 0x7fffffffu), (P.rsf >> 31) != 0,
+               x);
+        }
+  }
+  info[0] = L.vpieces.size();
+  info[1] = L.rpieces.size();
+  info[2] = L.t_rows;
+  return 0;
+}

@@ -74,11 +74,8 @@ __device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, u
 }
 
 template <typename S, typename R, int PG, int OP>
-__global__ void __launch_bounds__(kThreads) zmv_kernel(ZArgs a) {
-  __shared__ C2<R> Xs[kCh][PG];
-  __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
-  __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
-  const MvLeaf L = a.leaves[a.order[blockIdx.x]];
+__device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
+  const MvLeaf L = a.leaves[a.order[leaf]];
   const S* base = reinterpret_cast<const S*>(a.arena) + L.off;
   const uint32_t tid = threadIdx.x;
   constexpr bool kFwd = OP == kZOpN;
@@ -177,14 +174,31 @@ __global__ void __launch_bounds__(kThreads) zmv_kernel(ZArgs a) {
   }
 }
 
+template <typename S, typename R, int PG, int OP, bool GUARD>
+__global__ void __launch_bounds__(kThreads) zmv_kernel(ZArgs a) {
+  __shared__ C2<R> Xs[kCh][PG];
+  __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
+  __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
+  if (GUARD) {
+    if (*a.guard == 0) return;
+    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP>(a, l, Xs, Ts, red);
+  } else {
+    zmv_leaf<S, R, PG, OP>(a, blockIdx.x, Xs, Ts, red);
+  }
+}
+
 template <typename S, typename R, int OP>
 void launch_op(const ZArgs& a, cudaStream_t s) {
+  if (a.guard) {
+    zmv_kernel<S, R, 4, OP, true><<<std::min(a.nleaves, 1024u), kThreads, 0, s>>>(a);
+    return;
+  }
   const uint32_t grid = a.nleaves;
-  if (a.p == 1) zmv_kernel<S, R, 1, OP><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) zmv_kernel<S, R, 2, OP><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) zmv_kernel<S, R, 4, OP><<<grid, kThreads, 0, s>>>(a);
+  if (a.p == 1) zmv_kernel<S, R, 1, OP, false><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p == 2) zmv_kernel<S, R, 2, OP, false><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 4) zmv_kernel<S, R, 4, OP, false><<<grid, kThreads, 0, s>>>(a);
   // wider groups (16) measured slower: fewer columns per pass, lower occupancy
-  else zmv_kernel<S, R, 8, OP><<<grid, kThreads, 0, s>>>(a);
+  else zmv_kernel<S, R, 8, OP, false><<<grid, kThreads, 0, s>>>(a);
 }
 
 template <typename S, typename R>

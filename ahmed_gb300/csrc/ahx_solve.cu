@@ -293,7 +293,13 @@ struct HmatOp : Operator {
   }
   uint64_t product_bytes(int prec) const override { return H->prod[prec].bytes; }
   int prepare(int prec, uint32_t p) override {
-    int rc = prepare_product(H, prec);
+    int rc;
+    if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) {
+      bool usable = false;
+      if ((rc = prepare_dg(H, p, false, usable))) return rc;
+      if (usable) prec = kFP64;
+    }
+    rc = prepare_product(H, prec);
     if (rc || prec != kDF64) return rc;
     return prepare_df_x(H->prod[kDF64], ntot, p);
   }

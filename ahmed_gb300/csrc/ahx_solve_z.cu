@@ -359,6 +359,32 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     return AHX_OK;
   }
   if (H->tree.sym) op = kZOpN;  // A^T = A
+  // several right-hand sides on the complex128 leaves: the digit-sliced product;
+  // the plain kernels then only run when X does not fit the digits
+  const int* guard = nullptr;
+  if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p)) {
+    DgState& D = Z.dg[op];
+    if (!D.valid) {
+      const auto& Ls = H->tree.leaves;
+      const uint32_t mode = op == kZOpN ? kDgN : op == kZOpT ? kDgT : kDgH;
+      std::vector<DgLeaf> lv;
+      lv.reserve(Ls.size());
+      for (uint32_t l = 0; l < (uint32_t)Ls.size(); ++l) {
+        if (Z.rank[l] == 0) continue;
+        const Leaf& L = Ls[l];
+        lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], mode, Z.off[l]});
+        if (H->tree.sym && L.b1 != L.b2) lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], kDgT, Z.off[l]});
+      }
+      if ((rc = dg_prepare_state(D, lv, H->tree.n, Z.arena.p, 2 * Z.elems, kDgK / 2, Z.finite, H->device, H->stream)))
+        return rc;
+    }
+    if (D.usable && Z.finite == 1) {
+      if ((rc = H->dg_work.reserve(dg_work_bytes(true, H->tree.n, D.t_rows, p)))) return rc;
+      const DgPlan pl = dg_plan(D, H->tree.n, Z.arena.p, H->dg_work);
+      AHX_CUDA(launch_matvec_dg(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
+      guard = dg_flag(pl);
+    }
+  }
   ZArgs a;
   a.leaves = H->z.leaves.as<MvLeaf>();
   a.order = H->z.order.as<uint32_t>();
@@ -373,6 +399,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.Y = Y;
   a.ldY = ldY;
   a.op = op;
+  a.guard = guard;
   AHX_CUDA(launch_matvec_z(a, H->stream));
   if (Z.ntleaves) {
     // the blocks below the diagonal: the upper ones transposed
