@@ -594,9 +594,11 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     return AHX_OK;
   }
   // FP64 and its double-float stand-in: the digit-sliced product where it is the
-  // faster one; the plain kernel then only runs when X was not finite
+  // faster one; the plain kernel then only runs when X does not fit the digits
+  // (double-float would need a copy of the leaves: there always)
   const int* guard = nullptr;
-  if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) {
+  if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2 &&
+      (prec == kDF64 || dg_due(H->dg[transposed ? 1 : 0], H->arena64_elems, p, H->tree.leaves.size()))) {
     bool usable = false;
     if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
     if (usable) {

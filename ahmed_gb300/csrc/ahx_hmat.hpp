@@ -84,12 +84,14 @@ struct ProdCopy {
 struct DgState {
   bool valid = false;   // built (usable or not)
   bool usable = false;  // the layout's indices fit
+  double spent = 0.0;   // estimated us of the plain products before the layout
   DevBuf vpieces, rpieces, rowptr, pos;
   uint32_t nv = 0, nr = 0, t_rows = 0, t_split = 0;
   bool rs1 = true;
   void release() {
     for (DevBuf* b : {&vpieces, &rpieces, &rowptr, &pos}) b->release();
     valid = usable = false;
+    spent = 0.0;
   }
 };
 
@@ -212,6 +214,10 @@ bool um_enabled();
 // Whether p right-hand sides on leaves of `elems` real elements go through the
 // digit-sliced product.
 bool dg_wanted(uint64_t elems, uint32_t p);
+// Whether a product (of dg_wanted's size) should run sliced now: always once the
+// layout exists; before, when the plain products so far and this one cost as much
+// as the layout does.
+bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves);
 // Builds the layout of `leaves`; looks at the arena's elements once (finite).
 // count: its doubles.
 int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,

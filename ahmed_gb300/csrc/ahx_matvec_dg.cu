@@ -765,11 +765,24 @@ cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStre
 // 43 against 69 (p = 16).  One right-hand side leaves the FP64 pipe less work per
 // byte than the digits take: 0.99 ms against 0.64 ms (65,536 points; p = 2: 0.99
 // against 1.11 ms, p = 8: 0.99 against 4.2, p = 16: 1.41 against 8.35).
-// AHX_DG_MIN overrides the 10^7.
+// AHX_DG_MIN overrides the 10^7 (and lays out at the first product).
 bool dg_wanted(uint64_t elems, uint32_t p) {
   const char* e = std::getenv("AHX_DG_MIN");
   const uint64_t least = e && *e ? std::strtoull(e, nullptr, 10) : 10000000ull;
   return p >= 2 && elems * p >= least;
+}
+
+// A single product gains less than the layout takes (about 0.3 ms and 55 ns per
+// leaf: 1.9 ms in all against 1.1 ms of the plain kernel for 20,011 points and five
+// right-hand sides, 25,000 leaves), so a handle that multiplies once stays with the
+// plain kernel (2 p FP64 operations per element at 1 TFLOP/s); one that goes on
+// never spends more than about twice the better choice.
+bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves) {
+  if (D.valid || std::getenv("AHX_DG_MIN")) return true;
+  const double plain = 2e-6 * (double)elems * p, layout = 300.0 + 0.055 * (double)nleaves;
+  if (D.spent + plain >= layout) return true;
+  D.spent += plain;
+  return false;
 }
 
 int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,
@@ -840,41 +853,61 @@ bool build_dg_layout(const std::vector<DgLeaf>& leaves, uint32_t n, uint32_t cta
     const uint64_t u = l.off, v = l.off + (uint64_t)l.n1 * (uint32_t)std::max(l.rank, 0);
     return l.mode == kDgN ? Side{l.b2, l.n2, l.b1, l.n1, v, u} : Side{l.b1, l.n1, l.b2, l.n2, u, v};
   };
+  const uint32_t nl = (uint32_t)leaves.size();
+  std::vector<Side> sd(nl);
+  for (uint32_t l = 0; l < nl; ++l) sd[l] = side(leaves[l]);
   // ---- V sweep: factor columns by column cluster, long clusters first (their
-  // tiles are split along K, so their T rows come first)
-  std::vector<uint32_t> lr;
-  for (uint32_t l = 0; l < leaves.size(); ++l)
-    if (leaves[l].rank > 0) lr.push_back(l);
-  std::stable_sort(lr.begin(), lr.end(), [&](uint32_t x, uint32_t y) {
-    const Side a = side(leaves[x]), b = side(leaves[y]);
-    return a.in != b.in ? a.in > b.in : a.ib < b.ib;
-  });
-  std::vector<uint32_t> trow(leaves.size(), 0);
+  // tiles are split along K, so their T rows come first).  Clusters are found by
+  // their first row (a short list per row: one entry per level), the leaves of a
+  // cluster stay in leaf order.
+  struct Cluster {
+    uint32_t ib, in, rows, next;  // next: the next cluster with this first row + 1
+  };
+  std::vector<Cluster> cl;
+  std::vector<uint32_t> head(n, 0u), of(nl, 0u);
   uint64_t t_rows = 0, vwork = 0;
-  for (uint32_t l : lr) t_rows += (uint32_t)leaves[l].rank;
+  for (uint32_t l = 0; l < nl; ++l) {
+    if (leaves[l].rank <= 0) continue;
+    const Side& q = sd[l];
+    uint32_t c = head[q.ib];
+    while (c && cl[c - 1].in != q.in) c = cl[c - 1].next;
+    if (!c) {
+      cl.push_back({q.ib, q.in, 0u, head[q.ib]});
+      c = head[q.ib] = (uint32_t)cl.size();
+    }
+    of[l] = c - 1;
+    cl[c - 1].rows += (uint32_t)leaves[l].rank;
+    t_rows += (uint32_t)leaves[l].rank;
+  }
   if (t_rows + n > 0x3fffffffull) return false;
-  L.rowptr.reserve(t_rows);
+  std::vector<uint32_t> ord(cl.size()), at(cl.size());
+  for (uint32_t c = 0; c < ord.size(); ++c) ord[c] = c;
+  std::sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) {
+    return cl[x].in != cl[y].in ? cl[x].in > cl[y].in : cl[x].ib < cl[y].ib;
+  });
   struct Tile {
     uint32_t row0, nrows, in0, K;
   };
   std::vector<Tile> vt;
-  for (size_t i = 0; i < lr.size();) {
-    const Side s = side(leaves[lr[i]]);
-    const uint32_t t0 = (uint32_t)L.rowptr.size();
-    for (; i < lr.size(); ++i) {
-      const DgLeaf& q = leaves[lr[i]];
-      const Side b = side(q);
-      if (b.in != s.in || b.ib != s.ib) break;
-      trow[lr[i]] = (uint32_t)L.rowptr.size();
-      // U V^H: the input factor is conjugated unless the leaf acts transposed
-      const uint64_t cj = q.mode == kDgT ? 0ull : kDgConj;
-      for (int32_t k = 0; k < q.rank; ++k) L.rowptr.push_back((b.q + (uint64_t)k * b.in) | cj);
+  uint32_t t0 = 0;
+  for (uint32_t c : ord) {
+    at[c] = t0;
+    for (uint32_t t = 0; t < cl[c].rows; t += kDgRows) {
+      vt.push_back({t0 + t, std::min(kDgRows, cl[c].rows - t), cl[c].ib, cl[c].in});
+      vwork += cl[c].in;
     }
-    const uint32_t t1 = (uint32_t)L.rowptr.size();
-    for (uint32_t t = t0; t < t1; t += kDgRows) {
-      vt.push_back({t, std::min(kDgRows, t1 - t), s.ib, s.in});
-      vwork += s.in;
-    }
+    t0 += cl[c].rows;
+  }
+  std::vector<uint32_t> trow(nl, 0u);
+  L.rowptr.resize(t_rows);
+  for (uint32_t l = 0; l < nl; ++l) {
+    const DgLeaf& q = leaves[l];
+    if (q.rank <= 0) continue;
+    const uint32_t t = trow[l] = at[of[l]];
+    at[of[l]] += (uint32_t)q.rank;
+    // U V^H: the input factor is conjugated unless the leaf acts transposed
+    const uint64_t cj = q.mode == kDgT ? 0ull : kDgConj;
+    for (int32_t k = 0; k < q.rank; ++k) L.rowptr[t + k] = (sd[l].q + (uint64_t)k * sd[l].in) | cj;
   }
   L.t_rows = (uint32_t)t_rows;
   // K range of a piece: enough pieces to fill the GPU several times over, long
@@ -894,70 +927,94 @@ bool build_dg_layout(const std::vector<DgLeaf>& leaves, uint32_t n, uint32_t cta
     }
   }
   // ---- rows sweep: the finest row blocks, at most kDgRows rows each
-  std::vector<uint32_t> bd{0u, n};
-  for (const DgLeaf& q : leaves)
-    if (q.rank != 0) {
-      const Side s = side(q);
-      bd.push_back(s.ob);
-      bd.push_back(s.ob + s.on);
-    }
-  std::sort(bd.begin(), bd.end());
-  bd.erase(std::unique(bd.begin(), bd.end()), bd.end());
+  std::vector<uint32_t> blk(n + 1, 0u);  // first row of a block -> its number
+  blk[0] = 1;
+  for (uint32_t l = 0; l < nl; ++l)
+    if (leaves[l].rank != 0) blk[sd[l].ob] = blk[sd[l].ob + sd[l].on] = 1;
   std::vector<uint32_t> bs;
-  for (size_t i = 0; i + 1 < bd.size(); ++i) {
-    const uint32_t len = bd[i + 1] - bd[i];
+  for (uint32_t r = 0; r < n;) {
+    uint32_t e = r + 1;
+    while (e < n && !blk[e]) ++e;
     // parts of whole 16-row fragments (only the last one ragged)
-    const uint32_t np = (len + kDgRows - 1) / kDgRows, fr = ((len + 15) / 16 + np - 1) / np * 16;
-    for (uint32_t r = 0; r < len; r += fr) bs.push_back(bd[i] + r);
+    const uint32_t len = e - r, np = (len + kDgRows - 1) / kDgRows, fr = ((len + 15) / 16 + np - 1) / np * 16;
+    blk[r] = (uint32_t)bs.size();
+    for (uint32_t q = 0; q < len; q += fr) bs.push_back(r + q);
+    r = e;
   }
+  const uint32_t nb = (uint32_t)bs.size();
+  blk[n] = nb;
   bs.push_back(n);
-  const size_t nb = bs.size() - 1;
-  std::vector<uint32_t> first(nb + 1, 0);
-  auto each_block = [&](auto&& f) {
-    // low-rank leaves first: the dense ones hold a row's largest entries, and
-    // what a row has met before them keeps its own, finer scale
-    for (int pass = 0; pass < 2; ++pass)
-      for (uint32_t l = 0; l < leaves.size(); ++l) {
-        if (leaves[l].rank == 0 || (leaves[l].rank < 0) != (pass == 1)) continue;
-        const Side s = side(leaves[l]);
-        size_t i = (size_t)(std::lower_bound(bs.begin(), bs.end(), s.ob) - bs.begin());
-        for (; i < nb && bs[i] < s.ob + s.on; ++i) f(l, s, i);
-      }
-  };
-  each_block([&](uint32_t, const Side&, size_t i) { ++first[i + 1]; });
-  for (size_t i = 0; i < nb; ++i) first[i + 1] += first[i];
-  L.segs.resize(first[nb]);
-  {
-    std::vector<uint32_t> at(first.begin(), first.end() - 1);
-    each_block([&](uint32_t l, const Side& s, size_t i) {
-      const DgLeaf& q = leaves[l];
-      const uint32_t r = bs[i] - s.ob;
-      DgSeg g{};
-      if (q.rank > 0) {
-        // U V^H: only the transposed leaf conj(V) U^T conjugates its output factor
-        g = DgSeg{s.p + r, s.on, 1u | (q.mode == kDgT ? 0x80000000u : 0u), (uint32_t)q.rank, n + trow[l], 0u, 0u};
-      } else if (q.mode == kDgN) {
-        g = DgSeg{q.off + r, q.n1, 1u, q.n2, q.b2, 0u, 0u};
-      } else {
-        L.rs1 = false;
-        g = DgSeg{q.off + (uint64_t)r * q.n1, 1u, q.n1 | (q.mode == kDgH ? 0x80000000u : 0u), q.n1, q.b1, 0u, 0u};
-      }
-      L.segs[at[i]++] = g;
-    });
+  // segments and positions per block, by differences over the blocks of each leaf;
+  // low-rank leaves first: the dense ones hold a row's largest entries, and what
+  // a row has met before them keeps its own, finer scale
+  std::vector<uint32_t> seg[2] = {std::vector<uint32_t>(nb + 1, 0u), std::vector<uint32_t>(nb + 1, 0u)};
+  std::vector<uint64_t> kat[2] = {std::vector<uint64_t>(nb + 1, 0ull), std::vector<uint64_t>(nb + 1, 0ull)};
+  auto kn_of = [](const DgLeaf& q) { return q.rank > 0 ? (uint32_t)q.rank : q.mode == kDgN ? q.n2 : q.n1; };
+  for (uint32_t l = 0; l < nl; ++l) {
+    const DgLeaf& q = leaves[l];
+    if (q.rank == 0) continue;
+    const uint32_t d = q.rank < 0, i0 = blk[sd[l].ob], i1 = blk[sd[l].ob + sd[l].on];
+    ++seg[d][i0];
+    --seg[d][i1];
+    kat[d][i0] += kn_of(q);
+    kat[d][i1] -= kn_of(q);
   }
-  uint64_t npos = 0;
-  std::vector<uint64_t> bpos(nb + 1, 0);
-  for (size_t i = 0; i < nb; ++i) {
-    for (uint32_t s = first[i]; s < first[i + 1]; ++s) {
-      L.segs[s].pos0 = (uint32_t)npos;
-      npos += L.segs[s].kn;
-      if (npos > 0xffffffffull) return false;
+  std::vector<uint64_t> bpos(nb + 1, 0ull);
+  uint64_t npos = 0, nsegs = 0;
+  uint32_t run[2] = {0u, 0u};
+  uint64_t krun[2] = {0ull, 0ull};
+  for (uint32_t i = 0; i < nb; ++i) {
+    bpos[i] = npos;
+    for (int d = 0; d < 2; ++d) {
+      run[d] += seg[d][i];
+      krun[d] += kat[d][i];
+      seg[d][i] = (uint32_t)nsegs;
+      kat[d][i] = npos;
+      nsegs += run[d];
+      npos += krun[d];
     }
-    bpos[i + 1] = npos;
+    if (npos > 0xffffffffull) return false;
   }
+  bpos[nb] = npos;
   L.npos = npos;
+  L.segs.resize(nsegs);
+  for (uint32_t l = 0; l < nl; ++l) {
+    const DgLeaf& q = leaves[l];
+    if (q.rank == 0) continue;
+    const Side& s = sd[l];
+    const uint32_t d = q.rank < 0, kn = kn_of(q), i1 = blk[s.ob + s.on];
+    DgSeg g{};
+    g.kn = kn;
+    uint64_t step = 1;  // of base per row
+    if (q.rank > 0) {
+      // U V^H: only the transposed leaf conj(V) U^T conjugates its output factor
+      g.base = s.p;
+      g.ldk = s.on;
+      g.rsf = 1u | (q.mode == kDgT ? 0x80000000u : 0u);
+      g.z = n + trow[l];
+    } else if (q.mode == kDgN) {
+      g.base = q.off;
+      g.ldk = q.n1;
+      g.rsf = 1u;
+      g.z = q.b2;
+    } else {
+      L.rs1 = false;
+      g.base = q.off;
+      g.ldk = 1u;
+      g.rsf = q.n1 | (q.mode == kDgH ? 0x80000000u : 0u);
+      g.z = q.b1;
+      step = q.n1;
+    }
+    const uint64_t base = g.base;
+    for (uint32_t i = blk[s.ob]; i < i1; ++i) {
+      g.base = base + (bs[i] - s.ob) * step;
+      g.pos0 = (uint32_t)kat[d][i];
+      kat[d][i] += kn;
+      L.segs[seg[d][i]++] = g;
+    }
+  }
   const uint32_t kr = piece_len(npos);
-  for (size_t i = 0; i < nb; ++i)
+  for (uint32_t i = 0; i < nb; ++i)
     for (uint64_t k = bpos[i]; k < bpos[i + 1]; k += kr)
       L.rpieces.push_back({bs[i], bs[i + 1] - bs[i], (uint32_t)k, (uint32_t)std::min<uint64_t>(kr, bpos[i + 1] - k),
                            0u, 0u, {0, 0}});

@@ -362,7 +362,8 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   // several right-hand sides on the complex128 leaves: the digit-sliced product;
   // the plain kernels then only run when X does not fit the digits
   const int* guard = nullptr;
-  if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p)) {
+  if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) &&
+      dg_due(Z.dg[op], 4 * Z.elems, p, H->tree.leaves.size())) {
     DgState& D = Z.dg[op];
     if (!D.valid) {
       const auto& Ls = H->tree.leaves;
