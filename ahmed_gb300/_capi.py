@@ -90,6 +90,7 @@ SIGNATURES = [
     ("ahx_mlp_nparams", _u32, []),
     ("ahx_mlp_create", _i32, [_i32, _u64, _vp]),
     ("ahx_mlp_destroy", _i32, [_vp]),
+    ("ahx_mlp_moments", _i32, [_vp, _u32, _vp, _vp]),
     ("ahx_mlp_get_params", _i32, [_vp, _vp]),
     ("ahx_mlp_set_params", _i32, [_vp, _vp]),
     ("ahx_mlp_set_norm", _i32, [_vp, _vp, _vp]),

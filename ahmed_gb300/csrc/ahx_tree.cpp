@@ -287,6 +287,20 @@ void build_tree(Tree& T, const double* pts, uint32_t n, int kind, uint32_t bmin,
   else B.subdivide(root, root);
 }
 
+void column_moments(const float* x, uint32_t n, float mean[8], float stdev[8]) {
+  float s[8] = {};
+  for (uint32_t i = 0; i < n; ++i)
+    for (int j = 0; j < 8; ++j) s[j] += x[8 * (size_t)i + j];
+  for (int j = 0; j < 8; ++j) mean[j] = s[j] / (float)n;
+  float v[8] = {};
+  for (uint32_t i = 0; i < n; ++i)
+    for (int j = 0; j < 8; ++j) {
+      const float d = x[8 * (size_t)i + j] - mean[j];
+      v[j] += d * d;
+    }
+  for (int j = 0; j < 8; ++j) stdev[j] = std::sqrt(v[j] / (float)n);
+}
+
 void leaf_features(const Tree& T, const Leaf& L, double wavenumber, double eps, float out[8]) {
   const ClusterNode& a = T.nodes[L.row_cl];
   const ClusterNode& b = T.nodes[L.col_cl];

@@ -57,6 +57,10 @@ void build_tree(Tree& T, const double* pts, uint32_t n, int kind, uint32_t bmin,
 // sum order); *min_out (if given) receives the smallest one.
 double mean_nn(const double* pts, uint32_t n, double* min_out = nullptr);
 
+// Column means and standard deviations of n x 8 floats (rows contiguous), summed
+// row by row in single precision.
+void column_moments(const float* x, uint32_t n, float mean[8], float stdev[8]);
+
 // Geometric features of a leaf for the rank predictor (8 floats):
 //   log diam(row cluster), log diam(col cluster), log centre distance,
 //   min(diam) / distance, log n1, log n2, wavenumber * max(diam), -log10(eps)

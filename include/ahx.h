@@ -289,6 +289,8 @@ int ahx_mlp_destroy(ahx_mlp* M);
 int ahx_mlp_get_params(const ahx_mlp* M, float* out);
 int ahx_mlp_set_params(ahx_mlp* M, const float* in);
 int ahx_mlp_set_norm(ahx_mlp* M, const float* mean8, const float* std8);
+/* column means and standard deviations of X (host, n x 8), summed row by row in FP32 */
+int ahx_mlp_moments(const float* X, uint32_t n, float* mean8, float* std8);
 /* gradient of the mean squared error over n samples (host X n x 8, Y n) */
 int ahx_mlp_gradients(ahx_mlp* M, const float* X, const float* Y, uint32_t n, float* grad,
                       float* loss);
