@@ -1,405 +1,22 @@
-// Batched adaptive cross approximation (ACA) with SVD recompression, FP64.
-//
-// One cooperative group per admissible leaf: a warp for leaves up to 256 rows
-// and columns, a whole CTA for larger ones.  Every per-index array (rows of U,
-// the row counters Z, columns of V, the column counters S) is owned by the
-// thread with index % G == rank, so the only cross-thread traffic is through
-// the group's all-reduces plus one barrier per cross.
-//
-// Algorithm (same control flow, same stopping rule and counters as the
-// reference):
-//   ACA row/column steps      Include/ACA.h:29-213
-//   ACA driver                Include/ACA.h:217-350
-//   leaf policy (maxk, i0)    Include/apprx.h:136-172
-//   recompression addtrll     H/mblock_D.cpp:356-465 (Householder QR in place of
-//                             dgeqrf/dormqr, one-sided Jacobi in place of dgesvd)
+// Laplace assembly: the ACA launch over admissible leaves (ahx_lowrank.cuh; leaf policy
+// Include/apprx.h:136-172), dense and mirrored leaves, the recompression of unions of
+// leaves (agglomeration), and the ACA of one block without device allocation.
 #include <climits>
 #include <mutex>
 #include <string>
 
 #include "ahx_aca.cuh"
 #include "ahx_hmat.hpp"
+#include "ahx_lowrank.cuh"
 
 namespace ahx {
 namespace {
 
 constexpr int KSM = 32;        // ranks up to KSM keep the k x k SVD in shared memory
 constexpr int LDS = KSM + 1;   // padded row stride of the shared k x k arrays
-constexpr int kSmallWarps = 4; // warps (= leaves) per CTA of the small-leaf kernel
 
 // per-group shared scratch (doubles)
 constexpr int kSmemPerGroup = 2 * KSM * LDS + KSM + 2 * KSM + KSM;
-
-struct Blk {
-  PointsSoA P;
-  double diag;
-  uint32_t b1, n1, b2, n2;
-  double* U;
-  double* V;
-  int* Z;
-  int* S;
-};
-
-template <class Grp>
-__device__ __forceinline__ bool owns(const Grp& g, uint32_t i, int G) {
-  return (i % (uint32_t)G) == g.rank;
-}
-
-// next index >= j (cyclic) whose counter is not -1 (ACA.h:29-36)
-template <int G, class Grp>
-__device__ uint32_t nexti(const Grp& g, const int* Z, uint32_t n, uint32_t j) {
-  uint32_t d = 0xffffffffu;
-  for (uint32_t i = g.rank; i < n; i += G)
-    if (Z[i] != -1) d = min(d, i >= j ? i - j : i + n - j);
-  d = g.umin(d);
-  return d == 0xffffffffu ? j : (j + d) % n;
-}
-
-// ACA_row_step (ACA.h:46-130)
-template <int G, class Grp>
-__device__ bool row_step(const Grp& g, const Blk& B, uint32_t& klast, uint32_t& i0, uint32_t k,
-                         uint32_t& no, double& nrmlsk2, double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  double* const pu = B.U + (size_t)k * n1;
-  double* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    g.sync();
-    const uint32_t gi = B.b1 + i0;
-    const double xi = B.P.x[gi], yi = B.P.y[gi], zi = B.P.z[gi];
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t j = g.rank; j < n2; j += G) {
-      double v = lap_entry_aca(B.P, gi, B.b2 + j, xi, yi, zi, B.diag);
-      for (uint32_t l = 0; l < k; ++l) v = fma(-B.U[(size_t)l * n1 + i0], B.V[(size_t)l * n2 + j], v);
-      pv[j] = v;
-      if (B.S[j] >= 0) {
-        const double a = fabs(v);
-        if (gt_nonneg(a, am.v)) am = ArgMax{a, j, v};
-      }
-    }
-    am = g.argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (owns(g, i0, G)) B.Z[i0] = -1;
-    if (++no >= n1) return false;
-    g.sync();
-    i0 = nexti<G>(g, B.Z, n1, i0);
-  }
-  const uint32_t j0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const double sca = sqrtpiv / am.sv;
-  const double thr = 1e-8 * scale * sqrtpiv;
-  double nrmv2 = 0.0;
-  for (uint32_t j = g.rank; j < n2; j += G) {
-    if (B.S[j] >= 0) {
-      const double e = pv[j] * sca;
-      pv[j] = e;
-      nrmv2 += e * e;
-      if (gt_nonneg(fabs(e), thr)) ++B.S[j];
-    }
-  }
-  const uint32_t gj = B.b2 + j0;
-  const double xj = B.P.x[gj], yj = B.P.y[gj], zj = B.P.z[gj];
-  for (uint32_t i = g.rank; i < n1; i += G) {
-    double u = lap_entry_aca(B.P, gj, B.b1 + i, xj, yj, zj, B.diag);
-    for (uint32_t l = 0; l < k; ++l) u = fma(-B.V[(size_t)l * n2 + j0], B.U[(size_t)l * n1 + i], u);
-    pu[i] = u;
-  }
-  klast = (uint32_t)g.imax(owns(g, i0, G) ? B.Z[i0] : INT_MIN);
-  if (owns(g, i0, G)) B.Z[i0] = -1;
-  if (owns(g, j0, G)) B.S[j0] = -1;
-  ++no;
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmu2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t i = g.rank; i < n1; i += G) {
-    const double e = pu[i] * dsca;
-    pu[i] = e;
-    const double ea = fabs(e);
-    if (B.Z[i] >= 0 && gt_nonneg(ea, thr)) ++B.Z[i];
-    nrmu2 += ea * ea;
-    if (B.Z[i] >= 0 && gt_nonneg(ea, nm.v)) nm = ArgMax{ea, i, e};
-  }
-  g.sum2(nrmu2, nrmv2);
-  nm = g.argmax(nm);
-  if (nm.v > 0.0) i0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACA_col_step (ACA.h:134-213)
-template <int G, class Grp>
-__device__ bool col_step(const Grp& g, const Blk& B, uint32_t& j0, uint32_t k, uint32_t& no,
-                         double& nrmlsk2, double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  double* const pu = B.U + (size_t)k * n1;
-  double* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    g.sync();
-    const uint32_t gj = B.b2 + j0;
-    const double xj = B.P.x[gj], yj = B.P.y[gj], zj = B.P.z[gj];
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t i = g.rank; i < n1; i += G) {
-      double u = lap_entry_aca(B.P, gj, B.b1 + i, xj, yj, zj, B.diag);
-      for (uint32_t l = 0; l < k; ++l) u = fma(-B.V[(size_t)l * n2 + j0], B.U[(size_t)l * n1 + i], u);
-      pu[i] = u;
-      if (B.Z[i] >= 0) {
-        const double a = fabs(u);
-        if (gt_nonneg(a, am.v)) am = ArgMax{a, i, u};
-      }
-    }
-    am = g.argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (owns(g, j0, G)) B.S[j0] = -1;
-    if (++no >= n2) return false;
-    g.sync();
-    j0 = nexti<G>(g, B.S, n2, j0);
-  }
-  const uint32_t i0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const double sca = sqrtpiv / am.sv;
-  const double thr = 1e-8 * scale * sqrtpiv;
-  double nrmu2 = 0.0;
-  for (uint32_t i = g.rank; i < n1; i += G) {
-    if (B.Z[i] >= 0) {
-      const double e = pu[i] * sca;
-      pu[i] = e;
-      nrmu2 += e * e;
-      if (gt_nonneg(fabs(e), thr)) ++B.Z[i];
-    }
-  }
-  const uint32_t gi = B.b1 + i0;
-  const double xi = B.P.x[gi], yi = B.P.y[gi], zi = B.P.z[gi];
-  for (uint32_t j = g.rank; j < n2; j += G) {
-    double v = lap_entry_aca(B.P, gi, B.b2 + j, xi, yi, zi, B.diag);
-    for (uint32_t l = 0; l < k; ++l) v = fma(-B.U[(size_t)l * n1 + i0], B.V[(size_t)l * n2 + j], v);
-    pv[j] = v;
-  }
-  if (owns(g, i0, G)) B.Z[i0] = -1;
-  if (owns(g, j0, G)) B.S[j0] = -1;
-  ++no;
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmv2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t j = g.rank; j < n2; j += G) {
-    const double e = pv[j] * dsca;
-    pv[j] = e;
-    const double ea = fabs(e);
-    if (B.S[j] >= 0 && gt_nonneg(ea, thr)) ++B.S[j];
-    nrmv2 += ea * ea;
-    if (gt_nonneg(ea, nm.v)) nm = ArgMax{ea, j, e};  // no S filter here, as in the reference
-  }
-  g.sum2(nrmu2, nrmv2);
-  nm = g.argmax(nm);
-  if (nm.v > 0.0) j0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACA driver (ACA.h:217-350).  Returns the status, the rank in k.
-template <int G, class Grp>
-__device__ int aca(const Grp& g, const Blk& B, uint32_t i0, uint32_t kmax, uint32_t kcap,
-                   double eps, uint32_t& kout) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  for (uint32_t i = g.rank; i < n1; i += G) B.Z[i] = 0;
-  for (uint32_t j = g.rank; j < n2; j += G) B.S[j] = 0;
-  double scale;
-  {
-    const uint32_t a = B.b1, b = B.b2;
-    scale = fabs(lap_entry(B.P, a, b, B.P.x[a], B.P.y[a], B.P.z[a], B.diag));
-  }
-  uint32_t k = 0, no = 0, klast = 0, inext = i0, j0 = 0;
-  int kmin = -2, keps = -1;
-  double nrmlsk2 = 0.0, nrms2 = 0.0;
-  int outcome = -1;  // 0 NSUCC, 1 SUCC, 2 overflow
-  do {
-    if (k >= kcap) { outcome = kAcaOverflow; break; }
-    inext = i0;
-    if (!row_step<G>(g, B, klast, inext, k, no, nrmlsk2, scale)) {
-      nrmlsk2 = 0.0;
-      outcome = kAcaOk;
-      break;
-    }
-    double sum = 0.0;
-    const double* uk = B.U + (size_t)k * n1;
-    const double* vk = B.V + (size_t)k * n2;
-    for (uint32_t l = 0; l < k; ++l) {
-      double du = 0.0, dv = 0.0;
-      for (uint32_t i = g.rank; i < n1; i += G) du += B.U[(size_t)l * n1 + i] * uk[i];
-      for (uint32_t j = g.rank; j < n2; j += G) dv += B.V[(size_t)l * n2 + j] * vk[j];
-      g.sum2(du, dv);
-      sum += du * dv;
-    }
-    nrms2 += 2.0 * sum + nrmlsk2;
-    const bool stpcrit = nrmlsk2 < eps * eps * nrms2;
-    if (stpcrit && keps == -1) keps = (int)klast + 1;
-    ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
-    if (keps > 0) {
-      ArgMinI m{INT_MAX, 0xffffffffu};
-      for (uint32_t i = g.rank; i < n1; i += G)
-        if (B.Z[i] >= 0 && B.Z[i] < m.v) m = ArgMinI{B.Z[i], i};
-      m = g.argmin(m);
-      if (m.v == INT_MAX) {
-        nrmlsk2 = 0.0;
-        outcome = kAcaOk;
-        break;
-      }
-      kmin = m.v;
-      i0 = m.idx;
-      if ((uint32_t)kmin == k) i0 = inext;
-    } else {
-      i0 = inext;
-    }
-  } while (no < n1 && k < kmax && kmin < keps);
-
-  if (outcome < 0) {
-    if ((no == n1 || k == kmax) && kmin < keps) {
-      outcome = kAcaFail;
-    } else {
-      do {
-        ArgMinI m{INT_MAX, 0xffffffffu};
-        for (uint32_t j = g.rank; j < n2; j += G)
-          if (B.S[j] >= 0 && B.S[j] < m.v) m = ArgMinI{B.S[j], j};
-        m = g.argmin(m);
-        if (m.v == INT_MAX) {
-          nrmlsk2 = 0.0;
-          outcome = kAcaOk;
-          break;
-        }
-        kmin = m.v;
-        j0 = m.idx;
-        if (kmin >= keps) { outcome = kAcaOk; break; }
-        if (k >= kcap) { outcome = kAcaOverflow; break; }
-        if (!col_step<G>(g, B, j0, k, no, nrmlsk2, scale)) {
-          nrmlsk2 = 0.0;
-          outcome = kAcaOk;
-          break;
-        }
-        ++k;
-      } while (no < n2 && k < kmax);
-      if (outcome < 0) outcome = kAcaFail;
-    }
-  }
-  if (outcome == kAcaOk) {
-    const double epsa = sqrt(nrmlsk2 / nrms2);
-    if (epsa >= eps) outcome = kAcaFail;  // NaN (0/0) stays a success, as in the reference
-  }
-  kout = k;
-  g.sync();
-  return outcome;
-}
-
-// ACAr_step (ACA.h:579-655), the simplified cross of the symmetric assembly:
-// rows are skipped only for a small pivot, the pivot column is searched over
-// all columns, and the next row is the largest unused entry of the new column.
-template <int G, class Grp>
-__device__ bool acar_step(const Grp& g, const Blk& B, uint32_t& i0, uint32_t k, uint32_t& no, double& nrmlsk2,
-                          double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  double* const pu = B.U + (size_t)k * n1;
-  double* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    g.sync();
-    const uint32_t gi = B.b1 + i0;
-    const double xi = B.P.x[gi], yi = B.P.y[gi], zi = B.P.z[gi];
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t j = g.rank; j < n2; j += G) {
-      double v = lap_entry_aca(B.P, gi, B.b2 + j, xi, yi, zi, B.diag);
-      for (uint32_t l = 0; l < k; ++l) v = fma(-B.U[(size_t)l * n1 + i0], B.V[(size_t)l * n2 + j], v);
-      pv[j] = v;
-      const double a = fabs(v);
-      if (gt_nonneg(a, am.v)) am = ArgMax{a, j, v};
-    }
-    am = g.argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (owns(g, i0, G)) B.Z[i0] = -1;
-    if (++no >= n1) return false;
-    g.sync();
-    i0 = nexti<G>(g, B.Z, n1, i0);
-  }
-  const uint32_t j0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const double sca = sqrtpiv / am.sv;
-  double nrmv2 = 0.0;
-  for (uint32_t j = g.rank; j < n2; j += G) {
-    const double e = pv[j] * sca;
-    pv[j] = e;
-    nrmv2 += e * e;
-  }
-  const uint32_t gj = B.b2 + j0;
-  const double xj = B.P.x[gj], yj = B.P.y[gj], zj = B.P.z[gj];
-  for (uint32_t i = g.rank; i < n1; i += G) {
-    double u = lap_entry_aca(B.P, gj, B.b1 + i, xj, yj, zj, B.diag);
-    for (uint32_t l = 0; l < k; ++l) u = fma(-B.V[(size_t)l * n2 + j0], B.U[(size_t)l * n1 + i], u);
-    pu[i] = u;
-  }
-  if (owns(g, i0, G)) B.Z[i0] = -1;
-  ++no;
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmu2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t i = g.rank; i < n1; i += G) {
-    const double e = pu[i] * dsca;
-    pu[i] = e;
-    const double ea = fabs(e);
-    nrmu2 += ea * ea;
-    if (B.Z[i] >= 0 && gt_nonneg(ea, nm.v)) nm = ArgMax{ea, i, e};
-  }
-  g.sum2(nrmu2, nrmv2);
-  nm = g.argmax(nm);
-  if (nm.v > 0.0) i0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACAr driver (ACA.h:657-720): crosses until the last one is below eps of the
-// approximation's norm, no more than n2 rows used, or kmax crosses.
-template <int G, class Grp>
-__device__ int acar(const Grp& g, const Blk& B, uint32_t i0, uint32_t kmax, uint32_t kcap, double eps,
-                    uint32_t& kout) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  for (uint32_t i = g.rank; i < n1; i += G) B.Z[i] = 0;
-  double scale;
-  {
-    const uint32_t a = B.b1, b = B.b2;
-    scale = fabs(lap_entry(B.P, a, b, B.P.x[a], B.P.y[a], B.P.z[a], B.diag));
-  }
-  uint32_t k = 0, no = 0;
-  double nrmlsk2 = 0.0, nrms2 = 0.0;
-  int outcome = -1;
-  do {
-    if (k >= kcap) {
-      outcome = kAcaOverflow;
-      break;
-    }
-    if (!acar_step<G>(g, B, i0, k, no, nrmlsk2, scale)) {
-      nrmlsk2 = 0.0;
-      break;
-    }
-    double sum = 0.0;
-    const double* uk = B.U + (size_t)k * n1;
-    const double* vk = B.V + (size_t)k * n2;
-    for (uint32_t l = 0; l < k; ++l) {
-      double du = 0.0, dv = 0.0;
-      for (uint32_t i = g.rank; i < n1; i += G) du += B.U[(size_t)l * n1 + i] * uk[i];
-      for (uint32_t j = g.rank; j < n2; j += G) dv += B.V[(size_t)l * n2 + j] * vk[j];
-      g.sum2(du, dv);
-      sum += du * dv;
-    }
-    nrms2 += 2.0 * sum + nrmlsk2;
-    ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
-  } while (no < n2 && k < kmax && nrmlsk2 >= eps * eps * nrms2);
-  if (outcome < 0) {
-    const double epsa = sqrt(nrmlsk2 / nrms2);
-    outcome = epsa >= eps ? kAcaFail : kAcaOk;  // NaN (0/0) stays a success, as in the reference
-  }
-  kout = k;
-  g.sync();
-  return outcome;
-}
 
 // In-place Householder QR of A (m x k, column-major) by the group; tau[k].
 template <int G, class Grp>
@@ -899,49 +516,6 @@ __device__ uint32_t recompress_qrcp(const Grp& g, uint32_t n1, uint32_t n2, uint
   return kt;
 }
 
-template <int G, class Grp>
-__device__ void aca_task(const Grp& g, const AcaParams& p, uint32_t ti, double* smem) {
-  const AcaTask t = p.tasks[ti];
-  Blk B;
-  B.P = p.pts;
-  B.diag = p.diag;
-  B.b1 = t.b1;
-  B.n1 = t.n1;
-  B.b2 = t.b2;
-  B.n2 = t.n2;
-  double* ws = p.ws + t.ws;
-  const uint32_t kc = t.kcap;
-  B.U = ws;
-  B.V = B.U + (size_t)t.n1 * kc;
-  double* Un = B.V + (size_t)t.n2 * kc;
-  double* Vn = Un + (size_t)t.n1 * kc;
-  double* Rg = Vn + (size_t)t.n2 * kc;
-  double* Vsg = Rg + (size_t)kc * kc;
-  double* sigg = Vsg + (size_t)kc * kc;
-  double* taug = sigg + kc;
-  B.Z = p.zs + t.zs;
-  B.S = B.Z + t.n1;
-  uint32_t k = 0;
-  const int st = p.variant == kAcaVariantSym ? acar<G>(g, B, t.i0, t.kmax, t.kcap, p.eps, k)
-                                             : aca<G>(g, B, t.i0, t.kmax, t.kcap, p.eps, k);
-  uint32_t kt = 0;
-  if (st == kAcaOk && k > 0) {
-    // small ranks: k x k work arrays in shared memory; larger: in the workspace
-    const bool sm = k <= (uint32_t)KSM;
-    double* R = sm ? smem : Rg;
-    double* Vs = sm ? smem + KSM * LDS : Vsg;
-    double* sig = sm ? smem + 2 * KSM * LDS : sigg;
-    double* tau = sm ? smem + 2 * KSM * LDS + KSM : taug;
-    // perm needs nmin+1 ints: shared memory when small, else the dead Z/S counters
-    // (n1 + n2 ints >= nmin + 1)
-    int* perm = sm ? reinterpret_cast<int*>(smem + 2 * KSM * LDS + 3 * KSM) : B.Z;
-    g.sync();
-    kt = recompress<G>(g, t.n1, t.n2, k, B.U, B.V, Un, Vn, p.eps, R, Vs, sm ? LDS : kc, sig, tau,
-                       perm, !sm);
-  }
-  if (g.rank == 0) p.res[ti] = AcaResult{st, k, kt, 0u};
-}
-
 // Agglomeration (H/agglH.cpp:14-107): the concatenated factors of sibling
 // low-rank blocks (gathered into the task's workspace, zero elsewhere)
 // recompressed to the parent's rank with the relative threshold of
@@ -1005,24 +579,7 @@ __global__ void copy2d_kernel(const Seg2D* __restrict__ segs, const double* __re
   }
 }
 
-__global__ void __launch_bounds__(32 * kSmallWarps) aca_small_kernel(AcaParams p) {
-  extern __shared__ double smem_all[];
-  const uint32_t w = threadIdx.x >> 5;
-  const uint32_t task = blockIdx.x * kSmallWarps + w;
-  if (task >= p.ntasks) return;
-  Group<32> g(threadIdx.x & 31);
-  aca_task<32>(g, p, task, smem_all + (size_t)w * kSmemPerGroup);
-}
-
 constexpr int kLargeThreads = 256;
-
-__global__ void __launch_bounds__(kLargeThreads) aca_large_kernel(AcaParams p) {
-  extern __shared__ double smem_all[];
-  const uint32_t task = blockIdx.x;
-  if (task >= p.ntasks) return;
-  Group<kLargeThreads> g(threadIdx.x, smem_all + kSmemPerGroup);
-  aca_task<kLargeThreads>(g, p, task, smem_all);
-}
 
 __global__ void __launch_bounds__(kLargeThreads) merge_large_kernel(MergeParams p) {
   extern __shared__ double smem_all[];
@@ -1073,26 +630,10 @@ __global__ void copy_factors_kernel(const CopyTask* __restrict__ tasks, const do
 
 }  // namespace
 
-cudaError_t launch_aca_small(const AcaParams& p, cudaStream_t s) {
-  if (p.ntasks == 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * kSmemPerGroup * kSmallWarps;
-  cudaError_t e = cudaFuncSetAttribute(aca_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
-  const uint32_t grid = (p.ntasks + kSmallWarps - 1) / kSmallWarps;
-  aca_small_kernel<<<grid, 32 * kSmallWarps, smem, s>>>(p);
-  return cudaGetLastError();
+cudaError_t launch_aca(const AcaParams& p, uint32_t grid, cudaStream_t s) {
+  return lowrank::launch_aca_kernel(lowrank::LapGen{p.pts, p.diag}, p, grid, s);
 }
-
-cudaError_t launch_aca_large(const AcaParams& p, cudaStream_t s) {
-  if (p.ntasks == 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * (kSmemPerGroup + 3 * (kLargeThreads / 32) + 8);
-  cudaError_t e = cudaFuncSetAttribute(aca_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
-  aca_large_kernel<<<p.ntasks, kLargeThreads, smem, s>>>(p);
-  return cudaGetLastError();
-}
+cudaError_t resident_aca(int device, uint32_t& ctas) { return lowrank::resident_aca_kernel<lowrank::LapGen>(device, ctas); }
 
 cudaError_t launch_dense_fill(const PointsSoA& pts, double diag, const DenseTask* tasks,
                               uint32_t ntasks, double* arena, cudaStream_t s) {
@@ -1150,7 +691,7 @@ cudaError_t launch_copy_factors(const CopyTask* tasks, uint32_t ntasks, const do
 // scratch (the ACA columns, the row/column counters and the recompression
 // work arrays) from the file-scope array below instead of an allocation.
 //
-// The array is 8 MiB and lives on every GPU that loads the library until the
+// The array is 11 MiB and lives on every GPU that loads the library until the
 // process exits.  Every call shares it and it keeps the last call's contents;
 // the kernel rewrites every word it reads (the counters are set to zero by the
 // ACA itself), so nothing carries over between calls.  Calls whose kernels
@@ -1160,9 +701,15 @@ namespace ahx {
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = (size_t)8 << 20;
-constexpr size_t kNoAllocHeader = 256;  // task slot + result slot
+constexpr size_t kNoAllocHeader = 256;
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// Blocks are accepted by the size formula of noalloc_bytes, up to 8 MiB.  The workspace
+// of a leaf (aca_ws_bytes) can be larger where the rank bound reaches the block's sides:
+// with n = n1 + n2 and c columns it is at most n c + 4 min(c, n)^2 + O(n + c) elements,
+// and 2 n c + 2 c^2 elements fit 8 MiB: at most 10 MiB, at n = c = 512, and O(n + c)
+// (c <= n, or the formula's own 2 c^2 is the larger).
+constexpr size_t kNoAllocArrayBytes = (size_t)11 << 20;
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocArrayBytes];
 
 // Blocks beyond this many rows or columns, or rank bounds beyond kNoAllocMaxK,
 // are refused before any size arithmetic (they could never fit the array).
@@ -1176,52 +723,26 @@ uint64_t noalloc_bytes(uint32_t n1, uint32_t n2, uint32_t kmax) {
   return kNoAllocHeader + ws + ((uint64_t)n1 + n2) * sizeof(int);
 }
 
-template <int G>
-__global__ void __launch_bounds__(G < 64 ? 32 : G)
-    aca_noalloc_kernel(AcaTask t, uint64_t ws_doubles, PointsSoA P, double diag, double eps,
-                       unsigned char* scratch, double* __restrict__ Uout,
-                       double* __restrict__ Vout, int32_t* info) {
-  extern __shared__ double smem_na[];
-  AcaTask* slot = reinterpret_cast<AcaTask*>(scratch);
-  AcaResult* res = reinterpret_cast<AcaResult*>(scratch + 128);
-  double* ws = reinterpret_cast<double*>(scratch + kNoAllocHeader);
-  int* zs = reinterpret_cast<int*>(ws + ws_doubles);
+template <int W>
+__global__ void __launch_bounds__(32 * W)
+    aca_noalloc_kernel(AcaTask t, PointsSoA P, double diag, double eps, unsigned char* scratch,
+                       double* __restrict__ Uout, double* __restrict__ Vout, int32_t* info) {
+  extern __shared__ __align__(16) unsigned char smem_na[];
+  double* const sm = reinterpret_cast<double*>(smem_na);
+  lowrank::Team<W> g(threadIdx.x, reinterpret_cast<double*>(smem_na + lowrank::team_smem<double>()));
+  int st;
+  uint32_t k, kt;
+  lowrank::leaf(g, lowrank::LapGen{P, diag}, t, eps, kAcaVariantGeneral, scratch, sm,
+                [&](uint32_t, double*& Un, double*& Vn) {
+                  Un = Uout;
+                  Vn = Vout;
+                  return true;
+                },
+                st, k, kt);
   if (threadIdx.x == 0) {
-    t.ws = 0;
-    t.zs = 0;
-    *slot = t;
-    *res = AcaResult{kAcaFail, 0u, 0u, 0u};
-  }
-  __syncthreads();
-  AcaParams p;
-  p.pts = P;
-  p.diag = diag;
-  p.eps = eps;
-  p.tasks = slot;
-  p.ntasks = 1;
-  p.ws = ws;
-  p.zs = zs;
-  p.res = res;
-  if constexpr (G == 32) {
-    Group<32> g(threadIdx.x);
-    aca_task<32>(g, p, 0, smem_na);
-  } else {
-    Group<G> g(threadIdx.x, smem_na + kSmemPerGroup);
-    aca_task<G>(g, p, 0, smem_na);
-  }
-  __syncthreads();
-  const AcaResult r = *res;
-  const uint64_t kc = t.kcap;
-  const double* Un = ws + (uint64_t)(t.n1 + t.n2) * kc;
-  const double* Vn = Un + (uint64_t)t.n1 * kc;
-  if (r.status == kAcaOk) {
-    for (uint64_t e = threadIdx.x; e < (uint64_t)t.n1 * r.kt; e += blockDim.x) Uout[e] = Un[e];
-    for (uint64_t e = threadIdx.x; e < (uint64_t)t.n2 * r.kt; e += blockDim.x) Vout[e] = Vn[e];
-  }
-  if (threadIdx.x == 0) {
-    info[0] = r.status;
-    info[1] = (int32_t)r.k_aca;
-    info[2] = (int32_t)r.kt;
+    info[0] = st;
+    info[1] = (int32_t)k;
+    info[2] = (int32_t)kt;
   }
 }
 
@@ -1312,16 +833,17 @@ extern "C" int ahx_aca_block_noalloc(const double* px, const double* py, const d
   t.leaf = 0;
   const PointsSoA P{px, py, pz};
   const double diag = 1.0 / (kFourPi * h);
-  const uint64_t wsd = aca_ws_doubles(n1, n2, t.kcap);
+  if (aca_ws_bytes(n1, n2, t.kcap, sizeof(double)) > kNoAllocArrayBytes) {
+    set_error("ahx_aca_block_noalloc: workspace beyond the fixed scratch array");
+    return AHX_ERR_ARG;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   if (std::max(n1, n2) > 256) {
-    const size_t smem = sizeof(double) * (kSmemPerGroup + 3 * (kLargeThreads / 32) + 8);
-    aca_noalloc_kernel<kLargeThreads><<<1, kLargeThreads, smem, s>>>(t, wsd, P, diag, eps,
-                                                                     (unsigned char*)scratch, U, V, info);
+    const size_t smem = lowrank::team_smem<double>() + 64 * sizeof(double);
+    aca_noalloc_kernel<4><<<1, 128, smem, s>>>(t, P, diag, eps, (unsigned char*)scratch, U, V, info);
   } else {
-    const size_t smem = sizeof(double) * kSmemPerGroup;
-    aca_noalloc_kernel<32><<<1, 32, smem, s>>>(t, wsd, P, diag, eps, (unsigned char*)scratch, U, V,
-                                               info);
+    aca_noalloc_kernel<1><<<1, 32, lowrank::team_smem<double>(), s>>>(t, P, diag, eps, (unsigned char*)scratch, U, V,
+                                                                      info);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "aca_noalloc_kernel launch");

@@ -8,18 +8,13 @@
 
 namespace ahx {
 
-// One admissible leaf to approximate.  Workspace layout at `ws` (doubles):
-//   U[n1*kcap] V[n2*kcap] Un[n1*kcap] Vn[n2*kcap] R[kcap*kcap] Vs[kcap*kcap] sig[kcap]
-//   tau[2*kcap]
-// and at `zs` (ints): Z[n1] S[n2]  (ACA.h:38-42 row/column success counters).
+// One admissible leaf to approximate, with the capacity kcap of its cross columns.
 struct AcaTask {
   uint32_t b1, n1, b2, n2;
   uint32_t i0, kmax, kcap, leaf;
-  uint64_t ws;
-  uint64_t zs;
 };
 
-enum AcaStatus : int32_t { kAcaFail = 0, kAcaOk = 1, kAcaOverflow = 2 };
+enum AcaStatus : int32_t { kAcaFail = 0, kAcaOk = 1, kAcaOverflow = 2, kAcaNoSpace = 3 };
 
 // ACA of the general assembly (Include/ACA.h:217-350) or ACAr of the symmetric one
 // (Include/ACA.h:657-720, Include/apprx.h:86-132)
@@ -30,29 +25,53 @@ struct AcaResult {
   uint32_t k_aca;  // rank returned by ACA (before recompression)
   uint32_t kt;     // rank after recompression
   uint32_t pad;
+  uint64_t off;    // element offset of the factors (U, then V) in the arena
 };
 
-// 64-bit throughout: n1 + n2 and kcap * kcap overflow 32 bits for large blocks
+// Workspace of a leaf (ahx_lowrank.cuh): elements U[n1 kcap] V[n2 kcap], four squares of
+// kw x kw, tau[2 kw]; doubles [5 kw]; ints Z[n1] S[n2] (ACA.h:38-42 row/column success
+// counters).  kw bounds the crosses of a block: every cross uses up a row (row steps) or
+// a column, one more may follow the last row.  64-bit throughout.
+__host__ __device__ inline uint32_t aca_work_k(uint32_t n1, uint32_t n2, uint32_t kcap) {
+  const uint32_t n = n1 > n2 ? n1 : n2;
+  return kcap <= n ? kcap : n + 1u;
+}
+inline uint64_t aca_ws_bytes(uint32_t n1, uint32_t n2, uint32_t kcap, size_t elem) {
+  const uint64_t n = (uint64_t)n1 + n2, kw = aca_work_k(n1, n2, kcap);
+  return ((n * kcap + 4ull * kw * kw + 2ull * kw) * elem + 40ull * kw + 4ull * n + 255u) & ~255ull;
+}
+
+// Agglomeration's workspace: U[n1 k] V[n2 k] Un[n1 k] Vn[n2 k] R[k k] Vs[k k] sig[k] tau[2 k]
 inline uint64_t aca_ws_doubles(uint32_t n1, uint32_t n2, uint32_t kcap) {
   const uint64_t n = (uint64_t)n1 + n2, k = kcap;
   return 2ull * n * k + 2ull * k * k + 3ull * k;
 }
 
+// One launch over all leaves: the first nlarge tasks by a CTA each, the rest by a warp
+// each, by as many resident teams as there are slots; slots[i]: byte offset of a team's
+// workspace (large teams first).
+constexpr int kAcaThreads = 128;
 struct AcaParams {
   PointsSoA pts;
-  double diag;  // 1/(4 pi h)
+  double diag;  // Laplace: 1/(4 pi h)
+  double k, h;  // Helmholtz
   double eps;
   const AcaTask* tasks;
-  uint32_t ntasks;
-  double* ws;
-  int* zs;
   AcaResult* res;
-  int32_t variant = kAcaVariantGeneral;
+  const uint64_t* slots;
+  unsigned char* ws;
+  void* arena;
+  unsigned long long* used;  // arena elements taken
+  uint32_t* ctr;             // two task counters
+  uint64_t cap;              // arena capacity in elements
+  uint32_t nlarge, nsmall, nslot_l, nslot_s;
+  int32_t variant;
 };
 
-// Launchers (ahx_aca.cu)
-cudaError_t launch_aca_small(const AcaParams& p, cudaStream_t s);  // one warp per leaf
-cudaError_t launch_aca_large(const AcaParams& p, cudaStream_t s);  // one CTA per leaf
+cudaError_t launch_aca(const AcaParams& p, uint32_t grid, cudaStream_t s);   // Laplace (ahx_aca.cu)
+cudaError_t launch_zaca(const AcaParams& p, uint32_t grid, cudaStream_t s);  // Helmholtz (ahx_aca_helm.cu)
+cudaError_t resident_aca(int device, uint32_t& ctas);
+cudaError_t resident_zaca(int device, uint32_t& ctas);
 
 // Dense leaves: fill n1 x n2 column-major blocks of the generator.
 struct DenseTask {

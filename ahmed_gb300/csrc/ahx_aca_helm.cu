@@ -15,437 +15,40 @@
 
 #include "ahx_aca.cuh"
 #include "ahx_hmat.hpp"
+#include "ahx_lowrank.cuh"
 
 namespace ahx {
 namespace {
 
 constexpr int kWarps = 4;  // leaves per CTA
 
-struct Cx {
-  double re, im;
-};
+using lowrank::HelmGen;
+using lowrank::Team;
 
 __device__ __forceinline__ double cabs2(Cx a) { return __dadd_rn(__dmul_rn(a.re, a.re), __dmul_rn(a.im, a.im)); }
 __device__ __forceinline__ double cabs(Cx a) { return __dsqrt_rn(cabs2(a)); }
 __device__ __forceinline__ Cx cconj(Cx a) { return Cx{a.re, -a.im}; }
-__device__ __forceinline__ Cx nconj(Cx a) { return Cx{-a.re, a.im}; }
-// y += a x (zaxpy)
-__device__ __forceinline__ void caxpy(Cx a, Cx x, Cx& y) {
-  y.re += a.re * x.re - a.im * x.im;
-  y.im += a.re * x.im + a.im * x.re;
-}
-// a *= b (Include/cmplx.h:187-194)
-__device__ __forceinline__ void cmul_eq(Cx& a, Cx b) {
-  const double t = __dsub_rn(__dmul_rn(a.re, b.re), __dmul_rn(a.im, b.im));
-  a.im = __dmul_rn(a.im, b.re);
-  a.im = __dadd_rn(a.im, __dmul_rn(a.re, b.im));
-  a.re = t;
-}
-// real / complex (Include/cmplx.h:235-241)
-__device__ __forceinline__ Cx rdiv(double a, Cx b) {
-  const double d = __ddiv_rn(a, cabs2(b));
-  return Cx{__dmul_rn(b.re, d), __dmul_rn(b.im, -d)};
-}
 
-struct HBlk {
-  PointsSoA P;
-  double k, h;
-  uint32_t b1, n1, b2, n2;
-  Cx* U;
-  Cx* V;
-  int* Z;
-  int* S;
-};
-
-__device__ __forceinline__ Cx helm_entry(const HBlk& B, uint32_t i, uint32_t j) {
-  double r = B.h;
+// entry of a dense leaf, explicitly rounded
+__device__ __forceinline__ Cx helm_entry(const PointsSoA& P, double k, double h, uint32_t i, uint32_t j) {
+  double r = h;
   if (i != j) {
-    const double dx = __dsub_rn(B.P.x[i], B.P.x[j]);
-    const double dy = __dsub_rn(B.P.y[i], B.P.y[j]);
-    const double dz = __dsub_rn(B.P.z[i], B.P.z[j]);
+    const double dx = __dsub_rn(P.x[i], P.x[j]);
+    const double dy = __dsub_rn(P.y[i], P.y[j]);
+    const double dz = __dsub_rn(P.z[i], P.z[j]);
     r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
   }
   const double s = __ddiv_rn(1.0, __dmul_rn(kFourPi, r));
   double sn, cs;
-  sincos(__dmul_rn(B.k, r), &sn, &cs);
+  sincos(__dmul_rn(k, r), &sn, &cs);
   return Cx{__dmul_rn(cs, s), __dmul_rn(sn, s)};
 }
 
 using G32 = Group<32>;
 
-__device__ uint32_t nexti(const G32& g, const int* Z, uint32_t n, uint32_t j) {
-  uint32_t d = 0xffffffffu;
-  for (uint32_t i = g.rank; i < n; i += 32)
-    if (Z[i] != -1) d = min(d, i >= j ? i - j : i + n - j);
-  d = G32::umin(d);
-  return d == 0xffffffffu ? j : (j + d) % n;
-}
-
-// ACA_row_step (ACA.h:46-130), T = dcomp: V holds conjugated rows
-__device__ bool row_step(const G32& g, const HBlk& B, uint32_t& klast, uint32_t& i0, uint32_t k, uint32_t& no,
-                         double& nrmlsk2, double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  Cx* const pu = B.U + (size_t)k * n1;
-  Cx* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    __syncwarp();
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t j = g.rank; j < n2; j += 32) {
-      Cx v = cconj(helm_entry(B, B.b1 + i0, B.b2 + j));
-      for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.U[(size_t)l * n1 + i0]), B.V[(size_t)l * n2 + j], v);
-      pv[j] = v;
-      if (B.S[j] >= 0) {
-        const double a = cabs(v);
-        if (gt_nonneg(a, am.v)) am = ArgMax{a, j, 0.0};
-      }
-    }
-    am = G32::argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (i0 % 32 == g.rank) B.Z[i0] = -1;
-    if (++no >= n1) return false;
-    __syncwarp();
-    i0 = nexti(g, B.Z, n1, i0);
-  }
-  __syncwarp();
-  const uint32_t j0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const Cx sca = rdiv(sqrtpiv, pv[j0]);
-  const double thr = 1e-8 * scale * sqrtpiv;
-  __syncwarp();
-  double nrmv2 = 0.0;
-  for (uint32_t j = g.rank; j < n2; j += 32) {
-    if (B.S[j] >= 0) {
-      Cx e = pv[j];
-      cmul_eq(e, sca);
-      pv[j] = e;
-      nrmv2 += cabs2(e);
-      if (gt_nonneg(cabs(e), thr)) ++B.S[j];
-    }
-  }
-  for (uint32_t i = g.rank; i < n1; i += 32) {
-    Cx u = helm_entry(B, B.b1 + i, B.b2 + j0);
-    for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.V[(size_t)l * n2 + j0]), B.U[(size_t)l * n1 + i], u);
-    pu[i] = u;
-  }
-  klast = (uint32_t)G32::imax(i0 % 32 == g.rank ? B.Z[i0] : INT_MIN);
-  if (i0 % 32 == g.rank) B.Z[i0] = -1;
-  if (j0 % 32 == g.rank) B.S[j0] = -1;
-  ++no;
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmu2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t i = g.rank; i < n1; i += 32) {
-    Cx e = pu[i];
-    e.re *= dsca;
-    e.im *= dsca;
-    pu[i] = e;
-    const double ea = cabs(e);
-    if (B.Z[i] >= 0 && gt_nonneg(ea, thr)) ++B.Z[i];
-    nrmu2 += ea * ea;
-    if (B.Z[i] >= 0 && gt_nonneg(ea, nm.v)) nm = ArgMax{ea, i, 0.0};
-  }
-  G32::sum2(nrmu2, nrmv2);
-  nm = G32::argmax(nm);
-  if (nm.v > 0.0) i0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACA_col_step (ACA.h:134-213), T = dcomp
-__device__ bool col_step(const G32& g, const HBlk& B, uint32_t& j0, uint32_t k, uint32_t& no, double& nrmlsk2,
-                         double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  Cx* const pu = B.U + (size_t)k * n1;
-  Cx* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    __syncwarp();
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t i = g.rank; i < n1; i += 32) {
-      Cx u = helm_entry(B, B.b1 + i, B.b2 + j0);
-      for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.V[(size_t)l * n2 + j0]), B.U[(size_t)l * n1 + i], u);
-      pu[i] = u;
-      if (B.Z[i] >= 0) {
-        const double a = cabs(u);
-        if (gt_nonneg(a, am.v)) am = ArgMax{a, i, 0.0};
-      }
-    }
-    am = G32::argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (j0 % 32 == g.rank) B.S[j0] = -1;
-    if (++no >= n2) return false;
-    __syncwarp();
-    j0 = nexti(g, B.S, n2, j0);
-  }
-  __syncwarp();
-  const uint32_t i0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const Cx sca = rdiv(sqrtpiv, pu[i0]);
-  const double thr = 1e-8 * scale * sqrtpiv;
-  __syncwarp();
-  double nrmu2 = 0.0;
-  for (uint32_t i = g.rank; i < n1; i += 32) {
-    if (B.Z[i] >= 0) {
-      Cx e = pu[i];
-      cmul_eq(e, sca);
-      pu[i] = e;
-      nrmu2 += cabs2(e);
-      if (gt_nonneg(cabs(e), thr)) ++B.Z[i];
-    }
-  }
-  for (uint32_t j = g.rank; j < n2; j += 32) {
-    Cx v = cconj(helm_entry(B, B.b1 + i0, B.b2 + j));
-    for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.U[(size_t)l * n1 + i0]), B.V[(size_t)l * n2 + j], v);
-    pv[j] = v;
-  }
-  if (i0 % 32 == g.rank) B.Z[i0] = -1;
-  if (j0 % 32 == g.rank) B.S[j0] = -1;
-  ++no;
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmv2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t j = g.rank; j < n2; j += 32) {
-    Cx e = pv[j];
-    e.re *= dsca;
-    e.im *= dsca;
-    pv[j] = e;
-    const double ea = cabs(e);
-    if (B.S[j] >= 0 && gt_nonneg(ea, thr)) ++B.S[j];
-    nrmv2 += ea * ea;
-    if (gt_nonneg(ea, nm.v)) nm = ArgMax{ea, j, 0.0};  // no S filter, as in the reference
-  }
-  G32::sum2(nrmu2, nrmv2);
-  nm = G32::argmax(nm);
-  if (nm.v > 0.0) j0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACA driver (ACA.h:217-350), T = dcomp.  Returns the status, the rank in k.
-__device__ int aca(const G32& g, const HBlk& B, uint32_t i0, uint32_t kmax, uint32_t kcap, double eps,
-                   uint32_t& kout) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  for (uint32_t i = g.rank; i < n1; i += 32) B.Z[i] = 0;
-  for (uint32_t j = g.rank; j < n2; j += 32) B.S[j] = 0;
-  double scale = cabs(helm_entry(B, B.b1, B.b2));
-  uint32_t k = 0, no = 0, klast = 0, inext = i0, j0 = 0;
-  int kmin = -2, keps = -1;
-  double nrmlsk2 = 0.0, nrms2 = 0.0;
-  int outcome = -1;
-  do {
-    if (k >= kcap) { outcome = kAcaOverflow; break; }
-    inext = i0;
-    if (!row_step(g, B, klast, inext, k, no, nrmlsk2, scale)) {
-      nrmlsk2 = 0.0;
-      outcome = kAcaOk;
-      break;
-    }
-    __syncwarp();
-    // sum_l scpr(U_l, U_k) * scpr(V_l, V_k), scpr = sum conj(x) y
-    double sre = 0.0, sim = 0.0;
-    const Cx* uk = B.U + (size_t)k * n1;
-    const Cx* vk = B.V + (size_t)k * n2;
-    for (uint32_t l = 0; l < k; ++l) {
-      double ur = 0.0, ui = 0.0, vr = 0.0, vi = 0.0;
-      for (uint32_t i = g.rank; i < n1; i += 32) {
-        const Cx a = B.U[(size_t)l * n1 + i], b = uk[i];
-        ur += a.re * b.re + a.im * b.im;
-        ui += a.re * b.im - a.im * b.re;
-      }
-      for (uint32_t j = g.rank; j < n2; j += 32) {
-        const Cx a = B.V[(size_t)l * n2 + j], b = vk[j];
-        vr += a.re * b.re + a.im * b.im;
-        vi += a.re * b.im - a.im * b.re;
-      }
-      G32::sum2(ur, ui);
-      G32::sum2(vr, vi);
-      sre += ur * vr - ui * vi;
-      sim += ur * vi + ui * vr;
-    }
-    nrms2 += 2.0 * sre + nrmlsk2;
-    const bool stpcrit = nrmlsk2 < eps * eps * nrms2;
-    if (stpcrit && keps == -1) keps = (int)klast + 1;
-    ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
-    if (keps > 0) {
-      ArgMinI m{INT_MAX, 0xffffffffu};
-      for (uint32_t i = g.rank; i < n1; i += 32)
-        if (B.Z[i] >= 0 && B.Z[i] < m.v) m = ArgMinI{B.Z[i], i};
-      m = G32::argmin(m);
-      if (m.v == INT_MAX) {
-        nrmlsk2 = 0.0;
-        outcome = kAcaOk;
-        break;
-      }
-      kmin = m.v;
-      i0 = m.idx;
-      if ((uint32_t)kmin == k) i0 = inext;
-    } else {
-      i0 = inext;
-    }
-  } while (no < n1 && k < kmax && kmin < keps);
-
-  if (outcome < 0) {
-    if ((no == n1 || k == kmax) && kmin < keps) {
-      outcome = kAcaFail;
-    } else {
-      do {
-        ArgMinI m{INT_MAX, 0xffffffffu};
-        for (uint32_t j = g.rank; j < n2; j += 32)
-          if (B.S[j] >= 0 && B.S[j] < m.v) m = ArgMinI{B.S[j], j};
-        m = G32::argmin(m);
-        if (m.v == INT_MAX) {
-          nrmlsk2 = 0.0;
-          outcome = kAcaOk;
-          break;
-        }
-        kmin = m.v;
-        j0 = m.idx;
-        if (kmin >= keps) { outcome = kAcaOk; break; }
-        if (k >= kcap) { outcome = kAcaOverflow; break; }
-        if (!col_step(g, B, j0, k, no, nrmlsk2, scale)) {
-          nrmlsk2 = 0.0;
-          outcome = kAcaOk;
-          break;
-        }
-        ++k;
-      } while (no < n2 && k < kmax);
-      if (outcome < 0) outcome = kAcaFail;
-    }
-  }
-  if (outcome == kAcaOk) {
-    const double epsa = sqrt(nrmlsk2 / nrms2);
-    if (epsa >= eps) outcome = kAcaFail;
-  }
-  kout = k;
-  __syncwarp();
-  return outcome;
-}
-
-// ACAr_step (ACA.h:579-655) with T = dcomp, the cross of the symmetric assembly:
-// rows are skipped only for a small pivot, the pivot column is searched over all
-// columns, the next row is the largest unused entry of the new column.
-__device__ bool acar_step(const G32& g, const HBlk& B, uint32_t& i0, uint32_t k, uint32_t& no, double& nrmlsk2,
-                          double scale) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  Cx* const pu = B.U + (size_t)k * n1;
-  Cx* const pv = B.V + (size_t)k * n2;
-  ArgMax am;
-  for (;;) {
-    __syncwarp();
-    am = ArgMax{0.0, 0xffffffffu, 0.0};
-    for (uint32_t j = g.rank; j < n2; j += 32) {
-      Cx v = cconj(helm_entry(B, B.b1 + i0, B.b2 + j));
-      for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.U[(size_t)l * n1 + i0]), B.V[(size_t)l * n2 + j], v);
-      pv[j] = v;
-      const double a = cabs(v);
-      if (gt_nonneg(a, am.v)) am = ArgMax{a, j, 0.0};
-    }
-    am = G32::argmax(am);
-    if (!(am.v < 1e-14 * scale)) break;
-    if (i0 % 32 == g.rank) B.Z[i0] = -1;
-    if (++no >= n1) return false;
-    __syncwarp();
-    i0 = nexti(g, B.Z, n1, i0);
-  }
-  __syncwarp();
-  const uint32_t j0 = am.idx;
-  const double sqrtpiv = sqrt(am.v);
-  const Cx sca = rdiv(sqrtpiv, pv[j0]);
-  __syncwarp();
-  double nrmv2 = 0.0;
-  for (uint32_t j = g.rank; j < n2; j += 32) {
-    Cx e = pv[j];
-    cmul_eq(e, sca);
-    pv[j] = e;
-    nrmv2 += cabs2(e);
-  }
-  for (uint32_t i = g.rank; i < n1; i += 32) {
-    Cx u = helm_entry(B, B.b1 + i, B.b2 + j0);
-    for (uint32_t l = 0; l < k; ++l) caxpy(nconj(B.V[(size_t)l * n2 + j0]), B.U[(size_t)l * n1 + i], u);
-    pu[i] = u;
-  }
-  if (i0 % 32 == g.rank) B.Z[i0] = -1;
-  ++no;
-  __syncwarp();
-  const double dsca = 1.0 / sqrtpiv;
-  double nrmu2 = 0.0;
-  ArgMax nm{0.0, 0xffffffffu, 0.0};
-  for (uint32_t i = g.rank; i < n1; i += 32) {
-    Cx e = pu[i];
-    e.re *= dsca;
-    e.im *= dsca;
-    pu[i] = e;
-    const double ea = cabs(e);
-    nrmu2 += ea * ea;
-    if (B.Z[i] >= 0 && gt_nonneg(ea, nm.v)) nm = ArgMax{ea, i, 0.0};
-  }
-  G32::sum2(nrmu2, nrmv2);
-  nm = G32::argmax(nm);
-  if (nm.v > 0.0) i0 = nm.idx;
-  nrmlsk2 = nrmu2 * nrmv2;
-  return true;
-}
-
-// ACAr (ACA.h:657-720) with T = dcomp: crosses until the last one is below eps of
-// the approximation's norm, no more than n2 rows used, or kmax crosses.
-__device__ int acar(const G32& g, const HBlk& B, uint32_t i0, uint32_t kmax, uint32_t kcap, double eps,
-                    uint32_t& kout) {
-  const uint32_t n1 = B.n1, n2 = B.n2;
-  for (uint32_t i = g.rank; i < n1; i += 32) B.Z[i] = 0;
-  double scale = cabs(helm_entry(B, B.b1, B.b2));
-  uint32_t k = 0, no = 0;
-  double nrmlsk2 = 0.0, nrms2 = 0.0;
-  int outcome = -1;
-  do {
-    if (k >= kcap) {
-      outcome = kAcaOverflow;
-      break;
-    }
-    if (!acar_step(g, B, i0, k, no, nrmlsk2, scale)) {
-      nrmlsk2 = 0.0;
-      break;
-    }
-    __syncwarp();
-    // Re sum_l scpr(U_l, U_k) scpr(V_l, V_k)
-    double sre = 0.0;
-    const Cx* uk = B.U + (size_t)k * n1;
-    const Cx* vk = B.V + (size_t)k * n2;
-    for (uint32_t l = 0; l < k; ++l) {
-      double ur = 0.0, ui = 0.0, vr = 0.0, vi = 0.0;
-      for (uint32_t i = g.rank; i < n1; i += 32) {
-        const Cx a = B.U[(size_t)l * n1 + i], b = uk[i];
-        ur += a.re * b.re + a.im * b.im;
-        ui += a.re * b.im - a.im * b.re;
-      }
-      for (uint32_t j = g.rank; j < n2; j += 32) {
-        const Cx a = B.V[(size_t)l * n2 + j], b = vk[j];
-        vr += a.re * b.re + a.im * b.im;
-        vi += a.re * b.im - a.im * b.re;
-      }
-      G32::sum2(ur, ui);
-      G32::sum2(vr, vi);
-      sre += ur * vr - ui * vi;
-    }
-    nrms2 += 2.0 * sre + nrmlsk2;
-    ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
-  } while (no < n2 && k < kmax && nrmlsk2 >= eps * eps * nrms2);
-  if (outcome < 0) {
-    const double epsa = sqrt(nrmlsk2 / nrms2);
-    outcome = epsa >= eps ? kAcaFail : kAcaOk;  // NaN (0/0) stays a success, as in the reference
-  }
-  kout = k;
-  __syncwarp();
-  return outcome;
-}
-
 // ---------------------------------------------------------------------------
-// Recompression of a complex low-rank block U V^H (mblock<dcomp>::addtrll,
-// H/mblock_Z.cpp:200-300: QR of U and V, SVD of R1 R2^H after dropping entries
-// below delta |R|_F / sqrt(mmin nmin), truncation at delta sigma_0, Q applied),
-// by one warp.  The row i of every column belongs to lane i % 32.
+// Unions of complex low-rank blocks, by one warp.  The row i of every column belongs
+// to lane i % 32.
 
 __device__ __forceinline__ Cx cmul(Cx a, Cx b) { return Cx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 // conj(a) b
@@ -549,112 +152,6 @@ __device__ void zapply_q(const G32& g, uint32_t m, uint32_t kr, const Cx* A, con
       }
     }
   }
-}
-
-// Un (n1 x kt), Vn (n2 x kt) with Un Vn^H = the truncated U V^H (rank k); R, Vs:
-// column-major with stride ld >= k; sig: k doubles; tau: 2k; perm: nmin + 1 ints.
-__device__ uint32_t zrecompress(const G32& g, uint32_t n1, uint32_t n2, uint32_t k, Cx* U, Cx* V, Cx* Un, Cx* Vn,
-                                double delta, Cx* R, Cx* Vs, uint32_t ld, double* sig, Cx* tau, int* perm) {
-  const uint32_t mmin = min(n1, k), nmin = min(n2, k), amin = min(mmin, nmin);
-  Cx* tau1 = tau;
-  Cx* tau2 = tau + k;
-  zqr(g, n1, k, U, tau1);
-  zqr(g, n2, k, V, tau2);
-  __syncwarp();
-  // R = R1 R2^H (Include/blas.h utrmmh)
-  double fro = 0.0;
-  for (uint32_t i = g.rank; i < mmin; i += 32) {
-    for (uint32_t j = 0; j < nmin; ++j) {
-      double dr = 0.0, di = 0.0;
-      for (uint32_t l = max(i, j); l < k; ++l) {
-        const Cx u = U[i + (size_t)l * n1], v = V[j + (size_t)l * n2];
-        dr += u.re * v.re + u.im * v.im;
-        di += u.im * v.re - u.re * v.im;
-      }
-      R[i + (size_t)j * ld] = Cx{dr, di};
-      fro += dr * dr + di * di;
-    }
-  }
-  fro = G32::sum(fro);
-  const double thresh = delta * sqrt(fro) / (double)sqrtf((float)mmin * (float)nmin);
-  for (uint32_t i = g.rank; i < mmin; i += 32)
-    for (uint32_t j = 0; j < nmin; ++j)
-      if (cabs(R[i + (size_t)j * ld]) < thresh) R[i + (size_t)j * ld] = Cx{0.0, 0.0};
-  for (uint32_t i = g.rank; i < nmin; i += 32)
-    for (uint32_t j = 0; j < nmin; ++j) Vs[i + (size_t)j * ld] = Cx{i == j ? 1.0 : 0.0, 0.0};
-  // one-sided Jacobi (Hestenes) on the columns of R with complex rotations
-  // [x y] <- [c x - s e y, s x + c e y], e = conj(gamma) / |gamma|, gamma = x^H y
-  for (int sweep = 0; sweep < 40; ++sweep) {
-    bool rotated = false;
-    for (uint32_t p = 0; p + 1 < nmin; ++p) {
-      for (uint32_t q = p + 1; q < nmin; ++q) {
-        double al = 0.0, be = 0.0, gr = 0.0, gi = 0.0;
-        for (uint32_t i = g.rank; i < mmin; i += 32) {
-          const Cx x = R[i + (size_t)p * ld], y = R[i + (size_t)q * ld];
-          al += x.re * x.re + x.im * x.im;
-          be += y.re * y.re + y.im * y.im;
-          const Cx z = cmulc(x, y);
-          gr += z.re;
-          gi += z.im;
-        }
-        G32::sum2(al, be);
-        G32::sum2(gr, gi);
-        const double ga = sqrt(gr * gr + gi * gi);
-        if (ga == 0.0 || ga <= 1e-15 * sqrt(al * be)) continue;
-        rotated = true;
-        const double zeta = (be - al) / (2.0 * ga);
-        const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = 1.0 / sqrt(1.0 + t * t);
-        const double s = c * t;
-        const Cx e{gr / ga, -gi / ga};
-        for (uint32_t i = g.rank; i < mmin; i += 32) {
-          const Cx x = R[i + (size_t)p * ld], ey = cmul(e, R[i + (size_t)q * ld]);
-          R[i + (size_t)p * ld] = Cx{c * x.re - s * ey.re, c * x.im - s * ey.im};
-          R[i + (size_t)q * ld] = Cx{s * x.re + c * ey.re, s * x.im + c * ey.im};
-        }
-        for (uint32_t i = g.rank; i < nmin; i += 32) {
-          const Cx x = Vs[i + (size_t)p * ld], ey = cmul(e, Vs[i + (size_t)q * ld]);
-          Vs[i + (size_t)p * ld] = Cx{c * x.re - s * ey.re, c * x.im - s * ey.im};
-          Vs[i + (size_t)q * ld] = Cx{s * x.re + c * ey.re, s * x.im + c * ey.im};
-        }
-      }
-    }
-    if (!rotated) break;
-  }
-  for (uint32_t j = 0; j < nmin; ++j) {
-    double sj = 0.0;
-    for (uint32_t i = g.rank; i < mmin; i += 32) sj += cabs2(R[i + (size_t)j * ld]);
-    sj = G32::sum(sj);
-    if (g.rank == 0) sig[j] = sqrt(sj);
-  }
-  __syncwarp();
-  if (g.rank == 0) {
-    for (uint32_t j = 0; j < nmin; ++j) perm[j] = (int)j;
-    for (uint32_t j = 0; j < nmin; ++j) {
-      uint32_t b = j;
-      for (uint32_t q = j + 1; q < nmin; ++q)
-        if (sig[perm[q]] > sig[perm[b]]) b = q;
-      const int t = perm[j];
-      perm[j] = perm[b];
-      perm[b] = t;
-    }
-    uint32_t kt = min(amin, k);
-    const double s0 = nmin ? sig[perm[0]] : 0.0;
-    while (kt > 0 && (sig[perm[kt - 1]] <= delta * s0 || sig[perm[kt - 1]] < 1e-64)) --kt;
-    perm[nmin] = (int)kt;
-  }
-  __syncwarp();
-  const uint32_t kt = (uint32_t)perm[nmin];
-  // Un = Q1 [R(:, perm[:kt]); 0] (R's columns are sigma_j u_j), Vn = Q2 [Vs(:, perm[:kt]); 0]
-  for (uint32_t j = 0; j < kt; ++j) {
-    const int pj = perm[j];
-    for (uint32_t i = g.rank; i < n1; i += 32) Un[i + (size_t)j * n1] = i < mmin ? R[i + (size_t)pj * ld] : Cx{0.0, 0.0};
-    for (uint32_t i = g.rank; i < n2; i += 32) Vn[i + (size_t)j * n2] = i < nmin ? Vs[i + (size_t)pj * ld] : Cx{0.0, 0.0};
-  }
-  zapply_q(g, n1, mmin, U, tau1, kt, Un);
-  zapply_q(g, n2, nmin, V, tau2, kt, Vn);
-  __syncwarp();
-  return kt;
 }
 
 // Recompression of a union of complex low-rank blocks (agglomeration of mblock<dcomp>
@@ -957,49 +454,6 @@ __global__ void __launch_bounds__(32) zmerge_kernel(MergeParams p) {
   if (g.rank == 0) p.res[ti] = AcaResult{kAcaOk, kc, kt, 0u};
 }
 
-// One leaf of the Helmholtz assembly.  Workspace (complex, at ws):
-//   U[n1 kcap] V[n2 kcap] Un[n1 kcap] Vn[n2 kcap] R[kcap^2] Vs[kcap^2] sig[kcap] tau[2 kcap]
-// ints at zs: Z[n1] S[n2] (later the SVD permutation).
-struct ZTask {
-  uint32_t b1, n1, b2, n2, i0, kmax, kcap, leaf;
-  uint64_t ws, zs;
-};
-
-__global__ void __launch_bounds__(32 * kWarps)
-    helm_assemble_kernel(PointsSoA P, double k, double h, double eps, const ZTask* __restrict__ tasks, uint32_t n,
-                         Cx* __restrict__ ws, int* __restrict__ zs, AcaResult* __restrict__ res, int sym) {
-  const uint32_t t = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  if (t >= n) return;
-  const ZTask T = tasks[t];
-  G32 g(threadIdx.x & 31);
-  HBlk B;
-  B.P = P;
-  B.k = k;
-  B.h = h;
-  B.b1 = T.b1;
-  B.n1 = T.n1;
-  B.b2 = T.b2;
-  B.n2 = T.n2;
-  const uint32_t kc = T.kcap;
-  B.U = ws + T.ws;
-  B.V = B.U + (size_t)T.n1 * kc;
-  B.Z = zs + T.zs;
-  B.S = B.Z + T.n1;
-  uint32_t kk = 0, kt = 0;
-  const int st = sym ? acar(g, B, T.i0, T.kmax, kc, eps, kk) : aca(g, B, T.i0, T.kmax, kc, eps, kk);
-  if (st == kAcaOk && kk > 0) {
-    Cx* Un = B.V + (size_t)T.n2 * kc;
-    Cx* Vn = Un + (size_t)T.n1 * kc;
-    Cx* R = Vn + (size_t)T.n2 * kc;
-    Cx* Vs = R + (size_t)kc * kc;
-    double* sig = reinterpret_cast<double*>(Vs + (size_t)kc * kc);
-    Cx* tau = Vs + (size_t)kc * kc + kc;
-    __syncwarp();
-    kt = zrecompress(g, T.n1, T.n2, kk, B.U, B.V, Un, Vn, eps, R, Vs, kc, sig, tau, B.Z);
-  }
-  if (g.rank == 0) res[t] = AcaResult{st, kk, kt, 0u};
-}
-
 struct ZDense {
   uint32_t b1, n1, b2, n2;
   uint64_t off;
@@ -1008,29 +462,12 @@ struct ZDense {
 __global__ void helm_dense_kernel(PointsSoA P, double k, double h, const ZDense* __restrict__ tasks,
                                   Cx* __restrict__ arena) {
   const ZDense t = tasks[blockIdx.x];
-  HBlk B;
-  B.P = P;
-  B.k = k;
-  B.h = h;
   const uint64_t cnt = (uint64_t)t.n1 * t.n2;
   Cx* out = arena + t.off;
   for (uint64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
     const uint32_t i = (uint32_t)(e % t.n1), j = (uint32_t)(e / t.n1);
-    out[e] = helm_entry(B, t.b1 + i, t.b2 + j);
+    out[e] = helm_entry(P, k, h, t.b1 + i, t.b2 + j);
   }
-}
-
-struct ZCopy {
-  uint64_t src_u, src_v, dst;
-  uint32_t n1, n2, kt, pad;
-};
-
-__global__ void helm_copy_kernel(const ZCopy* __restrict__ tasks, const Cx* __restrict__ ws, Cx* __restrict__ arena) {
-  const ZCopy t = tasks[blockIdx.x];
-  const uint64_t nu = (uint64_t)t.n1 * t.kt, nv = (uint64_t)t.n2 * t.kt;
-  Cx* dst = arena + t.dst;
-  for (uint64_t e = threadIdx.x; e < nu; e += blockDim.x) dst[e] = ws[t.src_u + e];
-  for (uint64_t e = threadIdx.x; e < nv; e += blockDim.x) dst[nu + e] = ws[t.src_v + e];
 }
 
 struct HTask {
@@ -1045,11 +482,9 @@ __global__ void __launch_bounds__(32 * kWarps)
   const uint32_t t = blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (t >= n) return;
   const HTask T = tasks[t];
-  G32 g(threadIdx.x & 31);
-  HBlk B;
-  B.P = P;
-  B.k = k;
-  B.h = h;
+  Team<1> g(threadIdx.x & 31, nullptr);
+  lowrank::Blk<HelmGen> B;
+  B.gen = HelmGen{P, k, h};
   B.b1 = T.b1;
   B.n1 = T.n1;
   B.b2 = T.b2;
@@ -1058,8 +493,11 @@ __global__ void __launch_bounds__(32 * kWarps)
   B.V = B.U + (size_t)T.n1 * T.kcap;
   B.Z = zs + T.zs;
   B.S = B.Z + T.n1;
+  B.P = nullptr;  // the ranks alone: no recompression
+  B.d2 = nullptr;
+  B.ld = 0;
   uint32_t kk = 0;
-  const int st = aca(g, B, 0u, T.kmax, T.kcap, eps, kk);
+  const int st = lowrank::aca(g, B, 0u, T.kmax, T.kcap, eps, kk);
   if (g.rank == 0) res[t] = make_int2(st, (int)kk);
 }
 
@@ -1187,10 +625,6 @@ int zarena_append(ahx_hmat* H, uint64_t count, uint64_t& off) {
   return AHX_OK;
 }
 
-namespace {
-uint64_t zws_elems(const ZTask& t) { return aca_ws_doubles(t.n1, t.n2, t.kcap); }
-
-}  // namespace
 }  // namespace ahx
 
 extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, double eps, uint32_t rankmax) {
@@ -1213,105 +647,30 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
   Z.aca_rank.assign(nl, -1);
   Z.off.assign(nl, 0);
   H->stat_ws_bytes = H->stat_retries = H->stat_batches = 0;
-  std::vector<ZTask> tasks;
+  std::vector<AcaTask> tasks;
   std::vector<uint32_t> dense;
   const uint32_t kcap0 = aca_kcap_default();
   for (uint32_t l = 0; l < nl; ++l) {
     const Leaf& L = Ls[l];
     const uint32_t maxk = maxk_of(L.n1, L.n2, rankmax);
-    if (L.adm && maxk) {
-      ZTask t{};
-      t.b1 = L.b1;
-      t.n1 = L.n1;
-      t.b2 = L.b2;
-      t.n2 = L.n2;
-      t.i0 = L.i0;
-      t.kmax = maxk;
-      t.kcap = std::min(kcap_limit(maxk), kcap0);
-      t.leaf = l;
-      tasks.push_back(t);
-    } else {
-      dense.push_back(l);
-    }
+    if (L.adm && maxk) tasks.push_back(AcaTask{L.b1, L.n1, L.b2, L.n2, L.i0, maxk, std::min(kcap_limit(maxk), kcap0), l});
+    else dense.push_back(l);
   }
   uint64_t est = 0;
   for (uint32_t l : dense) est += (uint64_t)Ls[l].n1 * Ls[l].n2;
-  for (const ZTask& t : tasks) est += (uint64_t)(t.n1 + t.n2) * std::min(t.kmax, 16u);
+  for (const AcaTask& t : tasks) est += (uint64_t)(t.n1 + t.n2) * std::min(t.kmax, 16u);
   if (Z.arena.bytes < est * sizeof(Cx)) {
     Z.arena.release();
     if ((rc = Z.arena.reserve(std::max<uint64_t>(est, 1) * sizeof(Cx)))) return rc;
   }
-  const size_t budget = aca_ws_budget();
   const double* pts = H->pts.as<double>();
   const PointsSoA P{pts, pts + H->tree.n, pts + 2 * (size_t)H->tree.n};
-  ScopedBuf ws, zs, dtasks, dres, dcopy;
-  while (!tasks.empty()) {
-    std::sort(tasks.begin(), tasks.end(), [](const ZTask& a, const ZTask& b) {
-      return (uint64_t)(a.n1 + a.n2) * a.kcap > (uint64_t)(b.n1 + b.n2) * b.kcap;
-    });
-    std::vector<ZTask> retry;
-    size_t i = 0;
-    while (i < tasks.size()) {
-      uint64_t wsc = 0, zsi = 0;
-      size_t j = i;
-      for (; j < tasks.size(); ++j) {
-        const uint64_t w = zws_elems(tasks[j]);
-        if (j > i && (wsc + w) * sizeof(Cx) + (zsi + tasks[j].n1 + tasks[j].n2) * 4 > budget) break;
-        tasks[j].ws = wsc;
-        tasks[j].zs = zsi;
-        wsc += w;
-        zsi += tasks[j].n1 + tasks[j].n2;
-      }
-      std::vector<ZTask> batch(tasks.begin() + i, tasks.begin() + j);
-      i = j;
-      H->stat_ws_bytes = std::max<uint64_t>(H->stat_ws_bytes, wsc * sizeof(Cx) + zsi * 4);
-      H->stat_batches++;
-      if ((rc = ws.reserve(std::max<uint64_t>(wsc, 1) * sizeof(Cx)))) return rc;
-      if ((rc = zs.reserve(std::max<uint64_t>(zsi, 1) * 4))) return rc;
-      if ((rc = upload(dtasks, batch, H->stream))) return rc;
-      if ((rc = dres.reserve(batch.size() * sizeof(AcaResult)))) return rc;
-      const uint32_t nb = (uint32_t)batch.size();
-      helm_assemble_kernel<<<(nb + kWarps - 1) / kWarps, 32 * kWarps, 0, H->stream>>>(
-          P, wavenumber, h, eps, dtasks.as<ZTask>(), nb, ws.as<Cx>(), zs.as<int>(), dres.as<AcaResult>(),
-          H->tree.sym ? 1 : 0);
-      AHX_CUDA(cudaGetLastError());
-      std::vector<AcaResult> res(nb);
-      AHX_CUDA(cudaMemcpyAsync(res.data(), dres.p, nb * sizeof(AcaResult), cudaMemcpyDeviceToHost, H->stream));
-      AHX_CUDA(cudaStreamSynchronize(H->stream));
-      std::vector<ZCopy> copies;
-      for (uint32_t q = 0; q < nb; ++q) {
-        const ZTask& t = batch[q];
-        const AcaResult& r = res[q];
-        if (r.status == kAcaOverflow && t.kcap < kcap_limit(t.kmax)) {
-          ZTask u = t;
-          u.kcap = std::min(kcap_limit(t.kmax), std::max(t.kcap * 4, 16u));
-          retry.push_back(u);
-          H->stat_retries++;
-          continue;
-        }
-        if (r.status != kAcaOk) {
-          dense.push_back(t.leaf);
-          continue;
-        }
-        Z.aca_rank[t.leaf] = (int32_t)r.k_aca;
-        Z.rank[t.leaf] = (int32_t)r.kt;
-        if (r.kt == 0) continue;
-        uint64_t off = 0;
-        if ((rc = zarena_append(H, (uint64_t)r.kt * (t.n1 + t.n2), off))) return rc;
-        Z.off[t.leaf] = off;
-        const uint64_t un = t.ws + (uint64_t)(t.n1 + t.n2) * t.kcap;  // Un follows U and V
-        copies.push_back(ZCopy{un, un + (uint64_t)t.n1 * t.kcap, off, t.n1, t.n2, r.kt, 0u});
-      }
-      if (!copies.empty()) {
-        if ((rc = upload(dcopy, copies, H->stream))) return rc;
-        helm_copy_kernel<<<(uint32_t)copies.size(), 128, 0, H->stream>>>(dcopy.as<ZCopy>(), ws.as<Cx>(),
-                                                                          Z.arena.as<Cx>());
-        AHX_CUDA(cudaGetLastError());
-      }
-      AHX_CUDA(cudaStreamSynchronize(H->stream));
-    }
-    tasks.swap(retry);
-  }
+  AcaParams par{};
+  par.pts = P;
+  par.k = wavenumber;
+  par.h = h;
+  par.eps = eps;
+  if ((rc = run_aca(H, true, tasks, par, dense))) return rc;
   // dense leaves (inadmissible and failed ACA) in leaf order
   std::sort(dense.begin(), dense.end());
   std::vector<ZDense> dt;
@@ -1392,6 +751,13 @@ extern "C" int ahx_helm_get_leaf(const ahx_hmat* H, uint32_t l, double* out) {
 }
 
 namespace ahx {
+cudaError_t launch_zaca(const AcaParams& p, uint32_t grid, cudaStream_t s) {
+  return lowrank::launch_aca_kernel(HelmGen{p.pts, p.k, p.h}, p, grid, s);
+}
+cudaError_t resident_zaca(int device, uint32_t& ctas) {
+  return lowrank::resident_aca_kernel<HelmGen>(device, ctas);
+}
+
 cudaError_t launch_zmerge(const MergeParams& p, cudaStream_t s) {
   if (p.ntasks == 0) return cudaSuccess;
   zmerge_kernel<<<p.ntasks, 32, 0, s>>>(p);

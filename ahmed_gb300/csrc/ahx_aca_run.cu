@@ -1,0 +1,154 @@
+// Host side of an assembly's ACA: order of the leaves, workspace slots, retries.
+#include <algorithm>
+#include <cmath>
+
+#include "ahx_aca.cuh"
+#include "ahx_hmat.hpp"
+
+namespace ahx {
+namespace {
+
+// A leaf goes to a CTA instead of a warp when its rows and columns are more than half of
+// what a resident warp gets on average (a warp that takes longer ends after the others),
+// but never below 512, where the work on the k x k arrays (one warp, the others wait)
+// outweighs the rows.  A leaf's k x k work counts as 256 rows.
+constexpr uint64_t kLeafRows = 256, kLargeMin = 512;
+
+// Workspace sizes in steps of 1/16 octave: tasks sort by class in linear time.
+uint32_t size_class(uint64_t b) {
+  const int m = 63 - __builtin_clzll(b | 16);
+  return (uint32_t)(m * 16) + (uint32_t)((b >> (m - 4)) & 15);
+}
+uint64_t class_bytes(uint32_t c) {  // an upper bound of the class, a multiple of 256
+  const uint64_t top = (uint64_t)(16 + (c & 15) + 1) << (c / 16 - 4);
+  return (top + 255) & ~255ull;
+}
+
+void sort_descending(std::vector<AcaTask>& t, std::vector<uint32_t>& cls, size_t elem) {
+  std::vector<uint32_t> c(t.size()), at(1025, 0);
+  for (size_t i = 0; i < t.size(); ++i) {
+    c[i] = 1023 - size_class(aca_ws_bytes(t[i].n1, t[i].n2, t[i].kcap, elem));
+    ++at[c[i] + 1];
+  }
+  for (size_t i = 0; i < 1024; ++i) at[i + 1] += at[i];
+  std::vector<AcaTask> out(t.size());
+  cls.resize(t.size());
+  for (size_t i = 0; i < t.size(); ++i) {
+    const uint32_t p = at[c[i]]++;
+    out[p] = t[i];
+    cls[p] = 1023 - c[i];
+  }
+  t.swap(out);
+}
+
+}  // namespace
+
+int run_aca(ahx_hmat* H, bool cplx, std::vector<AcaTask>& tasks, AcaParams p, std::vector<uint32_t>& dense) {
+  const size_t elem = cplx ? 16 : 8;
+  DevBuf& arena = cplx ? H->z.arena : H->arena64;
+  uint64_t& elems = cplx ? H->z.elems : H->arena64_elems;
+  std::vector<int32_t>& rank = cplx ? H->z.rank : H->rank;
+  std::vector<int32_t>& aca_rank = cplx ? H->z.aca_rank : H->aca_rank;
+  std::vector<uint64_t>& offs = cplx ? H->z.off : H->off;
+  const uint64_t budget = aca_ws_budget();
+  p.variant = H->tree.sym ? kAcaVariantSym : kAcaVariantGeneral;
+  uint32_t ctas = 0;
+  AHX_CUDA(cplx ? resident_zaca(H->device, ctas) : resident_aca(H->device, ctas));
+  constexpr uint32_t kWarps = kAcaThreads / 32;
+  ScopedBuf ws, dtasks, dres, dslots, dctl;
+  int rc;
+  while (!tasks.empty()) {
+    uint64_t rows = 0;
+    for (const AcaTask& t : tasks) rows += (uint64_t)t.n1 + t.n2 + kLeafRows;
+    const uint64_t lim = std::max<uint64_t>(kLargeMin, rows / ((uint64_t)ctas * kWarps * 2));
+    std::vector<AcaTask> large, small;
+    for (const AcaTask& t : tasks) ((uint64_t)t.n1 + t.n2 > lim ? large : small).push_back(t);
+    std::vector<uint32_t> cl, cs;
+    sort_descending(large, cl, elem);
+    sort_descending(small, cs, elem);
+    // slots: each phase takes at most half the budget, and at least one team runs
+    std::vector<uint64_t> slots;
+    uint64_t bytes = 0, part = 0;
+    p.nlarge = (uint32_t)large.size();
+    p.nsmall = (uint32_t)small.size();
+    p.nslot_l = p.nslot_s = 0;
+    for (; p.nslot_l < std::min(ctas, p.nlarge); ++p.nslot_l) {
+      const uint64_t b = class_bytes(cl[p.nslot_l]);
+      if (p.nslot_l && part + b > budget / 2) break;
+      slots.push_back(bytes);
+      bytes += b;
+      part += b;
+    }
+    part = 0;
+    for (; p.nslot_s < std::min(ctas * kWarps, p.nsmall); ++p.nslot_s) {
+      const uint64_t b = class_bytes(cs[p.nslot_s]);
+      if (p.nslot_s && part + b > budget / 2) break;
+      slots.push_back(bytes);
+      bytes += b;
+      part += b;
+    }
+    H->stat_ws_bytes = std::max<uint64_t>(H->stat_ws_bytes, bytes);
+    H->stat_batches++;
+    std::vector<AcaTask> all(std::move(large));
+    all.insert(all.end(), small.begin(), small.end());
+    struct Ctl {
+      unsigned long long used;
+      uint32_t ctr[2];
+    };
+    const std::vector<Ctl> ctl{{elems, {0u, 0u}}};
+    if ((rc = ws.reserve(bytes)) || (rc = upload(dtasks, all, H->stream)) || (rc = upload(dslots, slots, H->stream)) ||
+        (rc = upload(dctl, ctl, H->stream)) || (rc = dres.reserve(all.size() * sizeof(AcaResult))))
+      return rc;
+    p.tasks = dtasks.as<AcaTask>();
+    p.res = dres.as<AcaResult>();
+    p.slots = dslots.as<uint64_t>();
+    p.ws = ws.as<unsigned char>();
+    p.arena = arena.p;
+    p.cap = arena.bytes / elem;
+    p.used = &dctl.as<Ctl>()->used;
+    p.ctr = dctl.as<Ctl>()->ctr;
+    const uint32_t grid = std::max(p.nslot_l, (p.nslot_s + kWarps - 1) / kWarps);
+    AHX_CUDA(cplx ? launch_zaca(p, grid, H->stream) : launch_aca(p, grid, H->stream));
+    std::vector<AcaResult> res(all.size());
+    AHX_CUDA(cudaMemcpyAsync(res.data(), dres.p, res.size() * sizeof(AcaResult), cudaMemcpyDeviceToHost, H->stream));
+    AHX_CUDA(cudaStreamSynchronize(H->stream));
+    std::vector<AcaTask> retry;
+    uint64_t end = elems, more = 0;
+    for (size_t q = 0; q < all.size(); ++q) {
+      const AcaTask& t = all[q];
+      const AcaResult& r = res[q];
+      const uint64_t size = (uint64_t)r.kt * ((uint64_t)t.n1 + t.n2);
+      // an overflow at the full capacity cannot happen (kcap_limit); were it
+      // to, the leaf is treated as an ACA failure so that the loop ends
+      if (r.status == kAcaOverflow && t.kcap < kcap_limit(t.kmax)) {
+        AcaTask u = t;
+        u.kcap = std::min(kcap_limit(t.kmax), std::max(t.kcap * 4, 16u));
+        retry.push_back(u);
+        H->stat_retries++;
+      } else if (r.status == kAcaNoSpace) {  // the arena was estimated too small
+        retry.push_back(t);
+        more += size;
+      } else if (r.status != kAcaOk) {
+        dense.push_back(t.leaf);
+      } else {
+        aca_rank[t.leaf] = (int32_t)r.k_aca;
+        rank[t.leaf] = (int32_t)r.kt;
+        if (r.kt == 0) continue;
+        offs[t.leaf] = r.off;
+        end = std::max(end, r.off + size);
+      }
+    }
+    elems = end;
+    if (!retry.empty()) {
+      // room for the retried leaves: what they needed, or twice the estimate's 16 columns
+      for (const AcaTask& t : retry) more += (uint64_t)(t.n1 + t.n2) * std::min(t.kmax, 32u);
+      uint64_t off = 0;
+      if ((rc = cplx ? zarena_append(H, more, off) : arena_append(H, more, off))) return rc;
+      elems = off;
+    }
+    tasks.swap(retry);
+  }
+  return AHX_OK;
+}
+
+}  // namespace ahx

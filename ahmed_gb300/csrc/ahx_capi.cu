@@ -17,118 +17,6 @@ namespace ahx {
 
 namespace {
 thread_local std::string g_err;
-
-// leaves with more rows or columns than this use the CTA-per-leaf kernel; the
-// rest run one warp per leaf (warp reductions; the FP64 pipe is the limit)
-constexpr uint32_t kLargeLeaf = 4096;
-
-// Runs ACA + recompression for `tasks` in workspace-bounded batches, appends the
-// factors to the arena; failed leaves go to `dense`, capacity overflows to `retry`.
-int run_aca(ahx_hmat* H, std::vector<AcaTask>& tasks, double diag, double eps,
-            std::vector<uint32_t>& dense, std::vector<AcaTask>& retry) {
-  const size_t budget = aca_ws_budget();
-  std::sort(tasks.begin(), tasks.end(), [](const AcaTask& a, const AcaTask& b) {
-    return (uint64_t)(a.n1 + a.n2) * a.kcap > (uint64_t)(b.n1 + b.n2) * b.kcap;
-  });
-  DevBuf ws, zs, dtasks, dres, dcopy;
-  size_t i = 0;
-  while (i < tasks.size()) {
-    // gather one batch
-    std::vector<AcaTask> small, large;
-    uint64_t wsd = 0, zsi = 0;
-    size_t j = i;
-    while (j < tasks.size()) {
-      AcaTask t = tasks[j];
-      const uint64_t w = aca_ws_doubles(t.n1, t.n2, t.kcap);
-      if (j > i && (wsd + w) * 8 + (zsi + t.n1 + t.n2) * 4 > budget) break;
-      t.ws = wsd;
-      t.zs = zsi;
-      wsd += w;
-      zsi += t.n1 + t.n2;
-      (std::max(t.n1, t.n2) > kLargeLeaf ? large : small).push_back(t);
-      ++j;
-    }
-    i = j;
-    H->stat_ws_bytes = std::max<uint64_t>(H->stat_ws_bytes, wsd * sizeof(double) + zsi * sizeof(int));
-    H->stat_batches++;
-    int rc = ws.reserve(std::max<uint64_t>(wsd, 1) * sizeof(double));
-    if (rc) return rc;
-    rc = zs.reserve(std::max<uint64_t>(zsi, 1) * sizeof(int));
-    if (rc) return rc;
-    std::vector<AcaTask> all(large);
-    all.insert(all.end(), small.begin(), small.end());
-    if ((rc = upload(dtasks, all, H->stream))) return rc;
-    rc = dres.reserve(all.size() * sizeof(AcaResult));
-    if (rc) return rc;
-    AcaParams p;
-    const double* pts = H->pts.as<double>();
-    p.pts = PointsSoA{pts, pts + H->tree.n, pts + 2 * (size_t)H->tree.n};
-    p.diag = diag;
-    p.eps = eps;
-    p.variant = H->tree.sym ? kAcaVariantSym : kAcaVariantGeneral;
-    p.ws = ws.as<double>();
-    p.zs = zs.as<int>();
-    p.tasks = dtasks.as<AcaTask>();
-    p.res = dres.as<AcaResult>();
-    p.ntasks = (uint32_t)large.size();
-    AHX_CUDA(launch_aca_large(p, H->stream));
-    p.tasks = dtasks.as<AcaTask>() + large.size();
-    p.res = dres.as<AcaResult>() + large.size();
-    p.ntasks = (uint32_t)small.size();
-    AHX_CUDA(launch_aca_small(p, H->stream));
-    std::vector<AcaResult> res(all.size());
-    AHX_CUDA(cudaMemcpyAsync(res.data(), dres.p, res.size() * sizeof(AcaResult),
-                             cudaMemcpyDeviceToHost, H->stream));
-    AHX_CUDA(cudaStreamSynchronize(H->stream));
-    std::vector<CopyTask> copies;
-    for (size_t q = 0; q < all.size(); ++q) {
-      const AcaTask& t = all[q];
-      const AcaResult& r = res[q];
-      // an overflow at the full capacity cannot happen (kcap_limit); were it
-      // to, the leaf is treated as an ACA failure so that the loop ends
-      if (r.status == kAcaOverflow && t.kcap < kcap_limit(t.kmax)) {
-        AcaTask u = t;
-        u.kcap = std::min(kcap_limit(t.kmax), std::max(t.kcap * 4, 16u));
-        retry.push_back(u);
-        H->stat_retries++;
-        continue;
-      }
-      if (r.status != kAcaOk) {
-        dense.push_back(t.leaf);
-        continue;
-      }
-      H->aca_rank[t.leaf] = (int32_t)r.k_aca;
-      H->rank[t.leaf] = (int32_t)r.kt;
-      if (r.kt == 0) continue;
-      uint64_t off = 0;
-      if ((rc = arena_append(H, (uint64_t)r.kt * (t.n1 + t.n2), off))) return rc;
-      H->off[t.leaf] = off;
-      const uint64_t un = t.ws + (uint64_t)(t.n1 + t.n2) * t.kcap;  // Un follows U and V
-      CopyTask c;
-      c.src_u = un;
-      c.src_v = un + (uint64_t)t.n1 * t.kcap;
-      c.dst = off;
-      c.n1 = t.n1;
-      c.n2 = t.n2;
-      c.kt = r.kt;
-      c.pad = 0;
-      copies.push_back(c);
-    }
-    if (!copies.empty()) {
-      if ((rc = upload(dcopy, copies, H->stream))) return rc;
-      AHX_CUDA(launch_copy_factors(dcopy.as<CopyTask>(), (uint32_t)copies.size(), ws.as<double>(),
-                                   H->arena64.as<double>(), H->stream));
-    }
-    AHX_CUDA(cudaStreamSynchronize(H->stream));
-  }
-  ws.release();
-  zs.release();
-  dtasks.release();
-  dres.release();
-  dcopy.release();
-  return AHX_OK;
-}
-
 }  // namespace
 
 // Append-only growable FP64 arena.
@@ -870,11 +758,12 @@ int ahx_assemble_hinted(ahx_hmat* H, double h, double eps, uint32_t rankmax,
     rc = H->arena64.reserve(std::max<uint64_t>(est, 1) * sizeof(double));
     if (rc) return rc;
   }
-  while (!tasks.empty()) {
-    std::vector<AcaTask> retry;
-    if ((rc = run_aca(H, tasks, diag, eps, dense, retry))) return rc;
-    tasks.swap(retry);
-  }
+  const double* pts = H->pts.as<double>();
+  AcaParams par{};
+  par.pts = PointsSoA{pts, pts + H->tree.n, pts + 2 * (size_t)H->tree.n};
+  par.diag = diag;
+  par.eps = eps;
+  if ((rc = run_aca(H, false, tasks, par, dense))) return rc;
   // dense leaves (inadmissible and failed ACA), filled in leaf order
   std::sort(dense.begin(), dense.end());
   std::vector<DenseTask> dt;
@@ -890,9 +779,7 @@ int ahx_assemble_hinted(ahx_hmat* H, double h, double eps, uint32_t rankmax,
   if (!dt.empty()) {
     DevBuf ddt;
     if ((rc = upload(ddt, dt, H->stream))) return rc;
-    const double* pts = H->pts.as<double>();
-    PointsSoA P{pts, pts + H->tree.n, pts + 2 * (size_t)H->tree.n};
-    AHX_CUDA(launch_dense_fill(P, diag, ddt.as<DenseTask>(), (uint32_t)dt.size(),
+    AHX_CUDA(launch_dense_fill(par.pts, diag, ddt.as<DenseTask>(), (uint32_t)dt.size(),
                                H->arena64.as<double>(), H->stream));
     AHX_CUDA(cudaStreamSynchronize(H->stream));
   }

@@ -232,6 +232,11 @@ int prepare_df_x(ahx::ProdCopy& pc, uint64_t n, uint32_t p);
 int run_df(const ahx::MvLeaf* leaves, const uint32_t* order, uint32_t nleaves, ahx::ProdCopy& pc, uint64_t n,
            double d, uint32_t p, const double* X, uint64_t ldX, double* Y, uint64_t ldY, cudaStream_t s);
 int ensure_device(ahx_hmat* H);
+// ACA + recompression of `tasks` into the leaf arena (cplx: the Helmholtz one), retried
+// with more columns where they overflow; failed leaves are appended to `dense`
+struct AcaTask;
+struct AcaParams;
+int run_aca(ahx_hmat* H, bool cplx, std::vector<AcaTask>& tasks, AcaParams p, std::vector<uint32_t>& dense);
 // Reserves count doubles at the end of the FP64 leaf arena (grows it, stream-ordered).
 int arena_append(ahx_hmat* H, uint64_t count, uint64_t& off);
 // Drops every precision's product copy (after the leaves change).
