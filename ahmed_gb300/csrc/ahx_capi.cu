@@ -488,7 +488,10 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2 &&
       (prec == kDF64 || dg_due(H->dg[transposed ? 1 : 0], H->arena64_elems, p, H->tree.leaves.size()))) {
     bool usable = false;
-    if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
+    // (nothing is laid out or allocated while the stream is captured)
+    const DgState& D = H->dg[transposed ? 1 : 0];
+    if ((D.valid && H->dg_work.bytes >= dg_work_bytes(false, H->tree.n, D.t_rows, p)) || !stream_captured(H->stream))
+      if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
     if (usable) {
       const DgPlan pl = dg_plan(H->dg[transposed ? 1 : 0], H->tree.n, H->arena64.p, H->dg_work);
       const DgArgs da{false, d, 0.0, p, X, ldX, Y, ldY};

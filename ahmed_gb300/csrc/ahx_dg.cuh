@@ -112,5 +112,10 @@ cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cuda
 // *bad |= any of the count doubles is not finite, or not zero and outside [2^-500, 2^500]
 cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStream_t s);
 cudaError_t launch_matvec_dg(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
+// complex64 leaves over the same layout (ahx_matvec_zt.cu; X, Y complex128): pl.arena the
+// complex64 copy, pl.work of zt_work_bytes
+size_t zt_work_bytes(uint32_t n, uint32_t t_rows, uint32_t p);
+cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
+bool zt_wanted(uint64_t elems, uint32_t p);
 
 }  // namespace ahx

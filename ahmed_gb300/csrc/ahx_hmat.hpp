@@ -106,6 +106,7 @@ struct ZState {
   DevBuf arena;                         // complex128 elements
   uint64_t elems = 0;
   DevBuf arena32;                       // complex64 copy (AHX_FP32 storage)
+  DevBuf xf;                            // X as complex64, 16 right-hand sides
   bool valid32 = false;
   DevBuf leaves, order;                 // product leaf table, launch order
   uint32_t nleaves = 0;
@@ -124,7 +125,7 @@ struct ZState {
   }
   void release_all() {
     drop_table();
-    for (DevBuf* b : {&arena, &arena32, &leaves, &order, &tleaves, &torder, &gm, &xc}) b->release();
+    for (DevBuf* b : {&arena, &arena32, &xf, &leaves, &order, &tleaves, &torder, &gm, &xc}) b->release();
     assembled = false;
     elems = 0;
     nleaves = ntleaves = 0;
@@ -218,6 +219,8 @@ bool dg_wanted(uint64_t elems, uint32_t p);
 // layout exists; before, when the plain products so far and this one cost as much
 // as the layout does.
 bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves);
+// Whether a graph capture is under way on the stream (nothing may be allocated or waited for).
+bool stream_captured(cudaStream_t s);
 // Builds the layout of `leaves`; looks at the arena's elements once (finite).
 // count: its doubles.
 int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,

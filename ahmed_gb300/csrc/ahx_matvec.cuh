@@ -82,9 +82,14 @@ struct ZArgs {
   double2* Y;
   uint64_t ldY;
   int op;
-  const int* guard = nullptr;  // as MvArgs::guard
+  const int* guard = nullptr;  // as MvArgs::guard; complex128 leaves only
+  uint64_t elems = 0;          // complex64 leaves: elements,
+  uint32_t n = 0;              //   rows of X,
+  float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes),
+  bool d_one = false;          //   d = 1 (set by the launcher)
 };
 cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s);
+size_t matvec_z_xf_bytes(uint64_t n);
 // dst[i] = (float) src[i], complex128 -> complex64
 cudaError_t launch_z_to_c64(const double2* src, uint64_t n, float2* dst, cudaStream_t s);
 

@@ -11,6 +11,16 @@
 // side has one row per thread (coalesced factor reads).  Complex128 leaves
 // accumulate in FP64, complex64 leaves in FP32; contributions reach Y through
 // FP64 atomics (leaves share rows).
+//
+// Complex64 leaves with more than four right-hand sides: FP64 instructions bound the
+// kernel (one warp instruction occupies the SM's FP64 pipe for 16 clocks, 64 FP32 issue
+// slots, also when it is predicated off; rounding X per leaf, widening the sums and
+// multiplying by d kept that pipe 73 % busy).  With PRE, X is rounded to complex64 once
+// (zc_x_kernel), sums are widened by integer operations, and d = 1 is not multiplied.
+// 16,384 points: 16 right-hand sides 665 -> 462 us, 8: 366 -> 269 us (then bound by the
+// L1: broadcast loads, atomic additions).  Up to four right-hand sides it gains nothing
+// (p = 3: 170 -> 171 us), below 3 10^7 (elements x right-hand sides) the extra launch
+// outweighs it (1,025 points, p = 8: 54 -> 56 us).
 #include <algorithm>
 
 #include "ahx_matvec.cuh"
@@ -20,6 +30,7 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kCh = 64;  // input rows per staged chunk
+constexpr int kXW = 16;  // right-hand sides of the rounded copy
 
 template <typename R>
 struct C2 {
@@ -44,36 +55,69 @@ __device__ __forceinline__ C2<float> ldz(const float2* p, bool cj) {
   return C2<float>{v.x, cj ? -v.y : v.y};
 }
 
-// Xs[j][r] = X[row0 + j, r0 + r] for j < jn (zero for r >= pg)
-template <typename R, int PG>
+// a float as a double by integer operations.  Zeros, denormals, infinities and NaN are
+// converted in a function of its own: predicated in line, the conversion would occupy
+// the FP64 pipe for every value.
+__device__ __noinline__ double widen_other(float f) { return (double)f; }
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xffu;
+  if (e == 0u || e == 255u) return widen_other(f);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __noinline__ void scale_pair(double dre, double dim, double& ar, double& ai) {
+  const double t = dre * ar - dim * ai;
+  ai = dre * ai + dim * ar;
+  ar = t;
+}
+
+// Xs[j][r] = X[row0 + j, r0 + r] for j < jn (zero for r >= pg); PRE: from the rounded
+// copy, rows of kXW
+template <typename R, int PG, bool PRE>
 __device__ __forceinline__ void stage(C2<R> (*Xs)[PG], const ZArgs& a, uint32_t r0, uint32_t pg, uint32_t row0,
                                       uint32_t jn) {
-  for (uint32_t e = threadIdx.x; e < jn * PG; e += kThreads) {
-    const uint32_t j = e % jn, r = e / jn;
-    C2<R> v{(R)0, (R)0};
-    if (r < pg) {
-      const double2 x = a.X[(uint64_t)(r0 + r) * a.ldX + row0 + j];
-      v = C2<R>{(R)x.x, (R)x.y};
+  if constexpr (PRE) {
+    for (uint32_t e = threadIdx.x; e < jn * PG; e += kThreads) {
+      const uint32_t j = e / PG, r = e % PG;
+      const float2 x = __ldg(a.xf + (uint64_t)(row0 + j) * kXW + r0 + r);
+      Xs[j][r] = C2<R>{x.x, x.y};
     }
-    Xs[j][r] = v;
+  } else {
+    for (uint32_t e = threadIdx.x; e < jn * PG; e += kThreads) {
+      const uint32_t j = e % jn, r = e / jn;
+      C2<R> v{(R)0, (R)0};
+      if (r < pg) {
+        const double2 x = a.X[(uint64_t)(r0 + r) * a.ldX + row0 + j];
+        v = C2<R>{(R)x.x, (R)x.y};
+      }
+      Xs[j][r] = v;
+    }
   }
 }
 
 // Y[row, r0 + r] += d acc[r]
-template <typename R, int PG>
+template <typename R, int PG, bool PRE>
 __device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, uint64_t row, const C2<R>* acc) {
 #pragma unroll
   for (int r = 0; r < PG; ++r) {
     if ((uint32_t)r < pg) {
-      const double ar = (double)acc[r].re, ai = (double)acc[r].im;
+      double ar, ai;
+      if constexpr (PRE) {
+        ar = widen(acc[r].re);
+        ai = widen(acc[r].im);
+        if (!a.d_one) scale_pair(a.dre, a.dim, ar, ai);
+      } else {
+        const double xr = (double)acc[r].re, xi = (double)acc[r].im;
+        ar = a.dre * xr - a.dim * xi;
+        ai = a.dre * xi + a.dim * xr;
+      }
       double* y = &a.Y[(uint64_t)(r0 + r) * a.ldY + row].x;
-      atomicAdd(y, a.dre * ar - a.dim * ai);
-      atomicAdd(y + 1, a.dre * ai + a.dim * ar);
+      atomicAdd(y, ar);
+      atomicAdd(y + 1, ai);
     }
   }
 }
 
-template <typename S, typename R, int PG, int OP>
+template <typename S, typename R, int PG, int OP, bool PRE>
 __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
   const MvLeaf L = a.leaves[a.order[leaf]];
   const S* base = reinterpret_cast<const S*>(a.arena) + L.off;
@@ -95,7 +139,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
         for (uint32_t jb = 0; jb < nc; jb += kCh) {
           const uint32_t jn = min((uint32_t)kCh, nc - jb);
           __syncthreads();
-          stage<R, PG>(Xs, a, r0, pg, co + jb, jn);
+          stage<R, PG, PRE>(Xs, a, r0, pg, co + jb, jn);
           __syncthreads();
           if (i < nr) {
             for (uint32_t j = 0; j < jn; ++j) {
@@ -106,7 +150,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
             }
           }
         }
-        if (i < nr) emit<R, PG>(a, r0, pg, ro + i, acc);
+        if (i < nr) emit<R, PG, PRE>(a, r0, pg, ro + i, acc);
       }
     } else if (L.rank > 0) {
       const uint32_t k = (uint32_t)L.rank;
@@ -127,7 +171,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
         for (uint32_t jb = 0; jb < nc; jb += kCh) {
           const uint32_t jn = min((uint32_t)kCh, nc - jb);
           __syncthreads();
-          stage<R, PG>(Xs, a, r0, pg, co + jb, jn);
+          stage<R, PG, PRE>(Xs, a, r0, pg, co + jb, jn);
           __syncthreads();
           if (sub < ns) {
             const S* qc = Q + (uint64_t)(lb + l) * nc + jb;
@@ -165,7 +209,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
 #pragma unroll
               for (int rr = 0; rr < PG; ++rr) cfma(acc[rr], pv, Ts[ll * PG + rr]);
             }
-            emit<R, PG>(a, r0, pg, ro + i, acc);
+            emit<R, PG, PRE>(a, r0, pg, ro + i, acc);
           }
         }
         __syncthreads();
@@ -174,16 +218,16 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
   }
 }
 
-template <typename S, typename R, int PG, int OP, bool GUARD>
+template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE = false>
 __global__ void __launch_bounds__(kThreads) zmv_kernel(ZArgs a) {
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
   if (GUARD) {
     if (*a.guard == 0) return;
-    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP>(a, l, Xs, Ts, red);
+    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP, PRE>(a, l, Xs, Ts, red);
   } else {
-    zmv_leaf<S, R, PG, OP>(a, blockIdx.x, Xs, Ts, red);
+    zmv_leaf<S, R, PG, OP, PRE>(a, blockIdx.x, Xs, Ts, red);
   }
 }
 
@@ -208,6 +252,28 @@ void launch_typed(const ZArgs& a, cudaStream_t s) {
   else launch_op<S, R, kZOpN>(a, s);
 }
 
+// xf[row * kXW + r] = (complex64) X[row, r], zero for r >= p; rows fastest in its reads, r in
+// its writes
+__global__ void zc_x_kernel(const double2* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t p,
+                            float2* __restrict__ xf) {
+  __shared__ float2 t[32][kXW + 1];
+  const uint32_t row0 = blockIdx.x * 32;
+  for (uint32_t e = threadIdx.x; e < 32 * kXW; e += blockDim.x) {
+    const uint32_t i = e & 31, r = e >> 5;
+    float2 v = make_float2(0.f, 0.f);
+    if (r < p && row0 + i < n) {
+      const double2 x = X[(uint64_t)r * ldX + row0 + i];
+      v = make_float2((float)x.x, (float)x.y);
+    }
+    t[i][r] = v;
+  }
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < 32 * kXW; e += blockDim.x) {
+    const uint32_t i = e / kXW, r = e % kXW;
+    if (row0 + i < n) xf[(uint64_t)(row0 + i) * kXW + r] = t[i][r];
+  }
+}
+
 __global__ void z_to_c64_kernel(const double2* __restrict__ src, uint64_t n, float2* __restrict__ dst) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const double2 v = src[i];
@@ -220,11 +286,32 @@ __global__ void z_to_c64_kernel(const double2* __restrict__ src, uint64_t n, flo
 cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
   if (a.op < kZOpN || a.op > kZOpT) return cudaErrorInvalidValue;
   if (a.nleaves == 0 || a.p == 0) return cudaSuccess;
-  if (a.single) launch_typed<float2, float>(a, s);
-  else launch_typed<double2, double>(a, s);
-  count_product_launches(1);
+  if (!a.single) {
+    launch_typed<double2, double>(a, s);
+    count_product_launches(1);
+    return cudaGetLastError();
+  }
+  if (a.p <= 4 || a.elems * a.p < 30000000ull) {
+    launch_typed<float2, float>(a, s);
+    count_product_launches(1);
+    return cudaGetLastError();
+  }
+  for (uint32_t r0 = 0; r0 < a.p; r0 += kXW) {
+    ZArgs b = a;
+    b.p = std::min<uint32_t>(kXW, a.p - r0);
+    b.X = a.X + (uint64_t)r0 * a.ldX;
+    b.Y = a.Y + (uint64_t)r0 * a.ldY;
+    b.d_one = a.dre == 1.0 && a.dim == 0.0;
+    zc_x_kernel<<<(a.n + 31) / 32, 128, 0, s>>>(b.X, b.ldX, a.n, b.p, a.xf);
+    if (a.op == kZOpH) zmv_kernel<float2, float, 8, kZOpH, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
+    else if (a.op == kZOpT) zmv_kernel<float2, float, 8, kZOpT, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
+    else zmv_kernel<float2, float, 8, kZOpN, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
+    count_product_launches(2);
+  }
   return cudaGetLastError();
 }
+
+size_t matvec_z_xf_bytes(uint64_t n) { return n * kXW * sizeof(float2); }
 
 cudaError_t launch_z_to_c64(const double2* src, uint64_t n, float2* dst, cudaStream_t s) {
   if (n == 0) return cudaSuccess;

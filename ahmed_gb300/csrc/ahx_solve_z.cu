@@ -151,6 +151,7 @@ int prepare_z(ahx_hmat* H, int prec) {
   if (rc) return rc;
   if (prec == kFP32 && !Z.valid32) {
     if ((rc = Z.arena32.reserve(std::max<uint64_t>(Z.elems, 1) * sizeof(float2)))) return rc;
+    if ((rc = Z.xf.reserve(std::max<size_t>(matvec_z_xf_bytes(H->tree.n), 16)))) return rc;
     AHX_CUDA(launch_z_to_c64(Z.arena.as<double2>(), Z.elems, Z.arena32.as<float2>(), H->stream));
     Z.valid32 = true;
   }
@@ -359,31 +360,51 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     return AHX_OK;
   }
   if (H->tree.sym) op = kZOpN;  // A^T = A
-  // several right-hand sides on the complex128 leaves: the digit-sliced product;
-  // the plain kernels then only run when X does not fit the digits
-  const int* guard = nullptr;
-  if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) &&
-      dg_due(Z.dg[op], 4 * Z.elems, p, H->tree.leaves.size())) {
-    DgState& D = Z.dg[op];
-    if (!D.valid) {
-      const auto& Ls = H->tree.leaves;
-      const uint32_t mode = op == kZOpN ? kDgN : op == kZOpT ? kDgT : kDgH;
-      std::vector<DgLeaf> lv;
-      lv.reserve(Ls.size());
-      for (uint32_t l = 0; l < (uint32_t)Ls.size(); ++l) {
-        if (Z.rank[l] == 0) continue;
-        const Leaf& L = Ls[l];
-        lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], mode, Z.off[l]});
-        if (H->tree.sym && L.b1 != L.b2) lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], kDgT, Z.off[l]});
-      }
-      if ((rc = dg_prepare_state(D, lv, H->tree.n, Z.arena.p, 2 * Z.elems, kDgK / 2, Z.finite, H->device, H->stream)))
-        return rc;
+  // the layout over which products run on the tensor cores (complex128: digits, several
+  // right-hand sides; complex64: TF32)
+  const uint64_t n = H->tree.n;
+  DgState& D = Z.dg[op];
+  auto laid_out = [&](uint64_t cost) -> bool {  // (not while the stream is captured: it waits)
+    return D.valid || (dg_due(D, cost, p, H->tree.leaves.size()) && !stream_captured(H->stream));
+  };
+  auto layout = [&]() -> int {
+    if (D.valid) return AHX_OK;
+    const auto& Ls = H->tree.leaves;
+    const uint32_t mode = op == kZOpN ? kDgN : op == kZOpT ? kDgT : kDgH;
+    std::vector<DgLeaf> lv;
+    lv.reserve(Ls.size());
+    for (uint32_t l = 0; l < (uint32_t)Ls.size(); ++l) {
+      if (Z.rank[l] == 0) continue;
+      const Leaf& L = Ls[l];
+      lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], mode, Z.off[l]});
+      if (H->tree.sym && L.b1 != L.b2) lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], kDgT, Z.off[l]});
     }
-    if (D.usable && Z.finite == 1) {
-      if ((rc = H->dg_work.reserve(dg_work_bytes(true, H->tree.n, D.t_rows, p)))) return rc;
-      const DgPlan pl = dg_plan(D, H->tree.n, Z.arena.p, H->dg_work);
+    return dg_prepare_state(D, lv, n, Z.arena.p, 2 * Z.elems, kDgK / 2, Z.finite, H->device, H->stream);
+  };
+  auto work = [&](size_t bytes) -> bool {
+    return H->dg_work.bytes >= bytes || !stream_captured(H->stream);
+  };
+  const int* guard = nullptr;
+  if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) && laid_out(4 * Z.elems)) {
+    // the plain kernels then only run when X does not fit the digits
+    if ((rc = layout())) return rc;
+    const size_t bytes = dg_work_bytes(true, n, D.t_rows, p);
+    if (D.usable && Z.finite == 1 && work(bytes)) {
+      if ((rc = H->dg_work.reserve(bytes))) return rc;
+      const DgPlan pl = dg_plan(D, n, Z.arena.p, H->dg_work);
       AHX_CUDA(launch_matvec_dg(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
       guard = dg_flag(pl);
+    }
+  }
+  // (the plain complex64 kernel costs a third of what dg_due counts for real elements)
+  if (prec == kFP32 && zt_wanted(Z.elems, p) && laid_out(Z.elems / 3)) {
+    if ((rc = layout())) return rc;
+    const size_t bytes = zt_work_bytes(n, D.t_rows, p);
+    if (D.usable && work(bytes)) {
+      if ((rc = H->dg_work.reserve(bytes))) return rc;
+      const DgPlan pl = dg_plan(D, n, Z.arena32.p, H->dg_work);
+      AHX_CUDA(launch_matvec_zt(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
+      return AHX_OK;
     }
   }
   ZArgs a;
@@ -401,6 +422,9 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.ldY = ldY;
   a.op = op;
   a.guard = guard;
+  a.elems = Z.elems;
+  a.n = (uint32_t)n;
+  a.xf = Z.xf.as<float2>();
   AHX_CUDA(launch_matvec_z(a, H->stream));
   if (Z.ntleaves) {
     // the blocks below the diagonal: the upper ones transposed
