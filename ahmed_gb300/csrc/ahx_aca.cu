@@ -592,12 +592,19 @@ __global__ void __launch_bounds__(kLargeThreads) merge_large_kernel(MergeParams 
 __global__ void dense_fill_kernel(PointsSoA P, double diag, const DenseTask* __restrict__ tasks,
                                   double* __restrict__ arena) {
   const DenseTask t = tasks[blockIdx.x];
-  const uint64_t cnt = (uint64_t)t.n1 * t.n2;
   double* out = arena + t.off;
-  for (uint64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const uint32_t i = (uint32_t)(e % t.n1), j = (uint32_t)(e / t.n1);
+  const uint32_t si = blockDim.x % t.n1, sj = blockDim.x / t.n1;
+  for (uint32_t i = threadIdx.x % t.n1, j = threadIdx.x / t.n1; j < t.n2;) {
     const uint32_t gj = t.b2 + j;
-    out[e] = lap_entry(P, gj, t.b1 + i, P.x[gj], P.y[gj], P.z[gj], diag);
+    const double v = lap_entry(P, gj, t.b1 + i, P.x[gj], P.y[gj], P.z[gj], diag);
+    out[(uint64_t)j * t.n1 + i] = v;
+    if (t.mirror != kNoMirror) arena[t.mirror + (uint64_t)i * t.n2 + j] = v;
+    i += si;
+    j += sj;
+    if (i >= t.n1) {
+      i -= t.n1;
+      ++j;
+    }
   }
 }
 

@@ -2,9 +2,11 @@
 // dense fill of inadmissible leaves (FP64 throughout).
 #pragma once
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "ahx_device.cuh"
+#include "ahx_tree.hpp"
 
 namespace ahx {
 
@@ -73,11 +75,17 @@ cudaError_t launch_zaca(const AcaParams& p, uint32_t grid, cudaStream_t s);  // 
 cudaError_t resident_aca(int device, uint32_t& ctas);
 cudaError_t resident_zaca(int device, uint32_t& ctas);
 
-// Dense leaves: fill n1 x n2 column-major blocks of the generator.
+// Dense leaves: fill n1 x n2 column-major blocks of the generator.  The generators are
+// symmetric, entry for entry: where the tree also has the block's mirror image, one task
+// writes both.
+constexpr uint64_t kNoMirror = ~0ull;
 struct DenseTask {
   uint32_t b1, n1, b2, n2;
-  uint64_t off;  // element offset in the arena
+  uint64_t off, mirror;  // element offsets in the arena
 };
+// The tasks of `leaves` (indices, ascending; off: their offsets), mirror images joined.
+std::vector<DenseTask> dense_tasks(const std::vector<Leaf>& Ls, uint32_t n, const std::vector<uint32_t>& leaves,
+                                   const std::vector<uint64_t>& off);
 cudaError_t launch_dense_fill(const PointsSoA& pts, double diag, const DenseTask* tasks,
                               uint32_t ntasks, double* arena, cudaStream_t s);
 

@@ -29,16 +29,11 @@ __device__ __forceinline__ double cabs2(Cx a) { return __dadd_rn(__dmul_rn(a.re,
 __device__ __forceinline__ double cabs(Cx a) { return __dsqrt_rn(cabs2(a)); }
 __device__ __forceinline__ Cx cconj(Cx a) { return Cx{a.re, -a.im}; }
 
-// entry of a dense leaf, explicitly rounded
+// entry of a dense leaf, r and 1 / (4 pi r) rounded as on the host
 __device__ __forceinline__ Cx helm_entry(const PointsSoA& P, double k, double h, uint32_t i, uint32_t j) {
-  double r = h;
-  if (i != j) {
-    const double dx = __dsub_rn(P.x[i], P.x[j]);
-    const double dy = __dsub_rn(P.y[i], P.y[j]);
-    const double dz = __dsub_rn(P.z[i], P.z[j]);
-    r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-  }
-  const double s = __ddiv_rn(1.0, __dmul_rn(kFourPi, r));
+  double r = h, s;
+  if (i != j) rounded_r_s(rounded_r2(P.x[i], P.y[i], P.z[i], P.x[j], P.y[j], P.z[j]), r, s);
+  else s = __ddiv_rn(1.0, __dmul_rn(kFourPi, r));
   double sn, cs;
   sincos(__dmul_rn(k, r), &sn, &cs);
   return Cx{__dmul_rn(cs, s), __dmul_rn(sn, s)};
@@ -454,19 +449,21 @@ __global__ void __launch_bounds__(32) zmerge_kernel(MergeParams p) {
   if (g.rank == 0) p.res[ti] = AcaResult{kAcaOk, kc, kt, 0u};
 }
 
-struct ZDense {
-  uint32_t b1, n1, b2, n2;
-  uint64_t off;
-};
-
-__global__ void helm_dense_kernel(PointsSoA P, double k, double h, const ZDense* __restrict__ tasks,
+__global__ void helm_dense_kernel(PointsSoA P, double k, double h, const DenseTask* __restrict__ tasks,
                                   Cx* __restrict__ arena) {
-  const ZDense t = tasks[blockIdx.x];
-  const uint64_t cnt = (uint64_t)t.n1 * t.n2;
+  const DenseTask t = tasks[blockIdx.x];
   Cx* out = arena + t.off;
-  for (uint64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const uint32_t i = (uint32_t)(e % t.n1), j = (uint32_t)(e / t.n1);
-    out[e] = helm_entry(P, k, h, t.b1 + i, t.b2 + j);
+  const uint32_t si = blockDim.x % t.n1, sj = blockDim.x / t.n1;
+  for (uint32_t i = threadIdx.x % t.n1, j = threadIdx.x / t.n1; j < t.n2;) {
+    const Cx v = helm_entry(P, k, h, t.b1 + i, t.b2 + j);
+    out[(uint64_t)j * t.n1 + i] = v;
+    if (t.mirror != kNoMirror) arena[t.mirror + (uint64_t)i * t.n2 + j] = v;
+    i += si;
+    j += sj;
+    if (i >= t.n1) {
+      i -= t.n1;
+      ++j;
+    }
   }
 }
 
@@ -673,7 +670,6 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
   if ((rc = run_aca(H, true, tasks, par, dense))) return rc;
   // dense leaves (inadmissible and failed ACA) in leaf order
   std::sort(dense.begin(), dense.end());
-  std::vector<ZDense> dt;
   for (uint32_t l : dense) {
     const Leaf& L = Ls[l];
     uint64_t off = 0;
@@ -681,12 +677,12 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
     Z.off[l] = off;
     Z.rank[l] = -1;
     Z.aca_rank[l] = -1;
-    dt.push_back(ZDense{L.b1, L.n1, L.b2, L.n2, off});
   }
+  const std::vector<DenseTask> dt = dense_tasks(Ls, H->tree.n, dense, Z.off);
   if (!dt.empty()) {
     ScopedBuf ddt;
     if ((rc = upload(ddt, dt, H->stream))) return rc;
-    helm_dense_kernel<<<(uint32_t)dt.size(), 256, 0, H->stream>>>(P, wavenumber, h, ddt.as<ZDense>(), Z.arena.as<Cx>());
+    helm_dense_kernel<<<(uint32_t)dt.size(), 256, 0, H->stream>>>(P, wavenumber, h, ddt.as<DenseTask>(), Z.arena.as<Cx>());
     AHX_CUDA(cudaGetLastError());
   }
   AHX_CUDA(cudaStreamSynchronize(H->stream));

@@ -14,34 +14,69 @@ namespace {
 // outweighs the rows.  A leaf's k x k work counts as 256 rows.
 constexpr uint64_t kLeafRows = 256, kLargeMin = 512;
 
-// Workspace sizes in steps of 1/16 octave: tasks sort by class in linear time.
-uint32_t size_class(uint64_t b) {
-  const int m = 63 - __builtin_clzll(b | 16);
-  return (uint32_t)(m * 16) + (uint32_t)((b >> (m - 4)) & 15);
-}
 uint64_t class_bytes(uint32_t c) {  // an upper bound of the class, a multiple of 256
   const uint64_t top = (uint64_t)(16 + (c & 15) + 1) << (c / 16 - 4);
   return (top + 255) & ~255ull;
 }
 
+// tasks by descending class of their workspace; cls: the classes
 void sort_descending(std::vector<AcaTask>& t, std::vector<uint32_t>& cls, size_t elem) {
-  std::vector<uint32_t> c(t.size()), at(1025, 0);
-  for (size_t i = 0; i < t.size(); ++i) {
-    c[i] = 1023 - size_class(aca_ws_bytes(t[i].n1, t[i].n2, t[i].kcap, elem));
-    ++at[c[i] + 1];
-  }
-  for (size_t i = 0; i < 1024; ++i) at[i + 1] += at[i];
+  std::vector<uint64_t> size(t.size());
+  for (size_t i = 0; i < t.size(); ++i) size[i] = aca_ws_bytes(t[i].n1, t[i].n2, t[i].kcap, elem);
+  std::vector<uint32_t> ord;
+  order_by_size(size, ord);
   std::vector<AcaTask> out(t.size());
   cls.resize(t.size());
   for (size_t i = 0; i < t.size(); ++i) {
-    const uint32_t p = at[c[i]]++;
-    out[p] = t[i];
-    cls[p] = 1023 - c[i];
+    out[i] = t[ord[i]];
+    cls[i] = size_class(size[ord[i]]);
   }
   t.swap(out);
 }
 
 }  // namespace
+
+uint32_t size_class(uint64_t size) {
+  const int m = 63 - __builtin_clzll(size | 16);
+  return (uint32_t)(m * 16) + (uint32_t)((size >> (m - 4)) & 15);
+}
+
+void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order) {
+  std::vector<uint32_t> at(1025, 0);
+  for (uint64_t s : size) ++at[1024 - size_class(s)];
+  for (size_t c = 0; c < 1024; ++c) at[c + 1] += at[c];
+  order.resize(size.size());
+  for (size_t i = 0; i < size.size(); ++i) order[at[1023 - size_class(size[i])]++] = (uint32_t)i;
+}
+
+std::vector<DenseTask> dense_tasks(const std::vector<Leaf>& Ls, uint32_t n, const std::vector<uint32_t>& leaves,
+                                   const std::vector<uint64_t>& off) {
+  // lists of the tasks by first row (their leaf has b1 < b2), for the mirror images
+  std::vector<DenseTask> t;
+  std::vector<uint32_t> head(n, 0u), next;
+  t.reserve(leaves.size());
+  next.reserve(leaves.size());
+  for (int pass = 0; pass < 2; ++pass)
+    for (uint32_t l : leaves) {
+      const Leaf& L = Ls[l];
+      if ((L.b1 > L.b2) != (pass == 1)) continue;
+      if (pass == 1) {
+        uint32_t q = head[L.b2];
+        while (q && (t[q - 1].b2 != L.b1 || t[q - 1].n1 != L.n2 || t[q - 1].n2 != L.n1)) q = next[q - 1];
+        if (q) {
+          t[q - 1].mirror = off[l];
+          continue;
+        }
+      }
+      t.push_back(DenseTask{L.b1, L.n1, L.b2, L.n2, off[l], kNoMirror});
+      next.push_back(0u);
+      if (L.b1 < L.b2) {
+        next.back() = head[L.b1];
+        head[L.b1] = (uint32_t)t.size();
+      }
+    }
+  return t;
+}
 
 int run_aca(ahx_hmat* H, bool cplx, std::vector<AcaTask>& tasks, AcaParams p, std::vector<uint32_t>& dense) {
   const size_t elem = cplx ? 16 : 8;

@@ -168,9 +168,10 @@ int upload_leaf_table(ahx_hmat* H, const std::vector<PlanLeaf>& pls, DevBuf& lea
     mv.push_back(m);
     cost.push_back(q.rank < 0 ? (uint64_t)q.n1 * q.n2 : (uint64_t)q.rank * (q.n1 + q.n2));
   }
-  std::vector<uint32_t> ord(mv.size());
-  std::iota(ord.begin(), ord.end(), 0u);
-  std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
+  // in steps of 1/16 octave, which is as good for the launch order as an exact one (92,497
+  // leaves: table and order in 2.0 ms instead of 5.6)
+  std::vector<uint32_t> ord;
+  order_by_size(cost, ord);
   int rc;
   if ((rc = upload(leaves, mv, H->stream))) return rc;
   if ((rc = upload(order, ord, H->stream))) return rc;
@@ -769,7 +770,6 @@ int ahx_assemble_hinted(ahx_hmat* H, double h, double eps, uint32_t rankmax,
   if ((rc = run_aca(H, false, tasks, par, dense))) return rc;
   // dense leaves (inadmissible and failed ACA), filled in leaf order
   std::sort(dense.begin(), dense.end());
-  std::vector<DenseTask> dt;
   for (uint32_t l : dense) {
     const Leaf& L = Ls[l];
     uint64_t off = 0;
@@ -777,8 +777,8 @@ int ahx_assemble_hinted(ahx_hmat* H, double h, double eps, uint32_t rankmax,
     H->off[l] = off;
     H->rank[l] = -1;
     H->aca_rank[l] = -1;
-    dt.push_back(DenseTask{L.b1, L.n1, L.b2, L.n2, off});
   }
+  const std::vector<DenseTask> dt = dense_tasks(Ls, H->tree.n, dense, H->off);
   if (!dt.empty()) {
     DevBuf ddt;
     if ((rc = upload(ddt, dt, H->stream))) return rc;

@@ -14,31 +14,73 @@ struct PointsSoA {
   const double* z;
 };
 
+// FP32 image of a double times 2^-shift, truncated, by integer operations (the
+// conversion instruction shares the FP64 pipe); 0 below FP32's range
+__device__ __forceinline__ float to_f32(double x, int shift) {
+  const int hi = __double2hiint(x);
+  const int f = (hi >> 20) & 0x7ff, e = f - shift - 896;
+  if (f == 0 || e <= 0) return 0.f;
+  const uint32_t m = __funnelshift_l((uint32_t)__double2loint(x), (uint32_t)hi & 0xfffffu, 3);
+  return __int_as_float((hi & 0x80000000) | (e << 23) | (int)(m & 0x7fffffu));
+}
+// a normal FP32 number as a double
+__device__ __forceinline__ double to_f64(float f) {
+  const int b = __float_as_int(f);
+  return __hiloint2double((b & 0x80000000) | (int)((((uint32_t)b & 0x7fffffffu) >> 3) + 0x38000000u), b << 29);
+}
+__device__ __forceinline__ float rsqrt_f32(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ bool f32_range(double x) {  // 2^-120 <= x < 2^120
+  return (uint32_t)(__double2hiint(x) - ((1023 - 120) << 20)) < (uint32_t)(240 << 20);
+}
+// 1 / sqrt(x) for f32_range(x): an FP32 seed y (relative error e < 2^-20) and one step
+// of Halley's series y (1 + e/2 + 3 e^2/8), remainder below 2^-61
+__device__ __forceinline__ double rsqrt_seeded(double x) {
+  const double y = to_f64(rsqrt_f32(to_f32(x, 0)));
+  const double e = fma(-x, y * y, 1.0);  // y * y is exact (24-bit y)
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// r = sqrt(r2) and s = 1 / (4 pi r), every operation rounded to nearest, so that entries
+// equal the host's bit for bit.  One reciprocal square root serves both: the final
+// steps r + (r2 - r^2) y / 2 and z + z (1 - t z) (Markstein) leave the unrounded results
+// within 2^-104 of the exact ones.  21 FP64 instructions an entry; with the mirror images
+// written by the same task, the dense leaves of 65,536 points take 2.7 ms instead of 5.1.
+// (The general case is a function of its own: predicated in line its FP64 instructions
+// would occupy the pipe for every entry.)
+static __device__ __noinline__ double2 rounded_r_s_any(double r2) {
+  const double r = __dsqrt_rn(r2);
+  return make_double2(r, __ddiv_rn(1.0, __dmul_rn(kFourPi, r)));
+}
+__device__ __forceinline__ void rounded_r_s(double r2, double& r, double& s) {
+  if (f32_range(r2)) {
+    const double y = rsqrt_seeded(r2), g = __dmul_rn(r2, y);
+    r = fma(fma(-g, g, r2), 0.5 * y, g);
+    const double t = __dmul_rn(kFourPi, r), z = __dmul_rn(1.0 / kFourPi, y);
+    s = fma(z, fma(-t, z, 1.0), z);
+  } else {
+    const double2 v = rounded_r_s_any(r2);
+    r = v.x;
+    s = v.y;
+  }
+}
+static __device__ __noinline__ double rsqrt_other(double x) { return rsqrt(x); }
+__device__ __forceinline__ double rsqrt_any(double x) { return f32_range(x) ? rsqrt_seeded(x) : rsqrt_other(x); }
+__device__ __forceinline__ double rounded_r2(double xi, double yi, double zi, double xj, double yj, double zj) {
+  const double dx = __dsub_rn(xi, xj), dy = __dsub_rn(yi, yj), dz = __dsub_rn(zi, zj);
+  return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+}
+
 // Laplace single-layer entry K(i,j) = 1/(4 pi |x_i - x_j|), diag = 1/(4 pi h).
-// Evaluated with explicitly rounded operations (no contraction to FMA) so that
-// every entry equals the host evaluation bit for bit.
 __device__ __forceinline__ double lap_entry(const PointsSoA& P, uint32_t i, uint32_t j,
                                             double xi, double yi, double zi, double diag) {
   if (i == j) return diag;
-  const double dx = __dsub_rn(xi, P.x[j]);
-  const double dy = __dsub_rn(yi, P.y[j]);
-  const double dz = __dsub_rn(zi, P.z[j]);
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  return __ddiv_rn(1.0, __dmul_rn(kFourPi, __dsqrt_rn(r2)));
-}
-
-// The same kernel inside the ACA steps, evaluated as (1/(4 pi)) * rsqrt(r^2):
-// within an ulp of lap_entry and several times fewer FP64 instructions (the
-// FP64 pipe is what bounds the assembly on this GPU).  Dense leaves use
-// lap_entry.
-__device__ __forceinline__ double lap_entry_aca(const PointsSoA& P, uint32_t i, uint32_t j,
-                                                double xi, double yi, double zi, double diag) {
-  if (i == j) return diag;
-  const double dx = xi - P.x[j];
-  const double dy = yi - P.y[j];
-  const double dz = zi - P.z[j];
-  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-  return (1.0 / kFourPi) * rsqrt(r2);
+  double r, s;
+  rounded_r_s(rounded_r2(xi, yi, zi, P.x[j], P.y[j], P.z[j]), r, s);
+  return s;
 }
 
 // a > b for non-negative doubles, on the integer pipe (IEEE order of the bit patterns)

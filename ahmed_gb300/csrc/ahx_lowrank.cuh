@@ -85,41 +85,12 @@ __device__ __forceinline__ Cx shfl_(Cx a, int src, int w = 32) {
   return Cx{__shfl_sync(0xffffffffu, a.re, src, w), __shfl_sync(0xffffffffu, a.im, src, w)};
 }
 
-// FP32 image of a double times 2^-shift, truncated, by integer operations (the
-// conversion instruction shares the FP64 pipe); 0 below FP32's range
-__device__ __forceinline__ float to_f32(double x, int shift) {
-  const int hi = __double2hiint(x);
-  const int f = (hi >> 20) & 0x7ff, e = f - shift - 896;
-  if (f == 0 || e <= 0) return 0.f;
-  const uint32_t m = __funnelshift_l((uint32_t)__double2loint(x), (uint32_t)hi & 0xfffffu, 3);
-  return __int_as_float((hi & 0x80000000) | (e << 23) | (int)(m & 0x7fffffu));
-}
-// a normal FP32 number as a double
-__device__ __forceinline__ double to_f64(float f) {
-  const int b = __float_as_int(f);
-  return __hiloint2double((b & 0x80000000) | (int)((((uint32_t)b & 0x7fffffffu) >> 3) + 0x38000000u), b << 29);
-}
-__device__ __forceinline__ float rsqrt_f32(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
+__device__ __forceinline__ double sqrt_any(double x) { return x > 0.0 ? x * rsqrt_any(x) : sqrt(x); }
 __device__ __forceinline__ float sqrt_f32(float x) {
   float y;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ bool f32_range(double x) {  // 2^-120 <= x < 2^120
-  return (uint32_t)(__double2hiint(x) - ((1023 - 120) << 20)) < (uint32_t)(240 << 20);
-}
-// 1 / sqrt(x) for f32_range(x): an FP32 seed y (relative error e < 2^-20) and one step
-// of Halley's series y (1 + e/2 + 3 e^2/8), remainder below 2^-61
-__device__ __forceinline__ double rsqrt_seeded(double x) {
-  const double y = to_f64(rsqrt_f32(to_f32(x, 0)));
-  const double e = fma(-x, y * y, 1.0);  // y * y is exact (24-bit y)
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-__device__ __forceinline__ double rsqrt_any(double x) { return f32_range(x) ? rsqrt_seeded(x) : rsqrt(x); }
 
 // ---------------------------------------------------------------------------
 // matrix entries
@@ -160,8 +131,9 @@ struct HelmGen {  // exp(i k r) / (4 pi r)
       r = fma(0.5 * y, fma(-r, r, r2), r);
       s = (1.0 / kFourPi) * y;
     } else {
-      r = f.i == j ? h : sqrt(r2);
-      s = 1.0 / (kFourPi * r);
+      const double2 v = rounded_r_s_any(f.i == j ? h * h : r2);
+      r = v.x;
+      s = v.y;
     }
     double sn, cs;
     sincos(k * r, &sn, &cs);
@@ -379,7 +351,7 @@ __device__ bool row_step(Team<W>& g, const Blk<Gen>& B, uint32_t& klast, uint32_
     i0 = nexti(g, B.Z, n1, i0);
   }
   // v *= sqrt|p| / p, u /= sqrt|p| (p: the pivot)
-  const double ap = abs_of_mag(T(), am), rs = rsqrt(ap), sq = ap * rs;
+  const double ap = abs_of_mag(T(), am), rs = rsqrt_any(ap), sq = ap * rs;
   T sca;
   if constexpr (sizeof(T) == 8) sca = copysign(rs, piv);
   else sca = scale_(conj_(piv), rs * (rs * rs));
@@ -466,7 +438,7 @@ __device__ bool col_step(Team<W>& g, const Blk<Gen>& B, uint32_t& j0, uint32_t k
     g.sync();
     j0 = nexti(g, B.S, n2, j0);
   }
-  const double ap = abs_of_mag(T(), am), rs = rsqrt(ap), sq = ap * rs;
+  const double ap = abs_of_mag(T(), am), rs = rsqrt_any(ap), sq = ap * rs;
   T sca;
   if constexpr (sizeof(T) == 8) sca = copysign(rs, piv);
   else sca = scale_(conj_(piv), rs * (rs * rs));
@@ -582,6 +554,7 @@ __device__ int aca(Team<W>& g, const Blk<Gen>& B, uint32_t i0, uint32_t kmax, ui
   for (uint32_t i = g.rank; i < n1; i += G) B.Z[i] = 0;
   for (uint32_t j = g.rank; j < n2; j += G) B.S[j] = 0;
   double scale = abs_of_mag(T(), mag(B.gen.entry(B.gen.fix(B.b1), B.b2)));
+  const double inv_n = 1.0 / (double)(uint32_t)(n1 * n2);
   uint32_t k = 0, no = 0, klast = 0, inext = i0, j0 = 0;
   int kmin = -2, keps = -1;
   double nrmlsk2 = 0.0, nrms2 = 0.0, nu, nv, w2;
@@ -599,7 +572,7 @@ __device__ int aca(Team<W>& g, const Blk<Gen>& B, uint32_t i0, uint32_t kmax, ui
     const bool stpcrit = nrmlsk2 < eps * eps * nrms2;
     if (stpcrit && keps == -1) keps = (int)klast + 1;
     ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
+    scale = sqrt_any(nrmlsk2 * inv_n);
     if (keps > 0) {
       int mv = INT_MAX;
       uint32_t mi = 0xffffffffu;
@@ -674,6 +647,7 @@ __device__ int acar(Team<W>& g, const Blk<Gen>& B, uint32_t i0, uint32_t kmax, u
   const uint32_t n1 = B.n1, n2 = B.n2;
   for (uint32_t i = g.rank; i < n1; i += Team<W>::G) B.Z[i] = 0;
   double scale = abs_of_mag(T(), mag(B.gen.entry(B.gen.fix(B.b1), B.b2)));
+  const double inv_n = 1.0 / (double)(uint32_t)(n1 * n2);
   uint32_t k = 0, no = 0, klast = 0;
   double nrmlsk2 = 0.0, nrms2 = 0.0, nu, nv, w2;
   int outcome = -1;
@@ -689,7 +663,7 @@ __device__ int acar(Team<W>& g, const Blk<Gen>& B, uint32_t i0, uint32_t kmax, u
     nrmlsk2 = nu * nv;
     nrms2 += 2.0 * gram(g, B, k, nu, w2) + nrmlsk2;
     ++k;
-    scale = sqrt(nrmlsk2 / (double)(uint32_t)(n1 * n2));
+    scale = sqrt_any(nrmlsk2 * inv_n);
   } while (no < n2 && k < kmax && nrmlsk2 >= eps * eps * nrms2);
   if (outcome < 0) {
     const double epsa = sqrt(nrmlsk2 / nrms2);
@@ -750,7 +724,7 @@ __device__ bool cholesky(const Work<T>& w, uint32_t k, uint32_t lane) {
           const double d = __shfl_sync(0xffffffffu, re_(s), 0, wd);
           g0 = __shfl_sync(0xffffffffu, g0, 0, wd);
           if (!__all_sync(0xffffffffu, d > kCholTau * g0 && d < 1e300 && d > 1e-290)) return false;
-          inv = rsqrt(d);
+          inv = rsqrt_any(d);
           if (hl == 0) w.dinv[side * (k <= 32 ? 32 : k) + c] = inv;
         }
         if (j < k) {
