@@ -601,61 +601,98 @@ __global__ void __launch_bounds__(kThreads, 1) um_sweep_kernel(const __grid_cons
   }
 }
 
-// max |X_j| over the rows, j < pg (FP32 bits, atomicMax; the words start at 0)
+// max |X_j| over the rows, j < pg (FP32 bits, atomicMax; the words start at 0; NaN does
+// not count).  Column blockIdx.y; magnitudes compare as integers, one conversion per warp.
 __global__ void __launch_bounds__(256) um_xmax_kernel(const double* __restrict__ X, uint64_t ldX, uint64_t n,
-                                                      uint32_t pg, uint32_t* __restrict__ xmax) {
-  __shared__ float wm[8][64];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                                                      uint32_t* __restrict__ xmax) {
+  constexpr int kB = 4;
+  const double* x = X + (uint64_t)blockIdx.y * ldX;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint32_t j = 0; j < pg; ++j) {
-    float m = 0.f;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride)
-      m = fmaxf(m, (float)fabs(X[r + (uint64_t)j * ldX]));
+  unsigned long long m = 0;
+  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += kB * stride) {
+    double v[kB];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) wm[warp][j] = m;
+    for (int u = 0; u < kB; ++u) v[u] = x[min(r + u * stride, n - 1)];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(v[u]) & 0x7fffffffffffffffull;
+      if (b <= 0x7ff0000000000000ull && b > m) m = b;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x < pg) {
-    float m = 0.f;
-    for (uint32_t w = 0; w < 8; ++w) m = fmaxf(m, wm[w][threadIdx.x]);
-    atomicMax(xmax + threadIdx.x, __float_as_uint(m));
+  const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32));
+  const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32) == hi ? (uint32_t)m : 0u);
+  if ((threadIdx.x & 31) == 0) atomicMax(xmax + blockIdx.y, __float_as_uint((float)__hiloint2double((int)hi, (int)lo)));
+}
+
+// x as FP32, to odd: rounding it on to FP16 gives x's own rounding to nearest
+__device__ __forceinline__ float odd_f32(double x) {
+  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 896;
+  if (e <= 0) return 0.f;
+  const uint32_t lo = (uint32_t)__double2loint(x), m = __funnelshift_l(lo, (uint32_t)hi & 0xfffffu, 3);
+  return __int_as_float((hi & 0x80000000) | (e << 23) | (int)(m & 0x7fffffu) | ((lo & 0x1fffffffu) ? 1 : 0));
+}
+__device__ __noinline__ __half2 um_parts_any(double v) {
+  const __half h1 = __double2half(v);
+  return __halves2half2(h1, __double2half(v - (double)__half2float(h1)));
+}
+// the two FP16 parts of x 2^-E, both to nearest: one FP64 instruction (a conversion takes
+// as long as a multiply-add; there were five)
+__device__ __forceinline__ void um_parts(double x, int E, __half& h1, __half& h2) {
+  const int hi = __double2hiint(x), ef = (hi >> 20) & 0x7ff, nf = ef - E;
+  const uint32_t lo = (uint32_t)__double2loint(x);
+  h1 = h2 = __ushort_as_half(0);
+  if (ef == 0 ? (((uint32_t)hi << 1) | lo) != 0u : (ef == 0x7ff || nf > 1023 + 15)) {
+    const __half2 h = um_parts_any(x * ldexp(1.0, -E));
+    h1 = __low2half(h);
+    h2 = __high2half(h);
+  } else if (ef != 0 && nf >= 1023 - 60) {  // (below: zero in FP16)
+    const double v = __hiloint2double(hi - E * (1 << 20), (int)lo);
+    h1 = __float2half_rn(odd_f32(v));
+    const float f = __half2float(h1);
+    const int b = __float_as_int(f);
+    const double d = f == 0.f ? 0.0
+                              : __hiloint2double((b & 0x80000000) | (int)((((uint32_t)b & 0x7fffffffu) >> 3) + 0x38000000u),
+                                                 b << 29);
+    h2 = __float2half_rn(odd_f32(v - d));
   }
 }
 
 // X (FP64, column-major, ld ldX), columns 0 .. pg-1 -> Z rows 0 .. n-1: X_j
 // scaled by a power of two (its largest |value| into [2^13, 2^14)) and split
-// into two FP16 parts; slots >= pg are zero.
+// into two FP16 parts; slots >= pg are zero.  32 rows a turn, a warp per 8 columns (those
+// past pg only write zeros); through shared memory so that rows are read and written whole.
 __global__ void __launch_bounds__(256) um_prep_kernel(const double* __restrict__ X, uint64_t ldX, uint64_t n,
                                                       uint32_t pg, const uint32_t* __restrict__ xmax,
                                                       uint16_t* __restrict__ z) {
-  __shared__ double tile[64][33];
-  __shared__ double sx[64];
-  if (threadIdx.x < 64) {
-    const float m = __uint_as_float(xmax[threadIdx.x]);
-    sx[threadIdx.x] = ldexp(1.0, -scale_exp((double)m));
-  }
+  constexpr uint32_t kPitch = 256 + 16;
+  __shared__ __align__(16) unsigned char out[32 * kPitch];
+  __shared__ int sx[64];
+  if (threadIdx.x < 64) sx[threadIdx.x] = scale_exp((double)__uint_as_float(xmax[threadIdx.x]));
   __syncthreads();
+  const uint32_t row = threadIdx.x & 31, c0 = (threadIdx.x >> 5) * 8;
   const uint64_t nblk = (n + 31) / 32;
   for (uint64_t b = blockIdx.x; b < nblk; b += gridDim.x) {
-    const uint64_t r0 = b * 32;
-    for (uint32_t e = threadIdx.x; e < 32u * 64u; e += blockDim.x) {
-      const uint32_t row = e & 31, col = e >> 5;
-      double v = 0.0;
-      if (col < pg && r0 + row < n) v = X[(r0 + row) + (uint64_t)col * ldX] * sx[col];
-      tile[col][row] = v;
+    const uint64_t r = b * 32 + row;
+    __align__(16) __half h[2][8];
+    if (c0 < pg) {
+      double x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = c0 + k < pg && r < n ? X[r + (uint64_t)(c0 + k) * ldX] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) um_parts(x[k], sx[c0 + k], h[0][k], h[1][k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) h[0][k] = h[1][k] = __ushort_as_half(0);
     }
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      *reinterpret_cast<uint4*>(out + row * kPitch + q * 128 + c0 * 2) = *reinterpret_cast<const uint4*>(h[q]);
     __syncthreads();
-    for (uint32_t e = threadIdx.x; e < 32u * 64u; e += blockDim.x) {
-      const uint32_t col = e & 63, row = e >> 6;
-      if (r0 + row < n) {
-        const double v = tile[col][row];
-        const __half h1 = __double2half(v);
-        const __half h2 = __double2half(v - (double)__half2float(h1));
-        __half* zp = reinterpret_cast<__half*>(z) + (r0 + row) * (kUmZPitch / 2);
-        zp[col] = h1;
-        zp[64 + col] = h2;
-      }
+    for (uint32_t e = threadIdx.x; e < 32 * 16; e += 256) {
+      const uint32_t i = e >> 4, w = e & 15;
+      if (b * 32 + i < n)
+        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(z) + (b * 32 + i) * kUmZPitch + w * 16) =
+            *reinterpret_cast<const uint4*>(out + i * kPitch + w * 16);
     }
     __syncthreads();
   }
@@ -898,8 +935,8 @@ cudaError_t run_um(const UmPlan& pl, double d, uint32_t r0, uint32_t pg, const d
   cudaError_t e = cudaMemsetAsync(pl.xmax, 0, 64 * sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
   const double* Xp = X + (uint64_t)r0 * ldX;
-  const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((pl.n + 255) / 256, (uint64_t)pl.grid * 4));
-  um_xmax_kernel<<<gx, 256, 0, s>>>(Xp, ldX, pl.n, pg, pl.xmax);
+  const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((pl.n + 1023) / 1024, 64));
+  um_xmax_kernel<<<dim3(gx, pg), 256, 0, s>>>(Xp, ldX, pl.n, pl.xmax);
   um_prep_kernel<<<grid, 256, 0, s>>>(Xp, ldX, pl.n, pg, pl.xmax, pl.z);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   uint64_t launches = 2;
