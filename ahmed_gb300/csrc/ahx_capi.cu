@@ -19,6 +19,41 @@ namespace {
 thread_local std::string g_err;
 }  // namespace
 
+int HostWord::reserve() {
+  if (p) return AHX_OK;
+  void* q = nullptr;
+  AHX_CUDA(cudaHostAlloc(&q, sizeof(unsigned long long), cudaHostAllocMapped | cudaHostAllocPortable));
+  p = static_cast<unsigned long long*>(q);
+  *p = 0;
+  return AHX_OK;
+}
+
+int HostWord::wait(uint32_t step, cudaStream_t s, uint32_t& value) {
+  const volatile unsigned long long* w = p;
+  for (uint32_t spin = 1;; ++spin) {
+    unsigned long long v = *w;
+    if ((uint32_t)(v >> 32) != step && spin % 4096 == 0) {
+      const cudaError_t e = cudaStreamQuery(s);
+      if (e == cudaErrorNotReady) continue;
+      if (e != cudaSuccess) return cuda_fail(e, "solver step");
+      v = *w;
+      if ((uint32_t)(v >> 32) != step) {
+        set_error("solver step ended without a count");
+        return AHX_ERR_CUDA;
+      }
+    }
+    if ((uint32_t)(v >> 32) == step) {
+      value = (uint32_t)v;
+      return AHX_OK;
+    }
+  }
+}
+
+void HostWord::release() {
+  if (p) cudaFreeHost(p);
+  p = nullptr;
+}
+
 // Append-only growable FP64 arena.
 int arena_append(ahx_hmat* H, uint64_t count, uint64_t& off) {
   const uint64_t need = (H->arena64_elems + count) * sizeof(double);
@@ -658,6 +693,7 @@ int ahx_hmat_destroy(ahx_hmat* H) {
   H->stage_y.release();
   H->scratch.release();
   H->dg_work.release();
+  H->gm_word.release();
   H->z.release_all();
   if (H->own_stream && H->stream) cudaStreamDestroy(H->stream);
   delete H;

@@ -42,6 +42,17 @@ struct ScopedBuf : DevBuf {
   ~ScopedBuf() { release(); }
 };
 
+// A word of host memory that kernels write and the host waits for: step << 32 | value.
+struct HostWord {
+  unsigned long long* p = nullptr;
+  int reserve();
+  unsigned long long* device() const { return p; }  // (unified addressing)
+  void clear() { *const_cast<volatile unsigned long long*>(p) = 0; }
+  // until the word is of `step`; ends with an error if the stream fails or finishes without it
+  int wait(uint32_t step, cudaStream_t s, uint32_t& value);
+  void release();
+};
+
 // The product's view of one storage precision.
 struct ProdCopy {
   bool valid = false;
@@ -201,6 +212,7 @@ struct ahx_hmat {
   // staging buffers for host vectors
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch
+  ahx::HostWord gm_word;
   // statistics of the last assembly
   uint64_t stat_ws_bytes = 0;   // largest ACA workspace batch (bytes)
   uint64_t stat_retries = 0;    // leaves re-run with a larger rank capacity

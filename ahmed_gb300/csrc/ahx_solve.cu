@@ -26,7 +26,9 @@
 namespace ahx {
 namespace {
 
-constexpr uint32_t kChunk = 4096;  // elements per reduction item
+// Elements per reduction item (a CTA).  1,024: a few hundred CTAs for 16 systems of 32,768
+// points; 4,096 left most SMs idle (a batch of 16 systems of 2,048 to 16,384: 27 CTAs).
+constexpr uint32_t kChunk = 1024;
 constexpr int kRedThreads = 256;
 constexpr int kPerThread = kChunk / kRedThreads;
 
@@ -36,6 +38,37 @@ struct Item {
   uint32_t q;     // system
 };
 
+// out[k] = sum_e V_k[e] w[e] over the CTA's item (v: V_0 at its base; a thread's elements:
+// threadIdx.x + e kRedThreads), summed in a fixed order
+__device__ __forceinline__ void item_dots(const double (&w)[kPerThread], uint32_t len, const double* v,
+                                          uint64_t vstride, uint32_t nk, double* out) {
+  constexpr uint32_t kTile = 64, kW = kRedThreads / 32;
+  __shared__ double red[kTile][kW];
+  for (uint32_t k0 = 0; k0 < nk; k0 += kTile) {
+    const uint32_t kn = min(kTile, nk - k0);
+#pragma unroll 4
+    for (uint32_t k = 0; k < kn; ++k) {
+      const double* vk = v + (uint64_t)(k0 + k) * vstride;
+      double s = 0.0;
+#pragma unroll
+      for (int e = 0; e < kPerThread; ++e) {
+        const uint32_t o = threadIdx.x + e * kRedThreads;
+        if (o < len) s = fma(vk[o], w[e], s);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < kn) {
+      double t = red[threadIdx.x][0];
+      for (uint32_t q = 1; q < kW; ++q) t += red[threadIdx.x][q];
+      out[k0 + threadIdx.x] = t;
+    }
+    __syncthreads();
+  }
+}
+
 // partial[it * ldp + k] = sum_e V_k[base+e] * W[base+e],  V_k = V + k * vstride
 __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restrict__ items,
                                                            const double* __restrict__ V,
@@ -43,7 +76,6 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restric
                                                            const double* __restrict__ W,
                                                            double* __restrict__ partial,
                                                            uint32_t ldp) {
-  __shared__ double red[kRedThreads / 32];
   const Item it = items[blockIdx.x];
   double w[kPerThread];
 #pragma unroll
@@ -51,14 +83,64 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restric
     const uint32_t o = threadIdx.x + e * kRedThreads;
     w[e] = o < it.len ? W[it.base + o] : 0.0;
   }
-  for (uint32_t k = 0; k < nk; ++k) {
-    const double* v = V + k * vstride + it.base;
+  item_dots(w, it.len, V + it.base, vstride, nk, partial + (uint64_t)blockIdx.x * ldp);
+}
+
+// One Gram-Schmidt pass on the CTA's item: the coefficients of its system from the item
+// sums `pin` of the pass before (each CTA adds them up itself, in item order; the system's
+// first one keeps them in coef), W -= sum_k coef_k V_k, and from the new W the item sums
+// of the next pass (LAST: of |W|^2).  One launch instead of a reduction, a combination
+// and the sums, one read of W, V from L1 the second time: a step's orthogonalisation
+// (16 systems of 32,768 points, steps 1 to 10) 93 us -> 62 us on average with cold caches.
+template <bool LAST>
+__global__ void __launch_bounds__(kRedThreads)
+    cgs_kernel(const Item* __restrict__ items, const uint32_t* __restrict__ first, const double* __restrict__ V,
+               uint64_t vstride, uint32_t nk, double* __restrict__ W, const double* __restrict__ pin, uint32_t ldp,
+               double* __restrict__ coef, uint32_t ldc, double* __restrict__ pout) {
+  constexpr uint32_t kTile = kRedThreads;
+  __shared__ double c[kTile];
+  const Item it = items[blockIdx.x];
+  const uint32_t i0 = first[it.q], i1 = first[it.q + 1];
+  double w[kPerThread];
+#pragma unroll
+  for (int e = 0; e < kPerThread; ++e) {
+    const uint32_t o = threadIdx.x + e * kRedThreads;
+    w[e] = o < it.len ? W[it.base + o] : 0.0;
+  }
+  for (uint32_t k0 = 0; k0 < nk; k0 += kTile) {
+    const uint32_t kn = min(kTile, nk - k0);
+    if (threadIdx.x < kn) {
+      double s = 0.0;
+#pragma unroll 8
+      for (uint32_t i = i0; i < i1; ++i) s += pin[(uint64_t)i * ldp + k0 + threadIdx.x];
+      c[threadIdx.x] = s;
+      if (blockIdx.x == i0) coef[(uint64_t)it.q * ldc + k0 + threadIdx.x] = s;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t k = 0; k < kn; ++k) {
+      const double* v = V + (k0 + k) * vstride + it.base;
+      const double ck = c[k];
+#pragma unroll
+      for (int e = 0; e < kPerThread; ++e) {
+        const uint32_t o = threadIdx.x + e * kRedThreads;
+        if (o < it.len) w[e] = fma(-ck, v[o], w[e]);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int e = 0; e < kPerThread; ++e) {
+    const uint32_t o = threadIdx.x + e * kRedThreads;
+    if (o < it.len) W[it.base + o] = w[e];
+  }
+  if (!LAST) {
+    item_dots(w, it.len, V + it.base, vstride, nk, pout + (uint64_t)blockIdx.x * ldp);
+  } else {
+    __shared__ double red[kRedThreads / 32];
     double s = 0.0;
 #pragma unroll
-    for (int e = 0; e < kPerThread; ++e) {
-      const uint32_t o = threadIdx.x + e * kRedThreads;
-      if (o < it.len) s = fma(v[o], w[e], s);
-    }
+    for (int e = 0; e < kPerThread; ++e) s = fma(w[e], w[e], s);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -66,9 +148,8 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restric
     if (threadIdx.x == 0) {
       double t = red[0];
       for (int q = 1; q < kRedThreads / 32; ++q) t += red[q];
-      partial[(uint64_t)blockIdx.x * ldp + k] = t;
+      pout[(uint64_t)blockIdx.x * ldp] = t;
     }
-    __syncthreads();
   }
 }
 
@@ -89,22 +170,6 @@ __device__ __forceinline__ uint32_t sys_of(uint64_t idx, uint64_t ntot, const ui
   const uint64_t c = idx / ntot;
   const uint32_t s = seg_id ? seg_id[idx - c * ntot] : 0u;
   return (uint32_t)c * nseg + s;
-}
-
-// W -= sum_{k < nk} coef[q * ldc + k] V_k   (per element's system q)
-__global__ void sub_combination_kernel(double* __restrict__ W, const double* __restrict__ V,
-                                       uint64_t vstride, uint32_t nk,
-                                       const double* __restrict__ coef, uint32_t ldc,
-                                       uint64_t total, uint64_t ntot,
-                                       const uint32_t* __restrict__ seg_id, uint32_t nseg) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t q = sys_of(i, ntot, seg_id, nseg);
-    const double* c = coef + (uint64_t)q * ldc;
-    double w = W[i];
-    for (uint32_t k = 0; k < nk; ++k) w = fma(-c[k], V[k * vstride + i], w);
-    W[i] = w;
-  }
 }
 
 // X += sum_{k < len[q]} y[q * ldy + k] V_k
@@ -180,69 +245,126 @@ __device__ __forceinline__ void appl_rot_d(double& dx, double& dy, double cs, do
 struct GmDev {
   double *R, *cs, *sn, *s, *y, *normb, *resid;
   uint32_t *flags;  // bit 0: running in this cycle, bit 1: converged
-  uint32_t *ylen, *iters, *jbase, *nactive;
+  uint32_t *ylen, *iters, *jbase;
   const double* tol;      // in device memory so that captured graphs stay valid
   const uint32_t* maxit;  // across calls with other tolerances and step limits
+  uint32_t *ticket, *stepno;  // of arnoldi_kernel's last warp; steps of this solve
+  unsigned long long* word;   // host memory: steps << 32 | systems still running
 };
 
-// y = R^{-1} s over the first k columns (solvers/GMRES.cpp:62-78, dtrsv)
-__device__ void tri_solve_d(const GmDev& g, uint32_t q, uint32_t k, uint32_t m, uint32_t K) {
+// y = R^{-1} s over the first k columns (solvers/GMRES.cpp:62-78, dtrsv), by one warp
+__device__ void tri_solve_d(const GmDev& g, uint32_t q, uint32_t k, uint32_t m, uint32_t K, uint32_t lane) {
   const double* Rq = g.R + (size_t)q * m * K;
   double* y = g.y + (size_t)q * K;
-  for (uint32_t i = 0; i < k; ++i) y[i] = g.s[(size_t)q * K + i];
+  for (uint32_t i = lane; i < k; i += 32) y[i] = g.s[(size_t)q * K + i];
+  __syncwarp();
   for (int jj = (int)k - 1; jj >= 0; --jj) {
-    y[jj] = __ddiv_rn(y[jj], Rq[(size_t)jj * K + jj]);
-    for (int i = 0; i < jj; ++i) y[i] = __dsub_rn(y[i], __dmul_rn(y[jj], Rq[(size_t)jj * K + i]));
+    const double yj = __ddiv_rn(y[jj], Rq[(size_t)jj * K + jj]);
+    __syncwarp();
+    if (lane == 0) y[jj] = yj;
+    for (int i = lane; i < jj; i += 32) y[i] = __dsub_rn(y[i], __dmul_rn(yj, Rq[(size_t)jj * K + i]));
+    __syncwarp();
   }
-  g.ylen[q] = k;
+  if (lane == 0) g.ylen[q] = k;
 }
 
-// One Arnoldi step i of every running system: Hessenberg column from the two
-// Gram-Schmidt passes (h1 + h2) and |w|, the rotations, the residual estimate.
-__global__ void arnoldi_kernel(GmDev g, uint32_t i, uint32_t m, uint32_t K, const double* __restrict__ h1,
-                               const double* __restrict__ h2, const double* __restrict__ nrm, uint32_t nsys) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsys) return;
+__device__ void arnoldi_system(const GmDev& g, uint32_t q, uint32_t i, uint32_t m, uint32_t K, const double* h1,
+                               const double* h2, double w2, uint32_t lane) {
   const uint32_t f = g.flags[q];
   if (!(f & 1u) || (f & 2u)) return;
   const uint32_t j = g.jbase[0] + i + 1;
   if (j > g.maxit[0]) return;
   double* col = g.R + ((size_t)q * m + i) * K;
-  for (uint32_t k = 0; k <= i; ++k) col[k] = __dadd_rn(h1[(size_t)q * K + k], h2[(size_t)q * K + k]);
-  col[i + 1] = __dsqrt_rn(nrm[(size_t)q * K]);
   double* csq = g.cs + (size_t)q * K;
   double* snq = g.sn + (size_t)q * K;
   double* sq = g.s + (size_t)q * K;
-  for (uint32_t k = 0; k < i; ++k) appl_rot_d(col[k], col[k + 1], csq[k], snq[k]);
-  gen_rot_d(col[i], col[i + 1], csq[i], snq[i]);
-  appl_rot_d(col[i], col[i + 1], csq[i], snq[i]);
-  appl_rot_d(sq[i], sq[i + 1], csq[i], snq[i]);
-  const double r = fabs(__ddiv_rn(sq[i + 1], g.normb[q]));
-  g.resid[q] = r;
-  g.iters[q] = j;
-  if (r < g.tol[0]) {
-    tri_solve_d(g, q, i + 1, m, K);
-    g.flags[q] = f | 2u;
+  const double* a = h1 + (size_t)q * K;
+  const double* b = h2 + (size_t)q * K;
+  double cur = 0.0;  // the entry that the next rotation takes with it
+  for (uint32_t k0 = 0; k0 <= i; k0 += 32) {
+    const uint32_t kn = min(32u, i + 1 - k0);
+    double h = 0.0, cs = 0.0, sn = 0.0;
+    if (lane < kn) {
+      h = __dadd_rn(a[k0 + lane], b[k0 + lane]);
+      if (k0 + lane > 0) {  // the rotation of entries k - 1 and k
+        cs = csq[k0 + lane - 1];
+        sn = snq[k0 + lane - 1];
+      }
+    }
+    for (uint32_t k = 0; k < kn; ++k) {
+      double hk = __shfl_sync(0xffffffffu, h, k);
+      const double c = __shfl_sync(0xffffffffu, cs, k), s = __shfl_sync(0xffffffffu, sn, k);
+      if (k0 + k > 0) {
+        appl_rot_d(cur, hk, c, s);
+        if (lane == 0) col[k0 + k - 1] = cur;
+      }
+      cur = hk;
+    }
+  }
+  double last = __dsqrt_rn(w2), cs, sn;
+  gen_rot_d(cur, last, cs, sn);
+  appl_rot_d(cur, last, cs, sn);
+  double s0 = sq[i], s1 = sq[i + 1];
+  __syncwarp();
+  appl_rot_d(s0, s1, cs, sn);
+  const double r = fabs(__ddiv_rn(s1, g.normb[q]));
+  const bool conv = r < g.tol[0];
+  if (lane == 0) {
+    col[i] = cur;
+    col[i + 1] = last;
+    csq[i] = cs;
+    snq[i] = sn;
+    sq[i] = s0;
+    sq[i + 1] = s1;
+    g.resid[q] = r;
+    g.iters[q] = j;
+    if (conv) g.flags[q] = f | 2u;
+  }
+  __syncwarp();
+  if (conv) tri_solve_d(g, q, i + 1, m, K, lane);
+}
+
+// One Arnoldi step i of every running system, a warp each: Hessenberg column from the two
+// Gram-Schmidt passes (h1 + h2) and |w| (item sums pn), the rotations, the residual
+// estimate.  fac[q] = 1 / |w| of every system (0 for w = 0).  The lanes load what the
+// rotations need 32 at a time, and the chain of rotations runs in registers.  The last
+// warp to finish counts the systems still running and tells the host, which prepares the
+// next step while w is scaled.
+__global__ void arnoldi_kernel(GmDev g, uint32_t i, uint32_t m, uint32_t K, const double* __restrict__ h1,
+                               const double* __restrict__ h2, const double* __restrict__ pn, uint32_t ldp,
+                               const uint32_t* __restrict__ first, double* __restrict__ fac, uint32_t nsys) {
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (q >= nsys) return;
+  double w2 = 0.0;
+  for (uint32_t it = first[q] + lane; it < first[q + 1]; it += 32) w2 += pn[(uint64_t)it * ldp];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) w2 += __shfl_xor_sync(0xffffffffu, w2, o);
+  if (lane == 0) fac[q] = w2 > 0.0 ? 1.0 / sqrt(w2) : 0.0;
+  arnoldi_system(g, q, i, m, K, h1, h2, w2, lane);
+  uint32_t t = 0;
+  if (lane == 0) {
+    __threadfence();
+    t = atomicAdd(g.ticket, 1u);
+  }
+  if (__shfl_sync(0xffffffffu, t, 0) != nsys - 1) return;
+  __threadfence();
+  uint32_t run = 0;
+  for (uint32_t s = lane; s < nsys; s += 32) run += (__ldcg(g.flags + s) & 3u) == 1u ? 1u : 0u;
+  run = __reduce_add_sync(0xffffffffu, run);
+  if (lane == 0) {
+    *g.ticket = 0u;
+    const uint32_t step = *g.stepno + 1u;
+    *g.stepno = step;
+    *reinterpret_cast<volatile unsigned long long*>(g.word) = ((unsigned long long)step << 32) | run;
   }
 }
 
 // running systems at the end of a cycle of `icount` steps: y from those steps
 __global__ void cycle_end_kernel(GmDev g, uint32_t icount, uint32_t m, uint32_t K, uint32_t nsys) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (q >= nsys) return;
   const uint32_t f = g.flags[q];
-  if ((f & 1u) && !(f & 2u) && icount > 0) tri_solve_d(g, q, icount, m, K);
-}
-
-__global__ void count_active_kernel(GmDev g, uint32_t nsys) {
-  __shared__ uint32_t c;
-  if (threadIdx.x == 0) c = 0;
-  __syncthreads();
-  uint32_t mine = 0;
-  for (uint32_t q = threadIdx.x; q < nsys; q += blockDim.x) mine += ((g.flags[q] & 3u) == 1u) ? 1u : 0u;
-  atomicAdd(&c, mine);
-  __syncthreads();
-  if (threadIdx.x == 0) g.nactive[0] = c;
+  if ((f & 1u) && !(f & 2u) && icount > 0) tri_solve_d(g, q, icount, m, K, threadIdx.x & 31);
 }
 
 }  // namespace
@@ -254,6 +376,7 @@ struct Operator {
   std::vector<uint64_t> seg_off;  // nseg + 1
   DevBuf seg_id;                  // ntot uint32 (only when nseg > 1)
   cudaStream_t stream = nullptr;
+  HostWord* word = nullptr;       // what the device tells the host between steps
   virtual ~Operator() { seg_id.release(); }
   // Y += d A X in storage precision prec
   virtual int apply(int prec, double d, uint32_t p, const double* X, double* Y) = 0;
@@ -287,6 +410,7 @@ struct HmatOp : Operator {
     ntot = h->tree.n;
     seg_off = {0, ntot};
     stream = h->stream;
+    word = &h->gm_word;
   }
   int apply(int prec, double d, uint32_t p, const double* X, double* Y) override {
     return product_device(H, prec, d, p, X, ntot, Y, ntot);
@@ -333,7 +457,7 @@ class Solver {
     int rc;
     if ((rc = items_.reserve(std::max<size_t>(items.size(), 1) * sizeof(Item)))) return rc;
     if ((rc = first_.reserve(first.size() * sizeof(uint32_t)))) return rc;
-    if ((rc = partial_.reserve((size_t)std::max(nitems_, 1u) * maxk * sizeof(double)))) return rc;
+    if ((rc = partial_.reserve(2 * (size_t)std::max(nitems_, 1u) * maxk * sizeof(double)))) return rc;
     if ((rc = small_.reserve((size_t)nsys_ * maxk * sizeof(double)))) return rc;
     if ((rc = small2_.reserve((size_t)nsys_ * maxk * sizeof(double)))) return rc;
     if ((rc = small3_.reserve((size_t)nsys_ * maxk * sizeof(double)))) return rc;
@@ -352,8 +476,22 @@ class Solver {
     dots_kernel<<<nitems_, kRedThreads, 0, op_.stream>>>(items_.as<Item>(), V, vstride, nk, W,
                                                          partial_.as<double>(), maxk_);
     const uint32_t nt = nsys_ * nk;
-    reduce_items_kernel<<<(nt + 255) / 256, 256, 0, op_.stream>>>(
+    reduce_items_kernel<<<(nt + 63) / 64, 64, 0, op_.stream>>>(
         partial_.as<double>(), maxk_, first_.as<uint32_t>(), nsys_, nk, out, maxk_);
+    AHX_CUDA(cudaGetLastError());
+    return AHX_OK;
+  }
+
+  // W -= V (V^T W), twice; the coefficients in h1 and h2, the items' |W|^2 in partial_
+  int gram_schmidt(const double* V, uint64_t vstride, uint32_t nk, double* W, double* h1, double* h2) {
+    if (nitems_ == 0) return AHX_OK;
+    const Item* it = items_.as<Item>();
+    const uint32_t* fi = first_.as<uint32_t>();
+    double *pa = partial_.as<double>(), *pb = pa + (size_t)nitems_ * maxk_;
+    cudaStream_t st = op_.stream;
+    dots_kernel<<<nitems_, kRedThreads, 0, st>>>(it, V, vstride, nk, W, pa, maxk_);
+    cgs_kernel<false><<<nitems_, kRedThreads, 0, st>>>(it, fi, V, vstride, nk, W, pa, maxk_, h1, maxk_, pb);
+    cgs_kernel<true><<<nitems_, kRedThreads, 0, st>>>(it, fi, V, vstride, nk, W, pb, maxk_, h2, maxk_, pa);
     AHX_CUDA(cudaGetLastError());
     return AHX_OK;
   }
@@ -424,7 +562,7 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
   double* d3 = sv.small3_.as<double>();
   // device state
   const size_t nd = (size_t)nsys * ((size_t)m * K + 4 * (size_t)K + 2) + 1;  // R, cs, sn, s, y, normb, resid, tol
-  const size_t nu = (size_t)nsys * 3 + 3;                                    // flags, ylen, iters, jbase, nactive, maxit
+  const size_t nu = (size_t)nsys * 3 + 4;                                    // flags, ylen, iters, jbase, ticket, maxit, stepno
   if ((rc = sv.gm_.reserve(nd * sizeof(double) + nu * sizeof(uint32_t)))) return rc;
   GmDev g;
   {
@@ -450,12 +588,16 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     g.ylen = u + nsys;
     g.iters = u + 2 * (size_t)nsys;
     g.jbase = u + 3 * (size_t)nsys;
-    g.nactive = g.jbase + 1;
+    g.ticket = g.jbase + 1;
+    g.stepno = g.jbase + 3;
     uint32_t* pmaxit = g.jbase + 2;
     g.tol = ptol;
     g.maxit = pmaxit;
     AHX_CUDA(cudaMemcpyAsync(ptol, &tol, sizeof(double), cudaMemcpyHostToDevice, st));
+    AHX_CUDA(cudaMemsetAsync(g.ticket, 0, 3 * sizeof(uint32_t), st));  // ticket, maxit, stepno
     AHX_CUDA(cudaMemcpyAsync(pmaxit, &maxit, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    if ((rc = op.word->reserve())) return rc;
+    g.word = op.word->device();
   }
   std::vector<double> hbuf((size_t)nsys * K);
   auto fetch = [&](const double* dev) -> int {
@@ -509,7 +651,6 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
       if (!done[q]) return true;
     return false;
   };
-  const unsigned sgrid = (nsys + 127) / 128;
   // steps i0 .. i1 - 1 of a cycle, then the count of systems still running
   auto steps = [&](uint32_t i0, uint32_t i1) -> int {
     for (uint32_t i = i0; i < i1; ++i) {
@@ -519,18 +660,12 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
       int e = op.apply(prec, 1.0, sv.p_, vi, w);
       if (e) return e;
       // CGS2: h = V^T w; w -= V h; h2 = V^T w; w -= V h2
-      if ((e = sv.dots(V, vstride, i + 1, w, d1))) return e;
-      sub_combination_kernel<<<grid_for(total), 256, 0, st>>>(w, V, vstride, i + 1, d1, K, total, op.ntot, sid,
-                                                              op.nseg);
-      if ((e = sv.dots(V, vstride, i + 1, w, d2))) return e;
-      sub_combination_kernel<<<grid_for(total), 256, 0, st>>>(w, V, vstride, i + 1, d2, K, total, op.ntot, sid,
-                                                              op.nseg);
-      if ((e = sv.dots(w, 0, 1, w, d3))) return e;
-      arnoldi_kernel<<<sgrid, 128, 0, st>>>(g, i, m, K, d1, d2, d3, nsys);
+      if ((e = sv.gram_schmidt(V, vstride, i + 1, w, d1, d2))) return e;
+      arnoldi_kernel<<<(nsys + 3) / 4, 128, 0, st>>>(g, i, m, K, d1, d2, sv.partial_.as<double>(), K, sv.first_.as<uint32_t>(),
+                                            d3, nsys);
       // w /= |w|
-      scale_kernel<<<grid_for(total), 256, 0, st>>>(w, w, d3, K, 1, total, op.ntot, sid, op.nseg);
+      scale_kernel<<<grid_for(total), 256, 0, st>>>(w, w, d3, 1, 0, total, op.ntot, sid, op.nseg);
     }
-    count_active_kernel<<<1, 256, 0, st>>>(g, nsys);
     AHX_CUDA(cudaGetLastError());
     return AHX_OK;
   };
@@ -543,7 +678,9 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     graphs->chunk = chunk;
   }
   auto run_chunk = [&](uint32_t c, uint32_t i0, uint32_t i1) -> int {
-    if (!graphs || graphs->failed) return steps(i0, i1);
+    // long steps: a graph of one of them costs the host more (0.1 ms to capture and
+    // instantiate, while the GPU waits) than its launches, which the GPU never catches up with
+    if (!graphs || graphs->failed || chunk == 1) return steps(i0, i1);
     if (graphs->exec.size() <= c) graphs->exec.resize(c + 1, nullptr);
     if (!graphs->exec[c]) {
       cudaGraph_t graph = nullptr;
@@ -569,6 +706,9 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     return AHX_OK;
   };
   uint32_t j = 1;  // global number of the next step
+  uint32_t launched = 0;  // steps (modulo 2^32, as the device counts them)
+  AHX_CUDA(cudaStreamSynchronize(st));
+  op.word->clear();
   std::vector<uint32_t> flags(nsys), hiters(nsys);
   std::vector<double> hres(nsys);
   while (active_left() && j <= maxit) {
@@ -592,12 +732,12 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
       const uint32_t i0 = c * chunk, i1 = std::min(m, i0 + chunk);
       if ((rc = run_chunk(c, i0, i1))) return rc;
       ran = std::min(i1, icap);
+      launched += i1 - i0;
       uint32_t nact = 0;
-      AHX_CUDA(cudaMemcpyAsync(&nact, g.nactive, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-      AHX_CUDA(cudaStreamSynchronize(st));
+      if ((rc = op.word->wait(launched, st, nact))) return rc;
       if (nact == 0) break;
     }
-    cycle_end_kernel<<<sgrid, 128, 0, st>>>(g, ran, m, K, nsys);
+    cycle_end_kernel<<<(nsys + 3) / 4, 128, 0, st>>>(g, ran, m, K, nsys);
     add_combination_kernel<<<grid_for(total), 256, 0, st>>>(X, V, vstride, g.ylen, g.y, K, total, op.ntot, sid,
                                                             op.nseg);
     AHX_CUDA(cudaGetLastError());
@@ -953,6 +1093,7 @@ struct ahx_batch : ahx::Operator {
     ahx::ProdCopy plan;  // mixed-precision plan over the concatenated leaves
   } tab[ahx::kNumPrecisions];
   ahx::DevBuf stx, sty;
+  ahx::HostWord steps;
 
   // FP64: concatenated leaf table and arena; mixed precisions: streams built
   // from the concatenated FP64 arena.
@@ -1250,6 +1391,7 @@ int ahx_batch_destroy(ahx_batch* b) {
   }
   b->stx.release();
   b->sty.release();
+  b->steps.release();
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   b->stream = nullptr;
   delete b;
@@ -1301,6 +1443,7 @@ int ahx_batch_gmres(ahx_batch* b, const double* B, double* X, double tol, uint32
   if ((rc = stage_in(X, n, n, 1, xb, Xc, b->stream))) return rc;
   double* Xd = const_cast<double*>(Xc);
   int status = AHX_OK;
+  b->word = &b->steps;
   rc = gmres_driver(*b, b->prec, 1, Bd, Xd, tol, m, maxit, iters, resid, status);
   if (rc) return rc;
   if (Xd != X) AHX_CUDA(cudaMemcpyAsync(X, Xd, n * 8, cudaMemcpyDefault, b->stream));
