@@ -521,13 +521,19 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   // faster one; the plain kernel then only runs when X does not fit the digits
   // (double-float would need a copy of the leaves: there always)
   const int* guard = nullptr;
-  if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2 &&
-      (prec == kDF64 || dg_due(H->dg[transposed ? 1 : 0], H->arena64_elems, p, H->tree.leaves.size()))) {
+  const bool one = prec == kFP64 && p == 1 && f1_wanted(H->arena64_elems, transposed);
+  if (one || ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2)) {
     bool usable = false;
     // (nothing is laid out or allocated while the stream is captured)
-    const DgState& D = H->dg[transposed ? 1 : 0];
-    if ((D.valid && H->dg_work.bytes >= dg_work_bytes(false, H->tree.n, D.t_rows, p)) || !stream_captured(H->stream))
+    DgState& D = H->dg[transposed ? 1 : 0];
+    const bool ready = D.valid && H->dg_work.bytes >= dg_work_bytes(false, H->tree.n, D.t_rows, p);
+    if (ready || ((prec == kDF64 || dg_due(D, H->arena64_elems, p, H->tree.leaves.size())) && !stream_captured(H->stream)))
       if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
+    if (usable && one) {
+      const DgPlan pl = dg_plan(D, H->tree.n, H->arena64.p, H->dg_work);
+      AHX_CUDA(launch_matvec_f1(pl, d, X, Y, H->stream));
+      return AHX_OK;
+    }
     if (usable) {
       const DgPlan pl = dg_plan(H->dg[transposed ? 1 : 0], H->tree.n, H->arena64.p, H->dg_work);
       const DgArgs da{false, d, 0.0, p, X, ldX, Y, ldY};
@@ -578,7 +584,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
 
 int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable) {
   usable = false;
-  if (H->finite == 2) return AHX_OK;
+  if (H->finite == 2 && p > 1) return AHX_OK;  // (one right-hand side takes any leaves)
   DgState& D = H->dg[transposed ? 1 : 0];
   int rc;
   if (!D.valid) {
@@ -596,7 +602,7 @@ int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable) {
     if ((rc = dg_prepare_state(D, lv, H->tree.n, H->arena64.p, H->arena64_elems, kDgK, H->finite, H->device, H->stream)))
       return rc;
   }
-  if (!D.usable || H->finite == 2) return AHX_OK;
+  if (!D.usable || (H->finite == 2 && p > 1)) return AHX_OK;
   if ((rc = H->dg_work.reserve(dg_work_bytes(false, H->tree.n, D.t_rows, p)))) return rc;
   usable = true;
   return AHX_OK;

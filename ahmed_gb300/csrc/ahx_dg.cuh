@@ -112,6 +112,10 @@ cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cuda
 // *bad |= any of the count doubles is not finite, or not zero and outside [2^-500, 2^500]
 cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStream_t s);
 cudaError_t launch_matvec_dg(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
+// FP64 leaves and one right-hand side over the same layout (ahx_matvec_f1.cu); pl.work:
+// dg_work_bytes
+cudaError_t launch_matvec_f1(const DgPlan& pl, double d, const double* X, double* Y, cudaStream_t s);
+bool f1_wanted(uint64_t elems, bool transposed);
 // complex64 leaves over the same layout (ahx_matvec_zt.cu; X, Y complex128): pl.arena the
 // complex64 copy, pl.work of zt_work_bytes
 size_t zt_work_bytes(uint32_t n, uint32_t t_rows, uint32_t p);

@@ -418,7 +418,8 @@ struct HmatOp : Operator {
   uint64_t product_bytes(int prec) const override { return H->prod[prec].bytes; }
   int prepare(int prec, uint32_t p) override {
     int rc;
-    if ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) {
+    if (((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) ||
+        (prec == kFP64 && p == 1 && f1_wanted(H->arena64_elems, false))) {
       bool usable = false;
       if ((rc = prepare_dg(H, p, false, usable))) return rc;
       if (usable) prec = kFP64;
