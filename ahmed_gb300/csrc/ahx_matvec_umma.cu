@@ -343,13 +343,21 @@ __global__ void __launch_bounds__(kThreads, 1) um_sweep_kernel(const __grid_cons
       unsigned long long zlat = 0;
       uint32_t c = 0;
       bool issued = false;
+      // A wait costs some 200 cycles even on a completed barrier, and three in turn for
+      // every chunk bounded this thread: they are tested together, and only what the test
+      // finds incomplete is waited for (the Z warps do the same).  A chunk takes 1,436
+      // cycles instead of 1,703 (65,536 points, leaf 32, 16 right-hand sides), 1,676
+      // instead of 1,969 (131,072 points, leaf 64, 64); four accumulators of 128 columns
+      // with tiles of 64 rows 1,362, but 14 % more chunks.
       while (true) {
-        const uint32_t sl = c % kSlots, q = c % kAcc;
+        const uint32_t sl = c % kSlots, q = c % kAcc, ps = (c / kSlots) & 1, pq = ((c / kAcc) - 1) & 1;
         long long tp = P.now();
-        if (!wait_bar(S.fimg(sl), (c / kSlots) & 1, a.err)) break;
+        const uint32_t tst = mbar_test3(S.fimg(sl), ps, S.accempty(q), pq, S.fz(sl), ps);
+        const bool ti = tst & 1u, ta = c < kAcc || (tst & 2u), tz = tst & 4u;
+        if (!ti && !wait_bar(S.fimg(sl), (c / kSlots) & 1, a.err)) break;
         P.add(0, tp);
         tp = P.now();
-        if (c >= kAcc && !wait_bar(S.accempty(q), ((c / kAcc) - 1) & 1, a.err)) break;
+        if (!ta && !wait_bar(S.accempty(q), ((c / kAcc) - 1) & 1, a.err)) break;
         P.add(1, tp);
         if (S.meta(sl)->hdr == 0u) {
           // forward the stop to the epilogue (both arrivals of the phase)
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) um_sweep_kernel(const __grid_cons
           break;
         }
         tp = P.now();
-        if (!wait_bar(S.fz(sl), (c / kSlots) & 1, a.err)) break;
+        if (!tz && !wait_bar(S.fz(sl), (c / kSlots) & 1, a.err)) break;
         P.add(2, tp);
         if (P.on) zlat += (unsigned long long)(clock64() - *S.issued(sl));  // issue -> Z rows landed
         tp = P.now();
@@ -429,10 +437,13 @@ __global__ void __launch_bounds__(kThreads, 1) um_sweep_kernel(const __grid_cons
     for (; c < ncb; ++c) {
       const uint32_t sl = c % kSlots, e = c % kQ;
       long long tp = P.now();
-      if (!__all_sync(0xffffffffu, wait_bar(S.idxbar(h, e), (c / kQ) & 1, a.err))) break;
+      // (both tested before either is waited for, as the MMA thread does)
+      const uint32_t tst = mbar_test2(S.idxbar(h, e), (c / kQ) & 1, S.empty(sl), ((c / kSlots) - 1) & 1);
+      const bool ti = tst & 1u, te = c < kSlots || (tst & 2u);
+      if (!__all_sync(0xffffffffu, ti || wait_bar(S.idxbar(h, e), (c / kQ) & 1, a.err))) break;
       P.add(0, tp);
       tp = P.now();
-      if (c >= kSlots && !__all_sync(0xffffffffu, wait_bar(S.empty(sl), ((c / kSlots) - 1) & 1, a.err))) break;
+      if (!__all_sync(0xffffffffu, te || wait_bar(S.empty(sl), ((c / kSlots) - 1) & 1, a.err))) break;
       P.add(1, tp);
       tp = P.now();
       // index of position 2 r + odd (of this warp's positions) in zi[r]
@@ -1208,12 +1219,16 @@ void build_um_layout(const std::vector<PlanLeaf>& leaves, uint64_t n, uint32_t g
   };
   place(L.vbuild, L.vtiles, L.vbytes, L.vchunks);
   place(L.rbuild, L.rtiles, L.rbytes, L.rchunks);
-  // contiguous tile ranges per CTA, balanced by stream bytes
+  // contiguous tile ranges per CTA, balanced by cost
   auto ranges = [&](const std::vector<UmBuild>& bl, std::vector<uint32_t>& first) {
-    std::vector<uint64_t> bytes(bl.size());
-    // stream bytes plus the chunks' Z rows (mostly L2 hits: weighted by half)
-    for (size_t t = 0; t < bl.size(); ++t) bytes[t] = chunk_bytes(bl[t]) + (uint64_t)bl[t].nchunks * kUmKc * kUmZRowBytes / 2;
-    balance_ranges(bytes, std::max<uint32_t>(grid, 1), first);
+    std::vector<uint64_t> cost(bl.size());
+    // In cycles: a chunk takes its share of the memory's rate (21 bytes a cycle and SM) or
+    // what its pass through the roles does (1,420 to 1,680 cycles with 14 KB a chunk as with
+    // 24), whichever is more; the end of a tile besides.  By bytes alone: 503 us instead of
+    // 480 (65,536 points, 16 right-hand sides), 1,094 instead of 1,065 (131,072, 64).
+    for (size_t t = 0; t < bl.size(); ++t)
+      cost[t] = std::max<uint64_t>(chunk_bytes(bl[t]) / 21, (uint64_t)bl[t].nchunks * 1300) + 500;
+    balance_ranges(cost, std::max<uint32_t>(grid, 1), first);
   };
   ranges(L.vbuild, L.vranges);
   ranges(L.rbuild, L.rranges);

@@ -21,6 +21,40 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
                : "memory");
 }
 
+// whether the phases of three (two) barriers have completed, without suspending the
+// thread; one asm block, so that the tests' latencies overlap (bit i: barrier i)
+__device__ __forceinline__ uint32_t mbar_test3(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2,
+                                               uint32_t p2) {
+  uint32_t m;
+  asm volatile(
+      "{\n\t.reg .pred a, b, c;\n\t.reg .b32 x, y;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 a, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 b, [%3], %4;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 c, [%5], %6;\n\t"
+      "selp.u32 %0, 1, 0, a;\n\t"
+      "selp.u32 x, 2, 0, b;\n\t"
+      "selp.u32 y, 4, 0, c;\n\t"
+      "or.b32 %0, %0, x;\n\t"
+      "or.b32 %0, %0, y;\n\t}"
+      : "=&r"(m)
+      : "r"(b0), "r"(p0), "r"(b1), "r"(p1), "r"(b2), "r"(p2)
+      : "memory");
+  return m;
+}
+__device__ __forceinline__ uint32_t mbar_test2(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1) {
+  uint32_t m;
+  asm volatile(
+      "{\n\t.reg .pred a, b;\n\t.reg .b32 x;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 a, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 b, [%3], %4;\n\t"
+      "selp.u32 %0, 1, 0, a;\n\t"
+      "selp.u32 x, 2, 0, b;\n\t"
+      "or.b32 %0, %0, x;\n\t}"
+      : "=&r"(m)
+      : "r"(b0), "r"(p0), "r"(b1), "r"(p1)
+      : "memory");
+  return m;
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
