@@ -20,11 +20,13 @@
 //     tolerances near rounding) take a Householder QR;
 //   * the Jacobi rotations are found in FP32 (the angle need not be exact, only
 //     c^2 + s^2 = 1 must: one more sweep at most), their right factor is not
-//     accumulated (Z = M^H (W S) S^-2 afterwards), column norms are updated;
+//     accumulated (Z = M^H (W S) S^-2 afterwards), column norms are updated; M is
+//     brought to triangular form first (lq: all of the assembly 31.6 -> 29.9 ms below,
+//     19.9 -> 17.5 ms complex);
 //   * matrix entries take a reciprocal square root seeded in FP32.
 // All admissible leaves of 65,536 sphere points (60,012, ranks about 10 before and 7
-// after the truncation): 95 ms with Householder QRs and one value per reduction, 22 ms
-// so; Helmholtz, 12,289 points, k = 8: 96 ms, 17 ms.  FP64 pipe 85 % busy (68 % complex).
+// after the truncation): 95 ms with Householder QRs and one value per reduction, 20 ms
+// so; Helmholtz, 12,289 points, k = 8: 96 ms, 15 ms.  FP64 pipe 85 % busy (68 % complex).
 #pragma once
 #include <climits>
 #include <cstdint>
@@ -869,10 +871,69 @@ __device__ void apply_q(Team<W>& g, uint32_t m, uint32_t kr, const T* A, const T
   }
 }
 
+// M := L with M = L Q^H, Q's columns orthonormal (modified Gram-Schmidt on M's rows,
+// whose triangular factor is as accurate as Householder's, Bjorck 1967): same left
+// singular vectors and singular values, L lower triangular.  The rows are R1's, in the
+// order of falling pivots, so that L's columns are nearly orthogonal already and Jacobi
+// needs about 3 sweeps less (7 -> 4-5; this costs 0.6 of one); rows that the threshold
+// has emptied leave no column: returns the number of columns to work on.
+// G: scratch (m x n, row-major, stride ldg), nrm: n.
+template <int NW, class T>
+__device__ uint32_t lq(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, T* G, uint32_t ldg, double* nrm) {
+  const uint32_t q = min(m, n);
+  for (uint32_t j = 0; j < q; ++j) {
+    const uint32_t rows = m - j;
+    const uint32_t L = rows <= 4 * NW ? 8 : rows <= 8 * NW ? 4 : rows <= 16 * NW ? 2 : 1;
+    const uint32_t sub = g.lane & (L - 1), grp = g.rank / L, groups = 32 * NW / L;
+    const T* const rj = M + j * ld;
+    for (uint32_t i0 = j; i0 < m; i0 += groups) {
+      const uint32_t i = i0 + grp;
+      T s = zero_of(T());
+      if (i < m)
+        for (uint32_t l = sub; l < n; l += L) s = maddc(s, rj[l], M[i * ld + l]);
+      for (uint32_t o = 1; o < L; o <<= 1) {
+        if constexpr (sizeof(T) == 16) {
+          s.re += __shfl_xor_sync(0xffffffffu, s.re, o);
+          s.im += __shfl_xor_sync(0xffffffffu, s.im, o);
+        } else {
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+        }
+      }
+      if (i < m && sub == 0) G[i * ldg + j] = s;
+    }
+    g.sync();
+    const double d = re_(G[j * ldg + j]);
+    const double rs = __double2hiint(d) >= 0x00100000 ? rsqrt_any(d) : 0.0;  // an empty row: no column
+    if (g.rank == 0) nrm[j] = rs;
+    const double r2 = rs * rs;
+    for (uint32_t i = j + 1 + grp; i < m; i += groups) {
+      const T f = scale_(G[i * ldg + j], r2);
+      for (uint32_t l = sub; l < n; l += L) M[i * ld + l] = msub(M[i * ld + l], f, rj[l]);
+    }
+    g.sync();
+  }
+  uint32_t cols = 0;
+  for (uint32_t j0 = 0; j0 < q; j0 += 32) {
+    const uint32_t b =
+        __ballot_sync(0xffffffffu, j0 + g.lane < q && __double_as_longlong(nrm[min(j0 + g.lane, q - 1)]) != 0);
+    if (b) cols = j0 + 32 - __clz(b);
+  }
+  for (uint32_t e = g.rank; e < m * n; e += 32 * NW) {
+    const uint32_t i = e / n, j = e - i * n;
+    M[i * ld + j] = j < cols && j <= i ? scale_(G[i * ldg + j], nrm[j]) : zero_of(T());
+  }
+  g.sync();
+  return cols;
+}
+
 // One-sided Jacobi (Hestenes) on the columns of M (m x n, row-major) in tournament
 // order (Brent-Luk round robin) by NW warps: 8, 4 or 2 lanes per column pair.  A pair
 // rotates unless |x^H y| <= 1e-15 |x| |y|.  The tangent is found in FP32, c and s from
-// it in FP64; the squared norms are computed once a sweep and updated between.
+// it in FP64; the squared norms are computed once a sweep and updated between.  A sweep
+// whose cosines and angles (against the columns' lengths) all stayed below kJacLast is
+// the last: a rotation leaves 1e-7 of its own cosine (FP32 angle) and changes the others
+// by products of two such numbers, so that all are below the threshold after it.
+constexpr float kJacLast = 3e-9f;
 template <int NW, class T>
 __device__ void jacobi(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, double* nrm) {
   constexpr bool CX = sizeof(T) == 16;
@@ -892,7 +953,7 @@ __device__ void jacobi(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, d
       nrm[j] = s;
     }
     g.sync();
-    bool rotated = false;
+    bool large = false;
     for (uint32_t r = 0; r + 1 < ne; ++r) {
       for (uint32_t p0 = 0; p0 < np; p0 += groups) {
         const uint32_t p = p0 + grp;
@@ -943,8 +1004,9 @@ __device__ void jacobi(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, d
           const float fd = to_f32(be - al, sh);
           const float g2 = 2.f * fg;
           const float t = __fdividef(g2, fd + copysignf(sqrt_f32(fmaf(fd, fd, g2 * g2)), fd));
-          if (fabsf(fg) > 1e-15f * sqrt_f32(fal) * sqrt_f32(fbe) && fabsf(t) > 1e-37f) {
-            rotated = true;
+          const float sa = sqrt_f32(fal), sb = sqrt_f32(fbe);
+          if (fabsf(fg) > 1e-15f * sa * sb && fabsf(t) > 1e-37f) {
+            large |= fabsf(fg) > kJacLast * sa * sb || fabsf(t) * fmaxf(sa, sb) > kJacLast * fminf(sa, sb);
             const double td = to_f64(t);
             const double c = rsqrt_seeded(fma(td, td, 1.0)), s = c * td;
             if constexpr (CX) {
@@ -972,11 +1034,11 @@ __device__ void jacobi(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, d
       g.sync();
     }
     if constexpr (NW > 1) {
-      if (rotated) again = 1;
+      if (large) again = 1;
       __syncthreads();
       if (!again) break;
     } else {
-      if (!__any_sync(0xffffffffu, rotated)) break;
+      if (!__any_sync(0xffffffffu, large)) break;
     }
   }
   g.sync();
@@ -1083,11 +1145,17 @@ __device__ bool compress(Team<W>& g, uint32_t n1, uint32_t n2, uint32_t k, T* U,
       w.M0[i * w.ld + j] = s;
     }
     __syncwarp();
-    if (W == 1 || k <= 32) jacobi<1>(g1, mm, nn, w.M, w.ldm, w.nrm);
+    if (W == 1 || k <= 32) {
+      const uint32_t cols = lq<1>(g1, mm, nn, w.M, w.ldm, w.C2, w.ld, w.nrm);
+      jacobi<1>(g1, mm, cols, w.M, w.ldm, w.nrm);
+    }
   }
   if constexpr (W > 1) {
     __syncthreads();
-    if (k > 32) jacobi<W>(g, mm, nn, w.M, w.ldm, w.nrm);
+    if (k > 32) {
+      const uint32_t cols = lq<W>(g, mm, nn, w.M, w.ldm, w.C2, w.ld, w.nrm);
+      jacobi<W>(g, mm, cols, w.M, w.ldm, w.nrm);
+    }
   }
   if (first) {
     // singular values in descending order (the first among equals first), the rank

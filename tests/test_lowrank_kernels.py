@@ -90,3 +90,32 @@ def test_a_cta_per_leaf(eps, cplx):
         U, V = d[:n1 * k].reshape(k, n1).T, d[n1 * k:].reshape(k, n2).T
         assert np.linalg.norm(U @ V.conj().T - B) <= (20 * eps + 6e-12) * np.linalg.norm(B), (l, n1, n2, k)
     H.close()
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n,bmin,eta,eps", [(2500, 8, 0.8, 1e-3), (2500, 40, 0.8, 1e-6), (6007, 200, 2.0, 1e-9)])
+def test_columns_of_u_are_orthogonal(n, bmin, eta, eps, cplx):
+    """The triangular form and the last Jacobi sweep: ranks of 1 to more than 32, rows that
+    the threshold empties, columns of very different lengths."""
+    pts = _points(n, n + 1)
+    H = A.HMatrix(pts, "bbx", bmin=bmin, eta=eta)
+    h = A.mean_nn(pts)
+    if cplx:
+        H.helmholtz_assemble(9.0, h, eps)
+        ranks, data = H.helm_ranks(), H.helm_leaf_data
+    else:
+        H.matgenGeH_omp(h, eps)
+        ranks, data = H.ranks(), H.leaf_data
+    lv = H.leaves()
+    low = np.nonzero(ranks > 1)[0]
+    assert len(low)
+    for l in low:
+        n1, k = int(lv[l, 1]), int(ranks[l])
+        U = data(int(l))[:n1 * k].reshape(k, n1).T
+        s = np.linalg.norm(U, axis=0)
+        assert (s[1:] <= s[:-1] * (1 + 1e-6)).all()
+        # Q1 = U R1^-1 is orthonormal to k u cond(R1)^2: column pivots above 1e-6 of their
+        # columns' squares keep that below 1e-6; a sweep too few leaves 1e-5 to 1
+        G = np.abs(U.conj().T @ U) / np.outer(s, s) - np.eye(k)
+        assert np.abs(G).max() <= 1e-6, (l, n1, k)
+    H.close()
