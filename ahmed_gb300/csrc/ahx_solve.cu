@@ -38,27 +38,62 @@ struct Item {
   uint32_t q;     // system
 };
 
+// Sums over the warp of R values a lane by halving exchanges: value u ends in the lanes
+// whose top log2(R) bits are u (9 additions for 8 values, 40 one by one).
+template <int R>
+__device__ __forceinline__ double warp_sums(double (&s)[R]) {
+  const uint32_t lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int r = R / 2; r > 0; r >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int u = 0; u < r; ++u) {
+      const double keep = up ? s[u + r] : s[u], give = up ? s[u] : s[u + r];
+      s[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+  return s[0];
+}
+
+// red[u][warp] = this warp's part of sum_e V_u[e] w[e], u < R
+template <int R>
+__device__ __forceinline__ void warp_dots(const double (&w)[kPerThread], uint32_t len, const double* v,
+                                          uint64_t vstride, double (*red)[kRedThreads / 32]) {
+  double s[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    s[u] = 0.0;
+#pragma unroll
+    for (int e = 0; e < kPerThread; ++e) {
+      const uint32_t o = threadIdx.x + e * kRedThreads;
+      s[u] = fma(o < len ? v[u * vstride + o] : 0.0, w[e], s[u]);
+    }
+  }
+  const double t = warp_sums<R>(s);
+  const uint32_t lane = threadIdx.x & 31;
+  if (lane % (32 / R) == 0) red[lane / (32 / R)][threadIdx.x >> 5] = t;
+}
+
 // out[k] = sum_e V_k[e] w[e] over the CTA's item (v: V_0 at its base; a thread's elements:
-// threadIdx.x + e kRedThreads), summed in a fixed order
+// threadIdx.x + e kRedThreads), summed in a fixed order.  The FP64 pipe bounds it (2
+// multiply-adds per clock and SM): 4 multiply-adds per vector and warp, so that 5 additions
+// per vector for its sum were more than half of the work; for 8 vectors at once they are 9.
+// 10 vectors of 524,288 elements (cold caches): 31 -> 21 us, a pass of cgs_kernel 45 -> 32.
 __device__ __forceinline__ void item_dots(const double (&w)[kPerThread], uint32_t len, const double* v,
                                           uint64_t vstride, uint32_t nk, double* out) {
   constexpr uint32_t kTile = 64, kW = kRedThreads / 32;
   __shared__ double red[kTile][kW];
   for (uint32_t k0 = 0; k0 < nk; k0 += kTile) {
     const uint32_t kn = min(kTile, nk - k0);
-#pragma unroll 4
-    for (uint32_t k = 0; k < kn; ++k) {
-      const double* vk = v + (uint64_t)(k0 + k) * vstride;
-      double s = 0.0;
-#pragma unroll
-      for (int e = 0; e < kPerThread; ++e) {
-        const uint32_t o = threadIdx.x + e * kRedThreads;
-        if (o < len) s = fma(vk[o], w[e], s);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = s;
-    }
+    const double* vt = v + (uint64_t)k0 * vstride;
+    uint32_t k = 0;
+    for (; k + 8 <= kn; k += 8) warp_dots<8>(w, len, vt + k * vstride, vstride, red + k);
+    if (kn & 4) warp_dots<4>(w, len, vt + k * vstride, vstride, red + k), k += 4;
+    if (kn & 2) warp_dots<2>(w, len, vt + k * vstride, vstride, red + k), k += 2;
+    if (kn & 1) warp_dots<1>(w, len, vt + k * vstride, vstride, red + k);
     __syncthreads();
     if (threadIdx.x < kn) {
       double t = red[threadIdx.x][0];
@@ -91,14 +126,14 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restric
 // first one keeps them in coef), W -= sum_k coef_k V_k, and from the new W the item sums
 // of the next pass (LAST: of |W|^2).  One launch instead of a reduction, a combination
 // and the sums, one read of W, V from L1 the second time: a step's orthogonalisation
-// (16 systems of 32,768 points, steps 1 to 10) 93 us -> 62 us on average with cold caches.
+// (16 systems of 32,768 points, steps 1 to 10) 93 us -> 50 us on average with cold caches.
 template <bool LAST>
 __global__ void __launch_bounds__(kRedThreads)
     cgs_kernel(const Item* __restrict__ items, const uint32_t* __restrict__ first, const double* __restrict__ V,
                uint64_t vstride, uint32_t nk, double* __restrict__ W, const double* __restrict__ pin, uint32_t ldp,
                double* __restrict__ coef, uint32_t ldc, double* __restrict__ pout) {
   constexpr uint32_t kTile = kRedThreads;
-  __shared__ double c[kTile];
+  __shared__ double c[kTile], parts[kTile];
   const Item it = items[blockIdx.x];
   const uint32_t i0 = first[it.q], i1 = first[it.q + 1];
   double w[kPerThread];
@@ -109,10 +144,17 @@ __global__ void __launch_bounds__(kRedThreads)
   }
   for (uint32_t k0 = 0; k0 < nk; k0 += kTile) {
     const uint32_t kn = min(kTile, nk - k0);
+    // up to 16 threads to a coefficient, each with every 16th item
+    const uint32_t kw = kn > 128 ? 256 : kn > 64 ? 128 : kn > 32 ? 64 : kn > 16 ? 32 : 16, np = kTile / kw;
+    const uint32_t kt = threadIdx.x & (kw - 1), part = threadIdx.x / kw;
+    double s = 0.0;
+    if (kt < kn)
+#pragma unroll 4
+      for (uint32_t i = i0 + part; i < i1; i += np) s += pin[(uint64_t)i * ldp + k0 + kt];
+    parts[threadIdx.x] = s;
+    __syncthreads();
     if (threadIdx.x < kn) {
-      double s = 0.0;
-#pragma unroll 8
-      for (uint32_t i = i0; i < i1; ++i) s += pin[(uint64_t)i * ldp + k0 + threadIdx.x];
+      for (uint32_t q = 1; q < np; ++q) s += parts[q * kw + threadIdx.x];
       c[threadIdx.x] = s;
       if (blockIdx.x == i0) coef[(uint64_t)it.q * ldc + k0 + threadIdx.x] = s;
     }
@@ -252,17 +294,33 @@ struct GmDev {
   unsigned long long* word;   // host memory: steps << 32 | systems still running
 };
 
-// y = R^{-1} s over the first k columns (solvers/GMRES.cpp:62-78, dtrsv), by one warp
+// y = R^{-1} s over the first k columns (solvers/GMRES.cpp:62-78, dtrsv), by one warp: 32
+// unknowns at a time in the lanes' registers, the next column loaded a step ahead (a chain
+// through memory cost 12 us for 10 columns)
 __device__ void tri_solve_d(const GmDev& g, uint32_t q, uint32_t k, uint32_t m, uint32_t K, uint32_t lane) {
   const double* Rq = g.R + (size_t)q * m * K;
   double* y = g.y + (size_t)q * K;
   for (uint32_t i = lane; i < k; i += 32) y[i] = g.s[(size_t)q * K + i];
   __syncwarp();
-  for (int jj = (int)k - 1; jj >= 0; --jj) {
-    const double yj = __ddiv_rn(y[jj], Rq[(size_t)jj * K + jj]);
+  for (int b = (int)((k - 1) / 32) * 32; b >= 0; b -= 32) {
+    const int kb = min(32, (int)k - b);
+    const double* Rb = Rq + (size_t)b * K + b + lane;
+    double v = (int)lane < kb ? y[b + lane] : 0.0;
+    double r = (int)lane < kb ? Rb[(size_t)(kb - 1) * K] : 0.0;
+    for (int jj = kb - 1; jj >= 0; --jj) {
+      const double rn = (int)lane < jj ? Rb[(size_t)(jj - 1) * K] : 0.0;
+      const double yj = __ddiv_rn(__shfl_sync(0xffffffffu, v, jj), __shfl_sync(0xffffffffu, r, jj));
+      if ((int)lane == jj) v = yj;
+      else if ((int)lane < jj) v = __dsub_rn(v, __dmul_rn(yj, r));
+      r = rn;
+    }
+    if ((int)lane < kb) y[b + lane] = v;
     __syncwarp();
-    if (lane == 0) y[jj] = yj;
-    for (int i = lane; i < jj; i += 32) y[i] = __dsub_rn(y[i], __dmul_rn(yj, Rq[(size_t)jj * K + i]));
+    for (int i = lane; i < b; i += 32) {
+      double t = y[i];
+      for (int jj = kb - 1; jj >= 0; --jj) t = __dsub_rn(t, __dmul_rn(y[b + jj], Rq[(size_t)(b + jj) * K + i]));
+      y[i] = t;
+    }
     __syncwarp();
   }
   if (lane == 0) g.ylen[q] = k;
