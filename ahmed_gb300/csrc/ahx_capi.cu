@@ -700,6 +700,7 @@ int ahx_hmat_destroy(ahx_hmat* H) {
   H->scratch.release();
   H->dg_work.release();
   H->gm_word.release();
+  H->solve_work.release();
   H->z.release_all();
   if (H->own_stream && H->stream) cudaStreamDestroy(H->stream);
   delete H;

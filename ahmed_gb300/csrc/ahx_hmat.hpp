@@ -53,6 +53,24 @@ struct HostWord {
   void release();
 };
 
+// Device scratch of the solvers, kept between the solves of a handle (which run one after
+// another): allocating and freeing it took 0.7 ms of a GMRES call of 8.8 ms (16 systems of
+// 32,768 points).  What is larger than kKeep goes back after each solve (a basis of 50
+// vectors at 1,048,576 points and 64 right-hand sides is 27 GB).
+struct SolveWork {
+  static constexpr size_t kKeep = 256ull << 20;
+  DevBuf items, first, partial, small[3], len, gm;  // reductions, GMRES state
+  DevBuf v, r, rr, z;                               // basis, residuals, correction
+  void release() {
+    for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) b->release();
+  }
+  void trim() {
+    size_t s = 0;
+    for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) s += b->bytes;
+    if (s > kKeep) release();
+  }
+};
+
 // The product's view of one storage precision.
 struct ProdCopy {
   bool valid = false;
@@ -213,6 +231,7 @@ struct ahx_hmat {
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch
   ahx::HostWord gm_word;
+  ahx::SolveWork solve_work;
   // statistics of the last assembly
   uint64_t stat_ws_bytes = 0;   // largest ACA workspace batch (bytes)
   uint64_t stat_retries = 0;    // leaves re-run with a larger rank capacity

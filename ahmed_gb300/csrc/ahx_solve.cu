@@ -435,6 +435,7 @@ struct Operator {
   DevBuf seg_id;                  // ntot uint32 (only when nseg > 1)
   cudaStream_t stream = nullptr;
   HostWord* word = nullptr;       // what the device tells the host between steps
+  SolveWork* work = nullptr;      // device scratch of the solvers
   virtual ~Operator() { seg_id.release(); }
   // Y += d A X in storage precision prec
   virtual int apply(int prec, double d, uint32_t p, const double* X, double* Y) = 0;
@@ -469,6 +470,7 @@ struct HmatOp : Operator {
     seg_off = {0, ntot};
     stream = h->stream;
     word = &h->gm_word;
+    work = &h->solve_work;
   }
   int apply(int prec, double d, uint32_t p, const double* X, double* Y) override {
     return product_device(H, prec, d, p, X, ntot, Y, ntot);
@@ -493,7 +495,8 @@ class Solver {
  public:
   Solver(Operator& op, uint32_t p) : op_(op), p_(p) {}
   ~Solver() {
-    for (DevBuf* b : {&items_, &first_, &partial_, &small_, &small2_, &small3_, &len_, &gm_}) b->release();
+    if (idle_) work_.trim();
+    else work_.release();  // (waits for kernels that an error left in flight)
   }
 
   int init(uint32_t maxk) {
@@ -558,10 +561,13 @@ class Solver {
   const uint32_t* segid() const { return op_.nseg > 1 ? op_.seg_id.as<uint32_t>() : nullptr; }
 
   Operator& op_;
+  SolveWork& work_{*op_.work};
+  bool idle_ = false;  // set once nothing in flight uses the scratch
   uint32_t p_, nsys_ = 0, nitems_ = 0, maxk_ = 0;
   uint64_t total_ = 0;
-  DevBuf items_, first_, partial_, small_, small2_, small3_, len_;
-  DevBuf gm_;  // device GMRES state (GmDev arrays)
+  DevBuf &items_{work_.items}, &first_{work_.first}, &partial_{work_.partial}, &small_{work_.small[0]},
+      &small2_{work_.small[1]}, &small3_{work_.small[2]}, &len_{work_.len};
+  DevBuf& gm_{work_.gm};  // device GMRES state (GmDev arrays)
 };
 
 // CUDA graphs of GMRES steps: one executable graph per chunk of kGraphChunk
@@ -664,21 +670,24 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     AHX_CUDA(cudaStreamSynchronize(st));
     return AHX_OK;
   };
-  // normb
+  // normb, and whether x = 0
   if ((rc = sv.dots(B, 0, 1, B, d1))) return rc;
+  if ((rc = sv.dots(X, 0, 1, X, d1 + 1))) return rc;
   if ((rc = fetch(d1))) return rc;
   std::vector<double> normb(nsys);
   for (uint32_t q = 0; q < nsys; ++q) normb[q] = std::sqrt(hbuf[(size_t)q * K]);
   AHX_CUDA(cudaMemcpyAsync(g.normb, normb.data(), nsys * sizeof(double), cudaMemcpyHostToDevice, st));
   // r = b - A x (no product for a zero initial guess: r = b)
-  if ((rc = sv.dots(X, 0, 1, X, d1))) return rc;
-  if ((rc = fetch(d1))) return rc;
   bool x_zero = true;
-  for (uint32_t q = 0; q < nsys; ++q) x_zero = x_zero && hbuf[(size_t)q * K] == 0.0;
-  AHX_CUDA(cudaMemcpyAsync(r, B, total * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  if (!x_zero && (rc = op.apply(prec, -1.0, sv.p_, X, r))) return rc;
-  if ((rc = sv.dots(r, 0, 1, r, d1))) return rc;
-  if ((rc = fetch(d1))) return rc;
+  for (uint32_t q = 0; q < nsys; ++q) x_zero = x_zero && hbuf[(size_t)q * K + 1] == 0.0;
+  const double* r0 = B;
+  if (!x_zero) {
+    r0 = r;
+    AHX_CUDA(cudaMemcpyAsync(r, B, total * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    if ((rc = op.apply(prec, -1.0, sv.p_, X, r))) return rc;
+    if ((rc = sv.dots(r, 0, 1, r, d1))) return rc;
+    if ((rc = fetch(d1))) return rc;
+  }
   std::vector<double> beta(nsys);
   std::vector<double> zero_fix(nsys, 0.0);
   for (uint32_t q = 0; q < nsys; ++q) {
@@ -774,7 +783,7 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     // V_0 = r / beta; a cycle of at most m steps for the running systems
     for (uint32_t q = 0; q < nsys; ++q) hbuf[q] = done[q] ? 0.0 : beta[q] * beta[q];
     AHX_CUDA(cudaMemcpyAsync(d2, hbuf.data(), nsys * sizeof(double), cudaMemcpyHostToDevice, st));
-    scale_kernel<<<grid_for(total), 256, 0, st>>>(V, r, d2, 1, 1, total, op.ntot, sid, op.nseg);
+    scale_kernel<<<grid_for(total), 256, 0, st>>>(V, r0, d2, 1, 1, total, op.ntot, sid, op.nseg);
     std::fill(hbuf.begin(), hbuf.end(), 0.0);
     for (uint32_t q = 0; q < nsys; ++q) {
       hbuf[(size_t)q * K] = beta[q];
@@ -813,6 +822,7 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
     }
     if (!active_left() || j > maxit) break;
     // r = b - A x for the running systems
+    r0 = r;
     AHX_CUDA(cudaMemcpyAsync(r, B, total * sizeof(double), cudaMemcpyDeviceToDevice, st));
     if ((rc = op.apply(prec, -1.0, sv.p_, X, r))) return rc;
     if ((rc = sv.dots(r, 0, 1, r, d1))) return rc;
@@ -890,7 +900,7 @@ int gmres_driver(Operator& op, int prec, uint32_t p, const double* B, double* X,
   std::vector<uint32_t> iters(nsys, 0);
   std::vector<double> resid(nsys, 0.0);
   std::vector<char> done(nsys, 0);
-  DevBuf vbuf, rbuf, rr, z;
+  DevBuf &vbuf = op.work->v, &rbuf = op.work->r, &rr = op.work->rr, &z = op.work->z;
   GmresGraphs graphs[kNumPrecisions];  // per operator precision
   if (prec == kFP64 || prec == kDF64) {
     rc = gmres_core(sv, kFP64, B, X, tol, m, maxit, iters, resid, done, vbuf, rbuf, &graphs[kFP64]);
@@ -910,6 +920,7 @@ int gmres_driver(Operator& op, int prec, uint32_t p, const double* B, double* X,
     const double inner_tol = prec == kFP32 ? 1e-6 : 1e-3;
     std::vector<double> normb(nsys), nb((size_t)nsys * sv.maxk_);
     if ((rc = sv.dots(B, 0, 1, B, sv.small_.as<double>()))) return rc;
+    if ((rc = sv.dots(X, 0, 1, X, sv.small_.as<double>() + 1))) return rc;
     AHX_CUDA(cudaMemcpyAsync(nb.data(), sv.small_.p, nb.size() * 8, cudaMemcpyDeviceToHost, st));
     AHX_CUDA(cudaStreamSynchronize(st));
     for (uint32_t q = 0; q < nsys; ++q) normb[q] = std::sqrt(nb[(size_t)q * sv.maxk_]);
@@ -921,22 +932,21 @@ int gmres_driver(Operator& op, int prec, uint32_t p, const double* B, double* X,
     int inner_prec = prec;
     bool undone = false;  // the residual just recomputed follows an undo: accept it
     std::vector<double> prev(nsys, INFINITY), undo(nsys, 0.0);
-    // a zero initial guess needs no product for the first residual
-    if ((rc = sv.dots(X, 0, 1, X, sv.small_.as<double>()))) return rc;
-    AHX_CUDA(cudaMemcpyAsync(nb.data(), sv.small_.p, nb.size() * 8, cudaMemcpyDeviceToHost, st));
-    AHX_CUDA(cudaStreamSynchronize(st));
+    // a zero initial guess needs no product for the first residual, b (its sums are in nb)
     bool x_zero = true;
-    for (uint32_t q = 0; q < nsys; ++q) x_zero = x_zero && nb[(size_t)q * sv.maxk_] == 0.0;
+    for (uint32_t q = 0; q < nsys; ++q) x_zero = x_zero && nb[(size_t)q * sv.maxk_ + 1] == 0.0;
     StepTrace trace(st);
     int outer = 0;
     for (;;) {
       trace.mark(0);
       AHX_CUDA(cudaMemcpyAsync(rr.p, B, total * 8, cudaMemcpyDeviceToDevice, st));
-      if (!x_zero && (rc = op.apply(resid_prec, -1.0, p, X, rr.as<double>()))) return rc;
+      if (!x_zero) {
+        if ((rc = op.apply(resid_prec, -1.0, p, X, rr.as<double>()))) return rc;
+        if ((rc = sv.dots(rr.as<double>(), 0, 1, rr.as<double>(), sv.small_.as<double>()))) return rc;
+        AHX_CUDA(cudaMemcpyAsync(nb.data(), sv.small_.p, nb.size() * 8, cudaMemcpyDeviceToHost, st));
+      }
       x_zero = false;
-      if ((rc = sv.dots(rr.as<double>(), 0, 1, rr.as<double>(), sv.small_.as<double>()))) return rc;
       trace.mark(1);
-      AHX_CUDA(cudaMemcpyAsync(nb.data(), sv.small_.p, nb.size() * 8, cudaMemcpyDeviceToHost, st));
       AHX_CUDA(cudaStreamSynchronize(st));
       bool worse = false;
       for (uint32_t q = 0; q < nsys; ++q) {
@@ -1014,11 +1024,8 @@ int gmres_driver(Operator& op, int prec, uint32_t p, const double* B, double* X,
       AHX_CUDA(cudaGetLastError());
     }
   }
-  vbuf.release();
-  rbuf.release();
-  rr.release();
-  z.release();
   if (rc) return rc;
+  sv.idle_ = true;
   status = AHX_OK;
   for (uint32_t q = 0; q < nsys; ++q) {
     if (!done[q]) status = AHX_NOT_CONVERGED;
@@ -1153,6 +1160,7 @@ struct ahx_batch : ahx::Operator {
   } tab[ahx::kNumPrecisions];
   ahx::DevBuf stx, sty;
   ahx::HostWord steps;
+  ahx::SolveWork solve_work;
 
   // FP64: concatenated leaf table and arena; mixed precisions: streams built
   // from the concatenated FP64 arena.
@@ -1451,6 +1459,7 @@ int ahx_batch_destroy(ahx_batch* b) {
   b->stx.release();
   b->sty.release();
   b->steps.release();
+  b->solve_work.release();
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   b->stream = nullptr;
   delete b;
@@ -1503,6 +1512,7 @@ int ahx_batch_gmres(ahx_batch* b, const double* B, double* X, double tol, uint32
   double* Xd = const_cast<double*>(Xc);
   int status = AHX_OK;
   b->word = &b->steps;
+  b->work = &b->solve_work;
   rc = gmres_driver(*b, b->prec, 1, Bd, Xd, tol, m, maxit, iters, resid, status);
   if (rc) return rc;
   if (Xd != X) AHX_CUDA(cudaMemcpyAsync(X, Xd, n * 8, cudaMemcpyDefault, b->stream));

@@ -39,3 +39,32 @@ def test_a_cycle_minimises_the_residual(m, p):
         # times the condition of the projected matrix, below 1e5)
         assert abs(got - best) <= 1e-8 * best
     H.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_solves_share_a_handles_scratch(precision):
+    """Solves of other sizes in turn, from zero and from a given x, equal those of a handle
+    of their own."""
+    n = 2111
+    pts = A.geometry.sphere_surface(n, 4)
+    g = np.random.default_rng(0)
+
+    def handle():
+        H = A.HMatrix(pts, "bbx")
+        H.matgenGeH_omp(A.min_nn(pts) / 2, 1e-6)  # positive definite, condition below 10
+        return H
+
+    kept = handle()
+    for p, m, steps, zero in ((1, 30, 60, True), (3, 5, 40, False), (1, 50, 50, False), (2, 30, 60, True), (1, 2, 3, True)):
+        B = g.standard_normal((p, n))
+        X = np.zeros((p, n)) if zero else g.standard_normal((p, n))
+        Y = X.copy()
+        own = handle()
+        s1 = kept.GMRes(B, X, 1e-8, m, steps, precision)
+        s2 = own.GMRes(B, Y, 1e-8, m, steps, precision)
+        own.close()
+        assert s1[0] == s2[0] and (s1[2] == s2[2]).all()
+        # products add with atomics, in another order each time: rounding (FP32-class products
+        # 1e-6 of the result) times the condition
+        assert np.linalg.norm(X - Y) <= (1e-9 if precision == "fp64" else 1e-5) * np.linalg.norm(Y)
+    kept.close()
