@@ -36,7 +36,7 @@
 //
 // What bounds it: the ALU work of cutting (about 30 integer operations per
 // element; ALU pipe 53%, issue 48%, tensor pipe 22% to 31% busy at 32,768 points).
-// 65,536 points (2.09 GB): 8.35 -> 1.41 ms with 16 right-hand sides, 4.21 -> 0.99
+// 65,536 points (2.09 GB): 8.35 -> 1.35 ms with 16 right-hand sides, 4.21 -> 0.99
 // ms with 8 (2.1 TB/s); 8,300 us of it were the FP64 pipe.
 #include <algorithm>
 #include <cstdlib>
@@ -598,26 +598,45 @@ __global__ void dg_xprep_kernel(const double* __restrict__ X, uint64_t ldX, uint
   if (bad) atomicOr(flag, 1);
 }
 
+// T rows: a lane per column pair (a complex T entry), so that a row is read and each of
+// its digit planes written by consecutive lanes; a thread per row left every access of a
+// warp in 32 places (65,536 points, 16 right-hand sides: 81 -> 24 us).
 template <int NT, int CW>
-__global__ void dg_tprep_kernel(const double* __restrict__ T, uint32_t t_rows, uint32_t pc,
-                                unsigned char* __restrict__ z, int* __restrict__ flag) {
-  constexpr int NP = 8 * NT;
-  const uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (q >= (uint64_t)t_rows * CW) return;
-  const uint64_t i = q / CW;
-  const uint32_t e = (uint32_t)(q % CW);
-  const double* t = T + i * NP;
+__global__ void __launch_bounds__(128) dg_tprep_kernel(const double* __restrict__ T, uint32_t t_rows, uint32_t pc,
+                                                       unsigned char* __restrict__ z, int* __restrict__ flag) {
+  constexpr uint32_t kL = 4 * NT;
+  const uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, q = id / kL;
+  const uint32_t l = (uint32_t)(id % kL), col = 2 * l;
+  const bool live = q < (uint64_t)t_rows * CW;
+  double v[2] = {0.0, 0.0};
+  if (live && col < pc) {
+    const double2 t = __ldg(reinterpret_cast<const double2*>(T + q / CW * (8 * NT) + col));
+    v[0] = CW == 2 && (q & 1) ? -t.y : t.x;
+    v[1] = CW == 2 ? (q & 1 ? t.x : t.y) : col + 1 < pc ? t.y : 0.0;
+  }
+  int m = kZeroZ, ex[2];
   bool bad = false;
-  auto val = [&](int col, int& sc) -> double {
-    sc = 1022;
-    double v;
-    if (CW == 1 || e == 0) v = t[col];
-    else v = (col & 1) ? t[col - 1] : -t[col + 1];
-    bad = bad || (((uint32_t)__double2hiint(v) >> 20) & 0x7ffu) == 0x7ffu || subnormal(v);
-    return v;
-  };
-  z_row<NT>(z + q * (kPR<NT> * 16), val, pc, flag);
-  if (bad) atomicOr(flag, 1);
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    ex[w] = ((uint32_t)__double2hiint(v[w]) >> 20) & 0x7ffu;
+    bad = bad || ex[w] == 0x7ff || subnormal(v[w]);
+    if (ex[w]) m = max(m, ex[w] - 1022);
+  }
+#pragma unroll
+  for (uint32_t o = 1; o < kL; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (!live) return;
+  Dig f[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+    f[w] = fix_f64((uint32_t)__double2hiint(v[w]), (uint32_t)__double2loint(v[w]),
+                   ex[w] ? (uint32_t)(m - (ex[w] - 1022)) : 64u);
+  uint32_t d[S];
+  digits(f[0], f[1], d);
+  unsigned char* zq = z + q * (kPR<NT> * 16);
+#pragma unroll
+  for (int k = 0; k < S; ++k) *reinterpret_cast<uint32_t*>(zq + k * NT * 16 + l * 4) = d[k];
+  if (l == 0) *reinterpret_cast<uint4*>(zq + S * NT * 16) = make_uint4((uint32_t)(m * (1 << 20)), 0u, 0u, 0u);
+  if (bad || (m != kZeroZ && (m < kZMin || m > kZMax))) atomicOr(flag, 1);
 }
 
 __global__ void dg_expand_kernel(const DgSeg* __restrict__ segs, uint32_t nsegs, DgPos* __restrict__ pos) {
@@ -703,7 +722,7 @@ cudaError_t run_pass(const DgPlan& pl, const DgArgs& a, const Work& w, uint32_t 
     if (pl.t_split && (e = cudaMemsetAsync(T, 0, (size_t)pl.t_split * NT * 64, s)) != cudaSuccess) return e;
     k.pieces = pl.vpieces;
     if ((e = sweep<NT, CW, false, false>(k, pl.nv, s)) != cudaSuccess) return e;
-    dg_tprep_kernel<NT, CW><<<(unsigned)((tr + 127) / 128), 128, 0, s>>>(T, pl.t_rows, pc,
+    dg_tprep_kernel<NT, CW><<<(unsigned)((tr * (4 * NT) + 127) / 128), 128, 0, s>>>(T, pl.t_rows, pc,
                                                                             z + xr * (kPR<NT> * 16), flag);
     count_product_launches(1);
   }
