@@ -10,8 +10,12 @@ namespace {
 
 // A leaf goes to a CTA instead of a warp when its rows and columns are more than half of
 // what a resident warp gets on average (a warp that takes longer ends after the others),
-// but never below 512, where the work on the k x k arrays (one warp, the others wait)
-// outweighs the rows.  A leaf's k x k work counts as 256 rows.
+// or when half the workspace budget would not hold a slot for every resident warp; but
+// never below 512, where the work on the k x k arrays (one warp, the others wait)
+// outweighs the rows.  A leaf's k x k work counts as 256 rows.  Where the budget does not
+// hold slots for half of the resident CTAs either, the leaves too large for that run first,
+// alone and in all of the budget.  (1,048,576 points, 440,940 leaves: with the first rule
+// only, 130 warps at a time, the assembly took 7.6 s; so 0.90 s; 262,144 points 0.35 -> 0.12 s.)
 constexpr uint64_t kLeafRows = 256, kLargeMin = 512;
 
 uint64_t class_bytes(uint32_t c) {  // an upper bound of the class, a multiple of 256
@@ -19,20 +23,44 @@ uint64_t class_bytes(uint32_t c) {  // an upper bound of the class, a multiple o
   return (top + 255) & ~255ull;
 }
 
-// tasks by descending class of their workspace; cls: the classes
-void sort_descending(std::vector<AcaTask>& t, std::vector<uint32_t>& cls, size_t elem) {
-  std::vector<uint64_t> size(t.size());
-  for (size_t i = 0; i < t.size(); ++i) size[i] = aca_ws_bytes(t[i].n1, t[i].n2, t[i].kcap, elem);
-  std::vector<uint32_t> ord;
-  order_by_size(size, ord);
-  std::vector<AcaTask> out(t.size());
-  cls.resize(t.size());
-  for (size_t i = 0; i < t.size(); ++i) {
-    out[i] = t[ord[i]];
-    cls[i] = size_class(size[ord[i]]);
+// A set of tasks in descending class of their workspace, with the classes' bytes
+struct Sorted {
+  std::vector<AcaTask> t;
+  std::vector<uint64_t> bytes;
+  Sorted() = default;
+  Sorted(const std::vector<AcaTask>& in, size_t elem) : t(in.size()), bytes(in.size()) {
+    std::vector<uint64_t> size(in.size());
+    for (size_t i = 0; i < in.size(); ++i) size[i] = aca_ws_bytes(in[i].n1, in[i].n2, in[i].kcap, elem);
+    std::vector<uint32_t> ord;
+    order_by_size(size, ord);
+    for (size_t i = 0; i < in.size(); ++i) {
+      t[i] = in[ord[i]];
+      bytes[i] = class_bytes(size_class(size[ord[i]]));
+    }
   }
-  t.swap(out);
-}
+  // slots for the first tasks from `at` on: at most n, one at least, within `room` bytes
+  uint32_t slots(size_t at, uint64_t n, uint64_t room) const {
+    n = std::min<uint64_t>(n, t.size() - at);
+    uint64_t part = 0;
+    uint32_t k = 0;
+    for (; k < n; ++k) {
+      part += bytes[at + k];
+      if (k && part > room) break;
+    }
+    return k;
+  }
+  // the first task from which on n slots (or as many as tasks are left) fit into `room` bytes
+  size_t fits(uint64_t n, uint64_t room) const {
+    uint64_t part = 0;
+    size_t i = 0, j = 0;
+    for (; i < t.size(); ++i) {
+      for (; j < t.size() && j < i + n; ++j) part += bytes[j];
+      if (part <= room) break;
+      part -= bytes[i];
+    }
+    return i;
+  }
+};
 
 }  // namespace
 
@@ -96,36 +124,47 @@ int run_aca(ahx_hmat* H, bool cplx, std::vector<AcaTask>& tasks, AcaParams p, st
     uint64_t rows = 0;
     for (const AcaTask& t : tasks) rows += (uint64_t)t.n1 + t.n2 + kLeafRows;
     const uint64_t lim = std::max<uint64_t>(kLargeMin, rows / ((uint64_t)ctas * kWarps * 2));
-    std::vector<AcaTask> large, small;
-    for (const AcaTask& t : tasks) ((uint64_t)t.n1 + t.n2 > lim ? large : small).push_back(t);
-    std::vector<uint32_t> cl, cs;
-    sort_descending(large, cl, elem);
-    sort_descending(small, cs, elem);
-    // slots: each phase takes at most half the budget, and at least one team runs
-    std::vector<uint64_t> slots;
-    uint64_t bytes = 0, part = 0;
-    p.nlarge = (uint32_t)large.size();
-    p.nsmall = (uint32_t)small.size();
-    p.nslot_l = p.nslot_s = 0;
-    for (; p.nslot_l < std::min(ctas, p.nlarge); ++p.nslot_l) {
-      const uint64_t b = class_bytes(cl[p.nslot_l]);
-      if (p.nslot_l && part + b > budget / 2) break;
-      slots.push_back(bytes);
-      bytes += b;
-      part += b;
+    const Sorted all_tasks(tasks, elem);
+    const size_t cut = all_tasks.fits((uint64_t)ctas * kWarps, budget / 2);
+    Sorted large, small;
+    small.t.reserve(tasks.size());
+    small.bytes.reserve(tasks.size());
+    for (size_t i = 0; i < all_tasks.t.size(); ++i) {
+      const uint64_t n = (uint64_t)all_tasks.t[i].n1 + all_tasks.t[i].n2;
+      Sorted& to = n > kLargeMin && (n > lim || i < cut) ? large : small;
+      to.t.push_back(all_tasks.t[i]);
+      to.bytes.push_back(all_tasks.bytes[i]);
     }
-    part = 0;
-    for (; p.nslot_s < std::min(ctas * kWarps, p.nsmall); ++p.nslot_s) {
-      const uint64_t b = class_bytes(cs[p.nslot_s]);
-      if (p.nslot_s && part + b > budget / 2) break;
+    // the largest leaves in a launch of their own?
+    std::vector<AcaTask> later;
+    const uint32_t ns = large.slots(0, ctas, budget / 2);
+    uint64_t room = budget / 2;
+    if (2 * (uint64_t)ns < std::min<uint64_t>(ctas, large.t.size())) {
+      const size_t first = large.fits(ctas, budget / 2);
+      if (first >= 2 * (size_t)ns) {
+        later.assign(large.t.begin() + (std::ptrdiff_t)first, large.t.end());
+        later.insert(later.end(), small.t.begin(), small.t.end());
+        large.t.resize(first);
+        large.bytes.resize(first);
+        small = Sorted();
+        room = budget;
+      }
+    }
+    // slots: each phase takes at most half the budget, and at least one team runs
+    p.nlarge = (uint32_t)large.t.size();
+    p.nsmall = (uint32_t)small.t.size();
+    p.nslot_l = large.slots(0, ctas, room);
+    p.nslot_s = small.slots(0, (uint64_t)ctas * kWarps, budget / 2);
+    std::vector<uint64_t> slots;
+    uint64_t bytes = 0;
+    for (uint32_t i = 0; i < p.nslot_l + p.nslot_s; ++i) {
       slots.push_back(bytes);
-      bytes += b;
-      part += b;
+      bytes += i < p.nslot_l ? large.bytes[i] : small.bytes[i - p.nslot_l];
     }
     H->stat_ws_bytes = std::max<uint64_t>(H->stat_ws_bytes, bytes);
     H->stat_batches++;
-    std::vector<AcaTask> all(std::move(large));
-    all.insert(all.end(), small.begin(), small.end());
+    std::vector<AcaTask> all(std::move(large.t));
+    all.insert(all.end(), small.t.begin(), small.t.end());
     struct Ctl {
       unsigned long long used;
       uint32_t ctr[2];
@@ -181,6 +220,7 @@ int run_aca(ahx_hmat* H, bool cplx, std::vector<AcaTask>& tasks, AcaParams p, st
       if ((rc = cplx ? zarena_append(H, more, off) : arena_append(H, more, off))) return rc;
       elems = off;
     }
+    retry.insert(retry.end(), later.begin(), later.end());
     tasks.swap(retry);
   }
   return AHX_OK;

@@ -2,7 +2,7 @@
 // (ahx_dg.cuh): Y += d op(A) X, op = A, A^T (mltaGeHVec / mltaGeHtVec,
 // H/mltaGeHVec.cpp:16-150), with plain FP64 multiply-adds.
 //
-// Two sweeps, a CTA of 96 threads per piece (<= 48 rows over a range of K):
+// Two sweeps, a CTA of 192 threads per piece (<= 48 rows over a range of K):
 //   V sweep     T = Q^T X: a lane quad per factor column reads 32 consecutive bytes of it,
 //               eight columns a warp load, two of them per lane
 //   rows sweep  Y += P T + D X: a thread per row and K slice, neighbouring rows of a column
@@ -12,7 +12,7 @@
 // 65,536 points at two lanes a clock and SM, above their memory time (307 us); the rows
 // sweep keeps the pipe 87 % busy, the V sweep 70 %.  The plain kernel (ahx_matvec.cu: a
 // CTA per leaf) reads its factors in a chain of dependent steps and half fills its
-// warps.  A x, 65,536 points: 628 -> 524 us; 10,007: 128 -> 92; 4,096: 65 -> 40 us.
+// warps.  A x, 65,536 points: 628 -> 524 us; 10,007: 128 -> 92; 4,096: 65 -> 39 us.
 #include <algorithm>
 #include <cstdlib>
 

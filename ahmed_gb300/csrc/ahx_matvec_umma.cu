@@ -4,7 +4,7 @@
 //
 // One persistent CTA per SM, 20 warps with fixed roles:
 //   warp 0      producer: walks the CTA's contiguous range of tiles (ranges
-//               balanced by bytes; descriptors fetched 32 at a time) and
+//               balanced by cycles; descriptors fetched 32 at a time) and
 //               bulk-copies (cp.async.bulk) each chunk image into one of
 //               kSlots ring slots
 //   warp 1      MMA issuer (one thread) and owner of the tensor memory: per

@@ -119,3 +119,40 @@ def test_columns_of_u_are_orthogonal(n, bmin, eta, eps, cplx):
         G = np.abs(U.conj().T @ U) / np.outer(s, s) - np.eye(k)
         assert np.abs(G).max() <= 1e-6, (l, n1, k)
     H.close()
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("budget,batches", [(1 << 22, 2), (1 << 26, 1), (1 << 33, 1)])
+def test_workspace_budgets(budget, batches, cplx, monkeypatch):
+    """The largest leaves in a launch of their own (4 MB hold slots for few of them), leaves
+    moved from warps to CTAs for want of slots, and neither."""
+    import ctypes
+
+    from ahmed_gb300._capi import lib
+    monkeypatch.setenv("AHX_ACA_WS_BYTES", str(budget))
+    n = 9001
+    pts = _points(n, 11)
+    H = A.HMatrix(pts, "bbx", bmin=16)
+    h = A.mean_nn(pts)
+    if cplx:
+        H.helmholtz_assemble(3.0, h, 1e-6)
+        ranks, data = H.helm_ranks(), H.helm_leaf_data
+    else:
+        H.matgenGeH_omp(h, 1e-6)
+        ranks, data = H.ranks(), H.leaf_data
+    stats = (ctypes.c_uint64 * 3)()
+    lib().ahx_hmat_assembly_stats(H._h, stats)
+    assert stats[0] <= budget and stats[2] == batches and stats[1] == 0
+    Q = pts[H.perm()[0]]
+    lv = H.leaves()
+    low = np.nonzero(lv[:, 4] == 1)[0]
+    assert (ranks[low] > 0).all()
+    size = lv[low, 1] + lv[low, 3]
+    for l in np.concatenate([low[np.argsort(size)[-6:]], low[:: len(low) // 40]]):
+        b1, n1, b2, n2 = (int(v) for v in lv[l, :4])
+        r = np.linalg.norm(Q[b1:b1 + n1, None] - Q[None, b2:b2 + n2], axis=2)
+        B = (np.exp(3j * r) if cplx else 1.0) / (4 * np.pi * r)
+        k, d = int(ranks[l]), data(int(l))
+        U, V = d[:n1 * k].reshape(k, n1).T, d[n1 * k:].reshape(k, n2).T
+        assert np.linalg.norm(U @ V.conj().T - B) <= 20 * 1e-6 * np.linalg.norm(B)
+    H.close()
