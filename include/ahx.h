@@ -304,9 +304,9 @@ int ahx_mlp_predict(ahx_mlp* M, const float* X, uint32_t n, float* out);
  * caching allocator holds the device memory, paths that cannot afford the
  * device synchronisation of cudaMalloc/cudaFree, and hosts that own every
  * device allocation and only lend buffers.  The scratch comes from a fixed
- * 8 MiB array inside the library (present on every GPU that loads it, until
- * exit); with c = kmax + 1 ACA columns (the reference's capacity) a block needs
- * 256 + 8*(2*(n1+n2)*c + 2*c^2 + 3*c) + 4*(n1+n2) bytes; larger requests, and
+ * 11 MiB array inside the library (present on every GPU that loads it, until
+ * exit); with c = kmax + 1 ACA columns (the reference's capacity) a block may need
+ * 256 + 8*(2*(n1+n2)*c + 2*c^2 + 3*c) + 4*(n1+n2) <= 8 MiB; larger requests, and
  * n1 or n2 above 2^20 or kmax above 2^16, return AHX_ERR_ARG.
  * Inputs (device): px/py/pz = point coordinates in permuted order; the block
  * is rows b1..b1+n1-1, columns b2..b2+n2-1, ACA start row i0 (< n1), kernel
