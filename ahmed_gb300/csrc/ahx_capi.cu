@@ -509,6 +509,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     set_error("transposed products use the FP64 leaves");
     return AHX_ERR_ARG;
   }
+  std::lock_guard<std::mutex> lk(H->product_mu);
   int rc;
   if (prec == kFP32 && p >= 2 && um_enabled()) {
     // FP32 leaves, several right-hand sides: the tcgen05 sweeps

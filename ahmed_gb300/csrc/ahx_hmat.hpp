@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/ahx.h"
@@ -54,13 +55,14 @@ struct HostWord {
 };
 
 // Device scratch of the solvers, kept between the solves of a handle (which run one after
-// another): allocating and freeing it took 0.7 ms of a GMRES call of 8.8 ms (16 systems of
+// another, from several threads too): allocating and freeing it took 0.7 ms of a GMRES call of 8.8 ms (16 systems of
 // 32,768 points).  What is larger than kKeep goes back after each solve (a basis of 50
 // vectors at 1,048,576 points and 64 right-hand sides is 27 GB).
 struct SolveWork {
   static constexpr size_t kKeep = 256ull << 20;
   DevBuf items, first, partial, small[3], len, gm;  // reductions, GMRES state
   DevBuf v, r, rr, z;                               // basis, residuals, correction
+  std::mutex mu;                                    // held by the solve that uses them
   void release() {
     for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) b->release();
   }
@@ -227,6 +229,9 @@ struct ahx_hmat {
   ahx::DgState dg[2];     // digit-sliced FP64 products: A, A^T
   int finite = 0;         // FP64 leaf elements: 0 not looked at, 1 fit for digits, 2 not
   ahx::DevBuf dg_work;    // their work buffer (real and complex)
+  // held while a product's kernels are queued: they share work buffers in stream order, so
+  // that products from several threads must not interleave (the plain kernels need no buffer)
+  std::mutex product_mu;
   // staging buffers for host vectors
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch

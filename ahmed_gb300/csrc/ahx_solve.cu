@@ -477,6 +477,7 @@ struct HmatOp : Operator {
   }
   uint64_t product_bytes(int prec) const override { return H->prod[prec].bytes; }
   int prepare(int prec, uint32_t p) override {
+    std::lock_guard<std::mutex> lk(H->product_mu);
     int rc;
     if (((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) ||
         (prec == kFP64 && p == 1 && f1_wanted(H->arena64_elems, false))) {
@@ -493,7 +494,7 @@ struct HmatOp : Operator {
 // Reduction plan + device scratch for a family of systems.
 class Solver {
  public:
-  Solver(Operator& op, uint32_t p) : op_(op), p_(p) {}
+  Solver(Operator& op, uint32_t p) : lock_(op.work->mu), op_(op), p_(p) {}
   ~Solver() {
     if (idle_) work_.trim();
     else work_.release();  // (waits for kernels that an error left in flight)
@@ -560,6 +561,7 @@ class Solver {
 
   const uint32_t* segid() const { return op_.nseg > 1 ? op_.seg_id.as<uint32_t>() : nullptr; }
 
+  std::unique_lock<std::mutex> lock_;
   Operator& op_;
   SolveWork& work_{*op_.work};
   bool idle_ = false;  // set once nothing in flight uses the scratch

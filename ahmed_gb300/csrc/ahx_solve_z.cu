@@ -340,8 +340,8 @@ int zgmres_one(ahx_hmat* H, int prec, const ZGm& g, const double2* b, double2* x
 
 }  // namespace
 
-int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
-                    uint64_t ldX, double2* Y, uint64_t ldY) {
+static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
+                           uint64_t ldX, double2* Y, uint64_t ldY) {
   int rc = prepare_z(H, prec);
   if (rc) return rc;
   ZState& Z = H->z;
@@ -354,7 +354,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     zconj_kernel<<<grid, 256, 0, H->stream>>>(X, ldX, Xc, n, n, p);
     zconj_kernel<<<grid, 256, 0, H->stream>>>(Y, ldY, Y, ldY, n, p);
     AHX_CUDA(cudaGetLastError());
-    if ((rc = zproduct_device(H, prec, kZOpN, dre, -dim, p, Xc, n, Y, ldY))) return rc;
+    if ((rc = zproduct_locked(H, prec, kZOpN, dre, -dim, p, Xc, n, Y, ldY))) return rc;
     zconj_kernel<<<grid, 256, 0, H->stream>>>(Y, ldY, Y, ldY, n, p);
     AHX_CUDA(cudaGetLastError());
     return AHX_OK;
@@ -435,6 +435,12 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     AHX_CUDA(launch_matvec_z(a, H->stream));
   }
   return AHX_OK;
+}
+
+int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
+                    uint64_t ldX, double2* Y, uint64_t ldY) {
+  std::lock_guard<std::mutex> lk(H->product_mu);
+  return zproduct_locked(H, prec, op, dre, dim, p, X, ldX, Y, ldY);
 }
 
 }  // namespace ahx
