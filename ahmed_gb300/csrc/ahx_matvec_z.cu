@@ -218,8 +218,15 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
   }
 }
 
+// CTAs an SM that the compiler is to leave registers for (0: its own choice).  Of its own it
+// takes 32 registers in these two, which costs loads in flight or spills: complex128 with one
+// right-hand side (9,000 points on a cube 296 us, with 48 registers 259; 40,000 on a sphere
+// the same) and complex64 A x with two (110 and 83 us; 16,000 on a sphere 130 and 136, which
+// is latency hidden by more CTAs).
+template <typename S, int PG, int OP>
+constexpr int kMinCtas = (sizeof(S) == 16 && PG == 1) || (sizeof(S) == 8 && PG == 2 && OP == kZOpN) ? 10 : 0;
 template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE = false>
-__global__ void __launch_bounds__(kThreads) zmv_kernel(ZArgs a) {
+__global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(ZArgs a) {
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
