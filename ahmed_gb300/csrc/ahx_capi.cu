@@ -539,7 +539,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
       const DgPlan pl = dg_plan(H->dg[transposed ? 1 : 0], H->tree.n, H->arena64.p, H->dg_work);
       const DgArgs da{false, d, 0.0, p, X, ldX, Y, ldY};
       AHX_CUDA(launch_matvec_dg(pl, da, H->stream));
-      guard = dg_flag(pl);
+      guard = dg_flags(pl);
       prec = kFP64;
     }
   }
@@ -571,6 +571,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   a.ldY = ldY;
   a.transposed = transposed ? 1u : 0u;
   a.guard = guard;
+  a.guard_cols = dg_pass_cols(false);
   AHX_CUDA(launch_matvec(prec, a, H->stream));
   if (pc.ntleaves) {
     // symmetric tree: the blocks below the diagonal are the upper ones transposed

@@ -102,11 +102,14 @@ struct DgArgs {
   uint64_t ldY;
 };
 
-// Bytes of the work buffer for p right-hand sides.  dg_flag: the word that is
-// non-zero after a product whose X (or V^T X) does not fit the digits (not finite,
-// or entries spread over more than 2^200), in which case Y was left as it was.
+// Bytes of the work buffer for p right-hand sides.  dg_flags: a word per pass of
+// dg_pass_cols right-hand sides, non-zero after a product in which those columns of X (or
+// of V^T X) do not fit the digits: an entry is not finite, the largest entry of a row is
+// below 2^-200 of its column's largest, or a column is subnormal.  Their columns of Y were
+// then left as they were.
 size_t dg_work_bytes(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p);
-inline const int* dg_flag(const DgPlan& pl) { return reinterpret_cast<const int*>(pl.work); }
+constexpr uint32_t dg_pass_cols(bool cplx) { return cplx ? 8u : 16u; }
+inline const int* dg_flags(const DgPlan& pl) { return reinterpret_cast<const int*>(pl.work); }
 
 cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cudaStream_t s);
 // *bad |= any of the count doubles is not finite, or not zero and outside [2^-500, 2^500]

@@ -46,7 +46,7 @@ __device__ __forceinline__ void stage_x(A (*Xs)[PG + 1], const MvArgs& a, uint32
 // leaves, H/mltaGeHVec.cpp:62-150): a low-rank leaf U V^T acts as V U^T (the
 // roles of the factors and of the row / column ranges swap); a dense leaf D
 // acts as D^T, one warp per column of D.
-template <typename SL, typename SD, typename A, int PG, bool TR>
+template <typename SL, typename SD, typename A, int PG, bool TR, bool GUARD>
 __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[PG + 1], A (*Ts)[PG], A* red) {
   MvLeaf L = a.leaves[a.order[leaf]];
   const uint32_t tid = threadIdx.x;
@@ -69,6 +69,7 @@ __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[
     const SD* Ad = L.dense_in_lr_arena ? reinterpret_cast<const SD*>(reinterpret_cast<const SL*>(a.arena_lr) + L.off)
                                        : reinterpret_cast<const SD*>(a.arena_dn) + L.off;
     for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
+      if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
       const uint32_t pg = min((uint32_t)PG, a.p - r0);
       for (uint32_t jb = 0; jb < L.n2; jb += kThreads) {
         const uint32_t j = jb + tid;
@@ -99,6 +100,7 @@ __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[
     return;
   }
   for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
+    if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
     const uint32_t pg = min((uint32_t)PG, a.p - r0);
     if (L.rank < 0) {
       const SD* Ad = L.dense_in_lr_arena ? reinterpret_cast<const SD*>(
@@ -215,10 +217,12 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
   __shared__ A Ts[kKt][PG];
   __shared__ A red[kThreads];
   if (GUARD) {
-    if (*a.guard == 0) return;
-    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) mv_leaf<SL, SD, A, PG, TR>(a, l, Xs, Ts, red);
+    bool any = false;
+    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q];
+    if (!__syncthreads_or(any)) return;
+    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) mv_leaf<SL, SD, A, PG, TR, true>(a, l, Xs, Ts, red);
   } else {
-    mv_leaf<SL, SD, A, PG, TR>(a, blockIdx.x, Xs, Ts, red);
+    mv_leaf<SL, SD, A, PG, TR, false>(a, blockIdx.x, Xs, Ts, red);
   }
 }
 

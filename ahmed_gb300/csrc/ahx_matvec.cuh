@@ -39,8 +39,10 @@ struct MvArgs {
   double* Y;
   uint64_t ldY;
   uint32_t transposed = 0;  // 1: Y += d A^T X (H/mltaGeHVec.cpp:62-150)
-  // when set: the product runs only if *guard is not zero (few CTAs, a leaf loop)
+  // when set: right-hand side r takes part only if guard[r / guard_cols] is not zero (few
+  // CTAs, a leaf loop; guard_cols a multiple of 8)
   const int* guard = nullptr;
+  uint32_t guard_cols = 0;
 };
 
 cudaError_t launch_matvec(int prec, const MvArgs& a, cudaStream_t s);
@@ -83,6 +85,7 @@ struct ZArgs {
   uint64_t ldY;
   int op;
   const int* guard = nullptr;  // as MvArgs::guard; complex128 leaves only
+  uint32_t guard_cols = 0;
   uint64_t elems = 0;          // complex64 leaves: elements,
   uint32_t n = 0;              //   rows of X,
   float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes),

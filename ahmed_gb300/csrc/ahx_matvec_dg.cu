@@ -501,20 +501,21 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 5 : 4) dg_sweep_kernel(con
 
 // ---- Z rows --------------------------------------------------------------
 
-// exponent field of the largest |X_r| per column (complex: of both parts), and
-// the flag of a value that is not finite
+// exponent field of the largest |X_r| per column r = r0 + blockIdx.y (complex: of both
+// parts), and the flag of its pass for a value that is not finite
 template <int CW>
-__global__ void dg_xmax_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, int* __restrict__ xmax,
-                               int* __restrict__ flag) {
-  const double* x = X + (uint64_t)blockIdx.y * ldX * CW;
+__global__ void dg_xmax_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t r0,
+                               int* __restrict__ xmax, int* __restrict__ flags) {
+  const uint32_t col = r0 + blockIdx.y;
+  const double* x = X + (uint64_t)col * ldX * CW;
   uint32_t m = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)n * CW;
        i += (uint64_t)gridDim.x * blockDim.x)
     m = max(m, ((uint32_t)__double2hiint(x[i]) >> 20) & 0x7ffu);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(xmax + blockIdx.y, (int)m);
-    if (m == 0x7ffu) atomicOr(flag, 1);
+    atomicMax(xmax + col, (int)m);
+    if (m == 0x7ffu) atomicOr(flags + col / dg_pass_cols(CW == 2), 1);
   }
 }
 
@@ -659,19 +660,20 @@ __global__ void dg_scan_kernel(const uint2* __restrict__ a, uint64_t count, int*
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Work {
-  size_t xmax, xexp, z, t, end;  // the flag word is at 0
+  size_t xmax, xexp, z, t, end;  // the passes' flags are at 0
 };
 
 // n-tiles of 8 columns per pass.  More than two per warp measured slower than
 // more passes (64 right-hand sides, 65,536 points: 6.2 ms with four, 5.6 ms with
 // two): their sums take the registers of half the warps.
-constexpr uint32_t kMaxCols = 16;
+constexpr uint32_t kMaxCols = dg_pass_cols(false);
 int nt_of(uint32_t cols) { return cols <= 8 ? 1 : 2; }
 
 Work work_of(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p) {
   const size_t cw = cplx ? 2 : 1, nt = nt_of(p * (uint32_t)cw);
   Work w;
-  w.xmax = 256;
+  const size_t per = dg_pass_cols(cplx);
+  w.xmax = align256(((size_t)p + per - 1) / per * 4);
   w.xexp = align256(w.xmax + (size_t)p * 4);
   w.z = align256(w.xexp + kMaxCols * 4);
   w.t = align256(w.z + ((size_t)n + t_rows) * cw * (S * nt + 1) * 16);
@@ -694,7 +696,7 @@ cudaError_t sweep(const KArgs& k, uint32_t n, cudaStream_t s) {
 template <int NT, int CW>
 cudaError_t run_pass(const DgPlan& pl, const DgArgs& a, const Work& w, uint32_t r0, uint32_t pr, cudaStream_t s) {
   unsigned char* wk = pl.work;
-  int* flag = reinterpret_cast<int*>(wk);
+  int* flag = reinterpret_cast<int*>(wk) + r0 / dg_pass_cols(CW == 2);
   int* xmax = reinterpret_cast<int*>(wk + w.xmax) + r0;
   int* xexp = reinterpret_cast<int*>(wk + w.xexp);
   unsigned char* z = wk + w.z;
@@ -737,16 +739,15 @@ template <int CW>
 cudaError_t run_all(const DgPlan& pl, const DgArgs& a, const Work& w, cudaStream_t s) {
   unsigned char* wk = pl.work;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(wk, 0, w.xexp, s)) != cudaSuccess) return e;  // flag, column maxima
+  if ((e = cudaMemsetAsync(wk, 0, w.xexp, s)) != cudaSuccess) return e;  // flags, column maxima
   const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.n * CW + 1023) / 1024, 64));
   for (uint32_t r0 = 0; r0 < a.p; r0 += 65535) {
     const uint32_t pr = std::min<uint32_t>(a.p - r0, 65535);
-    dg_xmax_kernel<CW><<<dim3(gx, pr), 256, 0, s>>>(static_cast<const double*>(a.X) + (uint64_t)r0 * a.ldX * CW,
-                                                    a.ldX, pl.n, reinterpret_cast<int*>(wk + w.xmax) + r0,
-                                                    reinterpret_cast<int*>(wk));
+    dg_xmax_kernel<CW><<<dim3(gx, pr), 256, 0, s>>>(static_cast<const double*>(a.X), a.ldX, pl.n, r0,
+                                                    reinterpret_cast<int*>(wk + w.xmax), reinterpret_cast<int*>(wk));
   }
   count_product_launches(1);
-  const uint32_t per = kMaxCols / CW;
+  const uint32_t per = dg_pass_cols(CW == 2);
   for (uint32_t r0 = 0; r0 < a.p; r0 += per) {
     const uint32_t pr = std::min(per, a.p - r0);
     e = nt_of(pr * CW) == 1 ? run_pass<1, CW>(pl, a, w, r0, pr, s) : run_pass<2, CW>(pl, a, w, r0, pr, s);

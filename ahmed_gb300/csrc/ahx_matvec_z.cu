@@ -117,7 +117,7 @@ __device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, u
   }
 }
 
-template <typename S, typename R, int PG, int OP, bool PRE>
+template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE>
 __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
   const MvLeaf L = a.leaves[a.order[leaf]];
   const S* base = reinterpret_cast<const S*>(a.arena) + L.off;
@@ -127,6 +127,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
   const uint32_t ro = kFwd ? L.b1 : L.b2, nr = kFwd ? L.n1 : L.n2;
   const uint32_t co = kFwd ? L.b2 : L.b1, nc = kFwd ? L.n2 : L.n1;
   for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
+    if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
     const uint32_t pg = min((uint32_t)PG, a.p - r0);
     if (L.rank < 0) {
       // dense: thread per output row; the forward product reads D by rows
@@ -231,10 +232,12 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(ZArg
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
   if (GUARD) {
-    if (*a.guard == 0) return;
-    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP, PRE>(a, l, Xs, Ts, red);
+    bool any = false;
+    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q];
+    if (!__syncthreads_or(any)) return;
+    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP, true, PRE>(a, l, Xs, Ts, red);
   } else {
-    zmv_leaf<S, R, PG, OP, PRE>(a, blockIdx.x, Xs, Ts, red);
+    zmv_leaf<S, R, PG, OP, false, PRE>(a, blockIdx.x, Xs, Ts, red);
   }
 }
 

@@ -393,7 +393,7 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
       if ((rc = H->dg_work.reserve(bytes))) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena.p, H->dg_work);
       AHX_CUDA(launch_matvec_dg(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
-      guard = dg_flag(pl);
+      guard = dg_flags(pl);
     }
   }
   // (the plain complex64 kernel costs a third of what dg_due counts for real elements)
@@ -422,6 +422,7 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
   a.ldY = ldY;
   a.op = op;
   a.guard = guard;
+  a.guard_cols = dg_pass_cols(true);
   a.elems = Z.elems;
   a.n = (uint32_t)n;
   a.xf = Z.xf.as<float2>();
