@@ -509,6 +509,7 @@ extern "C" int ahx_helm_aca_ranks(ahx_hmat* H, double wavenumber, double h, doub
     set_error("ahx_helm_aca_ranks: invalid argument (bounding-box trees only)");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   int rc = ensure_device(H);
   if (rc) return rc;
   const auto& Ls = H->tree.leaves;
@@ -629,6 +630,7 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
     set_error("ahx_helm_assemble: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   int rc = ensure_device(H);
   if (rc) return rc;
   ZState& Z = H->z;
@@ -692,6 +694,7 @@ extern "C" int ahx_helm_assemble(ahx_hmat* H, double wavenumber, double h, doubl
 
 extern "C" int ahx_helm_ranks(const ahx_hmat* H, int32_t* ranks) {
   if (!H || !ranks) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->z.assembled) {
     set_error("ahx_helm_ranks: Helmholtz leaves not assembled");
     return AHX_ERR_STATE;
@@ -709,7 +712,9 @@ bool packed_zleaf(const ahx_hmat* H, uint32_t l) {
 }  // namespace
 
 extern "C" uint64_t ahx_helm_leaf_size(const ahx_hmat* H, uint32_t l) {
-  if (!H || !H->z.assembled || l >= H->tree.leaves.size()) return 0;
+  if (!H) return 0;
+  const HandleLock lk(H->mu);
+  if (!H->z.assembled || l >= H->tree.leaves.size()) return 0;
   const Leaf& L = H->tree.leaves[l];
   const int32_t r = H->z.rank[l];
   if (packed_zleaf(H, l)) return (uint64_t)L.n1 * (L.n1 + 1) / 2;
@@ -717,7 +722,12 @@ extern "C" uint64_t ahx_helm_leaf_size(const ahx_hmat* H, uint32_t l) {
 }
 
 extern "C" int ahx_helm_get_leaf(const ahx_hmat* H, uint32_t l, double* out) {
-  if (!H || !out || l >= H->tree.leaves.size()) {
+  if (!H || !out) {
+    set_error("ahx_helm_get_leaf: invalid argument");
+    return AHX_ERR_ARG;
+  }
+  const HandleLock lk(H->mu);
+  if (l >= H->tree.leaves.size()) {
     set_error("ahx_helm_get_leaf: invalid argument");
     return AHX_ERR_ARG;
   }

@@ -120,6 +120,7 @@ namespace {
 // tree changes, so the other kind of leaves of the handle is dropped.
 int agglomerate_impl(ahx_hmat* H, double eps, uint32_t max_rank, uint32_t* nmerged, bool cplx) {
   if (!H || !(eps >= 0.0)) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!(cplx ? H->z.assembled : H->assembled)) {
     set_error("agglomerate: H-matrix not assembled");
     return AHX_ERR_STATE;

@@ -509,7 +509,6 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     set_error("transposed products use the FP64 leaves");
     return AHX_ERR_ARG;
   }
-  std::lock_guard<std::mutex> lk(H->product_mu);
   int rc;
   if (prec == kFP32 && p >= 2 && um_enabled()) {
     // FP32 leaves, several right-hand sides: the tcgen05 sweeps
@@ -711,6 +710,7 @@ int ahx_hmat_destroy(ahx_hmat* H) {
 
 int ahx_hmat_set_stream(ahx_hmat* H, void* stream) {
   if (!H) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (H->stream) {
     AHX_CUDA(cudaSetDevice(H->device));
     AHX_CUDA(cudaStreamSynchronize(H->stream));
@@ -734,6 +734,7 @@ int ahx_hmat_perm(const ahx_hmat* H, uint32_t* op_perm, uint32_t* po_perm) {
 
 int ahx_hmat_leaves(const ahx_hmat* H, uint32_t* out) {
   if (!H || !out) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   for (size_t l = 0; l < H->tree.leaves.size(); ++l) {
     const Leaf& L = H->tree.leaves[l];
     uint32_t* o = out + 7 * l;
@@ -758,6 +759,7 @@ int ahx_assemble_hinted(ahx_hmat* H, double h, double eps, uint32_t rankmax,
     set_error("ahx_assemble: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   int rc = ensure_device(H);
   if (rc) return rc;
   invalidate_products(H);
@@ -855,6 +857,7 @@ int ahx_hmat_autotune(ahx_hmat* H, int precision, uint32_t p, uint32_t* out4) {
     set_error("ahx_hmat_autotune: invalid argument (mixed precisions only)");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -939,6 +942,7 @@ int ahx_hmat_autotune(ahx_hmat* H, int precision, uint32_t p, uint32_t* out4) {
 
 int ahx_hmat_features(const ahx_hmat* H, double wavenumber, double eps, float* out) {
   if (!H || !out) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   for (size_t l = 0; l < H->tree.leaves.size(); ++l)
     leaf_features(H->tree, H->tree.leaves[l], wavenumber, eps, out + 8 * l);
   return AHX_OK;
@@ -946,6 +950,7 @@ int ahx_hmat_features(const ahx_hmat* H, double wavenumber, double eps, float* o
 
 int ahx_hmat_ranks(const ahx_hmat* H, int32_t* ranks) {
   if (!H || !ranks) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -956,6 +961,7 @@ int ahx_hmat_ranks(const ahx_hmat* H, int32_t* ranks) {
 
 int ahx_hmat_aca_ranks(const ahx_hmat* H, int32_t* ranks) {
   if (!H || !ranks) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -972,7 +978,9 @@ static bool packed_leaf(const ahx_hmat* H, uint32_t l) {
 }
 
 uint64_t ahx_hmat_leaf_size(const ahx_hmat* H, uint32_t l) {
-  if (!H || !H->assembled || l >= H->tree.leaves.size()) return 0;
+  if (!H) return 0;
+  const HandleLock lk(H->mu);
+  if (!H->assembled || l >= H->tree.leaves.size()) return 0;
   const Leaf& L = H->tree.leaves[l];
   const int32_t r = H->rank[l];
   if (packed_leaf(H, l)) return (uint64_t)L.n1 * (L.n1 + 1) / 2;
@@ -980,7 +988,9 @@ uint64_t ahx_hmat_leaf_size(const ahx_hmat* H, uint32_t l) {
 }
 
 int ahx_hmat_get_leaf(const ahx_hmat* H, uint32_t l, double* out) {
-  if (!H || !out || l >= H->tree.leaves.size()) return AHX_ERR_ARG;
+  if (!H || !out) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
+  if (l >= H->tree.leaves.size()) return AHX_ERR_ARG;
   if (!H->assembled) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -1007,6 +1017,7 @@ int ahx_hmat_get_leaf(const ahx_hmat* H, uint32_t l, double* out) {
 int ahx_hmat_set_leaves(ahx_hmat* H, const int32_t* ranks, const double* data,
                         const uint64_t* offsets) {
   if (!H || !ranks || !offsets) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   const auto& Ls = H->tree.leaves;
   const uint32_t nl = (uint32_t)Ls.size();
   // dense diagonal leaves of a symmetric tree may come packed (mblock HeM data)
@@ -1074,7 +1085,9 @@ int ahx_hmat_set_leaves(ahx_hmat* H, const int32_t* ranks, const double* data,
 }
 
 uint64_t ahx_hmat_storage_bytes(ahx_hmat* H, int precision) {
-  if (!H || !H->assembled) return 0;
+  if (!H) return 0;
+  const HandleLock lk(H->mu);
+  if (!H->assembled) return 0;
   if (ensure_device(H)) return 0;
   if (precision == kFP32 && um_enabled()) {
     if (prepare_um(H)) return 0;
@@ -1086,6 +1099,7 @@ uint64_t ahx_hmat_storage_bytes(ahx_hmat* H, int precision) {
 
 int ahx_hmat_stream_bytes(ahx_hmat* H, int precision, uint64_t* out) {
   if (!H || !out || precision != kFP32) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->assembled) return AHX_ERR_STATE;
   int rc = ensure_device(H);
   if (rc) return rc;
@@ -1107,6 +1121,7 @@ int ahx_timing_read(double* ms2, uint64_t* count2, int reset) {
 
 int ahx_hmat_prepare(ahx_hmat* H, int precision) {
   if (!H) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -1122,6 +1137,7 @@ int ahx_hmat_prepare(ahx_hmat* H, int precision) {
 int ahx_hmat_release(ahx_hmat* H, int precision) {
   if (!H || precision < 0 || precision >= kNumPrecisions) return AHX_ERR_ARG;
   if (precision == kFP64) return AHX_OK;  // the handle's own leaves
+  const HandleLock lk(H->mu);
   int rc = ensure_device(H);
   if (rc) return rc;
   AHX_CUDA(cudaStreamSynchronize(H->stream));
@@ -1136,6 +1152,7 @@ int matvec_any(ahx_hmat* H, int precision, double d, uint32_t p, const double* X
     set_error("ahx_matvec: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("ahx_matvec: H-matrix not assembled");
     return AHX_ERR_STATE;

@@ -55,14 +55,13 @@ struct HostWord {
 };
 
 // Device scratch of the solvers, kept between the solves of a handle (which run one after
-// another, from several threads too): allocating and freeing it took 0.7 ms of a GMRES call of 8.8 ms (16 systems of
-// 32,768 points).  What is larger than kKeep goes back after each solve (a basis of 50
-// vectors at 1,048,576 points and 64 right-hand sides is 27 GB).
+// another: ahx_hmat::mu): allocating and freeing it took 0.7 ms of a GMRES call of 8.8 ms
+// (16 systems of 32,768 points).  What is larger than kKeep goes back after each solve (a
+// basis of 50 vectors at 1,048,576 points and 64 right-hand sides is 27 GB).
 struct SolveWork {
   static constexpr size_t kKeep = 256ull << 20;
   DevBuf items, first, partial, small[3], len, gm;  // reductions, GMRES state
   DevBuf v, r, rr, z;                               // basis, residuals, correction
-  std::mutex mu;                                    // held by the solve that uses them
   void release() {
     for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) b->release();
   }
@@ -229,9 +228,12 @@ struct ahx_hmat {
   ahx::DgState dg[2];     // digit-sliced FP64 products: A, A^T
   int finite = 0;         // FP64 leaf elements: 0 not looked at, 1 fit for digits, 2 not
   ahx::DevBuf dg_work;    // their work buffer (real and complex)
-  // held while a product's kernels are queued: they share work buffers in stream order, so
-  // that products from several threads must not interleave (the plain kernels need no buffer)
-  std::mutex product_mu;
+  // Calls of one handle from several threads take turns: each call that queues device work
+  // or changes the handle's state holds this from its first copy to its last (recursive: some
+  // calls are made of others).  Staging, work and solver buffers are the handle's, used in
+  // stream order, and a solve records and replays its steps as graphs that address them: a
+  // product queued in between would be recorded too, or find its buffers in use.
+  mutable std::recursive_mutex mu;
   // staging buffers for host vectors
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch
@@ -244,6 +246,7 @@ struct ahx_hmat {
 };
 
 namespace ahx {
+using HandleLock = std::lock_guard<std::recursive_mutex>;
 int prepare_product(ahx_hmat* H, int prec);
 // FP32 leaves as tcgen05 streams (ahx_umma.cuh); AHX_UMMA=0 keeps every FP32 product on the mma.sync sweeps
 int prepare_um(ahx_hmat* H);

@@ -116,6 +116,7 @@ int64_t file_read(void* ctx, void* buf, uint64_t bytes) {
 // cplx: the Helmholtz leaves (mblock<dcomp>: two doubles per element; packed
 // symmetric diagonal blocks are status 5, SyM) instead of the real ones.
 int save_impl(ahx_hmat* H, double eta, uint32_t bmin, Writer& w, bool cplx) {
+  const HandleLock lk(H->mu);
   if (!(cplx ? H->z.assembled : H->assembled)) {
     set_error("not assembled");
     return AHX_ERR_STATE;
@@ -276,6 +277,7 @@ struct Stager {
 };
 
 int load_impl(ahx_hmat* H, Reader& rd, double* eta_out, uint32_t* bmin_out, bool cplx) {
+  const HandleLock lk(H->mu);
   double eta = 0.0;
   uint32_t bmin = 0, nfile = 0;
   if (!rd.get(&eta, sizeof eta) || !rd.get(&bmin, sizeof bmin) || !rd.get(&nfile, sizeof nfile)) {

@@ -477,7 +477,6 @@ struct HmatOp : Operator {
   }
   uint64_t product_bytes(int prec) const override { return H->prod[prec].bytes; }
   int prepare(int prec, uint32_t p) override {
-    std::lock_guard<std::mutex> lk(H->product_mu);
     int rc;
     if (((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p)) ||
         (prec == kFP64 && p == 1 && f1_wanted(H->arena64_elems, false))) {
@@ -494,7 +493,7 @@ struct HmatOp : Operator {
 // Reduction plan + device scratch for a family of systems.
 class Solver {
  public:
-  Solver(Operator& op, uint32_t p) : lock_(op.work->mu), op_(op), p_(p) {}
+  Solver(Operator& op, uint32_t p) : op_(op), p_(p) {}
   ~Solver() {
     if (idle_) work_.trim();
     else work_.release();  // (waits for kernels that an error left in flight)
@@ -561,7 +560,6 @@ class Solver {
 
   const uint32_t* segid() const { return op_.nseg > 1 ? op_.seg_id.as<uint32_t>() : nullptr; }
 
-  std::unique_lock<std::mutex> lock_;
   Operator& op_;
   SolveWork& work_{*op_.work};
   bool idle_ = false;  // set once nothing in flight uses the scratch
@@ -1160,6 +1158,7 @@ struct ahx_batch : ahx::Operator {
     uint64_t elems = 0;  // FP64 arena elements (kFP64 table)
     ahx::ProdCopy plan;  // mixed-precision plan over the concatenated leaves
   } tab[ahx::kNumPrecisions];
+  std::mutex mu;  // calls of a batch from several threads take turns (ahx_hmat::mu)
   ahx::DevBuf stx, sty;
   ahx::HostWord steps;
   ahx::SolveWork solve_work;
@@ -1199,6 +1198,7 @@ struct ahx_batch : ahx::Operator {
     std::vector<std::pair<const void*, uint64_t>> src;  // (ptr, bytes)
     for (size_t i = 0; i < mats.size(); ++i) {
       ahx_hmat* H = mats[i];
+      const HandleLock lk(H->mu);
       int rc = prepare_product(H, kFP64);
       if (rc) return rc;
       ProdCopy& pc = H->prod[kFP64];
@@ -1290,6 +1290,7 @@ int ahx_gmres(ahx_hmat* H, int precision, uint32_t p, const double* B, uint64_t 
     set_error("ahx_gmres: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("ahx_gmres: H-matrix not assembled");
     return AHX_ERR_STATE;
@@ -1320,6 +1321,7 @@ int ahx_gmres(ahx_hmat* H, int precision, uint32_t p, const double* B, uint64_t 
 // (FP64 products; A^T by the transposed product), the square root of the last norm.
 int ahx_spctrlnrm(ahx_hmat* H, uint32_t it_num, double* out) {
   if (!H || !out) return AHX_ERR_ARG;
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("ahx_spctrlnrm: H-matrix not assembled");
     return AHX_ERR_STATE;
@@ -1362,6 +1364,7 @@ int ahx_cg(ahx_hmat* H, uint32_t p, const double* B, uint64_t ldB, double* X, ui
     set_error("ahx_cg: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   if (!H->assembled) {
     set_error("ahx_cg: H-matrix not assembled");
     return AHX_ERR_STATE;
@@ -1409,7 +1412,11 @@ int ahx_batch_create(ahx_hmat* const* mats, uint32_t count, int precision, ahx_b
   b->mats.assign(mats, mats + count);
   b->prec = precision;
   b->device = mats[0]->device;
-  int rc = ensure_device(mats[0]);
+  int rc;
+  {
+    const HandleLock lk(mats[0]->mu);
+    rc = ensure_device(mats[0]);
+  }
   if (rc) {
     delete b;
     return rc;
@@ -1433,6 +1440,7 @@ int ahx_batch_create(ahx_hmat* const* mats, uint32_t count, int precision, ahx_b
   }
   for (uint32_t i = 0; i < count; ++i) {
     // instances share the first instance's stream for the duration of the batch
+    const HandleLock lk(mats[i]->mu);
     if ((rc = ensure_device(mats[i]))) {
       delete b;
       return rc;
@@ -1472,6 +1480,7 @@ uint64_t ahx_batch_n(const ahx_batch* b) { return b ? b->ntot : 0; }
 
 int ahx_batch_prepare(ahx_batch* b, int precision) {
   if (!b || precision < 0 || precision >= kNumPrecisions) return AHX_ERR_ARG;
+  const std::lock_guard<std::mutex> lk(b->mu);
   AHX_CUDA(cudaSetDevice(b->device));
   if (precision == kFP64) return AHX_OK;
   if (precision == kDF64) return b->prepare(kDF64, 1);
@@ -1482,6 +1491,7 @@ int ahx_batch_prepare(ahx_batch* b, int precision) {
 int ahx_batch_matvec(ahx_batch* b, double d, uint32_t p, const double* X, double* Y) {
   if (!b || !X || !Y) return AHX_ERR_ARG;
   if (p == 0) return AHX_OK;
+  const std::lock_guard<std::mutex> lk(b->mu);
   AHX_CUDA(cudaSetDevice(b->device));
   const uint64_t n = b->ntot;
   const double* Xd = nullptr;
@@ -1503,6 +1513,7 @@ int ahx_batch_matvec(ahx_batch* b, double d, uint32_t p, const double* X, double
 int ahx_batch_gmres(ahx_batch* b, const double* B, double* X, double tol, uint32_t m,
                     uint32_t maxit, uint32_t* iters, double* resid) {
   if (!b || !B || !X) return AHX_ERR_ARG;
+  const std::lock_guard<std::mutex> lk(b->mu);
   AHX_CUDA(cudaSetDevice(b->device));
   const uint64_t n = b->ntot;
   DevBuf bb, xb;

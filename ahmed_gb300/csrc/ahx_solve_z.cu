@@ -340,8 +340,8 @@ int zgmres_one(ahx_hmat* H, int prec, const ZGm& g, const double2* b, double2* x
 
 }  // namespace
 
-static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
-                           uint64_t ldX, double2* Y, uint64_t ldY) {
+int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
+                    uint64_t ldX, double2* Y, uint64_t ldY) {
   int rc = prepare_z(H, prec);
   if (rc) return rc;
   ZState& Z = H->z;
@@ -354,7 +354,7 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
     zconj_kernel<<<grid, 256, 0, H->stream>>>(X, ldX, Xc, n, n, p);
     zconj_kernel<<<grid, 256, 0, H->stream>>>(Y, ldY, Y, ldY, n, p);
     AHX_CUDA(cudaGetLastError());
-    if ((rc = zproduct_locked(H, prec, kZOpN, dre, -dim, p, Xc, n, Y, ldY))) return rc;
+    if ((rc = zproduct_device(H, prec, kZOpN, dre, -dim, p, Xc, n, Y, ldY))) return rc;
     zconj_kernel<<<grid, 256, 0, H->stream>>>(Y, ldY, Y, ldY, n, p);
     AHX_CUDA(cudaGetLastError());
     return AHX_OK;
@@ -366,6 +366,9 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
   DgState& D = Z.dg[op];
   auto laid_out = [&](uint64_t cost) -> bool {  // (not while the stream is captured: it waits)
     return D.valid || (dg_due(D, cost, p, H->tree.leaves.size()) && !stream_captured(H->stream));
+  };
+  auto work = [&](size_t bytes) -> bool {
+    return H->dg_work.bytes >= bytes || !stream_captured(H->stream);
   };
   auto layout = [&]() -> int {
     if (D.valid) return AHX_OK;
@@ -380,9 +383,6 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
       if (H->tree.sym && L.b1 != L.b2) lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], kDgT, Z.off[l]});
     }
     return dg_prepare_state(D, lv, n, Z.arena.p, 2 * Z.elems, kDgK / 2, Z.finite, H->device, H->stream);
-  };
-  auto work = [&](size_t bytes) -> bool {
-    return H->dg_work.bytes >= bytes || !stream_captured(H->stream);
   };
   const int* guard = nullptr;
   if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) && laid_out(4 * Z.elems)) {
@@ -438,12 +438,6 @@ static int zproduct_locked(ahx_hmat* H, int prec, int op, double dre, double dim
   return AHX_OK;
 }
 
-int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint32_t p, const double2* X,
-                    uint64_t ldX, double2* Y, uint64_t ldY) {
-  std::lock_guard<std::mutex> lk(H->product_mu);
-  return zproduct_locked(H, prec, op, dre, dim, p, X, ldX, Y, ldY);
-}
-
 }  // namespace ahx
 
 using namespace ahx;
@@ -451,7 +445,9 @@ using namespace ahx;
 extern "C" {
 
 uint64_t ahx_helm_storage_bytes(const ahx_hmat* H, int precision) {
-  if (!H || !H->z.assembled) return 0;
+  if (!H) return 0;
+  const HandleLock lk(H->mu);
+  if (!H->z.assembled) return 0;
   if (precision == AHX_FP64) return H->z.elems * 16;
   if (precision == AHX_FP32) return H->z.elems * 8;
   return 0;
@@ -463,6 +459,7 @@ int ahx_helm_matvec(ahx_hmat* H, int precision, int op, double d_re, double d_im
     set_error("ahx_helm_matvec: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   int rc = check_z(H, precision, "ahx_helm_matvec");
   if (rc) return rc;
   if (p == 0) return AHX_OK;
@@ -500,6 +497,7 @@ int ahx_helm_gmres(ahx_hmat* H, int precision, uint32_t p, const double* B, uint
     set_error("ahx_helm_gmres: invalid argument");
     return AHX_ERR_ARG;
   }
+  const HandleLock lk(H->mu);
   int rc = check_z(H, precision, "ahx_helm_gmres");
   if (rc) return rc;
   if ((rc = ensure_device(H))) return rc;
