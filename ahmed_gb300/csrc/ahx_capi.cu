@@ -522,7 +522,8 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   // (double-float would need a copy of the leaves: there always)
   const int* guard = nullptr;
   const bool one = prec == kFP64 && p == 1 && f1_wanted(H->arena64_elems, transposed);
-  if (one || ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2)) {
+  if ((one || ((prec == kFP64 || prec == kDF64) && dg_wanted(H->arena64_elems, p) && H->finite != 2)) &&
+      !caller_captures(H)) {
     bool usable = false;
     // (nothing is laid out or allocated while the stream is captured)
     DgState& D = H->dg[transposed ? 1 : 0];
@@ -530,6 +531,7 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     if (ready || ((prec == kDF64 || dg_due(D, H->arena64_elems, p, H->tree.leaves.size())) && !stream_captured(H->stream)))
       if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
     if (usable && one) {
+      if ((rc = prepare_product(H, kFP64))) return rc;  // (a product that the caller captures takes these)
       const DgPlan pl = dg_plan(D, H->tree.n, H->arena64.p, H->dg_work);
       AHX_CUDA(launch_matvec_f1(pl, d, X, Y, H->stream));
       return AHX_OK;

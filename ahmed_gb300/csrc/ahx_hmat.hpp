@@ -234,6 +234,7 @@ struct ahx_hmat {
   // stream order, and a solve records and replays its steps as graphs that address them: a
   // product queued in between would be recorded too, or find its buffers in use.
   mutable std::recursive_mutex mu;
+  bool recording = false;  // a solve of this handle is recording steps (which it replays itself)
   // staging buffers for host vectors
   ahx::DevBuf stage_x, stage_y;
   ahx::DevBuf scratch;  // solver scratch
@@ -260,6 +261,10 @@ bool dg_wanted(uint64_t elems, uint32_t p);
 bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves);
 // Whether a graph capture is under way on the stream (nothing may be allocated or waited for).
 bool stream_captured(cudaStream_t s);
+// Whether the caller is capturing the product: its graph may be replayed at any time, beside
+// other products of the handle or after its work buffers have grown, so that it gets the
+// kernels that address nothing but leaves, X and Y.
+inline bool caller_captures(const ahx_hmat* H) { return !H->recording && stream_captured(H->stream); }
 // Builds the layout of `leaves`; looks at the arena's elements once (finite).
 // count: its doubles.
 int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,

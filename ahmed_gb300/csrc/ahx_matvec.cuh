@@ -88,7 +88,7 @@ struct ZArgs {
   uint32_t guard_cols = 0;
   uint64_t elems = 0;          // complex64 leaves: elements,
   uint32_t n = 0;              //   rows of X,
-  float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes),
+  float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes; null: none is made),
   bool d_one = false;          //   d = 1 (set by the launcher)
 };
 cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s);

@@ -301,7 +301,7 @@ cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
     count_product_launches(1);
     return cudaGetLastError();
   }
-  if (a.p <= 4 || a.elems * a.p < 30000000ull) {
+  if (a.p <= 4 || a.elems * a.p < 30000000ull || !a.xf) {
     launch_typed<float2, float>(a, s);
     count_product_launches(1);
     return cudaGetLastError();

@@ -444,6 +444,8 @@ struct Operator {
     (void)prec;
     return 0;
   }
+  // the calls of apply until record(false) are captured into graphs that this solve replays
+  virtual void record(bool on) { (void)on; }
   // everything apply(prec, ...) allocates, done ahead (graph capture allows no allocation)
   virtual int prepare(int prec, uint32_t p) {
     (void)prec;
@@ -488,6 +490,7 @@ struct HmatOp : Operator {
     if (rc || prec != kDF64) return rc;
     return prepare_df_x(H->prod[kDF64], ntot, p);
   }
+  void record(bool on) override { H->recording = on; }
 };
 
 // Reduction plan + device scratch for a family of systems.
@@ -757,7 +760,9 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
         graphs->failed = true;
         return steps(i0, i1);
       }
+      op.record(true);
       const int e = steps(i0, i1);
+      op.record(false);
       const cudaError_t ce = cudaStreamEndCapture(st, &graph);
       cudaGraphExec_t ex = nullptr;
       if (e || ce != cudaSuccess || !graph || cudaGraphInstantiate(&ex, graph, 0) != cudaSuccess) {

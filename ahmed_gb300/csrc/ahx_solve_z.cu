@@ -362,13 +362,11 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   if (H->tree.sym) op = kZOpN;  // A^T = A
   // the layout over which products run on the tensor cores (complex128: digits, several
   // right-hand sides; complex64: TF32)
+  const bool captured = caller_captures(H);
   const uint64_t n = H->tree.n;
   DgState& D = Z.dg[op];
-  auto laid_out = [&](uint64_t cost) -> bool {  // (not while the stream is captured: it waits)
-    return D.valid || (dg_due(D, cost, p, H->tree.leaves.size()) && !stream_captured(H->stream));
-  };
-  auto work = [&](size_t bytes) -> bool {
-    return H->dg_work.bytes >= bytes || !stream_captured(H->stream);
+  auto laid_out = [&](uint64_t cost) -> bool {
+    return !captured && (D.valid || dg_due(D, cost, p, H->tree.leaves.size()));
   };
   auto layout = [&]() -> int {
     if (D.valid) return AHX_OK;
@@ -389,7 +387,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     // the plain kernels then only run when X does not fit the digits
     if ((rc = layout())) return rc;
     const size_t bytes = dg_work_bytes(true, n, D.t_rows, p);
-    if (D.usable && Z.finite == 1 && work(bytes)) {
+    if (D.usable && Z.finite == 1) {
       if ((rc = H->dg_work.reserve(bytes))) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena.p, H->dg_work);
       AHX_CUDA(launch_matvec_dg(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
@@ -400,7 +398,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   if (prec == kFP32 && zt_wanted(Z.elems, p) && laid_out(Z.elems / 3)) {
     if ((rc = layout())) return rc;
     const size_t bytes = zt_work_bytes(n, D.t_rows, p);
-    if (D.usable && work(bytes)) {
+    if (D.usable) {
       if ((rc = H->dg_work.reserve(bytes))) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena32.p, H->dg_work);
       AHX_CUDA(launch_matvec_zt(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
@@ -425,7 +423,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.guard_cols = dg_pass_cols(true);
   a.elems = Z.elems;
   a.n = (uint32_t)n;
-  a.xf = Z.xf.as<float2>();
+  a.xf = captured ? nullptr : Z.xf.as<float2>();
   AHX_CUDA(launch_matvec_z(a, H->stream));
   if (Z.ntleaves) {
     // the blocks below the diagonal: the upper ones transposed

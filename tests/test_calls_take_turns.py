@@ -1,5 +1,6 @@
 """One handle used from several threads at once, products beside solves, host vectors beside
-device ones, different numbers of right-hand sides."""
+device ones, different numbers of right-hand sides; and products that the caller captures
+into a graph, replayed after the handle's work buffers have grown."""
 import threading
 
 import numpy as np
@@ -86,4 +87,42 @@ def test_products_beside_solves(device, monkeypatch):
     for q, b in enumerate(B):
         for x in sols[q]:
             _close(_reference(H, np.ascontiguousarray(take(x))), b, 1e-9)
+    H.close()
+
+
+@pytest.mark.parametrize("kind,p,op", [("real", 1, "n"), ("real", 5, "n"), ("real", 5, "t"), ("c128", 3, "n"),
+                                       ("c128", 3, "h"), ("c64", 6, "n")])
+def test_captured_products(kind, p, op, monkeypatch):
+    for v in ("AHX_DG_MIN", "AHX_ZT_MIN", "AHX_F1_MIN"):
+        monkeypatch.setenv(v, "1")
+    n = 2111
+    s = torch.cuda.Stream()
+    H = _handle(n, s)
+    cplx = kind != "real"
+    if cplx:
+        H.helmholtz_assemble(4.0, 0.02, 1e-6)
+    prec = "fp32" if kind == "c64" else "fp64"
+    t = torch.complex128 if cplx else torch.float64
+    f = {"n": H.mltaGeHVec, "t": H.mltaGeHtVec, "h": H.mltaGeHhVec}[op]
+    big = torch.randn(40, n, dtype=t, device="cuda")
+    X = torch.randn(p, n, dtype=t, device="cuda")
+    X = X[0] if p == 1 else X
+    want, Y, Z = torch.zeros_like(X), torch.zeros_like(X), torch.zeros_like(big)
+    torch.cuda.synchronize()
+    f(1.0, X, want, precision=prec)  # (layout and buffers are there)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        f(1.0, X, Y, precision=prec)
+    f(1.0, big, Z, precision=prec)  # more right-hand sides: the work buffer grows
+    torch.cuda.synchronize()
+    junk = torch.full((64 << 20,), float("nan"), device="cuda")  # (what has been freed is reused)
+    with torch.cuda.stream(s):
+        for _ in range(3):
+            Y.zero_()
+            g.replay()
+    torch.cuda.synchronize()
+    tol = 1e-6 if kind == "c64" else 1e-13
+    assert float((Y - want).norm() / want.norm()) <= tol
+    del junk
     H.close()
