@@ -602,7 +602,7 @@ int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable) {
       if (H->tree.sym && L.b1 != L.b2)
         lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, H->rank[l], kDgT, H->off[l]});
     }
-    if ((rc = dg_prepare_state(D, lv, H->tree.n, H->arena64.p, H->arena64_elems, kDgK, H->finite, H->device, H->stream)))
+    if ((rc = dg_prepare_state(D, lv, H->tree.n, H->arena64.p, false, H->finite, H->device, H->stream)))
       return rc;
   }
   if (!D.usable || (H->finite == 2 && p > 1)) return AHX_OK;

@@ -87,6 +87,7 @@ struct DgPlan {
   const DgPos* pos;
   uint32_t nv, nr, t_rows, t_split, n;
   bool rs1;
+  const int* weight;  // per X row, then their maximum (DgState::weight)
   const void* arena;
   // work buffers of one product (dg_work_bytes)
   unsigned char* work;
@@ -105,15 +106,20 @@ struct DgArgs {
 // Bytes of the work buffer for p right-hand sides.  dg_flags: a word per pass of
 // dg_pass_cols right-hand sides, non-zero after a product in which those columns of X (or
 // of V^T X) do not fit the digits: an entry is not finite, the largest entry of a row is
-// below 2^-200 of its column's largest, or a column is subnormal.  Their columns of Y were
-// then left as they were.
+// below 2^-200 of its column's largest, a column is subnormal, or one column weighs too
+// little against the others (dg_xprep_kernel).  Their columns of Y were then left as they were.
 size_t dg_work_bytes(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p);
 constexpr uint32_t dg_pass_cols(bool cplx) { return cplx ? 8u : 16u; }
 inline const int* dg_flags(const DgPlan& pl) { return reinterpret_cast<const int*>(pl.work); }
 
 cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cudaStream_t s);
-// *bad |= any of the count doubles is not finite, or not zero and outside [2^-500, 2^500]
-cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStream_t s);
+// Every element of the leaves: *bad |= it is not finite, or not zero and outside [2^-500,
+// 2^500].  weight[i] (n of them, *wmax their maximum; kDgNoWeight to begin with): the binary
+// exponent of the largest entry that meets input row i, of a low-rank leaf P Q^H the largest
+// |Q_il| max |P_l|.
+constexpr int kDgNoWeight = (int)0x80808080;
+cudaError_t launch_dg_weigh(const DgLeaf* leaves, uint32_t nleaves, bool cplx, const void* arena, int* weight,
+                            int* wmax, int* bad, cudaStream_t s);
 cudaError_t launch_matvec_dg(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
 // FP64 leaves and one right-hand side over the same layout (ahx_matvec_f1.cu); pl.work:
 // dg_work_bytes

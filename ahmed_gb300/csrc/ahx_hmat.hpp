@@ -115,11 +115,11 @@ struct DgState {
   bool valid = false;   // built (usable or not)
   bool usable = false;  // the layout's indices fit
   double spent = 0.0;   // estimated us of the plain products before the layout
-  DevBuf vpieces, rpieces, rowptr, pos;
+  DevBuf vpieces, rpieces, rowptr, pos, weight;
   uint32_t nv = 0, nr = 0, t_rows = 0, t_split = 0;
   bool rs1 = true;
   void release() {
-    for (DevBuf* b : {&vpieces, &rpieces, &rowptr, &pos}) b->release();
+    for (DevBuf* b : {&vpieces, &rpieces, &rowptr, &pos, &weight}) b->release();
     valid = usable = false;
     spent = 0.0;
   }
@@ -265,10 +265,9 @@ bool stream_captured(cudaStream_t s);
 // other products of the handle or after its work buffers have grown, so that it gets the
 // kernels that address nothing but leaves, X and Y.
 inline bool caller_captures(const ahx_hmat* H) { return !H->recording && stream_captured(H->stream); }
-// Builds the layout of `leaves`; looks at the arena's elements once (finite).
-// count: its doubles.
-int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,
-                     uint32_t kmax, int& finite, int device, cudaStream_t s);
+// Builds the layout of `leaves`; looks at their elements once (finite, weights).
+int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
+                     int& finite, int device, cudaStream_t s);
 DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& work);
 // FP64 leaves: layout and work buffer ahead of products with p right-hand sides
 // (and of graph capture); sets usable.

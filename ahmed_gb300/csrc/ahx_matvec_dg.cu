@@ -29,8 +29,9 @@
 // are added up in 32-bit integers; those of 2^-36 gather in FP32 for one chunk
 // and are then moved to the integers too; those of 2^-45 and 2^-54 stay in FP32.
 // Pairs below are left out (2^-63).  So the error is that of the digits: 2^-58 of
-// the row's largest term so far per entry, below what the FP64 kernel rounds away
-// in its own sums.  Against long double on the same leaves (2,000 to 4,096 points,
+// the row's largest term so far per entry, over all columns of the pass; that it stays
+// below what the FP64 kernel rounds away in the sums of each column is seen to by
+// dg_xprep_kernel.  Against long double on the same leaves (2,000 to 4,096 points,
 // 2 to 20 right-hand sides): 0.9e-16 to 2.7e-16 per right-hand side, the FP64
 // kernel 1.5e-16 to 5.0e-16.
 //
@@ -56,7 +57,7 @@ constexpr int kMagic = 0x4B400000;  // 1.5 * 2^23
 
 // Exponents.  Leaf elements other than zero lie in [2^-500, 2^500] and the
 // exponents of the Z rows in [-200, 200] (anything else is left to the plain
-// kernel: dg_scan_kernel, the flag), zero Z rows have kZeroZ.  So exponent + Z
+// kernel: dg_weigh_kernel, the flag), zero Z rows have kZeroZ.  So exponent + Z
 // exponent is at least 323 for a term that counts, at most 200 for a zero element
 // and at most 123 for a zero Z row: neither moves a row's exponent, and both are
 // more than 63 bits below it.
@@ -524,62 +525,62 @@ __device__ __forceinline__ bool subnormal(double v) {
   return (hi & 0x7ff00000u) == 0u && ((hi << 1) | (uint32_t)__double2loint(v)) != 0u;
 }
 
-// Digits of one Z row (8 NT columns of real values v(col), exponents rel(col)
-// relative to the columns' scales), written at z with the row's exponent.
-// Exponents out of range raise the flag.
-template <int NT, typename V>
-__device__ __forceinline__ void z_row(unsigned char* z, const V& val, uint32_t pc, int* flag) {
-  constexpr int NP = 8 * NT;
-  int m = kZeroZ;
-#pragma unroll 4
-  for (int j = 0; j < NP; ++j) {
-    if ((uint32_t)j >= pc) break;
-    int sc;
-    const double v = val(j, sc);
-    const int e = ((uint32_t)__double2hiint(v) >> 20) & 0x7ffu;
-    if (e) m = max(m, e - sc);
-  }
+// Sums over the rows of a pass, of squared entries rounded down to powers of two, times the
+// rows' squared weights (relative to the largest weight and column): of each column, and of
+// the largest column of each row.
+struct PassSums {
+  float col[16], all;
+  uint32_t ticket, pad[2];
+};
+
+// sums over the warp of R values a lane: value u ends in the lanes whose top log2(R) bits are u
+template <int R>
+__device__ __forceinline__ float warp_sums(float (&v)[R], uint32_t lane) {
+  int o = 16;
 #pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    uint32_t o[S][4];
+  for (int r = R / 2; r > 0; r >>= 1, o >>= 1) {
+    const bool up = lane & o;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      Dig f[2];
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const int j = 8 * t + 2 * u + w;
-        int sc = 0;
-        const double v = (uint32_t)j < pc ? val(j, sc) : 0.0;
-        const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
-        const int e = (hi >> 20) & 0x7ffu;
-        f[w] = fix_f64(hi, lo, e ? (uint32_t)(m - (e - sc)) : 64u);
-      }
-      uint32_t d[S];
-      digits(f[0], f[1], d);
-#pragma unroll
-      for (int k = 0; k < S; ++k) o[k][u] = d[k];
+    for (int u = 0; u < r; ++u) {
+      const float keep = up ? v[u + r] : v[u], give = up ? v[u] : v[u + r];
+      v[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
-#pragma unroll
-    for (int k = 0; k < S; ++k)
-      *reinterpret_cast<uint4*>(z + (k * NT + t) * 16) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
   }
-  if (m != kZeroZ && (m < kZMin || m > kZMax)) atomicOr(flag, 1);
-  *reinterpret_cast<uint4*>(z + S * NT * 16) = make_uint4((uint32_t)(m * (1 << 20)), 0u, 0u, 0u);
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
 }
 
-// X rows (blocks past them do nothing); real row CW i + e of a complex row: e = 0
-// (re | im), e = 1 (-im | re)
+// X rows, a thread each; real row CW i + e of a complex row: e = 0 (re | im), e = 1 (-im | re):
+// the digits of the 8 NT columns and the row's exponent.
+//
+// One exponent serves a row's columns, and one scale the terms that meet a row of A.  So what a
+// column's result loses is relative to the largest terms of all columns of the pass: its norm
+// is at most 2^-58 W, W^2 = sum_k c_k^2 z_k^2 with c_k the largest |A_ik| and z_k the row's
+// largest entry, each column scaled to 1.  A column r whose own terms are small beside the
+// others' (S_r^2 = sum_k c_k^2 z_kr^2; a unit vector beside dense ones, columns of A of very
+// different size) would lose bits that the FP64 kernel keeps.  So S_r >= 2^-5 W is asked of
+// every column that is not zero (the loss is then below 2^-53 S_r, the FP64 kernel's own
+// rounding); the last CTA raises the pass's flag otherwise.  Random right-hand sides have S_r =
+// W / 2, at least W / 6 (random clouds of 1,024 to 65,536 points, whose closest pairs weigh
+// most).  The sums cost 3 us of 236 (complex128 A^H, 6,007 points, 3 right-hand sides), 7 of
+// 1,354 (65,536 points, 16).
+constexpr float kLightest = 1024.f;  // W^2 / S_r^2
+constexpr int kXPrepThreads = 128;
 template <int NT, int CW>
-__global__ void dg_xprep_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t pc,
-                                const int* __restrict__ xmax, int* __restrict__ xexp, unsigned char* __restrict__ z,
-                                int* __restrict__ flag) {
+__global__ void __launch_bounds__(kXPrepThreads)
+    dg_xprep_kernel(const double* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t pc, const int* __restrict__ xmax,
+                    const int* __restrict__ weight, int* __restrict__ xexp, unsigned char* __restrict__ z,
+                    PassSums* __restrict__ sums, int* __restrict__ flag) {
+  constexpr int NP = 8 * NT, kW = kXPrepThreads / 32;
+  __shared__ float part[kW][NP + 1];
   const uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // unit of column col: 2^(xexp - 0), xexp = field - 1022 (complex: the column pair shares it)
-  if (q < (uint64_t)8 * NT) xexp[q] = q < pc ? xmax[q / CW] - 1022 : 0;
-  const uint64_t total = (uint64_t)n * CW;
-  if (q >= total) return;
+  if (q < (uint64_t)NP) xexp[q] = q < pc ? xmax[q / CW] - 1022 : 0;
+  const bool live = q < (uint64_t)n * CW;
   // e-major order: consecutive threads read consecutive rows of X
-  const uint32_t e = (uint32_t)(q / n), i = (uint32_t)(q - (uint64_t)e * n);
+  const uint32_t e = live ? (uint32_t)(q / n) : 0u, i = live ? (uint32_t)(q - (uint64_t)e * n) : 0u;
   bool bad = false;
   auto val = [&](int col, int& sc) -> double {
     sc = __ldg(xmax + col / CW);
@@ -594,9 +595,78 @@ __global__ void dg_xprep_kernel(const double* __restrict__ X, uint64_t ldX, uint
     bad = bad || (sc < 100 && subnormal(r));
     return r;
   };
-  const uint64_t zr = (uint64_t)CW * i + e;
-  z_row<NT>(z + zr * (kPR<NT> * 16), val, pc, flag);
-  if (bad) atomicOr(flag, 1);
+  float t[NP], all = 0.f;
+#pragma unroll
+  for (int j = 0; j < NP; ++j) t[j] = 0.f;
+  if (live) {
+    const int wt = max(__ldg(weight + i) - __ldg(weight + n), -4096);
+    int m = kZeroZ;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      if ((uint32_t)j < pc) {
+        int sc;
+        const double v = val(j, sc);
+        const int x = ((uint32_t)__double2hiint(v) >> 20) & 0x7ffu;
+        if (x) m = max(m, x - sc);
+        const int s2 = 2 * (wt + x - sc);
+        if (x && e == 0 && s2 >= -126) t[j] = __int_as_float((127 + min(s2, 0)) << 23);
+        all = fmaxf(all, t[j]);
+      }
+    }
+    unsigned char* const zq = z + ((uint64_t)CW * i + e) * (kPR<NT> * 16);
+#pragma unroll
+    for (int g = 0; g < NT; ++g) {
+      uint32_t o[S][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        Dig f[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const int j = 8 * g + 2 * u + w;
+          int sc = 0;
+          const double v = (uint32_t)j < pc ? val(j, sc) : 0.0;
+          const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+          const int x = (hi >> 20) & 0x7ffu;
+          f[w] = fix_f64(hi, lo, x ? (uint32_t)(m - (x - sc)) : 64u);
+        }
+        uint32_t d[S];
+        digits(f[0], f[1], d);
+#pragma unroll
+        for (int k = 0; k < S; ++k) o[k][u] = d[k];
+      }
+#pragma unroll
+      for (int k = 0; k < S; ++k)
+        *reinterpret_cast<uint4*>(zq + (k * NT + g) * 16) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+    }
+    *reinterpret_cast<uint4*>(zq + S * NT * 16) = make_uint4((uint32_t)(m * (1 << 20)), 0u, 0u, 0u);
+    if (bad || (m != kZeroZ && (m < kZMin || m > kZMax))) atomicOr(flag, 1);
+  }
+  // ---- the columns' weights
+  constexpr int kSh = NT == 1 ? 2 : 1;  // lanes that share a column's sum: 2^kSh
+  const float cs = warp_sums<NP>(t, lane);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+  if ((lane & ((1u << kSh) - 1u)) == 0) part[warp][lane >> kSh] = cs;
+  if (lane == 0) part[warp][NP] = all;
+  __syncthreads();
+  if (threadIdx.x <= NP) {
+    float s = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < kW; ++w) s += part[w][threadIdx.x];
+    if (s != 0.f) atomicAdd(threadIdx.x == NP ? &sums->all : &sums->col[threadIdx.x], s);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(&sums->ticket, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const float least = __ldcg(&sums->all) / kLightest;
+  bool light = false;
+  for (uint32_t c = 0; c < pc; c += CW) {
+    float s = __ldcg(&sums->col[c]);
+    if (CW == 2) s += __ldcg(&sums->col[c + 1]);
+    light = light || (xmax[c / CW] != 0 && s < least);
+  }
+  if (light) atomicOr(flag, 1);
 }
 
 // T rows: a lane per column pair (a complex T entry), so that a row is read and each of
@@ -647,20 +717,96 @@ __global__ void dg_expand_kernel(const DgSeg* __restrict__ segs, uint32_t nsegs,
   for (uint32_t k = l; k < g.kn; k += 8) pos[(uint64_t)g.pos0 + k] = DgPos{g.base + (uint64_t)k * g.ldk, g.z + k, g.rsf};
 }
 
-__global__ void dg_scan_kernel(const uint2* __restrict__ a, uint64_t count, int* __restrict__ bad) {
-  bool b = false;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint2 u = __ldg(a + i);
-    const uint32_t e = (u.y >> 20) & 0x7ffu;
-    b = b || (((u.y << 1) | u.x) != 0 && (e < kLeafMin || e > kLeafMax));
+// exponent field of an element (complex: the larger of its parts'), 0 for zero; b |= it does not
+// fit the digits
+template <int CW>
+__device__ __forceinline__ int leaf_exp(const uint2* a, uint64_t at, bool& b) {
+  int m = 0;
+#pragma unroll
+  for (int c = 0; c < CW; ++c) {
+    const uint2 u = __ldg(a + at * CW + c);
+    const int e = (u.y >> 20) & 0x7ffu;
+    if (((u.y << 1) | u.x) != 0) {
+      b = b || e < kLeafMin || e > kLeafMax;
+      m = max(m, e);
+    }
   }
-  if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
+  return m;
+}
+
+// a CTA per leaf; see launch_dg_weigh
+constexpr int kWeighThreads = 128;
+template <int CW>
+__global__ void __launch_bounds__(kWeighThreads)
+    dg_weigh_kernel(const DgLeaf* __restrict__ leaves, const uint2* __restrict__ a, int* __restrict__ weight,
+                    int* __restrict__ wmax, int* __restrict__ bad) {
+  constexpr uint32_t kL = 32, kW = kWeighThreads / 32;
+  __shared__ int ep[kL];
+  const DgLeaf q = leaves[blockIdx.x];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  bool b = false;
+  int most = kDgNoWeight;
+  auto put = [&](uint32_t i, int w) {
+    most = max(most, w);
+    if (w > __ldcg(weight + i)) atomicMax(weight + i, w);
+  };
+  if (q.rank < 0) {
+    if (q.mode == kDgN) {
+      for (uint32_t j = warp; j < q.n2; j += kW) {
+        int m = 0;
+#pragma unroll 2
+        for (uint32_t i = lane; i < q.n1; i += 32) m = max(m, leaf_exp<CW>(a, q.off + (uint64_t)j * q.n1 + i, b));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0 && m) put(q.b2 + j, m - 1023);
+      }
+    } else {
+      for (uint32_t i = tid; i < q.n1; i += kWeighThreads) {
+        int m = 0;
+#pragma unroll 4
+        for (uint32_t j = 0; j < q.n2; ++j) m = max(m, leaf_exp<CW>(a, q.off + (uint64_t)j * q.n1 + i, b));
+        if (m) put(q.b1 + i, m - 1023);
+      }
+    }
+  } else {
+    const uint32_t k = (uint32_t)q.rank;
+    const uint64_t u = q.off, v = q.off + (uint64_t)q.n1 * k;
+    const bool fwd = q.mode == kDgN;
+    const uint32_t in = fwd ? q.n2 : q.n1, on = fwd ? q.n1 : q.n2, ib = fwd ? q.b2 : q.b1;
+    const uint64_t Q = fwd ? v : u, P = fwd ? u : v;
+    for (uint32_t l0 = 0; l0 < k; l0 += kL) {
+      const uint32_t ln = min(kL, k - l0);
+      for (uint32_t l = warp; l < ln; l += kW) {
+        int m = 0;
+#pragma unroll 2
+        for (uint32_t i = lane; i < on; i += 32) m = max(m, leaf_exp<CW>(a, P + (uint64_t)(l0 + l) * on + i, b));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) ep[l] = m;
+      }
+      __syncthreads();
+      for (uint32_t j = tid; j < in; j += kWeighThreads) {
+        int m = 0;
+#pragma unroll 4
+        for (uint32_t l = 0; l < ln; ++l) {
+          const int e = leaf_exp<CW>(a, Q + (uint64_t)(l0 + l) * in + j, b);
+          if (e && ep[l]) m = max(m, e + ep[l]);
+        }
+        if (m) put(ib + j, m - 2046);
+      }
+      __syncthreads();
+    }
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  const bool any = __any_sync(0xffffffffu, b);
+  if (lane == 0) {
+    if (most > __ldcg(wmax)) atomicMax(wmax, most);
+    if (any) atomicOr(bad, 1);
+  }
 }
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Work {
-  size_t xmax, xexp, z, t, end;  // the passes' flags are at 0
+  size_t sums, xmax, xexp, z, t, end;  // the passes' flags are at 0
 };
 
 // n-tiles of 8 columns per pass.  More than two per warp measured slower than
@@ -673,7 +819,9 @@ Work work_of(bool cplx, uint32_t n, uint32_t t_rows, uint32_t p) {
   const size_t cw = cplx ? 2 : 1, nt = nt_of(p * (uint32_t)cw);
   Work w;
   const size_t per = dg_pass_cols(cplx);
-  w.xmax = align256(((size_t)p + per - 1) / per * 4);
+  const size_t passes = ((size_t)p + per - 1) / per;
+  w.sums = align256(passes * 4);
+  w.xmax = align256(w.sums + passes * sizeof(PassSums));
   w.xexp = align256(w.xmax + (size_t)p * 4);
   w.z = align256(w.xexp + kMaxCols * 4);
   w.t = align256(w.z + ((size_t)n + t_rows) * cw * (S * nt + 1) * 16);
@@ -704,8 +852,9 @@ cudaError_t run_pass(const DgPlan& pl, const DgArgs& a, const Work& w, uint32_t 
   const uint32_t pc = pr * CW;
   const double* X = static_cast<const double*>(a.X) + (uint64_t)r0 * a.ldX * CW;
   const uint64_t xr = (uint64_t)pl.n * CW, tr = (uint64_t)pl.t_rows * CW;
-  dg_xprep_kernel<NT, CW><<<(unsigned)((std::max<uint64_t>(xr, 32) + 127) / 128), 128, 0, s>>>(
-      X, a.ldX, pl.n, pc, xmax, xexp, z, flag);
+  PassSums* sums = reinterpret_cast<PassSums*>(wk + w.sums) + r0 / dg_pass_cols(CW == 2);
+  dg_xprep_kernel<NT, CW><<<(unsigned)((xr + kXPrepThreads - 1) / kXPrepThreads), kXPrepThreads, 0, s>>>(
+      X, a.ldX, pl.n, pc, xmax, pl.weight, xexp, z, sums, flag);
   KArgs k;
   k.arena = pl.arena;
   k.rowptr = pl.rowptr;
@@ -739,7 +888,7 @@ template <int CW>
 cudaError_t run_all(const DgPlan& pl, const DgArgs& a, const Work& w, cudaStream_t s) {
   unsigned char* wk = pl.work;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(wk, 0, w.xexp, s)) != cudaSuccess) return e;  // flags, column maxima
+  if ((e = cudaMemsetAsync(wk, 0, w.xexp, s)) != cudaSuccess) return e;  // flags, sums, column maxima
   const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.n * CW + 1023) / 1024, 64));
   for (uint32_t r0 = 0; r0 < a.p; r0 += 65535) {
     const uint32_t pr = std::min<uint32_t>(a.p - r0, 65535);
@@ -772,10 +921,12 @@ cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cuda
   return cudaGetLastError();
 }
 
-cudaError_t launch_dg_scan(const void* arena, uint64_t count, int* bad, cudaStream_t s) {
-  if (!count) return cudaSuccess;
-  const unsigned grid = (unsigned)std::min<uint64_t>((count + 1023) / 1024, 152ull * 16);
-  dg_scan_kernel<<<grid, 256, 0, s>>>(static_cast<const uint2*>(arena), count, bad);
+cudaError_t launch_dg_weigh(const DgLeaf* leaves, uint32_t nleaves, bool cplx, const void* arena, int* weight,
+                            int* wmax, int* bad, cudaStream_t s) {
+  if (!nleaves) return cudaSuccess;
+  const uint2* a = static_cast<const uint2*>(arena);
+  if (cplx) dg_weigh_kernel<2><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, wmax, bad);
+  else dg_weigh_kernel<1><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, wmax, bad);
   return cudaGetLastError();
 }
 
@@ -815,28 +966,28 @@ bool stream_captured(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, uint64_t count,
-                     uint32_t kmax, int& finite, int device, cudaStream_t s) {
-  int rc;
-  if (finite == 0) {
-    ScopedBuf bad;
-    int b = 0;
-    if ((rc = bad.reserve(sizeof(int)))) return rc;
-    AHX_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-    AHX_CUDA(launch_dg_scan(arena, count, bad.as<int>(), s));
-    AHX_CUDA(cudaMemcpyAsync(&b, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    AHX_CUDA(cudaStreamSynchronize(s));
-    finite = b ? 2 : 1;
-  }
+int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
+                     int& finite, int device, cudaStream_t s) {
   if (D.valid) return AHX_OK;
-  int sms = 0;
+  int rc, sms = 0;
   AHX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   DgHost L;
   D.release();
-  D.valid = true;
-  if (!build_dg_layout(leaves, n, (uint32_t)std::max(sms, 1) * 16, kmax, L)) return AHX_OK;
-  D.valid = false;
-  ScopedBuf segs;
+  ScopedBuf segs, dl;
+  int bad = 0;
+  if ((rc = upload(dl, leaves, s)) || (rc = D.weight.reserve(((size_t)n + 2) * sizeof(int)))) return rc;
+  int* const w = D.weight.as<int>();
+  AHX_CUDA(cudaMemsetAsync(w, kDgNoWeight & 0xff, ((size_t)n + 1) * sizeof(int), s));
+  AHX_CUDA(cudaMemsetAsync(w + n + 1, 0, sizeof(int), s));
+  AHX_CUDA(launch_dg_weigh(dl.as<DgLeaf>(), (uint32_t)leaves.size(), cplx, arena, w, w + n, w + n + 1, s));
+  const bool fits = build_dg_layout(leaves, n, (uint32_t)std::max(sms, 1) * 16, cplx ? kDgK / 2 : kDgK, L);
+  AHX_CUDA(cudaMemcpyAsync(&bad, w + n + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  AHX_CUDA(cudaStreamSynchronize(s));
+  finite = bad ? 2 : 1;
+  if (!fits) {
+    D.valid = true;
+    return AHX_OK;
+  }
   if ((rc = upload(D.vpieces, L.vpieces, s))) return rc;
   if ((rc = upload(D.rpieces, L.rpieces, s))) return rc;
   if ((rc = upload(D.rowptr, L.rowptr, s))) return rc;
@@ -859,6 +1010,7 @@ DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& wo
   p.rpieces = D.rpieces.as<DgPiece>();
   p.rowptr = D.rowptr.as<uint64_t>();
   p.pos = D.pos.as<DgPos>();
+  p.weight = D.weight.as<int>();
   p.nv = D.nv;
   p.nr = D.nr;
   p.t_rows = D.t_rows;

@@ -380,7 +380,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
       lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], mode, Z.off[l]});
       if (H->tree.sym && L.b1 != L.b2) lv.push_back(DgLeaf{L.b1, L.n1, L.b2, L.n2, Z.rank[l], kDgT, Z.off[l]});
     }
-    return dg_prepare_state(D, lv, n, Z.arena.p, 2 * Z.elems, kDgK / 2, Z.finite, H->device, H->stream);
+    return dg_prepare_state(D, lv, (uint32_t)n, Z.arena.p, true, Z.finite, H->device, H->stream);
   };
   const int* guard = nullptr;
   if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) && laid_out(4 * Z.elems)) {
