@@ -606,9 +606,9 @@ int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable) {
       return rc;
   }
   if (!D.usable || (H->finite == 2 && p > 1)) return AHX_OK;
-  if ((rc = H->dg_work.reserve(dg_work_bytes(false, H->tree.n, D.t_rows, p)))) return rc;
-  usable = true;
-  return AHX_OK;
+  rc = H->dg_work.reserve(dg_work_bytes(false, H->tree.n, D.t_rows, p));
+  usable = rc == AHX_OK;
+  return rc == AHX_ERR_NOMEM ? AHX_OK : rc;
 }
 
 int ensure_device(ahx_hmat* H) {

@@ -265,12 +265,13 @@ bool stream_captured(cudaStream_t s);
 // other products of the handle or after its work buffers have grown, so that it gets the
 // kernels that address nothing but leaves, X and Y.
 inline bool caller_captures(const ahx_hmat* H) { return !H->recording && stream_captured(H->stream); }
-// Builds the layout of `leaves`; looks at their elements once (finite, weights).
+// Builds the layout of `leaves`; looks at their elements once (finite, weights).  Leaves it
+// unbuilt (D.usable is false) when there is no room for it.
 int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
                      int& finite, int device, cudaStream_t s);
 DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& work);
 // FP64 leaves: layout and work buffer ahead of products with p right-hand sides
-// (and of graph capture); sets usable.
+// (and of graph capture); sets usable, to false when there is no room for them.
 int prepare_dg(ahx_hmat* H, uint32_t p, bool transposed, bool& usable);
 // kDF64 product scratch for p right-hand sides (the split X), ahead of graph capture
 int prepare_df_x(ahx::ProdCopy& pc, uint64_t n, uint32_t p);

@@ -41,6 +41,7 @@
 // ms with 8 (2.1 TB/s); 8,300 us of it were the FP64 pipe.
 #include <algorithm>
 #include <cstdlib>
+#include <new>
 
 #include <cuda_fp16.h>
 
@@ -966,9 +967,8 @@ bool stream_captured(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
-                     int& finite, int device, cudaStream_t s) {
-  if (D.valid) return AHX_OK;
+static int build_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
+                       int& finite, int device, cudaStream_t s) {
   int rc, sms = 0;
   AHX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   DgHost L;
@@ -1002,6 +1002,24 @@ int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, 
   D.rs1 = L.rs1;
   D.valid = D.usable = true;
   return AHX_OK;
+}
+
+int dg_prepare_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n, const void* arena, bool cplx,
+                     int& finite, int device, cudaStream_t s) {
+  if (D.valid) return AHX_OK;
+  int rc;
+  try {
+    rc = build_state(D, leaves, n, arena, cplx, finite, device, s);
+  } catch (const std::bad_alloc&) {
+    rc = AHX_ERR_NOMEM;
+  }
+  if (rc == AHX_ERR_NOMEM) {
+    // no room: the plain kernels, which need none, go on (and are counted from zero for the
+    // next attempt)
+    D.release();
+    rc = AHX_OK;
+  }
+  return rc;
 }
 
 DgPlan dg_plan(const DgState& D, uint32_t n, const void* arena, const DevBuf& work) {

@@ -151,7 +151,8 @@ int prepare_z(ahx_hmat* H, int prec) {
   if (rc) return rc;
   if (prec == kFP32 && !Z.valid32) {
     if ((rc = Z.arena32.reserve(std::max<uint64_t>(Z.elems, 1) * sizeof(float2)))) return rc;
-    if ((rc = Z.xf.reserve(std::max<size_t>(matvec_z_xf_bytes(H->tree.n), 16)))) return rc;
+    rc = Z.xf.reserve(std::max<size_t>(matvec_z_xf_bytes(H->tree.n), 16));
+    if (rc && rc != AHX_ERR_NOMEM) return rc;  // (products do without it)
     AHX_CUDA(launch_z_to_c64(Z.arena.as<double2>(), Z.elems, Z.arena32.as<float2>(), H->stream));
     Z.valid32 = true;
   }
@@ -361,7 +362,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   }
   if (H->tree.sym) op = kZOpN;  // A^T = A
   // the layout over which products run on the tensor cores (complex128: digits, several
-  // right-hand sides; complex64: TF32)
+  // right-hand sides; complex64: TF32); without room for it or its work buffer the plain ones
   const bool captured = caller_captures(H);
   const uint64_t n = H->tree.n;
   DgState& D = Z.dg[op];
@@ -387,8 +388,8 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     // the plain kernels then only run when X does not fit the digits
     if ((rc = layout())) return rc;
     const size_t bytes = dg_work_bytes(true, n, D.t_rows, p);
-    if (D.usable && Z.finite == 1) {
-      if ((rc = H->dg_work.reserve(bytes))) return rc;
+    if (D.usable && Z.finite == 1 && (rc = H->dg_work.reserve(bytes)) != AHX_ERR_NOMEM) {
+      if (rc) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena.p, H->dg_work);
       AHX_CUDA(launch_matvec_dg(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
       guard = dg_flags(pl);
@@ -398,8 +399,8 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   if (prec == kFP32 && zt_wanted(Z.elems, p) && laid_out(Z.elems / 3)) {
     if ((rc = layout())) return rc;
     const size_t bytes = zt_work_bytes(n, D.t_rows, p);
-    if (D.usable) {
-      if ((rc = H->dg_work.reserve(bytes))) return rc;
+    if (D.usable && (rc = H->dg_work.reserve(bytes)) != AHX_ERR_NOMEM) {
+      if (rc) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena32.p, H->dg_work);
       AHX_CUDA(launch_matvec_zt(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
       return AHX_OK;
