@@ -226,20 +226,26 @@ __global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
   }
 }
 
+template <typename SL, typename SD, typename A, bool TR, bool GUARD>
+void launch_groups(const MvArgs& a, uint32_t grid, cudaStream_t s) {
+  if (a.p == 1) mv_kernel<SL, SD, A, 1, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p == 2) mv_kernel<SL, SD, A, 2, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 4) mv_kernel<SL, SD, A, 4, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 8) mv_kernel<SL, SD, A, 8, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else mv_kernel<SL, SD, A, 16, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+}
+
 template <typename SL, typename SD, typename A, bool TR>
 cudaError_t launch_typed(const MvArgs& a, cudaStream_t s) {
   if (a.nleaves == 0 || a.p == 0) return cudaSuccess;
-  if (a.guard) {
-    mv_kernel<SL, SD, A, 8, TR, true><<<std::min(a.nleaves, 1024u), kThreads, 0, s>>>(a);
-    count_product_launches(1);
-    return cudaGetLastError();
+  if constexpr (sizeof(SL) == 8) {
+    if (a.guard) {
+      launch_groups<SL, SD, A, TR, true>(a, std::min(a.nleaves, kGuardCtas), s);
+      count_product_launches(1);
+      return cudaGetLastError();
+    }
   }
-  const uint32_t grid = a.nleaves;
-  if (a.p == 1) mv_kernel<SL, SD, A, 1, TR, false><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) mv_kernel<SL, SD, A, 2, TR, false><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) mv_kernel<SL, SD, A, 4, TR, false><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 8) mv_kernel<SL, SD, A, 8, TR, false><<<grid, kThreads, 0, s>>>(a);
-  else mv_kernel<SL, SD, A, 16, TR, false><<<grid, kThreads, 0, s>>>(a);
+  launch_groups<SL, SD, A, TR, false>(a, a.nleaves, s);
   count_product_launches(1);
   return cudaGetLastError();
 }

@@ -40,10 +40,16 @@ struct MvArgs {
   uint64_t ldY;
   uint32_t transposed = 0;  // 1: Y += d A^T X (H/mltaGeHVec.cpp:62-150)
   // when set: right-hand side r takes part only if guard[r / guard_cols] is not zero (few
-  // CTAs, a leaf loop; guard_cols a multiple of 8)
+  // CTAs, a leaf loop; guard_cols a multiple of 16).  FP64 leaves only.
   const int* guard = nullptr;
   uint32_t guard_cols = 0;
 };
+
+// CTAs of a guarded product: as many as the SMs hold of the plain kernels (128 threads, 32 to
+// 64 registers).  65,536 points, 5 right-hand sides that do not fit: 4.74 ms (digits' first
+// kernels included), with 152 * 12 CTAs 5.20, the plain kernel alone 4.11; 2: 1.37 and 1.11
+// (groups of 8 columns: 4.77); that nothing runs takes 2 us more than with 1,024 CTAs.
+constexpr uint32_t kGuardCtas = 152 * 16;
 
 cudaError_t launch_matvec(int prec, const MvArgs& a, cudaStream_t s);
 

@@ -241,18 +241,19 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(ZArg
   }
 }
 
+template <typename S, typename R, int OP, bool GUARD>
+void launch_groups(const ZArgs& a, uint32_t grid, cudaStream_t s) {
+  if (a.p == 1) zmv_kernel<S, R, 1, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p == 2) zmv_kernel<S, R, 2, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 4) zmv_kernel<S, R, 4, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
+  // wider groups (16) measured slower: fewer columns per pass, lower occupancy
+  else zmv_kernel<S, R, 8, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
+}
+
 template <typename S, typename R, int OP>
 void launch_op(const ZArgs& a, cudaStream_t s) {
-  if (a.guard) {
-    zmv_kernel<S, R, 4, OP, true><<<std::min(a.nleaves, 1024u), kThreads, 0, s>>>(a);
-    return;
-  }
-  const uint32_t grid = a.nleaves;
-  if (a.p == 1) zmv_kernel<S, R, 1, OP, false><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) zmv_kernel<S, R, 2, OP, false><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) zmv_kernel<S, R, 4, OP, false><<<grid, kThreads, 0, s>>>(a);
-  // wider groups (16) measured slower: fewer columns per pass, lower occupancy
-  else zmv_kernel<S, R, 8, OP, false><<<grid, kThreads, 0, s>>>(a);
+  if (a.guard) launch_groups<S, R, OP, true>(a, std::min(a.nleaves, kGuardCtas), s);
+  else launch_groups<S, R, OP, false>(a, a.nleaves, s);
 }
 
 template <typename S, typename R>
