@@ -113,22 +113,33 @@ constexpr uint32_t dg_pass_cols(bool cplx) { return cplx ? 8u : 16u; }
 inline const int* dg_flags(const DgPlan& pl) { return reinterpret_cast<const int*>(pl.work); }
 
 cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cudaStream_t s);
-// Every element of the leaves: *bad |= it is not finite, or not zero and outside [2^-500,
-// 2^500].  weight[i] (n of them, *wmax their maximum; kDgNoWeight to begin with): the binary
-// exponent of the largest entry that meets input row i, of a low-rank leaf P Q^H the largest
-// |Q_il| max |P_l|.
+// Looks at every element of the leaves.  weight[i] (n of them, kDgNoWeight to begin with): the
+// binary exponent of the largest entry that meets input row i, of a low-rank leaf P Q^H the
+// largest |Q_il| max |P_l|.
 constexpr int kDgNoWeight = (int)0x80808080;
+struct DgRange {
+  int wmax;  // largest weight (kDgNoWeight to begin with)
+  int bad;   // an element is not finite, or not zero and outside [2^-500, 2^500] (0)
+  int emax;  // largest exponent of an element (kDgNoWeight; 1024: not finite)
+  int drop;  // wmax - smallest weight other than kDgNoWeight (0)
+};
 cudaError_t launch_dg_weigh(const DgLeaf* leaves, uint32_t nleaves, bool cplx, const void* arena, int* weight,
-                            int* wmax, int* bad, cudaStream_t s);
+                            uint32_t n, DgRange* range, cudaStream_t s);
 cudaError_t launch_matvec_dg(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
 // FP64 leaves and one right-hand side over the same layout (ahx_matvec_f1.cu); pl.work:
 // dg_work_bytes
 cudaError_t launch_matvec_f1(const DgPlan& pl, double d, const double* X, double* Y, cudaStream_t s);
 bool f1_wanted(uint64_t elems, bool transposed);
 // complex64 leaves over the same layout (ahx_matvec_zt.cu; X, Y complex128): pl.arena the
-// complex64 copy, pl.work of zt_work_bytes
+// complex64 copy, pl.work of zt_work_bytes, control: zt_control_bytes, zero before the first
+// product (each leaves its counters zero).  Every kZtPassWords words of it belong to a pass of
+// kZtPassCols right-hand sides; the one at kZtFlagAt is as dg_flags (out of the range in which
+// split operands are exact to FP32).
+constexpr uint32_t kZtPassCols = 16, kZtPassWords = kZtPassCols + 2, kZtFlagAt = kZtPassCols + 1;
+size_t zt_control_bytes(uint32_t p);
+bool zt_fits(const DgRange& r);  // whether the leaves' elements are in that range
 size_t zt_work_bytes(uint32_t n, uint32_t t_rows, uint32_t p);
-cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, cudaStream_t s);
+cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, int* control, cudaStream_t s);
 bool zt_wanted(uint64_t elems, uint32_t p);
 
 }  // namespace ahx

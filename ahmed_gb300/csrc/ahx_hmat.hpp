@@ -117,6 +117,7 @@ struct DgState {
   double spent = 0.0;   // estimated us of the plain products before the layout
   DevBuf vpieces, rpieces, rowptr, pos, weight;
   uint32_t nv = 0, nr = 0, t_rows = 0, t_split = 0;
+  DgRange range{};
   bool rs1 = true;
   void release() {
     for (DevBuf* b : {&vpieces, &rpieces, &rowptr, &pos, &weight}) b->release();
@@ -137,6 +138,7 @@ struct ZState {
   uint64_t elems = 0;
   DevBuf arena32;                       // complex64 copy (AHX_FP32 storage)
   DevBuf xf;                            // X as complex64, 16 right-hand sides
+  DevBuf control;                       // of the complex64 products on the tensor cores
   bool valid32 = false;
   DevBuf leaves, order;                 // product leaf table, launch order
   uint32_t nleaves = 0;
@@ -155,7 +157,7 @@ struct ZState {
   }
   void release_all() {
     drop_table();
-    for (DevBuf* b : {&arena, &arena32, &xf, &leaves, &order, &tleaves, &torder, &gm, &xc}) b->release();
+    for (DevBuf* b : {&arena, &arena32, &xf, &control, &leaves, &order, &tleaves, &torder, &gm, &xc}) b->release();
     assembled = false;
     elems = 0;
     nleaves = ntleaves = 0;

@@ -90,8 +90,8 @@ struct ZArgs {
   double2* Y;
   uint64_t ldY;
   int op;
-  const int* guard = nullptr;  // as MvArgs::guard; complex128 leaves only
-  uint32_t guard_cols = 0;
+  const int* guard = nullptr;  // as MvArgs::guard, the words guard_step apart
+  uint32_t guard_cols = 0, guard_step = 1;
   uint64_t elems = 0;          // complex64 leaves: elements,
   uint32_t n = 0;              //   rows of X,
   float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes; null: none is made),

@@ -740,13 +740,18 @@ constexpr int kWeighThreads = 128;
 template <int CW>
 __global__ void __launch_bounds__(kWeighThreads)
     dg_weigh_kernel(const DgLeaf* __restrict__ leaves, const uint2* __restrict__ a, int* __restrict__ weight,
-                    int* __restrict__ wmax, int* __restrict__ bad) {
+                    DgRange* __restrict__ range) {
   constexpr uint32_t kL = 32, kW = kWeighThreads / 32;
   __shared__ int ep[kL];
   const DgLeaf q = leaves[blockIdx.x];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   bool b = false;
-  int most = kDgNoWeight;
+  int most = kDgNoWeight, top = 0;
+  auto look = [&](uint64_t at) -> int {
+    const int e = leaf_exp<CW>(a, at, b);
+    top = max(top, e);
+    return e;
+  };
   auto put = [&](uint32_t i, int w) {
     most = max(most, w);
     if (w > __ldcg(weight + i)) atomicMax(weight + i, w);
@@ -756,7 +761,7 @@ __global__ void __launch_bounds__(kWeighThreads)
       for (uint32_t j = warp; j < q.n2; j += kW) {
         int m = 0;
 #pragma unroll 2
-        for (uint32_t i = lane; i < q.n1; i += 32) m = max(m, leaf_exp<CW>(a, q.off + (uint64_t)j * q.n1 + i, b));
+        for (uint32_t i = lane; i < q.n1; i += 32) m = max(m, look(q.off + (uint64_t)j * q.n1 + i));
         m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0 && m) put(q.b2 + j, m - 1023);
       }
@@ -764,7 +769,7 @@ __global__ void __launch_bounds__(kWeighThreads)
       for (uint32_t i = tid; i < q.n1; i += kWeighThreads) {
         int m = 0;
 #pragma unroll 4
-        for (uint32_t j = 0; j < q.n2; ++j) m = max(m, leaf_exp<CW>(a, q.off + (uint64_t)j * q.n1 + i, b));
+        for (uint32_t j = 0; j < q.n2; ++j) m = max(m, look(q.off + (uint64_t)j * q.n1 + i));
         if (m) put(q.b1 + i, m - 1023);
       }
     }
@@ -779,7 +784,7 @@ __global__ void __launch_bounds__(kWeighThreads)
       for (uint32_t l = warp; l < ln; l += kW) {
         int m = 0;
 #pragma unroll 2
-        for (uint32_t i = lane; i < on; i += 32) m = max(m, leaf_exp<CW>(a, P + (uint64_t)(l0 + l) * on + i, b));
+        for (uint32_t i = lane; i < on; i += 32) m = max(m, look(P + (uint64_t)(l0 + l) * on + i));
         m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0) ep[l] = m;
       }
@@ -788,7 +793,7 @@ __global__ void __launch_bounds__(kWeighThreads)
         int m = 0;
 #pragma unroll 4
         for (uint32_t l = 0; l < ln; ++l) {
-          const int e = leaf_exp<CW>(a, Q + (uint64_t)(l0 + l) * in + j, b);
+          const int e = look(Q + (uint64_t)(l0 + l) * in + j);
           if (e && ep[l]) m = max(m, e + ep[l]);
         }
         if (m) put(ib + j, m - 2046);
@@ -797,11 +802,24 @@ __global__ void __launch_bounds__(kWeighThreads)
     }
   }
   most = __reduce_max_sync(0xffffffffu, most);
+  top = __reduce_max_sync(0xffffffffu, top);
   const bool any = __any_sync(0xffffffffu, b);
   if (lane == 0) {
-    if (most > __ldcg(wmax)) atomicMax(wmax, most);
-    if (any) atomicOr(bad, 1);
+    if (most > __ldcg(&range->wmax)) atomicMax(&range->wmax, most);
+    if (top && top - 1023 > __ldcg(&range->emax)) atomicMax(&range->emax, top - 1023);
+    if (any) atomicOr(&range->bad, 1);
   }
+}
+
+__global__ void dg_drop_kernel(const int* __restrict__ weight, uint32_t n, DgRange* __restrict__ range) {
+  const int wmax = range->wmax;
+  int drop = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const int w = weight[i];
+    if (w != kDgNoWeight) drop = max(drop, wmax - w);
+  }
+  drop = __reduce_max_sync(0xffffffffu, drop);
+  if ((threadIdx.x & 31) == 0 && drop) atomicMax(&range->drop, drop);
 }
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -923,11 +941,12 @@ cudaError_t launch_dg_expand(const DgSeg* segs, uint32_t nsegs, DgPos* pos, cuda
 }
 
 cudaError_t launch_dg_weigh(const DgLeaf* leaves, uint32_t nleaves, bool cplx, const void* arena, int* weight,
-                            int* wmax, int* bad, cudaStream_t s) {
+                            uint32_t n, DgRange* range, cudaStream_t s) {
   if (!nleaves) return cudaSuccess;
   const uint2* a = static_cast<const uint2*>(arena);
-  if (cplx) dg_weigh_kernel<2><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, wmax, bad);
-  else dg_weigh_kernel<1><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, wmax, bad);
+  if (cplx) dg_weigh_kernel<2><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, range);
+  else dg_weigh_kernel<1><<<nleaves, kWeighThreads, 0, s>>>(leaves, a, weight, range);
+  dg_drop_kernel<<<std::min((n + 255) / 256, 152u), 256, 0, s>>>(weight, n, range);
   return cudaGetLastError();
 }
 
@@ -974,16 +993,17 @@ static int build_state(DgState& D, const std::vector<DgLeaf>& leaves, uint32_t n
   DgHost L;
   D.release();
   ScopedBuf segs, dl;
-  int bad = 0;
-  if ((rc = upload(dl, leaves, s)) || (rc = D.weight.reserve(((size_t)n + 2) * sizeof(int)))) return rc;
+  if ((rc = upload(dl, leaves, s)) || (rc = D.weight.reserve((size_t)n * sizeof(int) + sizeof(DgRange)))) return rc;
   int* const w = D.weight.as<int>();
-  AHX_CUDA(cudaMemsetAsync(w, kDgNoWeight & 0xff, ((size_t)n + 1) * sizeof(int), s));
-  AHX_CUDA(cudaMemsetAsync(w + n + 1, 0, sizeof(int), s));
-  AHX_CUDA(launch_dg_weigh(dl.as<DgLeaf>(), (uint32_t)leaves.size(), cplx, arena, w, w + n, w + n + 1, s));
+  DgRange* const range = reinterpret_cast<DgRange*>(w + n);
+  D.range = DgRange{kDgNoWeight, 0, kDgNoWeight, 0};
+  AHX_CUDA(cudaMemsetAsync(w, kDgNoWeight & 0xff, (size_t)n * sizeof(int), s));
+  AHX_CUDA(cudaMemcpyAsync(range, &D.range, sizeof(DgRange), cudaMemcpyHostToDevice, s));
+  AHX_CUDA(launch_dg_weigh(dl.as<DgLeaf>(), (uint32_t)leaves.size(), cplx, arena, w, n, range, s));
   const bool fits = build_dg_layout(leaves, n, (uint32_t)std::max(sms, 1) * 16, cplx ? kDgK / 2 : kDgK, L);
-  AHX_CUDA(cudaMemcpyAsync(&bad, w + n + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  AHX_CUDA(cudaMemcpyAsync(&D.range, range, sizeof(DgRange), cudaMemcpyDeviceToHost, s));
   AHX_CUDA(cudaStreamSynchronize(s));
-  finite = bad ? 2 : 1;
+  finite = D.range.bad ? 2 : 1;
   if (!fits) {
     D.valid = true;
     return AHX_OK;

@@ -127,7 +127,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
   const uint32_t ro = kFwd ? L.b1 : L.b2, nr = kFwd ? L.n1 : L.n2;
   const uint32_t co = kFwd ? L.b2 : L.b1, nc = kFwd ? L.n2 : L.n1;
   for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
-    if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
+    if (GUARD && !a.guard[r0 / a.guard_cols * a.guard_step]) continue;
     const uint32_t pg = min((uint32_t)PG, a.p - r0);
     if (L.rank < 0) {
       // dense: thread per output row; the forward product reads D by rows
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(ZArg
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
   if (GUARD) {
     bool any = false;
-    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q];
+    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q * a.guard_step];
     if (!__syncthreads_or(any)) return;
     for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP, true, PRE>(a, l, Xs, Ts, red);
   } else {
@@ -252,7 +252,9 @@ void launch_groups(const ZArgs& a, uint32_t grid, cudaStream_t s) {
 
 template <typename S, typename R, int OP>
 void launch_op(const ZArgs& a, cudaStream_t s) {
-  if (a.guard) launch_groups<S, R, OP, true>(a, std::min(a.nleaves, kGuardCtas), s);
+  // (complex64: only after right-hand sides of 2^40 or infinity, so that a short launch counts more)
+  constexpr uint32_t kCtas = sizeof(R) == 4 ? 152 * 4 : kGuardCtas;
+  if (a.guard) launch_groups<S, R, OP, true>(a, std::min(a.nleaves, kCtas), s);
   else launch_groups<S, R, OP, false>(a, a.nleaves, s);
 }
 
@@ -302,7 +304,7 @@ cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
     count_product_launches(1);
     return cudaGetLastError();
   }
-  if (a.p <= 4 || a.elems * a.p < 30000000ull || !a.xf) {
+  if (a.guard || a.p <= 4 || a.elems * a.p < 30000000ull || !a.xf) {
     launch_typed<float2, float>(a, s);
     count_product_launches(1);
     return cudaGetLastError();

@@ -13,17 +13,23 @@
 // load, full sectors in either sweep.
 //
 // Accuracy: a = ah + al with ah its 11 bits to nearest, and al bh + ah bl + ah bh is
-// summed over one step (8 positions) by the tensor core, steps and then chunks of eight by
-// FP32 additions: what is left out (al bl, the last bits of al and bl) is 2^-24 of a
-// term, and no long sum is truncated or rounded at every term.  Against the complex128
-// product: 1.3e-7 (4,096 points) and 1.5e-7 (16,384), the plain kernel 1.9e-7 in both;
-// truncated splits gave 4.8e-7, one FP32 sum per piece 2.3e-7.
+// summed over one step (8 positions) by the tensor core, steps by FP32 additions, chunks of
+// eight by FP32 additions whose rounding goes on into the next chunk: what is left out (al
+// bl, the last bits of al and bl) is 2^-24 of a term, and no long sum is rounded at every
+// term.  Against the complex128 product on the same leaves (8 right-hand sides, 1,024 to
+// 16,384 points on sphere, cube and ellipsoid, k 1 to 12; norms per right-hand side):
+//   random vectors   1.2e-7 to 1.9e-7   the plain kernel 1.9e-7 to 3.0e-7
+//   plane waves      6e-8 to 1.0e-7                      5e-8 to 3.5e-7
+//   constants        7e-8 to 1.0e-7                      3e-8 to 3.1e-7
+// 5e-8 of it is that the tensor core cuts its sums off (a second MMA that finds half a unit
+// of each sum to add halves plane waves' and takes 13 % longer); truncated splits
+// gave 4.8e-7, one FP32 sum per piece 2.3e-7.
 //
 // What bounds it: latency (DRAM 22 %, tensor 30 % busy; 27 warps a multiprocessor).  The
 // plain kernel (ahx_matvec_z.cu) reads X and adds to Y once per leaf; its atomic
 // additions and shared-memory broadcasts take 72 % of the L1's bandwidth.  Here a row of
 // Y meets a few dozen additions, and leaf values go from memory into fragments.
-// 16,384 points (474 MB): 16 right-hand sides 462 -> 305 us, 8: 269 -> 207 us.
+// 16,384 points (445 MB): 16 right-hand sides 433 -> 296 us, 8: 253 -> 199 us (cold caches).
 #include <algorithm>
 
 #include "ahx_dg.cuh"
@@ -34,7 +40,17 @@ namespace {
 
 constexpr int kThreads = 2 * kDgRows;
 constexpr uint32_t kCE = 32;     // elements per staged chunk
-constexpr uint32_t kBlock = 16;  // right-hand sides per pass
+constexpr uint32_t kBlock = kZtPassCols;  // right-hand sides per pass
+
+// Range.  The low part of a split operand must not fall below FP32's normal numbers, no sum
+// may reach infinity, and an infinite or NaN operand has no split (inf - inf; the GPU's NaN
+// 0x7fffffff rounds to -0).  So: elements of the leaves up to 2^kExp and a largest entry of
+// 2^-kExp at least in every column (zt_fits), right-hand sides whose largest entries lie in
+// [2^-kExp, 2^kExp] or are zero (zt_x_kernel), V^H X below 2^kTExp a piece (the V sweep).  A pass of
+// other right-hand sides raises its flag before anything is added to Y, and the plain kernel
+// runs instead.
+constexpr int kExp = 40, kTExp = 50;
+constexpr uint32_t kXLeast = (uint32_t)(127 - kExp) << 23, kXMost = (uint32_t)(127 + kExp) << 23;
 
 // floats of a staged Z row: four rows apart in the banks, 16-byte multiples
 template <int NT>
@@ -45,6 +61,7 @@ struct KArgs {
   const uint64_t* rowptr;
   const DgPos* pos;
   const float2* arena;
+  int* flag;    // of the pass (zt_x_kernel writes it)
   float* z;     // Z rows of 8 NT floats: X rows, then T rows (at zt)
   float* zt;
   double2* Y;   // first column of the pass
@@ -78,7 +95,9 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
   constexpr int ZS = kZS<NT>;
   __shared__ __align__(16) float z[2][kCE * ZS];
   __shared__ __align__(16) DgPos pos[3][kCE];
+  __shared__ float sum[NT * 4][kThreads];  // of the chunks before (registers would be spilled)
   const DgPiece pc = a.pieces[blockIdx.x];
+  const int out_of_range = *a.flag;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
   const uint32_t nch = (pc.kn + kCE - 1) / kCE;
   // this lane's rows of the fragment (rows past the tile repeat its last one)
@@ -138,11 +157,11 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
       v[s][1].y = __uint_as_float(__float_as_uint(v[s][1].y) ^ sb);
     }
   };
-  float acc[NT][4], sum[NT][4];  // of the present chunk, of the ones before
+  float acc[NT][4];  // of the present chunk
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[t][j] = sum[t][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[t][j] = sum[4 * t + j][tid] = 0.f;
   auto multiply = [&](const float2 (&v)[4][2], uint32_t ch, uint32_t h) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
@@ -172,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
   copy_pos(1);
   cp_commit();
   cp_wait_all();
-  __syncthreads();
+  if (__syncthreads_or(out_of_range)) return;  // (the V sweep may raise it meanwhile)
   copy_z(0);
   cp_commit();
   if (active) {
@@ -194,8 +213,9 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
     for (int t = 0; t < NT; ++t)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        sum[t][j] += acc[t][j];
-        acc[t][j] = 0.f;
+        const float old = sum[4 * t + j][tid], s = old + acc[t][j];
+        acc[t][j] -= s - old;  // (what the addition rounded off goes on with the next chunk)
+        sum[4 * t + j][tid] = s;
       }
   }
   if (!active) return;
@@ -206,8 +226,9 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
     for (int h = 0; h < 2; ++h) {
       const uint32_t row = warp * 16 + g + 8 * h;
       if (row >= pc.nrows) continue;
-      const float2 v = make_float2(sum[t][2 * h] + acc[t][2 * h], sum[t][2 * h + 1] + acc[t][2 * h + 1]);
+      const float2 v = make_float2(sum[4 * t + 2 * h][tid] + acc[t][2 * h], sum[4 * t + 2 * h + 1][tid] + acc[t][2 * h + 1]);
       if (!ROWS) {
+        if (!(fmaxf(fabsf(v.x), fabsf(v.y)) < (float)(1ull << kTExp))) atomicOr(a.flag, 1);
         float2* T = reinterpret_cast<float2*>(a.zt + (uint64_t)(pc.row0 + row) * (8 * NT) + 8 * t + 2 * c);
         if (pc.add) atomicAdd(T, v);
         else *T = v;
@@ -226,10 +247,14 @@ __global__ void __launch_bounds__(kThreads, 9) zt_sweep_kernel(const KArgs a) {
   }
 }
 
-// Z rows of X: z[row][r] = (complex64) X[row, r], zero for p <= r < W
-__global__ void zt_x_kernel(const double2* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t p, uint32_t W,
-                            float2* __restrict__ z) {
+// Z rows of X: z[row][r] = (complex64) X[row, r], zero for p <= r < W.  most[r]: the largest
+// part of column r (as bits: NaN above infinity); the last CTA looks whether they are in range.
+// (128 threads: a warp has 32 rows of one column at a time)
+__global__ void __launch_bounds__(128) zt_x_kernel(const double2* __restrict__ X, uint64_t ldX, uint32_t n, uint32_t p,
+                                                   uint32_t W, float2* __restrict__ z, uint32_t* __restrict__ most,
+                                                   uint32_t* __restrict__ ticket, int* __restrict__ flag) {
   __shared__ float2 t[32][kBlock + 1];
+  __shared__ uint32_t part[kBlock];
   const uint32_t row0 = blockIdx.x * 32;
   for (uint32_t e = threadIdx.x; e < 32 * W; e += blockDim.x) {
     const uint32_t i = e & 31, r = e >> 5;
@@ -239,19 +264,45 @@ __global__ void zt_x_kernel(const double2* __restrict__ X, uint64_t ldX, uint32_
       v = make_float2((float)x.x, (float)x.y);
     }
     t[i][r] = v;
+    const uint32_t m = __reduce_max_sync(
+        0xffffffffu, max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu));
+    if (i == 0) part[r] = m;
   }
   __syncthreads();
+  if (threadIdx.x < p && part[threadIdx.x]) atomicMax(most + threadIdx.x, part[threadIdx.x]);
   for (uint32_t e = threadIdx.x; e < 32 * W; e += blockDim.x) {
     const uint32_t i = e / W, r = e - i * W;
     if (row0 + i < n) z[(uint64_t)(row0 + i) * W + r] = t[i][r];
   }
+  if (threadIdx.x >= 32) return;
+  __threadfence();
+  __syncwarp();
+  uint32_t last = threadIdx.x == 0 ? (atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u) : 0u;
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  bool bad = false;
+  if (threadIdx.x < p) {
+    const uint32_t m = __ldcg(most + threadIdx.x);
+    bad = m != 0u && (m < kXLeast || m > kXMost);
+    most[threadIdx.x] = 0u;  // (for the next product)
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    *flag = bad;
+  }
 }
+
+// Control words of a pass: column maxima and ticket (zero between products), flag
+constexpr uint32_t kPassWords = kZtPassWords;
+static_assert(kZtFlagAt == kBlock + 1 && kPassWords == kBlock + 2, "maxima, ticket, flag");
 
 int nt_of(uint32_t p) { return p <= 4 ? 1 : p <= 8 ? 2 : 4; }
 
 template <int NT>
-cudaError_t pass(const DgPlan& pl, KArgs k, const double2* X, uint64_t ldX, cudaStream_t s) {
-  zt_x_kernel<<<(pl.n + 31) / 32, 128, 0, s>>>(X, ldX, pl.n, k.p, 4 * NT, reinterpret_cast<float2*>(k.z));
+cudaError_t pass(const DgPlan& pl, KArgs k, uint32_t* most, const double2* X, uint64_t ldX, cudaStream_t s) {
+  zt_x_kernel<<<(pl.n + 31) / 32, 128, 0, s>>>(X, ldX, pl.n, k.p, 4 * NT, reinterpret_cast<float2*>(k.z), most,
+                                               most + kBlock, k.flag);
   k.zt = k.z + (uint64_t)pl.n * (8 * NT);
   cudaError_t e;
   if (pl.nv) {
@@ -270,8 +321,11 @@ cudaError_t pass(const DgPlan& pl, KArgs k, const double2* X, uint64_t ldX, cuda
 }  // namespace
 
 size_t zt_work_bytes(uint32_t n, uint32_t t_rows, uint32_t p) { return ((size_t)n + t_rows) * nt_of(p) * 32; }
+size_t zt_control_bytes(uint32_t p) { return ((size_t)p + kBlock - 1) / kBlock * kPassWords * sizeof(int); }
 
-cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, cudaStream_t s) {
+bool zt_fits(const DgRange& r) { return r.emax <= kExp && r.wmax - r.drop >= -kExp; }
+
+cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, int* control, cudaStream_t s) {
   const double2* X = static_cast<const double2*>(a.X);
   double2* Y = static_cast<double2*>(a.Y);
   KArgs k{};
@@ -279,6 +333,7 @@ cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, cudaStream_t s) 
   k.pos = pl.pos;
   k.arena = static_cast<const float2*>(pl.arena);
   k.z = reinterpret_cast<float*>(pl.work);
+  cudaError_t e;
   k.ldY = a.ldY;
   k.dre = a.dre;
   k.dim = a.dim;
@@ -287,19 +342,23 @@ cudaError_t launch_matvec_zt(const DgPlan& pl, const DgArgs& a, cudaStream_t s) 
     k.p = std::min(kBlock, a.p - r0);
     k.Y = Y + (uint64_t)r0 * a.ldY;
     const double2* x = X + (uint64_t)r0 * a.ldX;
+    uint32_t* const most = reinterpret_cast<uint32_t*>(control) + r0 / kBlock * kPassWords;
+    k.flag = control + r0 / kBlock * kPassWords + kZtFlagAt;
     const int nt = nt_of(k.p);
-    const cudaError_t e = nt == 1   ? pass<1>(pl, k, x, a.ldX, s)
-                          : nt == 2 ? pass<2>(pl, k, x, a.ldX, s)
-                                    : pass<4>(pl, k, x, a.ldX, s);
+    e = nt == 1 ? pass<1>(pl, k, most, x, a.ldX, s)
+        : nt == 2 ? pass<2>(pl, k, most, x, a.ldX, s)
+                  : pass<4>(pl, k, most, x, a.ldX, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
-// Five right-hand sides and 9 10^7 (complex elements x right-hand sides) on.  4,096 points
-// (10^7 elements): p = 5: 84 us against 71 of the plain kernel, p = 8: 82 against 75, p =
-// 11: 107 against 124; 16,384 points: p = 3: 222 against 171, p = 5: 207 against 256.
-// AHX_ZT_MIN overrides both (and lays out at the first product).
+// Five right-hand sides and 9 10^7 (complex elements x right-hand sides) on.  Where the line
+// is best depends on the leaves (cold caches; this against the plain kernel): sphere of 4,096
+// points (10^7 elements), p = 8: 70 us against 58, 16: 94 against 91; of 6,007, 8: 105
+// against 86, 16: 146 against 135; of 9,000, 5: 123 against 127, 16: 171 against 218; cube
+// surface of 6,007 points, 5: 111 against 122, 16: 153 against 204; of 9,000, 5: 140 against
+// 196.  AHX_ZT_MIN overrides both (and lays out at the first product).
 bool zt_wanted(uint64_t elems, uint32_t p) {
   const char* e = std::getenv("AHX_ZT_MIN");
   if (e && *e) return elems * p >= std::strtoull(e, nullptr, 10);

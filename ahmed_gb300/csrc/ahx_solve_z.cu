@@ -159,6 +159,16 @@ int prepare_z(ahx_hmat* H, int prec) {
   return AHX_OK;
 }
 
+// Work buffer and control words of a complex64 product on the tensor cores.
+int zt_room(ahx_hmat* H, size_t bytes, uint32_t p) {
+  DevBuf& c = H->z.control;
+  const size_t cb = zt_control_bytes(p), had = c.bytes;
+  int rc;
+  if ((rc = H->dg_work.reserve(bytes)) || (rc = c.reserve(cb))) return rc;
+  if (c.bytes != had) AHX_CUDA(cudaMemsetAsync(c.p, 0, c.bytes, H->stream));
+  return AHX_OK;
+}
+
 int check_z(const ahx_hmat* H, int prec, const char* who) {
   if (!H->z.assembled) {
     set_error(std::string(who) + ": Helmholtz leaves not assembled");
@@ -384,6 +394,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
     return dg_prepare_state(D, lv, (uint32_t)n, Z.arena.p, true, Z.finite, H->device, H->stream);
   };
   const int* guard = nullptr;
+  uint32_t guard_cols = dg_pass_cols(true), guard_step = 1;
   if (prec == kFP64 && Z.finite != 2 && dg_wanted(4 * Z.elems, p) && laid_out(4 * Z.elems)) {
     // the plain kernels then only run when X does not fit the digits
     if ((rc = layout())) return rc;
@@ -395,15 +406,18 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
       guard = dg_flags(pl);
     }
   }
-  // (the plain complex64 kernel costs a third of what dg_due counts for real elements)
+  // (the plain complex64 kernel costs a third of what dg_due counts for real elements; it then
+  // only takes the right-hand sides that are out of range)
   if (prec == kFP32 && zt_wanted(Z.elems, p) && laid_out(Z.elems / 3)) {
     if ((rc = layout())) return rc;
     const size_t bytes = zt_work_bytes(n, D.t_rows, p);
-    if (D.usable && (rc = H->dg_work.reserve(bytes)) != AHX_ERR_NOMEM) {
+    if (D.usable && zt_fits(D.range) && (rc = zt_room(H, bytes, p)) != AHX_ERR_NOMEM) {
       if (rc) return rc;
       const DgPlan pl = dg_plan(D, n, Z.arena32.p, H->dg_work);
-      AHX_CUDA(launch_matvec_zt(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, H->stream));
-      return AHX_OK;
+      AHX_CUDA(launch_matvec_zt(pl, DgArgs{true, dre, dim, p, X, ldX, Y, ldY}, Z.control.as<int>(), H->stream));
+      guard = Z.control.as<int>() + kZtFlagAt;
+      guard_cols = kZtPassCols;
+      guard_step = kZtPassWords;
     }
   }
   ZArgs a;
@@ -421,7 +435,8 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.ldY = ldY;
   a.op = op;
   a.guard = guard;
-  a.guard_cols = dg_pass_cols(true);
+  a.guard_cols = guard_cols;
+  a.guard_step = guard_step;
   a.elems = Z.elems;
   a.n = (uint32_t)n;
   a.xf = captured ? nullptr : Z.xf.as<float2>();
