@@ -45,22 +45,32 @@ __device__ __forceinline__ double rsqrt_seeded(double x) {
 }
 
 // r = sqrt(r2) and s = 1 / (4 pi r), every operation rounded to nearest, so that entries
-// equal the host's bit for bit.  One reciprocal square root serves both: the final
-// steps r + (r2 - r^2) y / 2 and z + z (1 - t z) (Markstein) leave the unrounded results
-// within 2^-104 of the exact ones.  21 FP64 instructions an entry; with the mirror images
-// written by the same task, the dense leaves of 65,536 points take 2.7 ms instead of 5.1.
-// (The general case is a function of its own: predicated in line its FP64 instructions
-// would occupy the pipe for every entry.)
+// equal the host's bit for bit.  One reciprocal square root serves both, by the final steps
+// r + (r2 - r^2) y / 2 and z + z (1 - t z) (Markstein).
+//   root: before its last rounding within 2^-102.  Arguments X 2^q whose root lies closer to
+//     the middle of two doubles have M^2 = X 2^q + c with M odd of 54 bits, |c| < 95: 37 in
+//     all, which all round right.
+//   reciprocal: z is off by up to 2.6 2^-53, the result before rounding by its square; that
+//     rounds wrong for some t (T M = 2^106 - 2: T = 5276938686109394).  So the remainder 1 -
+//     t s, which is exact, is looked at: below half a unit of s times t (by its high word, one
+//     in 2^18 is not) s is the rounded one, otherwise the division decides.
+// 22 FP64 instructions an entry; with the mirror images written by the same task, the dense
+// leaves of 65,536 points take 2.7 ms instead of 5.1.  (The general case is a function of
+// its own: predicated in line its FP64 instructions would occupy the pipe for every entry.)
 static __device__ __noinline__ double2 rounded_r_s_any(double r2) {
   const double r = __dsqrt_rn(r2);
   return make_double2(r, __ddiv_rn(1.0, __dmul_rn(kFourPi, r)));
 }
+static __device__ __noinline__ double reciprocal_rounded(double t) { return __ddiv_rn(1.0, t); }
 __device__ __forceinline__ void rounded_r_s(double r2, double& r, double& s) {
   if (f32_range(r2)) {
     const double y = rsqrt_seeded(r2), g = __dmul_rn(r2, y);
     r = fma(fma(-g, g, r2), 0.5 * y, g);
     const double t = __dmul_rn(kFourPi, r), z = __dmul_rn(1.0 / kFourPi, y);
     s = fma(z, fma(-t, z, 1.0), z);
+    const int left = __double2hiint(fma(-t, s, 1.0)) & 0x7fffffff;
+    const int half = __double2hiint(t) + (__double2hiint(s) & 0x7ff00000) - ((1023 + 53) << 20);  // t ulp(s) / 2
+    if (left >= half) s = reciprocal_rounded(t);
   } else {
     const double2 v = rounded_r_s_any(r2);
     r = v.x;
