@@ -32,7 +32,7 @@ struct Sorted {
     std::vector<uint64_t> size(in.size());
     for (size_t i = 0; i < in.size(); ++i) size[i] = aca_ws_bytes(in[i].n1, in[i].n2, in[i].kcap, elem);
     std::vector<uint32_t> ord;
-    order_by_size(size, ord);
+    order_by_size(size, ord, 4);
     for (size_t i = 0; i < in.size(); ++i) {
       t[i] = in[ord[i]];
       bytes[i] = class_bytes(size_class(size[ord[i]]));
@@ -64,17 +64,23 @@ struct Sorted {
 
 }  // namespace
 
-uint32_t size_class(uint64_t size) {
-  const int m = 63 - __builtin_clzll(size | 16);
-  return (uint32_t)(m * 16) + (uint32_t)((size >> (m - 4)) & 15);
+namespace {
+// the leading 1 + bits binary digits of size, as a number that grows with it (below 2^bits: size)
+inline uint32_t leading(uint64_t size, int bits) {
+  const int m = 63 - __builtin_clzll(size | (1ull << bits));
+  return (uint32_t)(m << bits) + (uint32_t)((size >> (m - bits)) & ((1u << bits) - 1));
 }
+}  // namespace
 
-void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order) {
-  std::vector<uint32_t> at(1025, 0);
-  for (uint64_t s : size) ++at[1024 - size_class(s)];
-  for (size_t c = 0; c < 1024; ++c) at[c + 1] += at[c];
+uint32_t size_class(uint64_t size) { return leading(size, 4); }
+
+void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order, int bits) {
+  const uint32_t n = 64u << bits;
+  std::vector<uint32_t> at(n + 1, 0);
+  for (uint64_t s : size) ++at[n - leading(s, bits)];
+  for (uint32_t c = 0; c < n; ++c) at[c + 1] += at[c];
   order.resize(size.size());
-  for (size_t i = 0; i < size.size(); ++i) order[at[1023 - size_class(size[i])]++] = (uint32_t)i;
+  for (size_t i = 0; i < size.size(); ++i) order[at[n - 1 - leading(size[i], bits)]++] = (uint32_t)i;
 }
 
 std::vector<DenseTask> dense_tasks(const std::vector<Leaf>& Ls, uint32_t n, const std::vector<uint32_t>& leaves,

@@ -281,9 +281,10 @@ int prepare_df_x(ahx::ProdCopy& pc, uint64_t n, uint32_t p);
 int run_df(const ahx::MvLeaf* leaves, const uint32_t* order, uint32_t nleaves, ahx::ProdCopy& pc, uint64_t n,
            double d, uint32_t p, const double* X, uint64_t ldX, double* Y, uint64_t ldY, cudaStream_t s);
 int ensure_device(ahx_hmat* H);
-// order: the indices of `size` by descending size_class, equal ones in order; linear time
 uint32_t size_class(uint64_t size);  // 16 classes per octave
-void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order);
+// order: the indices of `size` by descending size in steps of 2^-bits octave, equal ones in
+// order; linear time
+void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order, int bits);
 // ACA + recompression of `tasks` into the leaf arena (cplx: the Helmholtz one), retried
 // with more columns where they overflow; failed leaves are appended to `dense`
 struct AcaTask;
