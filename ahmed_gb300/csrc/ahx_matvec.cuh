@@ -90,14 +90,21 @@ struct ZArgs {
   double2* Y;
   uint64_t ldY;
   int op;
-  const int* guard = nullptr;  // as MvArgs::guard, the words guard_step apart
-  uint32_t guard_cols = 0, guard_step = 1;
+};
+// (apart from ZArgs: fields beside those changed the registers that the compiler gives the
+// plain kernels, 36 to 32 for A^T with one right-hand side, and with them their times by
+// -10 to +27 %)
+struct ZGuard {
+  const int* flags;        // as MvArgs::guard, the words `step` apart
+  uint32_t cols, step;
+};
+struct ZRun : ZArgs {
+  ZGuard guard{nullptr, 0u, 1u};
   uint64_t elems = 0;          // complex64 leaves: elements,
   uint32_t n = 0;              //   rows of X,
-  float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes; null: none is made),
-  bool d_one = false;          //   d = 1 (set by the launcher)
+  float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes; null: none is made)
 };
-cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s);
+cudaError_t launch_matvec_z(const ZRun& a, cudaStream_t s);
 size_t matvec_z_xf_bytes(uint64_t n);
 // dst[i] = (float) src[i], complex128 -> complex64
 cudaError_t launch_z_to_c64(const double2* src, uint64_t n, float2* dst, cudaStream_t s);

@@ -72,13 +72,17 @@ __device__ __noinline__ void scale_pair(double dre, double dim, double& ar, doub
 
 // Xs[j][r] = X[row0 + j, r0 + r] for j < jn (zero for r >= pg); PRE: from the rounded
 // copy, rows of kXW
+struct Rounded {
+  const float2* xf;
+  bool d_one;  // d = 1
+};
 template <typename R, int PG, bool PRE>
-__device__ __forceinline__ void stage(C2<R> (*Xs)[PG], const ZArgs& a, uint32_t r0, uint32_t pg, uint32_t row0,
-                                      uint32_t jn) {
+__device__ __forceinline__ void stage(C2<R> (*Xs)[PG], const ZArgs& a, const Rounded& w, uint32_t r0, uint32_t pg,
+                                      uint32_t row0, uint32_t jn) {
   if constexpr (PRE) {
     for (uint32_t e = threadIdx.x; e < jn * PG; e += kThreads) {
       const uint32_t j = e / PG, r = e % PG;
-      const float2 x = __ldg(a.xf + (uint64_t)(row0 + j) * kXW + r0 + r);
+      const float2 x = __ldg(w.xf + (uint64_t)(row0 + j) * kXW + r0 + r);
       Xs[j][r] = C2<R>{x.x, x.y};
     }
   } else {
@@ -96,7 +100,8 @@ __device__ __forceinline__ void stage(C2<R> (*Xs)[PG], const ZArgs& a, uint32_t 
 
 // Y[row, r0 + r] += d acc[r]
 template <typename R, int PG, bool PRE>
-__device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, uint64_t row, const C2<R>* acc) {
+__device__ __forceinline__ void emit(const ZArgs& a, const Rounded& w, uint32_t r0, uint32_t pg, uint64_t row,
+                                     const C2<R>* acc) {
 #pragma unroll
   for (int r = 0; r < PG; ++r) {
     if ((uint32_t)r < pg) {
@@ -104,7 +109,7 @@ __device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, u
       if constexpr (PRE) {
         ar = widen(acc[r].re);
         ai = widen(acc[r].im);
-        if (!a.d_one) scale_pair(a.dre, a.dim, ar, ai);
+        if (!w.d_one) scale_pair(a.dre, a.dim, ar, ai);
       } else {
         const double xr = (double)acc[r].re, xi = (double)acc[r].im;
         ar = a.dre * xr - a.dim * xi;
@@ -118,7 +123,8 @@ __device__ __forceinline__ void emit(const ZArgs& a, uint32_t r0, uint32_t pg, u
 }
 
 template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE>
-__device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
+__device__ __forceinline__ void zmv_leaf(const ZArgs& a, const ZGuard& gd, const Rounded& w, uint32_t leaf,
+                                         C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
   const MvLeaf L = a.leaves[a.order[leaf]];
   const S* base = reinterpret_cast<const S*>(a.arena) + L.off;
   const uint32_t tid = threadIdx.x;
@@ -127,7 +133,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
   const uint32_t ro = kFwd ? L.b1 : L.b2, nr = kFwd ? L.n1 : L.n2;
   const uint32_t co = kFwd ? L.b2 : L.b1, nc = kFwd ? L.n2 : L.n1;
   for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
-    if (GUARD && !a.guard[r0 / a.guard_cols * a.guard_step]) continue;
+    if (GUARD && !gd.flags[r0 / gd.cols * gd.step]) continue;
     const uint32_t pg = min((uint32_t)PG, a.p - r0);
     if (L.rank < 0) {
       // dense: thread per output row; the forward product reads D by rows
@@ -140,7 +146,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
         for (uint32_t jb = 0; jb < nc; jb += kCh) {
           const uint32_t jn = min((uint32_t)kCh, nc - jb);
           __syncthreads();
-          stage<R, PG, PRE>(Xs, a, r0, pg, co + jb, jn);
+          stage<R, PG, PRE>(Xs, a, w, r0, pg, co + jb, jn);
           __syncthreads();
           if (i < nr) {
             for (uint32_t j = 0; j < jn; ++j) {
@@ -151,7 +157,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
             }
           }
         }
-        if (i < nr) emit<R, PG, PRE>(a, r0, pg, ro + i, acc);
+        if (i < nr) emit<R, PG, PRE>(a, w, r0, pg, ro + i, acc);
       }
     } else if (L.rank > 0) {
       const uint32_t k = (uint32_t)L.rank;
@@ -172,7 +178,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
         for (uint32_t jb = 0; jb < nc; jb += kCh) {
           const uint32_t jn = min((uint32_t)kCh, nc - jb);
           __syncthreads();
-          stage<R, PG, PRE>(Xs, a, r0, pg, co + jb, jn);
+          stage<R, PG, PRE>(Xs, a, w, r0, pg, co + jb, jn);
           __syncthreads();
           if (sub < ns) {
             const S* qc = Q + (uint64_t)(lb + l) * nc + jb;
@@ -210,7 +216,7 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
 #pragma unroll
               for (int rr = 0; rr < PG; ++rr) cfma(acc[rr], pv, Ts[ll * PG + rr]);
             }
-            emit<R, PG, PRE>(a, r0, pg, ro + i, acc);
+            emit<R, PG, PRE>(a, w, r0, pg, ro + i, acc);
           }
         }
         __syncthreads();
@@ -220,46 +226,62 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, uint32_t leaf, C2<R> (*
 }
 
 // CTAs an SM that the compiler is to leave registers for (0: its own choice).  Of its own it
-// takes 32 registers in these two, which costs loads in flight or spills: complex128 with one
-// right-hand side (9,000 points on a cube 296 us, with 48 registers 259; 40,000 on a sphere
-// the same) and complex64 A x with two (110 and 83 us; 16,000 on a sphere 130 and 136, which
-// is latency hidden by more CTAs).
-template <typename S, int PG, int OP>
-constexpr int kMinCtas = (sizeof(S) == 16 && PG == 1) || (sizeof(S) == 8 && PG == 2 && OP == kZOpN) ? 10 : 0;
-template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE = false>
-__global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(ZArgs a) {
+// takes 32 registers in the complex128 A^H with one right-hand side, which costs loads in
+// flight (9,000 points on a cube 332 us, with 48 registers 255; 40,000 on a sphere the same).
+template <typename S, int PG>
+constexpr int kMinCtas = sizeof(S) == 16 && PG == 1 ? 10 : 0;
+template <typename S, typename R, int PG, int OP>
+__global__ void __launch_bounds__(kThreads, kMinCtas<S, PG>) zmv_kernel(ZArgs a) {
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
-  if (GUARD) {
-    bool any = false;
-    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q * a.guard_step];
-    if (!__syncthreads_or(any)) return;
-    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) zmv_leaf<S, R, PG, OP, true, PRE>(a, l, Xs, Ts, red);
-  } else {
-    zmv_leaf<S, R, PG, OP, false, PRE>(a, blockIdx.x, Xs, Ts, red);
-  }
+  zmv_leaf<S, R, PG, OP, false, false>(a, ZGuard{}, Rounded{}, blockIdx.x, Xs, Ts, red);
 }
 
-template <typename S, typename R, int OP, bool GUARD>
-void launch_groups(const ZArgs& a, uint32_t grid, cudaStream_t s) {
-  if (a.p == 1) zmv_kernel<S, R, 1, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) zmv_kernel<S, R, 2, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) zmv_kernel<S, R, 4, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
-  // wider groups (16) measured slower: fewer columns per pass, lower occupancy
-  else zmv_kernel<S, R, 8, OP, GUARD><<<grid, kThreads, 0, s>>>(a);
+// the right-hand sides of the passes whose flag is set
+template <typename S, typename R, int PG, int OP>
+__global__ void __launch_bounds__(kThreads) zmv_guard_kernel(ZArgs a, ZGuard gd) {
+  __shared__ C2<R> Xs[kCh][PG];
+  __shared__ C2<R> Ts[kThreads];
+  __shared__ C2<R> red[kThreads * PG];
+  bool any = false;
+  for (uint32_t q = threadIdx.x; q * gd.cols < a.p; q += kThreads) any = any || gd.flags[q * gd.step];
+  if (!__syncthreads_or(any)) return;
+  for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x)
+    zmv_leaf<S, R, PG, OP, true, false>(a, gd, Rounded{}, l, Xs, Ts, red);
+}
+
+// X rounded beforehand
+template <int PG, int OP>
+__global__ void __launch_bounds__(kThreads) zmv_rounded_kernel(ZArgs a, Rounded w) {
+  __shared__ C2<float> Xs[kCh][PG];
+  __shared__ C2<float> Ts[kThreads];
+  __shared__ C2<float> red[kThreads * PG];
+  zmv_leaf<float2, float, PG, OP, false, true>(a, ZGuard{}, w, blockIdx.x, Xs, Ts, red);
 }
 
 template <typename S, typename R, int OP>
-void launch_op(const ZArgs& a, cudaStream_t s) {
-  // (complex64: only after right-hand sides of 2^40 or infinity, so that a short launch counts more)
-  constexpr uint32_t kCtas = sizeof(R) == 4 ? 152 * 4 : kGuardCtas;
-  if (a.guard) launch_groups<S, R, OP, true>(a, std::min(a.nleaves, kCtas), s);
-  else launch_groups<S, R, OP, false>(a, a.nleaves, s);
+void launch_op(const ZRun& a, cudaStream_t s) {
+  if (a.guard.flags) {
+    // (complex64: only after right-hand sides of 2^40 or infinity, so that a short launch counts more)
+    constexpr uint32_t kCtas = sizeof(R) == 4 ? 152 * 4 : kGuardCtas;
+    const uint32_t grid = std::min(a.nleaves, kCtas);
+    if (a.p == 1) zmv_guard_kernel<S, R, 1, OP><<<grid, kThreads, 0, s>>>(a, a.guard);
+    else if (a.p == 2) zmv_guard_kernel<S, R, 2, OP><<<grid, kThreads, 0, s>>>(a, a.guard);
+    else if (a.p <= 4) zmv_guard_kernel<S, R, 4, OP><<<grid, kThreads, 0, s>>>(a, a.guard);
+    else zmv_guard_kernel<S, R, 8, OP><<<grid, kThreads, 0, s>>>(a, a.guard);
+    return;
+  }
+  const uint32_t grid = a.nleaves;
+  if (a.p == 1) zmv_kernel<S, R, 1, OP><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p == 2) zmv_kernel<S, R, 2, OP><<<grid, kThreads, 0, s>>>(a);
+  else if (a.p <= 4) zmv_kernel<S, R, 4, OP><<<grid, kThreads, 0, s>>>(a);
+  // wider groups (16) measured slower: fewer columns per pass, lower occupancy
+  else zmv_kernel<S, R, 8, OP><<<grid, kThreads, 0, s>>>(a);
 }
 
 template <typename S, typename R>
-void launch_typed(const ZArgs& a, cudaStream_t s) {
+void launch_typed(const ZRun& a, cudaStream_t s) {
   if (a.op == kZOpH) launch_op<S, R, kZOpH>(a, s);
   else if (a.op == kZOpT) launch_op<S, R, kZOpT>(a, s);
   else launch_op<S, R, kZOpN>(a, s);
@@ -296,7 +318,7 @@ __global__ void z_to_c64_kernel(const double2* __restrict__ src, uint64_t n, flo
 
 }  // namespace
 
-cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
+cudaError_t launch_matvec_z(const ZRun& a, cudaStream_t s) {
   if (a.op < kZOpN || a.op > kZOpT) return cudaErrorInvalidValue;
   if (a.nleaves == 0 || a.p == 0) return cudaSuccess;
   if (!a.single) {
@@ -304,7 +326,7 @@ cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
     count_product_launches(1);
     return cudaGetLastError();
   }
-  if (a.guard || a.p <= 4 || a.elems * a.p < 30000000ull || !a.xf) {
+  if (a.guard.flags || a.p <= 4 || a.elems * a.p < 30000000ull || !a.xf) {
     launch_typed<float2, float>(a, s);
     count_product_launches(1);
     return cudaGetLastError();
@@ -314,11 +336,11 @@ cudaError_t launch_matvec_z(const ZArgs& a, cudaStream_t s) {
     b.p = std::min<uint32_t>(kXW, a.p - r0);
     b.X = a.X + (uint64_t)r0 * a.ldX;
     b.Y = a.Y + (uint64_t)r0 * a.ldY;
-    b.d_one = a.dre == 1.0 && a.dim == 0.0;
+    const Rounded w{a.xf, a.dre == 1.0 && a.dim == 0.0};
     zc_x_kernel<<<(a.n + 31) / 32, 128, 0, s>>>(b.X, b.ldX, a.n, b.p, a.xf);
-    if (a.op == kZOpH) zmv_kernel<float2, float, 8, kZOpH, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
-    else if (a.op == kZOpT) zmv_kernel<float2, float, 8, kZOpT, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
-    else zmv_kernel<float2, float, 8, kZOpN, false, true><<<a.nleaves, kThreads, 0, s>>>(b);
+    if (a.op == kZOpH) zmv_rounded_kernel<8, kZOpH><<<a.nleaves, kThreads, 0, s>>>(b, w);
+    else if (a.op == kZOpT) zmv_rounded_kernel<8, kZOpT><<<a.nleaves, kThreads, 0, s>>>(b, w);
+    else zmv_rounded_kernel<8, kZOpN><<<a.nleaves, kThreads, 0, s>>>(b, w);
     count_product_launches(2);
   }
   return cudaGetLastError();

@@ -420,7 +420,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
       guard_step = kZtPassWords;
     }
   }
-  ZArgs a;
+  ZRun a;
   a.leaves = H->z.leaves.as<MvLeaf>();
   a.order = H->z.order.as<uint32_t>();
   a.nleaves = H->z.nleaves;
@@ -434,9 +434,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.Y = Y;
   a.ldY = ldY;
   a.op = op;
-  a.guard = guard;
-  a.guard_cols = guard_cols;
-  a.guard_step = guard_step;
+  a.guard = ZGuard{guard, guard_cols, guard_step};
   a.elems = Z.elems;
   a.n = (uint32_t)n;
   a.xf = captured ? nullptr : Z.xf.as<float2>();
