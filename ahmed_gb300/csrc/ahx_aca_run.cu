@@ -64,23 +64,24 @@ struct Sorted {
 
 }  // namespace
 
-namespace {
-// the leading 1 + bits binary digits of size, as a number that grows with it (below 2^bits: size)
-inline uint32_t leading(uint64_t size, int bits) {
-  const int m = 63 - __builtin_clzll(size | (1ull << bits));
-  return (uint32_t)(m << bits) + (uint32_t)((size >> (m - bits)) & ((1u << bits) - 1));
+uint32_t size_class(uint64_t size) {
+  const int m = 63 - __builtin_clzll(size | 16);
+  return (uint32_t)(m * 16) + (uint32_t)((size >> (m - 4)) & 15);
 }
-}  // namespace
-
-uint32_t size_class(uint64_t size) { return leading(size, 4); }
 
 void order_by_size(const std::vector<uint64_t>& size, std::vector<uint32_t>& order, int bits) {
-  const uint32_t n = 64u << bits;
+  // sizes below 2^bits as they are, from there on 2^bits steps an octave
+  auto key = [bits](uint64_t s) -> uint32_t {
+    if (s >> bits == 0) return (uint32_t)s;
+    const int m = 63 - __builtin_clzll(s);
+    return ((uint32_t)(m - bits) << bits) + (uint32_t)(s >> (m - bits));
+  };
+  const uint32_t n = (uint32_t)(65 - bits) << bits;
   std::vector<uint32_t> at(n + 1, 0);
-  for (uint64_t s : size) ++at[n - leading(s, bits)];
+  for (uint64_t s : size) ++at[n - key(s)];
   for (uint32_t c = 0; c < n; ++c) at[c + 1] += at[c];
   order.resize(size.size());
-  for (size_t i = 0; i < size.size(); ++i) order[at[n - 1 - leading(size[i], bits)]++] = (uint32_t)i;
+  for (size_t i = 0; i < size.size(); ++i) order[at[n - 1 - key(size[i])]++] = (uint32_t)i;
 }
 
 std::vector<DenseTask> dense_tasks(const std::vector<Leaf>& Ls, uint32_t n, const std::vector<uint32_t>& leaves,
