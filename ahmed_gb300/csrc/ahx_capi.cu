@@ -571,16 +571,15 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
   a.Y = Y;
   a.ldY = ldY;
   a.transposed = transposed ? 1u : 0u;
-  a.guard = guard;
-  a.guard_cols = dg_pass_cols(false);
-  AHX_CUDA(launch_matvec(prec, a, H->stream));
+  const Guard gd{guard, dg_pass_cols(false), 1u};
+  AHX_CUDA(launch_matvec(prec, a, gd, H->stream));
   if (pc.ntleaves) {
     // symmetric tree: the blocks below the diagonal are the upper ones transposed
     a.leaves = pc.tleaves.as<MvLeaf>();
     a.order = pc.torder.as<uint32_t>();
     a.nleaves = pc.ntleaves;
     a.transposed = 1u;
-    AHX_CUDA(launch_matvec(prec, a, H->stream));
+    AHX_CUDA(launch_matvec(prec, a, gd, H->stream));
   }
   return AHX_OK;
 }

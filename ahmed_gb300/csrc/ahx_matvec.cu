@@ -47,7 +47,8 @@ __device__ __forceinline__ void stage_x(A (*Xs)[PG + 1], const MvArgs& a, uint32
 // roles of the factors and of the row / column ranges swap); a dense leaf D
 // acts as D^T, one warp per column of D.
 template <typename SL, typename SD, typename A, int PG, bool TR, bool GUARD>
-__device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[PG + 1], A (*Ts)[PG], A* red) {
+__device__ __forceinline__ void mv_leaf(const MvArgs& a, const Guard& gd, uint32_t leaf, A (*Xs)[PG + 1], A (*Ts)[PG],
+                                        A* red) {
   MvLeaf L = a.leaves[a.order[leaf]];
   const uint32_t tid = threadIdx.x;
   const double d = a.d;
@@ -69,7 +70,7 @@ __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[
     const SD* Ad = L.dense_in_lr_arena ? reinterpret_cast<const SD*>(reinterpret_cast<const SL*>(a.arena_lr) + L.off)
                                        : reinterpret_cast<const SD*>(a.arena_dn) + L.off;
     for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
-      if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
+      if (GUARD && !gd.flags[r0 / gd.cols * gd.step]) continue;
       const uint32_t pg = min((uint32_t)PG, a.p - r0);
       for (uint32_t jb = 0; jb < L.n2; jb += kThreads) {
         const uint32_t j = jb + tid;
@@ -100,7 +101,7 @@ __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[
     return;
   }
   for (uint32_t r0 = 0; r0 < a.p; r0 += PG) {
-    if (GUARD && !a.guard[r0 / a.guard_cols]) continue;
+    if (GUARD && !gd.flags[r0 / gd.cols * gd.step]) continue;
     const uint32_t pg = min((uint32_t)PG, a.p - r0);
     if (L.rank < 0) {
       const SD* Ad = L.dense_in_lr_arena ? reinterpret_cast<const SD*>(
@@ -211,41 +212,38 @@ __device__ __forceinline__ void mv_leaf(const MvArgs& a, uint32_t leaf, A (*Xs)[
   }
 }
 
-template <typename SL, typename SD, typename A, int PG, bool TR, bool GUARD>
+template <typename SL, typename SD, typename A, int PG, bool TR>
 __global__ void __launch_bounds__(kThreads) mv_kernel(MvArgs a) {
   __shared__ A Xs[kCh][PG + 1];
   __shared__ A Ts[kKt][PG];
   __shared__ A red[kThreads];
-  if (GUARD) {
-    bool any = false;
-    for (uint32_t q = threadIdx.x; q * a.guard_cols < a.p; q += kThreads) any = any || a.guard[q];
-    if (!__syncthreads_or(any)) return;
-    for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) mv_leaf<SL, SD, A, PG, TR, true>(a, l, Xs, Ts, red);
-  } else {
-    mv_leaf<SL, SD, A, PG, TR, false>(a, blockIdx.x, Xs, Ts, red);
-  }
+  mv_leaf<SL, SD, A, PG, TR, false>(a, Guard{}, blockIdx.x, Xs, Ts, red);
 }
 
-template <typename SL, typename SD, typename A, bool TR, bool GUARD>
-void launch_groups(const MvArgs& a, uint32_t grid, cudaStream_t s) {
-  if (a.p == 1) mv_kernel<SL, SD, A, 1, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p == 2) mv_kernel<SL, SD, A, 2, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 4) mv_kernel<SL, SD, A, 4, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else if (a.p <= 8) mv_kernel<SL, SD, A, 8, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
-  else mv_kernel<SL, SD, A, 16, TR, GUARD><<<grid, kThreads, 0, s>>>(a);
+template <typename SL, typename SD, typename A, int PG, bool TR>
+__global__ void __launch_bounds__(kThreads) mv_guard_kernel(MvArgs a, Guard gd) {
+  __shared__ A Xs[kCh][PG + 1];
+  __shared__ A Ts[kKt][PG];
+  __shared__ A red[kThreads];
+  bool any = false;
+  for (uint32_t q = threadIdx.x; q * gd.cols < a.p; q += kThreads) any = any || gd.flags[q * gd.step];
+  if (!__syncthreads_or(any)) return;
+  for (uint32_t l = blockIdx.x; l < a.nleaves; l += gridDim.x) mv_leaf<SL, SD, A, PG, TR, true>(a, gd, l, Xs, Ts, red);
 }
 
 template <typename SL, typename SD, typename A, bool TR>
-cudaError_t launch_typed(const MvArgs& a, cudaStream_t s) {
+cudaError_t launch_typed(const MvArgs& a, const Guard& gd, cudaStream_t s) {
   if (a.nleaves == 0 || a.p == 0) return cudaSuccess;
-  if constexpr (sizeof(SL) == 8) {
-    if (a.guard) {
-      launch_groups<SL, SD, A, TR, true>(a, std::min(a.nleaves, kGuardCtas), s);
-      count_product_launches(1);
-      return cudaGetLastError();
-    }
-  }
-  launch_groups<SL, SD, A, TR, false>(a, a.nleaves, s);
+  const uint32_t grid = gd.flags ? std::min(a.nleaves, kGuardCtas) : a.nleaves;
+  auto group = [&](auto plain, auto guarded) {
+    if (gd.flags) guarded<<<grid, kThreads, 0, s>>>(a, gd);
+    else plain<<<grid, kThreads, 0, s>>>(a);
+  };
+  if (a.p == 1) group(mv_kernel<SL, SD, A, 1, TR>, mv_guard_kernel<SL, SD, A, 1, TR>);
+  else if (a.p == 2) group(mv_kernel<SL, SD, A, 2, TR>, mv_guard_kernel<SL, SD, A, 2, TR>);
+  else if (a.p <= 4) group(mv_kernel<SL, SD, A, 4, TR>, mv_guard_kernel<SL, SD, A, 4, TR>);
+  else if (a.p <= 8) group(mv_kernel<SL, SD, A, 8, TR>, mv_guard_kernel<SL, SD, A, 8, TR>);
+  else group(mv_kernel<SL, SD, A, 16, TR>, mv_guard_kernel<SL, SD, A, 16, TR>);
   count_product_launches(1);
   return cudaGetLastError();
 }
@@ -253,10 +251,10 @@ cudaError_t launch_typed(const MvArgs& a, cudaStream_t s) {
 }  // namespace
 
 // the plain (FP64) form; the mixed forms run the tensor-core sweeps
-cudaError_t launch_matvec(int prec, const MvArgs& a, cudaStream_t s) {
+cudaError_t launch_matvec(int prec, const MvArgs& a, const Guard& g, cudaStream_t s) {
   if (prec != kFP64) return cudaErrorInvalidValue;
-  return a.transposed ? launch_typed<double, double, double, true>(a, s)
-                      : launch_typed<double, double, double, false>(a, s);
+  return a.transposed ? launch_typed<double, double, double, true>(a, g, s)
+                      : launch_typed<double, double, double, false>(a, g, s);
 }
 
 }  // namespace ahx

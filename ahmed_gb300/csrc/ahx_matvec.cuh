@@ -39,10 +39,15 @@ struct MvArgs {
   double* Y;
   uint64_t ldY;
   uint32_t transposed = 0;  // 1: Y += d A^T X (H/mltaGeHVec.cpp:62-150)
-  // when set: right-hand side r takes part only if guard[r / guard_cols] is not zero (few
-  // CTAs, a leaf loop; guard_cols a multiple of 16).  FP64 leaves only.
-  const int* guard = nullptr;
-  uint32_t guard_cols = 0;
+};
+
+// With flags, right-hand side r takes part only if flags[r / cols * step] is not zero (few
+// CTAs, a leaf loop; cols a multiple of the kernels' groups).  Apart from the arguments above:
+// fields beside those changed the registers that the compiler gives the plain kernels, and
+// with them their times by up to 27 %.
+struct Guard {
+  const int* flags = nullptr;
+  uint32_t cols = 0, step = 1;
 };
 
 // CTAs of a guarded product: as many as the SMs hold of the plain kernels (128 threads, 32 to
@@ -51,7 +56,7 @@ struct MvArgs {
 // (groups of 8 columns: 4.77); that nothing runs takes 2 us more than with 1,024 CTAs.
 constexpr uint32_t kGuardCtas = 152 * 16;
 
-cudaError_t launch_matvec(int prec, const MvArgs& a, cudaStream_t s);
+cudaError_t launch_matvec(int prec, const MvArgs& a, const Guard& g, cudaStream_t s);
 
 // Double-float product Y += A X (ahx_matvec_df.cu): arena = the FP64 arena's
 // elements as (hi, lo) float pairs at the same offsets; X = d X split the same
@@ -91,15 +96,8 @@ struct ZArgs {
   uint64_t ldY;
   int op;
 };
-// (apart from ZArgs: fields beside those changed the registers that the compiler gives the
-// plain kernels, 36 to 32 for A^T with one right-hand side, and with them their times by
-// -10 to +27 %)
-struct ZGuard {
-  const int* flags;        // as MvArgs::guard, the words `step` apart
-  uint32_t cols, step;
-};
 struct ZRun : ZArgs {
-  ZGuard guard{nullptr, 0u, 1u};
+  Guard guard;
   uint64_t elems = 0;          // complex64 leaves: elements,
   uint32_t n = 0;              //   rows of X,
   float2* xf = nullptr;        //   room for its rounded copy (matvec_z_xf_bytes; null: none is made)

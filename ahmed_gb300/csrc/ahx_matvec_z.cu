@@ -123,7 +123,7 @@ __device__ __forceinline__ void emit(const ZArgs& a, const Rounded& w, uint32_t 
 }
 
 template <typename S, typename R, int PG, int OP, bool GUARD, bool PRE>
-__device__ __forceinline__ void zmv_leaf(const ZArgs& a, const ZGuard& gd, const Rounded& w, uint32_t leaf,
+__device__ __forceinline__ void zmv_leaf(const ZArgs& a, const Guard& gd, const Rounded& w, uint32_t leaf,
                                          C2<R> (*Xs)[PG], C2<R>* Ts, C2<R>* red) {
   const MvLeaf L = a.leaves[a.order[leaf]];
   const S* base = reinterpret_cast<const S*>(a.arena) + L.off;
@@ -235,12 +235,12 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<S, PG>) zmv_kernel(ZArgs a)
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
-  zmv_leaf<S, R, PG, OP, false, false>(a, ZGuard{}, Rounded{}, blockIdx.x, Xs, Ts, red);
+  zmv_leaf<S, R, PG, OP, false, false>(a, Guard{}, Rounded{}, blockIdx.x, Xs, Ts, red);
 }
 
 // the right-hand sides of the passes whose flag is set
 template <typename S, typename R, int PG, int OP>
-__global__ void __launch_bounds__(kThreads) zmv_guard_kernel(ZArgs a, ZGuard gd) {
+__global__ void __launch_bounds__(kThreads) zmv_guard_kernel(ZArgs a, Guard gd) {
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];
   __shared__ C2<R> red[kThreads * PG];
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kThreads) zmv_rounded_kernel(ZArgs a, Rounded 
   __shared__ C2<float> Xs[kCh][PG];
   __shared__ C2<float> Ts[kThreads];
   __shared__ C2<float> red[kThreads * PG];
-  zmv_leaf<float2, float, PG, OP, false, true>(a, ZGuard{}, w, blockIdx.x, Xs, Ts, red);
+  zmv_leaf<float2, float, PG, OP, false, true>(a, Guard{}, w, blockIdx.x, Xs, Ts, red);
 }
 
 template <typename S, typename R, int OP>

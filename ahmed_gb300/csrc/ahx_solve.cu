@@ -1278,7 +1278,7 @@ struct ahx_batch : ahx::Operator {
     a.ldX = ntot;
     a.Y = Y;
     a.ldY = ntot;
-    AHX_CUDA(launch_matvec(pr, a, stream));
+    AHX_CUDA(launch_matvec(pr, a, Guard{}, stream));
     return AHX_OK;
   }
 };

@@ -434,7 +434,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   a.Y = Y;
   a.ldY = ldY;
   a.op = op;
-  a.guard = ZGuard{guard, guard_cols, guard_step};
+  a.guard = Guard{guard, guard_cols, guard_step};
   a.elems = Z.elems;
   a.n = (uint32_t)n;
   a.xf = captured ? nullptr : Z.xf.as<float2>();
