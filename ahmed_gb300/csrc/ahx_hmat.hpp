@@ -60,14 +60,14 @@ struct HostWord {
 // basis of 50 vectors at 1,048,576 points and 64 right-hand sides is 27 GB).
 struct SolveWork {
   static constexpr size_t kKeep = 256ull << 20;
-  DevBuf items, first, partial, small[3], len, gm;  // reductions, GMRES state
+  DevBuf items, first, partial, groups, small[3], len, gm;  // reductions, GMRES state
   DevBuf v, r, rr, z;                               // basis, residuals, correction
   void release() {
-    for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) b->release();
+    for (DevBuf* b : {&items, &first, &partial, &groups, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) b->release();
   }
   void trim() {
     size_t s = 0;
-    for (DevBuf* b : {&items, &first, &partial, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) s += b->bytes;
+    for (DevBuf* b : {&items, &first, &partial, &groups, small, small + 1, small + 2, &len, &gm, &v, &r, &rr, &z}) s += b->bytes;
     if (s > kKeep) release();
   }
 };

@@ -121,21 +121,53 @@ __global__ void __launch_bounds__(kRedThreads) dots_kernel(const Item* __restric
   item_dots(w, it.len, V + it.base, vstride, nk, partial + (uint64_t)blockIdx.x * ldp);
 }
 
-// One Gram-Schmidt pass on the CTA's item: the coefficients of its system from the item
-// sums `pin` of the pass before (each CTA adds them up itself, in item order; the system's
-// first one keeps them in coef), W -= sum_k coef_k V_k, and from the new W the item sums
+// A large system's item sums, kGroup items to one: with kDirect items and fewer (262,144
+// points) every CTA of cgs_kernel adds them all up itself, which takes less than a launch
+// (131,072 points, 10 vectors, 8 systems: 118 us a step's orthogonalisation, with groups 129),
+// but those reads grow with the square of the points: 524,288 points, 30 vectors, 4 systems
+// 687 us and 576, 1,048,576 points, 16 systems 6,110 and 4,120, 4,194,304 points, one system
+// 3,340 and 1,100 (reductions as launches of their own: 4,440 and 1,490).
+constexpr uint32_t kGroup = 64;
+constexpr uint32_t kDirect = 256;
+// pout[g * ldp + k] = sum of pin[i * ldp + k] over the items groups[g].x <= i < groups[g].y, k < nk
+__global__ void __launch_bounds__(kRedThreads) group_sums_kernel(const uint2* __restrict__ groups,
+                                                                 const double* __restrict__ pin, uint32_t ldp,
+                                                                 uint32_t nk, double* __restrict__ pout) {
+  constexpr uint32_t kw = 64, np = kRedThreads / kw;
+  __shared__ double part[np][kw];
+  const uint2 g = groups[blockIdx.x];
+  const uint32_t kt = threadIdx.x % kw, q = threadIdx.x / kw;
+  for (uint32_t k0 = 0; k0 < nk; k0 += kw) {
+    double s = 0.0;
+    if (k0 + kt < nk)
+#pragma unroll 4
+      for (uint32_t i = g.x + q; i < g.y; i += np) s += pin[(uint64_t)i * ldp + k0 + kt];
+    part[q][kt] = s;
+    __syncthreads();
+    if (q == 0 && k0 + kt < nk) {
+      for (uint32_t w = 1; w < np; ++w) s += part[w][kt];
+      pout[(uint64_t)blockIdx.x * ldp + k0 + kt] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// One Gram-Schmidt pass on the CTA's item: the coefficients of its system from the item (or
+// group) sums `pin` of the pass before, rows sfirst[q] to sfirst[q + 1] (each CTA adds them up
+// itself, in order; the system's first one keeps them in coef), W -= sum_k coef_k V_k, and from the new W the item sums
 // of the next pass (LAST: of |W|^2).  One launch instead of a reduction, a combination
 // and the sums, one read of W, V from L1 the second time: a step's orthogonalisation
 // (16 systems of 32,768 points, steps 1 to 10) 93 us -> 50 us on average with cold caches.
 template <bool LAST>
 __global__ void __launch_bounds__(kRedThreads)
-    cgs_kernel(const Item* __restrict__ items, const uint32_t* __restrict__ first, const double* __restrict__ V,
-               uint64_t vstride, uint32_t nk, double* __restrict__ W, const double* __restrict__ pin, uint32_t ldp,
+    cgs_kernel(const Item* __restrict__ items, const uint32_t* __restrict__ first,
+               const uint32_t* __restrict__ sfirst, const double* __restrict__ V, uint64_t vstride, uint32_t nk, double* __restrict__ W, const double* __restrict__ pin, uint32_t ldp,
                double* __restrict__ coef, uint32_t ldc, double* __restrict__ pout) {
   constexpr uint32_t kTile = kRedThreads;
   __shared__ double c[kTile], parts[kTile];
   const Item it = items[blockIdx.x];
-  const uint32_t i0 = first[it.q], i1 = first[it.q + 1];
+  const uint32_t i0 = sfirst[it.q], i1 = sfirst[it.q + 1];
+  const bool keeps = blockIdx.x == first[it.q];
   double w[kPerThread];
 #pragma unroll
   for (int e = 0; e < kPerThread; ++e) {
@@ -156,7 +188,7 @@ __global__ void __launch_bounds__(kRedThreads)
     if (threadIdx.x < kn) {
       for (uint32_t q = 1; q < np; ++q) s += parts[q * kw + threadIdx.x];
       c[threadIdx.x] = s;
-      if (blockIdx.x == i0) coef[(uint64_t)it.q * ldc + k0 + threadIdx.x] = s;
+      if (keeps) coef[(uint64_t)it.q * ldc + k0 + threadIdx.x] = s;
     }
     __syncthreads();
 #pragma unroll 4
@@ -518,6 +550,18 @@ class Solver {
     // systems are numbered c * nseg + s, which is the order items were produced in
     first[nsys_] = (uint32_t)items.size();
     nitems_ = (uint32_t)items.size();
+    // groups of the items, when a system has many; their first ones follow in `first`
+    std::vector<uint2> groups;
+    uint32_t most = 0;
+    for (uint32_t q = 0; q < nsys_; ++q) most = std::max(most, first[q + 1] - first[q]);
+    if (most > kDirect)
+      for (uint32_t q = 0; q < nsys_; ++q) {
+        first.push_back((uint32_t)groups.size());
+        for (uint32_t i = first[q]; i < first[q + 1]; i += kGroup)
+          groups.push_back(make_uint2(i, std::min(i + kGroup, first[q + 1])));
+      }
+    ngroups_ = (uint32_t)groups.size();
+    if (ngroups_) first.push_back(ngroups_);
     maxk_ = maxk;
     int rc;
     if ((rc = items_.reserve(std::max<size_t>(items.size(), 1) * sizeof(Item)))) return rc;
@@ -527,6 +571,10 @@ class Solver {
     if ((rc = small2_.reserve((size_t)nsys_ * maxk * sizeof(double)))) return rc;
     if ((rc = small3_.reserve((size_t)nsys_ * maxk * sizeof(double)))) return rc;
     if ((rc = len_.reserve((size_t)nsys_ * sizeof(uint32_t)))) return rc;
+    if (ngroups_) {
+      if ((rc = groups_.reserve(ngroups_ * (sizeof(uint2) + (size_t)maxk * sizeof(double))))) return rc;
+      AHX_CUDA(cudaMemcpyAsync(groups_.p, groups.data(), ngroups_ * sizeof(uint2), cudaMemcpyHostToDevice, op_.stream));
+    }
     if (!items.empty())
       AHX_CUDA(cudaMemcpyAsync(items_.p, items.data(), items.size() * sizeof(Item),
                                cudaMemcpyHostToDevice, op_.stream));
@@ -547,29 +595,40 @@ class Solver {
     return AHX_OK;
   }
 
-  // W -= V (V^T W), twice; the coefficients in h1 and h2, the items' |W|^2 in partial_
+  // W -= V (V^T W), twice; the coefficients in h1 and h2, parts of |W|^2 in norm_parts()
   int gram_schmidt(const double* V, uint64_t vstride, uint32_t nk, double* W, double* h1, double* h2) {
     if (nitems_ == 0) return AHX_OK;
     const Item* it = items_.as<Item>();
-    const uint32_t* fi = first_.as<uint32_t>();
+    const uint32_t *fi = first_.as<uint32_t>(), *fs = sum_rows();
     double *pa = partial_.as<double>(), *pb = pa + (size_t)nitems_ * maxk_;
     cudaStream_t st = op_.stream;
+    // the sums that the next kernel reads
+    auto sums = [&](double* p, uint32_t k) -> const double* {
+      if (!ngroups_) return p;
+      group_sums_kernel<<<ngroups_, kRedThreads, 0, st>>>(groups_.as<uint2>(), p, maxk_, k, gpart());
+      return gpart();
+    };
     dots_kernel<<<nitems_, kRedThreads, 0, st>>>(it, V, vstride, nk, W, pa, maxk_);
-    cgs_kernel<false><<<nitems_, kRedThreads, 0, st>>>(it, fi, V, vstride, nk, W, pa, maxk_, h1, maxk_, pb);
-    cgs_kernel<true><<<nitems_, kRedThreads, 0, st>>>(it, fi, V, vstride, nk, W, pb, maxk_, h2, maxk_, pa);
+    cgs_kernel<false><<<nitems_, kRedThreads, 0, st>>>(it, fi, fs, V, vstride, nk, W, sums(pa, nk), maxk_, h1, maxk_, pb);
+    cgs_kernel<true><<<nitems_, kRedThreads, 0, st>>>(it, fi, fs, V, vstride, nk, W, sums(pb, nk), maxk_, h2, maxk_, pa);
+    sums(pa, 1);
     AHX_CUDA(cudaGetLastError());
     return AHX_OK;
   }
+  // |W|^2 after gram_schmidt: rows sum_rows()[q] to sum_rows()[q + 1] of norm_parts(), maxk_ apart
+  const double* norm_parts() const { return ngroups_ ? gpart() : partial_.as<double>(); }
+  const uint32_t* sum_rows() const { return ngroups_ ? first_.as<uint32_t>() + nsys_ + 1 : first_.as<uint32_t>(); }
+  double* gpart() const { return reinterpret_cast<double*>(groups_.as<uint2>() + ngroups_); }
 
   const uint32_t* segid() const { return op_.nseg > 1 ? op_.seg_id.as<uint32_t>() : nullptr; }
 
   Operator& op_;
   SolveWork& work_{*op_.work};
   bool idle_ = false;  // set once nothing in flight uses the scratch
-  uint32_t p_, nsys_ = 0, nitems_ = 0, maxk_ = 0;
+  uint32_t p_, nsys_ = 0, nitems_ = 0, ngroups_ = 0, maxk_ = 0;
   uint64_t total_ = 0;
   DevBuf &items_{work_.items}, &first_{work_.first}, &partial_{work_.partial}, &small_{work_.small[0]},
-      &small2_{work_.small[1]}, &small3_{work_.small[2]}, &len_{work_.len};
+      &small2_{work_.small[1]}, &small3_{work_.small[2]}, &len_{work_.len}, &groups_{work_.groups};  // groups, then their sums
   DevBuf& gm_{work_.gm};  // device GMRES state (GmDev arrays)
 };
 
@@ -732,7 +791,7 @@ int gmres_core(Solver& sv, int prec, const double* B, double* X, double tol, uin
       if (e) return e;
       // CGS2: h = V^T w; w -= V h; h2 = V^T w; w -= V h2
       if ((e = sv.gram_schmidt(V, vstride, i + 1, w, d1, d2))) return e;
-      arnoldi_kernel<<<(nsys + 3) / 4, 128, 0, st>>>(g, i, m, K, d1, d2, sv.partial_.as<double>(), K, sv.first_.as<uint32_t>(),
+      arnoldi_kernel<<<(nsys + 3) / 4, 128, 0, st>>>(g, i, m, K, d1, d2, sv.norm_parts(), K, sv.sum_rows(),
                                             d3, nsys);
       // w /= |w|
       scale_kernel<<<grid_for(total), 256, 0, st>>>(w, w, d3, 1, 0, total, op.ntot, sid, op.nseg);
