@@ -132,8 +132,11 @@ struct HelmGen {  // exp(i k r) / (4 pi r)
       r = r2 * y;
       r = fma(0.5 * y, fma(-r, r, r2), r);
       s = (1.0 / kFourPi) * y;
+    } else if (f.i == j) {
+      r = h;
+      s = reciprocal_rounded(kFourPi * h);
     } else {
-      const double2 v = rounded_r_s_any(f.i == j ? h * h : r2);
+      const double2 v = rounded_r_s_any(r2);
       r = v.x;
       s = v.y;
     }
