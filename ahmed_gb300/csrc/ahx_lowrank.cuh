@@ -906,7 +906,9 @@ __device__ uint32_t lq(Team<NW>& g, uint32_t m, uint32_t n, T* M, uint32_t ld, T
     }
     g.sync();
     const double d = re_(G[j * ldg + j]);
-    const double rs = __double2hiint(d) >= 0x00100000 ? rsqrt_any(d) : 0.0;  // an empty row: no column
+    // an empty row: no column (a NaN, which the FP64 unit makes with its sign set, is no empty
+    // row: the leaf is to show it)
+    const double rs = (__double2hiint(d) & 0x7fffffff) >= 0x00100000 ? rsqrt_any(d) : 0.0;
     if (g.rank == 0) nrm[j] = rs;
     const double r2 = rs * rs;
     for (uint32_t i = j + 1 + grp; i < m; i += groups) {
