@@ -528,7 +528,9 @@ int product_device(ahx_hmat* H, int prec, double d, uint32_t p, const double* X,
     // (nothing is laid out or allocated while the stream is captured)
     DgState& D = H->dg[transposed ? 1 : 0];
     const bool ready = D.valid && H->dg_work.bytes >= dg_work_bytes(false, H->tree.n, D.t_rows, p);
-    if (ready || ((prec == kDF64 || dg_due(D, H->arena64_elems, p, H->tree.leaves.size())) && !stream_captured(H->stream)))
+    const char* at_once = one ? "AHX_F1_MIN" : "AHX_DG_MIN";
+    if (ready || ((prec == kDF64 || dg_due(D, H->arena64_elems, p, H->tree.leaves.size(), at_once)) &&
+                  !stream_captured(H->stream)))
       if ((rc = prepare_dg(H, p, transposed, usable))) return rc;
     if (usable && one) {
       if ((rc = prepare_product(H, kFP64))) return rc;  // (a product that the caller captures takes these)

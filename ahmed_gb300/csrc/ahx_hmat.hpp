@@ -259,8 +259,9 @@ bool um_enabled();
 bool dg_wanted(uint64_t elems, uint32_t p);
 // Whether a product (of dg_wanted's size) should run sliced now: always once the
 // layout exists; before, when the plain products so far and this one cost as much
-// as the layout does.
-bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves);
+// as the layout does.  at_once: the environment variable that, when set, has it laid out at the
+// first product (AHX_DG_MIN, AHX_F1_MIN or AHX_ZT_MIN, by the kind of product).
+bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves, const char* at_once);
 // Whether a graph capture is under way on the stream (nothing may be allocated or waited for).
 bool stream_captured(cudaStream_t s);
 // Whether the caller is capturing the product: its graph may be replayed at any time, beside

@@ -968,9 +968,8 @@ bool dg_wanted(uint64_t elems, uint32_t p) {
 // right-hand sides, 25,000 leaves), so a handle that multiplies once stays with the
 // plain kernel (2 p FP64 operations per element at 1 TFLOP/s); one that goes on
 // never spends more than about twice the better choice.
-bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves) {
-  if (D.valid || std::getenv("AHX_DG_MIN") || std::getenv("AHX_ZT_MIN") || std::getenv("AHX_F1_MIN"))
-    return true;
+bool dg_due(DgState& D, uint64_t elems, uint32_t p, size_t nleaves, const char* at_once) {
+  if (D.valid || std::getenv(at_once)) return true;
   const double plain = 2e-6 * (double)elems * p, layout = 300.0 + 0.055 * (double)nleaves;
   if (D.spent + plain >= layout) return true;
   D.spent += plain;

@@ -377,7 +377,7 @@ int zproduct_device(ahx_hmat* H, int prec, int op, double dre, double dim, uint3
   const uint64_t n = H->tree.n;
   DgState& D = Z.dg[op];
   auto laid_out = [&](uint64_t cost) -> bool {
-    return !captured && (D.valid || dg_due(D, cost, p, H->tree.leaves.size()));
+    return !captured && (D.valid || dg_due(D, cost, p, H->tree.leaves.size(), prec == kFP64 ? "AHX_DG_MIN" : "AHX_ZT_MIN"));
   };
   auto layout = [&]() -> int {
     if (D.valid) return AHX_OK;
