@@ -10,7 +10,7 @@
 //               memory first
 // What bounds it: one multiply-add per value on the FP64 pipe, 412 us for the 2.09 GB of
 // 65,536 points at two lanes a clock and SM, above their memory time (307 us); the rows
-// sweep keeps the pipe 87 % busy, the V sweep 70 %.  The plain kernel (ahx_matvec.cu: a
+// sweep keeps the pipe 94 % busy, the V sweep 88 %.  The plain kernel (ahx_matvec.cu: a
 // CTA per leaf) reads its factors in a chain of dependent steps and half fills its
 // warps.  A x, 65,536 points: 628 -> 524 us; 10,007: 128 -> 92; 4,096: 65 -> 39 us.
 #include <algorithm>

@@ -34,8 +34,9 @@ extern "C" {
 #define AHX_FP64 0      /* plain form: FP64 leaves (mblock<double>) */
 #define AHX_FP32 1      /* all leaves FP32, FP32 accumulation */
 #define AHX_BF16_FP32 2 /* low-rank factors BF16, dense leaves FP32, FP32 accumulation */
-#define AHX_DF64 3      /* FP64 leaves as float pairs, double-float arithmetic on the FP32
-                           pipes (about 2^-44 relative; FP64-class): the refinement's outer
+#define AHX_DF64 3      /* FP64-class: the FP64 product on digits where there is room for its
+                           layout, else FP64 leaves as float pairs in double-float arithmetic
+                           on the FP32 pipes (about 2^-44 relative).  The refinement's outer
                            residual from two right-hand sides per system on (one: the FP64
                            product; AHX_REFINE_RESIDUAL=fp64 / df64 forces either) */
 
