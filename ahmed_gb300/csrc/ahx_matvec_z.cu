@@ -22,6 +22,7 @@
 // (p = 3: 170 -> 171 us), below 3 10^7 (elements x right-hand sides) the extra launch
 // outweighs it (1,025 points, p = 8: 54 -> 56 us).
 #include <algorithm>
+#include <type_traits>
 
 #include "ahx_matvec.cuh"
 
@@ -227,11 +228,19 @@ __device__ __forceinline__ void zmv_leaf(const ZArgs& a, const Guard& gd, const 
 
 // CTAs an SM that the compiler is to leave registers for (0: its own choice).  Of its own it
 // takes 32 registers in the complex128 A^H with one right-hand side, which costs loads in
-// flight (9,000 points on a cube 332 us, with 48 registers 255; 40,000 on a sphere the same).
-template <typename S, int PG>
-constexpr int kMinCtas = sizeof(S) == 16 && PG == 1 ? 10 : 0;
+// flight (9,000 points on a cube 332 us, with 48 registers 255; 40,000 on a sphere the same),
+// and 44 in the complex64 A with two (48 with the bound: sphere of 9,000 points 72 -> 70 us,
+// 16,384 142 -> 138, cube of 9,000 68 -> 67, ellipsoid of 5,497 78 both).
+template <typename S, int PG, int OP>
+constexpr int kMinCtas = (sizeof(S) == 16 && PG == 1) || (sizeof(S) == 8 && PG == 2 && OP == kZOpN) ? 10 : 0;
+// What a kernel is passed.  The complex64 A with one right-hand side reads no more of ZRun than
+// of ZArgs, but the compiler schedules it better with the longer parameter block (31 registers
+// against 32: sphere of 9,000 points 52 -> 50 us, 16,384 101 -> 97, cube of 9,000 83 -> 81);
+// A^T with one right-hand side is the other way round (cube of 9,000 points 112 us with ZRun, 88).
+template <typename S, int PG, int OP>
+using PlainArgs = std::conditional_t<sizeof(S) == 8 && PG == 1 && OP == kZOpN, ZRun, ZArgs>;
 template <typename S, typename R, int PG, int OP>
-__global__ void __launch_bounds__(kThreads, kMinCtas<S, PG>) zmv_kernel(ZArgs a) {
+__global__ void __launch_bounds__(kThreads, kMinCtas<S, PG, OP>) zmv_kernel(PlainArgs<S, PG, OP> a) {
   __shared__ C2<R> Xs[kCh][PG];
   __shared__ C2<R> Ts[kThreads];       // kThreads / PG columns x PG right-hand sides
   __shared__ C2<R> red[kThreads * PG];  // per-slice partial inner products
