@@ -37,7 +37,7 @@
 //
 // What bounds it: the ALU work of cutting (about 30 integer operations per
 // element; ALU pipe 53%, issue 48%, tensor pipe 22% to 31% busy at 32,768 points).
-// 65,536 points (2.09 GB): 8.35 -> 1.35 ms with 16 right-hand sides, 4.21 -> 0.99
+// 65,536 points (2.09 GB): 8.35 -> 1.36 ms with 16 right-hand sides, 4.21 -> 0.99
 // ms with 8 (2.1 TB/s); 8,300 us of it were the FP64 pipe.
 #include <algorithm>
 #include <cstdlib>
